@@ -9,8 +9,8 @@
 //     wq    = (Q) round(w / scale)          round = hrint for f16 / bf16, roundf for f32
 //     w'    = (T) wq * scale
 //
-// in w's own type T, with CUDA's own operators for __half / __nv_bfloat16 (their division is an
-// approximate reciprocal times the dividend, rounded once; that is part of the result).  This file
+// in w's own type T, with CUDA's own operators for __half / __nv_bfloat16 or with operations shown to give
+// the same values.  This file
 // is compiled with -ftz=true -prec-div=false, the flags the reference compiles its kernels with
 // (python/hidet/backend/build.py:142-177), because they decide the f32 division.
 //
@@ -43,36 +43,18 @@ struct Arith<__half> {
     static __device__ __forceinline__ __half max_(__half a, __half b) { return __hmax(a, b); }
     static __device__ __forceinline__ __half div_(__half a, __half b) { return a / b; }
     static __device__ __forceinline__ __half qmax(int q) { return (__half)(float)q; }
-    // w / scale for many w and one scale.  CUDA's __half division (cuda_fp16.hpp, __hdiv) converts both
-    // operands to f32, takes rcp.approx.ftz.f32 of the divisor, multiplies, rounds to half, and redoes
-    // the last steps with one correction when the result is a non-zero value below 0x008F.  The
-    // reciprocal depends on the divisor only, so it is taken once per scale; every other operation is
-    // the same one, in the same order, which keeps the quotient bit-identical to `w / scale`.
-    struct Divisor {
-        float fb;
-        float rcp;
-    };
-    static __device__ __forceinline__ Divisor prepare(__half scale) {
-        Divisor d;
-        d.fb = __half2float(scale);
-        asm("{rcp.approx.ftz.f32 %0, %1;\n}" : "=f"(d.rcp) : "f"(d.fb));
-        return d;
-    }
-    static __device__ __forceinline__ __half div_prepared(__half a, const Divisor &d) {
-        const float fa = __half2float(a);
-        float fv = d.rcp * fa;
-        __half v = __float2half(fv);
-        const __half av = __habs(v);
-        if (__hlt(av, __ushort_as_half((unsigned short)0x008FU)) && __hlt(__float2half(0.0f), av)) {
-            const float err = __fmaf_rn(-d.fb, fv, fa);
-            fv = __fmaf_rn(d.rcp, err, fv);
-            v = __float2half(fv);
-        }
-        return v;
-    }
+    // w / scale for many w and one scale, as the correctly rounded reciprocal of the scale times w in f32, rounded to
+    // half: that is the correctly rounded quotient, the value of `w / scale`, wherever the quotient is a normal half.
+    // Let w and scale have the significands a, b < 2^11.  A midpoint between two halves has an odd 12-bit significand m,
+    // so a / b - m / 2^j (j <= 12) is a non-zero multiple of 1 / (b 2^j), at least 1 / (a 2^12) of the quotient (j = 12
+    // needs a < b <= 2047, so a <= 2046), which exceeds 2^-23 (1 + 2^-11); the two f32 roundings move it by less than
+    // 2^-23 (1 + 2^-24).  A quotient below the normal halves rounds to the integer 0 either way, and zero, infinite
+    // and NaN operands give the zeros, infinities and NaN of a division.
+    typedef float Divisor;
+    static __device__ __forceinline__ Divisor prepare(__half scale) { return __frcp_rn(__half2float(scale)); }
     template <typename Q>
-    static __device__ __forceinline__ Q quant(__half w, const Divisor &d) {
-        return (Q)(short)(hrint(div_prepared(w, d)));
+    static __device__ __forceinline__ Q quant(__half w, Divisor rcp) {
+        return (Q)(short)(hrint(__float2half(rcp * __half2float(w))));
     }
     template <typename Q>
     static __device__ __forceinline__ __half dequant(Q q, __half scale) {
@@ -161,8 +143,7 @@ struct QuantVec {
 
 // f16 -> int8, eight at a time, two per instruction where the arithmetic allows it, with the same bits as the
 // general form:
-//   * the quotient v is f16(rcp * f32(w)) as in Arith<__half>::div_prepared; the correction step there only touches
-//     non-zero quotients below 0x008F (8.5e-6), which round to zero either way, so it is left out;
+//   * the quotient v is f16(rcp * f32(w)) as in Arith<__half>::quant;
 //   * b = v + 1536 in f16 (1536 = 0x6600, where one ulp is 1) is v rounded to an integer, ties to even, plus 1536
 //     for |v| < 512: the same integer hrint gives, and 1536 being even the same ties.  For |hrint(v)| <= 127 the
 //     low mantissa byte of b is that integer's two's-complement byte, which replaces hrint and the two conversions
@@ -179,9 +160,9 @@ struct QuantVec<__half, int8_t, 8, Arith<__half>::Divisor> {
         __half2 b[4], far[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const Arith<__half>::Divisor &d0 = s[PER_ELEMENT ? 2 * j : 0], &d1 = s[PER_ELEMENT ? 2 * j + 1 : 0];
+            const float d0 = s[PER_ELEMENT ? 2 * j : 0], d1 = s[PER_ELEMENT ? 2 * j + 1 : 0];
             const float2 f = __half22float2(x2[j]);
-            b[j] = __hadd2(__floats2half2_rn(d0.rcp * f.x, d1.rcp * f.y), magic);
+            b[j] = __hadd2(__floats2half2_rn(d0 * f.x, d1 * f.y), magic);
             far[j] = __habs2(__hsub2(b[j], magic));
         }
         // one test for the eight: the largest magnitude, a NaN if there is any

@@ -19,7 +19,6 @@ import numpy as np
 _DIR = os.path.dirname(os.path.abspath(__file__))
 SOURCE = os.path.join(_DIR, 'quant_oracle.c')
 LIBRARY = os.path.join(_DIR, 'libquant_oracle.so')
-RCP_TABLE_FILE = os.path.join(_DIR, '..', 'tests', 'golden', 'rcp_approx_ftz_f32_of_f16.npy')
 
 # Portable, strict IEEE build: the checker must give the same bits on every host.
 STRICT_FLAGS = ['-O2', '-fPIC', '-shared', '-fopenmp', '-ffp-contract=off', '-fno-fast-math', '-fvisibility=hidden']
@@ -45,7 +44,7 @@ def load(path: Optional[str] = None) -> ctypes.CDLL:
         path = build()
     if path not in _libs:
         lib = ctypes.CDLL(path)
-        lib.oracle_quantize_f16.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_void_p]
+        lib.oracle_quantize_f16.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int]
         lib.oracle_dequantize_f16.argtypes = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int]
         lib.oracle_qmatmul_f16.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_int64]
         lib.oracle_qmatmul_f16_fused.argtypes = lib.oracle_qmatmul_f16.argtypes
@@ -58,30 +57,13 @@ def load(path: Optional[str] = None) -> ctypes.CDLL:
         lib.oracle_half_to_float.restype = ctypes.c_float
         lib.oracle_float_to_half.argtypes = [ctypes.c_float]
         lib.oracle_float_to_half.restype = ctypes.c_uint16
-        lib.oracle_hdiv.argtypes = [ctypes.c_uint16, ctypes.c_uint16, c_void_p]
+        lib.oracle_hdiv.argtypes = [ctypes.c_uint16, ctypes.c_uint16]
         lib.oracle_hdiv.restype = ctypes.c_uint16
         for name in ('oracle_quantize_f16', 'oracle_dequantize_f16', 'oracle_qmatmul_f16', 'oracle_qmatmul_f16_fused',
                      'oracle_quantize_f32', 'oracle_dequantize_f32', 'oracle_matmul_f32', 'oracle_qmatmul_f32'):
             getattr(lib, name).restype = None
         _libs[path] = lib
     return _libs[path]
-
-
-_rcp_table: Optional[np.ndarray] = None
-_rcp_table_loaded = False
-
-
-def rcp_table() -> Optional[np.ndarray]:
-    """uint32[65536]: bits of rcp.approx.ftz.f32(x) for every half bit pattern x, as measured on a
-    B200 (tests/golden/make_rcp_table.py), or None if the measurement is not in the tree."""
-    global _rcp_table, _rcp_table_loaded
-    if not _rcp_table_loaded:
-        _rcp_table_loaded = True
-        if os.path.exists(RCP_TABLE_FILE):
-            t = np.load(RCP_TABLE_FILE)
-            assert t.dtype == np.uint32 and t.shape == (65536,)
-            _rcp_table = np.ascontiguousarray(t)
-    return _rcp_table
 
 
 def _ptr(a: Optional[np.ndarray]):
@@ -111,7 +93,7 @@ def _as_2d(shape, dims) -> Tuple[int, int, int, list]:
     raise NotImplementedError('oracle: dims must be leading or trailing')
 
 
-def symmetric_quantize(w: np.ndarray, quant_type='int8', dims: Union[int, Sequence[int]] = -1, use_rcp_table: bool = True,
+def symmetric_quantize(w: np.ndarray, quant_type='int8', dims: Union[int, Sequence[int]] = -1,
                        x86_fast_math: bool = False, lib: Optional[ctypes.CDLL] = None):
     """(wq, scale) as the reference computes them for a float16 (CUDA arithmetic) or float32 input.
 
@@ -124,8 +106,7 @@ def symmetric_quantize(w: np.ndarray, quant_type='int8', dims: Union[int, Sequen
     wq = np.empty(w.shape, dtype=np.int8 if bits == 8 else np.int16)
     scale = np.empty(scale_shape, dtype=w.dtype)
     if w.dtype == np.float16:
-        table = rcp_table() if use_rcp_table else None
-        lib.oracle_quantize_f16(_ptr(w), _ptr(wq), _ptr(scale), rows, cols, reduce_dim, bits, _ptr(table))
+        lib.oracle_quantize_f16(_ptr(w), _ptr(wq), _ptr(scale), rows, cols, reduce_dim, bits)
     elif w.dtype == np.float32:
         lib.oracle_quantize_f32(_ptr(w), _ptr(wq), _ptr(scale), rows, cols, reduce_dim, bits, 1 if x86_fast_math else 0)
     else:

@@ -10,19 +10,13 @@
  *       f32 : the code its CPU (x86) backend generates -- fmaxf, '/', roundf
  *             (python/hidet/ir/primitives/cpu/math/float32.py:40), loops as generated by the
  *             auto-scheduler (one output per iteration, serial reduction);
- *       f16 : the code its CUDA backend generates -- __hmax, __half operator/ (= __hdiv),
- *             hrint, (int8_t)(short) cast (python/hidet/ir/primitives/cuda/math/float16.py:62-76,
- *             python/hidet/backend/codegen.py:452-453), with __hdiv restated from CUDA 12.9's public
- *             cuda_fp16.hpp: rcp.approx.ftz.f32 of the divisor, one f32 multiply, one rounding to
- *             half, and a correction step for results below 0x008F.
+ *       f16 : the code its CUDA backend generates -- __hmax, __half operator/, hrint, (int8_t)(short)
+ *             cast (python/hidet/ir/primitives/cuda/math/float16.py:62-76,
+ *             python/hidet/backend/codegen.py:452-453).  The division is taken as what it is documented to
+ *             be, the quotient rounded to the nearest half, ties to even.
  *   - SymmetricQuantizedMatmulTask, python/hidet/graph/ops/quant/matmul.py:24-74, and the
  *     dequantize-then-matmul composition the quantization pass builds first
  *     (python/hidet/graph/transforms/graph_patterns/quant/linear.py:37-49).
- *
- * rcp.approx.ftz.f32 is a hardware approximation with no published bit-level definition.  The f16
- * functions therefore take an optional table with the instruction's result for each of the 65536
- * half bit patterns (measured once on a B200 by tests/golden/make_rcp_table.py).  Without the table
- * the correctly rounded reciprocal is used.
  *
  * Parity status: the f32 functions are pinned against outputs of the reference's own compiled CPU
  * tasks (tests/golden/reference_cpu_*.npz).  The reference's own tests hold no bit-level vectors for
@@ -126,27 +120,10 @@ static inline uint16_t h_abs_ref(uint16_t w) {
     return le ? w : (uint16_t)(w ^ 0x8000u);
 }
 
-/* rcp.approx.ftz.f32 of a value that is exactly a half: table lookup or the correctly rounded value */
-static inline float rcp_of_half(uint16_t b, const uint32_t *rcp_table) {
-    if (rcp_table != NULL) return bits_to_float(rcp_table[b]);
-    return 1.0f / half_to_float(b);
-}
-
-/* __hdiv of cuda_fp16.hpp (device path) */
-static inline uint16_t h_div(uint16_t a, uint16_t b, const uint32_t *rcp_table) {
-    const float fa = half_to_float(a);
-    const float fb = half_to_float(b);
-    const float rcp = rcp_of_half(b, rcp_table);
-    float fv = rcp * fa;
-    uint16_t v = float_to_half(fv);
-    const uint16_t av = (uint16_t)(v & 0x7fffu);
-    if (av < 0x008fu && av > 0u) { /* __hlt(abs, den) && __hlt(0, abs); never true for NaN */
-        const float err = fmaf(-fb, fv, fa);
-        fv = fmaf(rcp, err, fv);
-        v = float_to_half(fv);
-    }
-    return v;
-}
+/* a / b, rounded to the nearest half.  The IEEE f32 quotient in between changes nothing: a quotient of two 11-bit
+ * significands is either exactly half-way between two halves, and then f32 holds it exactly, or at least 2^-23 of its
+ * value away from there, and one f32 rounding moves it by at most 2^-24. */
+static inline uint16_t h_div(uint16_t a, uint16_t b) { return float_to_half(half_to_float(a) / half_to_float(b)); }
 
 /* hrint: cvt.rni.f16.f16 */
 static inline uint16_t h_rint(uint16_t h) {
@@ -179,7 +156,7 @@ static inline uint16_t h_mul(uint16_t a, uint16_t b) { return float_to_half(half
  * Follows the three generated kernels: y (absmax), quantize, scaling.
  */
 ORACLE_API void oracle_quantize_f16(const uint16_t *w, void *wq, uint16_t *scale, int64_t rows, int64_t cols,
-                                    int reduce_dim, int q_bits, const uint32_t *rcp_table) {
+                                    int reduce_dim, int q_bits) {
     const uint16_t qmax = float_to_half(q_bits == 8 ? 127.0f : 32767.0f);
     const int64_t n_out = reduce_dim == 0 ? cols : rows;
     const int64_t n_red = reduce_dim == 0 ? rows : cols;
@@ -189,11 +166,11 @@ ORACLE_API void oracle_quantize_f16(const uint16_t *w, void *wq, uint16_t *scale
     for (int64_t o = 0; o < n_out; ++o) {
         uint16_t acc = 0xfbffu; /* (half)-65504.0f */
         for (int64_t v = 0; v < n_red; ++v) acc = h_max(acc, h_abs_ref(w[o * out_stride + v * red_stride]));
-        const uint16_t s = h_div(acc, qmax, rcp_table);
+        const uint16_t s = h_div(acc, qmax);
         scale[o] = s;
         for (int64_t v = 0; v < n_red; ++v) {
             const int64_t idx = o * out_stride + v * red_stride;
-            const int16_t q = h_to_short_rz(h_rint(h_div(w[idx], s, rcp_table)));
+            const int16_t q = h_to_short_rz(h_rint(h_div(w[idx], s)));
             if (q_bits == 8) ((int8_t *)wq)[idx] = (int8_t)q; /* (int8_t)(short): keeps the low byte */
             else ((int16_t *)wq)[idx] = q;
         }
@@ -352,4 +329,4 @@ ORACLE_API int oracle_num_threads(void) {
 /* conversions exported for the tests of this file */
 ORACLE_API float oracle_half_to_float(uint16_t h) { return half_to_float(h); }
 ORACLE_API uint16_t oracle_float_to_half(float f) { return float_to_half(f); }
-ORACLE_API uint16_t oracle_hdiv(uint16_t a, uint16_t b, const uint32_t *rcp_table) { return h_div(a, b, rcp_table); }
+ORACLE_API uint16_t oracle_hdiv(uint16_t a, uint16_t b) { return h_div(a, b); }
