@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from typing import Dict, List
 
@@ -22,6 +23,8 @@ OBJ_DIR = os.path.join(PKG_DIR, 'csrc', 'build')
 LIB_DIR = os.path.join(PKG_DIR, 'lib')
 LIB_NAME = 'libhidet_b200q.so'
 LIB_PATH = os.path.join(LIB_DIR, LIB_NAME)
+HOST_SOURCE = os.path.join(SRC_DIR, 'host.cpp')
+HOST_PATH = os.path.join(LIB_DIR, 'hidet_b200_host.so')
 
 ARCH_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a']
 COMMON_FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xcompiler', '-fvisibility=hidden']
@@ -65,6 +68,27 @@ def _compile(nvcc: str, src: str, verbose: bool) -> str:
     return obj
 
 
+def build_host_module(force: bool = False) -> str:
+    """The CPython module of csrc/host.cpp: host code only, against torch's headers and libraries.  Returns its path."""
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(
+            os.path.getmtime(HOST_SOURCE), os.path.getmtime(__file__), os.path.getmtime(os.path.join(PKG_DIR, '..', 'include', 'hidet_b200q.h'))):
+        return HOST_PATH
+    import torch
+
+    torch_dir = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda_dir = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    include = [os.path.join(torch_dir, 'include'), os.path.join(torch_dir, 'include', 'torch', 'csrc', 'api', 'include'),
+               os.path.join(cuda_dir, 'include'), sysconfig.get_paths()['include']]
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cmd = [os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-fvisibility=hidden',
+           '-D_GLIBCXX_USE_CXX11_ABI={}'.format(int(torch._C._GLIBCXX_USE_CXX11_ABI)), *('-isystem' + d for d in include), HOST_SOURCE, '-o', HOST_PATH,
+           '-L' + os.path.join(torch_dir, 'lib'), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch_python']
+    res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        raise RuntimeError('g++ failed for host.cpp:\n{}\n{}'.format(' '.join(cmd), res.stdout))
+    return HOST_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
     """Compile what is out of date and link the shared library.  Returns its path."""
     nvcc = find_nvcc()
@@ -81,6 +105,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         with ThreadPoolExecutor(max_workers=min(8, len(stale))) as pool:
             list(pool.map(lambda s: _compile(nvcc, s, verbose), stale))
     objs = [os.path.join(OBJ_DIR, s[:-3] + '.o') for s in sources()]
+    build_host_module(force)
     if stale or not os.path.exists(LIB_PATH):
         cmd = [nvcc, *ARCH_FLAGS, '-shared', '-o', LIB_PATH, *objs, '-cudart', 'static']
         res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)

@@ -16,6 +16,8 @@ from typing import Any, Callable, List, Optional, Sequence
 
 import torch
 
+from .runtime import workspaces
+
 
 class CudaGraph:
     def __init__(self, f_create_inputs: Callable[[], List[torch.Tensor]], f_run: Callable[[List[torch.Tensor]], List[torch.Tensor]],
@@ -27,13 +29,17 @@ class CudaGraph:
         device = self._inputs[0].device
         self._stream = torch.cuda.Stream(device)
         self._stream.wait_stream(torch.cuda.current_stream(device))
-        with torch.cuda.stream(self._stream):
-            for _ in range(max(num_warmup, 1)):  # allocates per-stream workspaces before the capture
-                f_run(self._inputs)
-            self._stream.synchronize()
-            self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph, stream=self._stream):
-                outputs = f_run(self._inputs)
+        around = workspaces.swap(device, self._stream.cuda_stream, None)
+        try:
+            with torch.cuda.stream(self._stream):
+                for _ in range(max(num_warmup, 1)):  # allocates the graph's scratch before the capture
+                    f_run(self._inputs)
+                self._stream.synchronize()
+                self._graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(self._graph, stream=self._stream):
+                    outputs = f_run(self._inputs)
+        finally:
+            self._scratch = workspaces.swap(device, self._stream.cuda_stream, around)  # kept for the replays
         self._outputs: List[torch.Tensor] = list(outputs) if isinstance(outputs, (list, tuple)) else [outputs]
 
     @property

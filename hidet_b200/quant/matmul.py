@@ -12,7 +12,7 @@ from typing import Optional
 
 import torch
 
-from .. import ffi
+from .. import ffi, native
 from ..runtime import current_stream_ptr, require_cuda, workspaces
 
 _LAYOUTS = {'KN': ffi.LAYOUT_KN, 'NK': ffi.LAYOUT_NK}
@@ -78,6 +78,9 @@ def symmetric_quant_matmul(a: torch.Tensor, weight: torch.Tensor, scale: torch.T
     columns are (gate_j, up_j) pairs (see interleave_gate_up) and the result, N / 2 wide, is
     silu(gate) * up.  residual has the shape of the result.
     """
+    c = native.linear(a, weight, scale, weight_layout, out, bias, residual, activation)
+    if c is not None:
+        return c
     m, n, k = _check_operands(a, weight, scale, weight_layout)
     if activation not in _ACTIVATIONS:
         raise ValueError("activation must be None or 'silu_mul', got {!r}".format(activation))

@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .. import ffi
+from .. import ffi, native
 from ..runtime import current_stream_ptr, require_cuda, workspaces
 
 
@@ -62,6 +62,9 @@ class FpAIntBGemm:
         self.name, self.k, self.n, self.group_size, self.with_zp = name, k, n, group_size, with_zp
 
     def __call__(self, a: torch.Tensor, b: torch.Tensor, scale: torch.Tensor, zeros: torch.Tensor = None) -> torch.Tensor:
+        c = native.w4(a, b, scale, zeros if self.with_zp else None, self.k, self.n, self.group_size) if zeros is not None or not self.with_zp else None
+        if c is not None:
+            return c
         require_cuda(a, 'a')
         require_cuda(b, 'b')
         require_cuda(scale, 'scale')

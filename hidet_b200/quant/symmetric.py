@@ -9,7 +9,7 @@ from typing import List, Sequence, Tuple, Union
 
 import torch
 
-from .. import ffi
+from .. import ffi, native
 from ..runtime import FLOAT_CODES, QUANT_CODES, QUANT_NAMES, current_stream_ptr, require_cuda
 
 
@@ -70,6 +70,9 @@ def symmetric_quantize(w: torch.Tensor, quant_type: Union[str, torch.dtype] = 'i
     wq has w's shape; scale has w's dtype and w's shape without `dims`.  Bit-identical to the
     reference's result for the same input (python/hidet/graph/ops/quant/symmetric.py:23-47).
     """
+    pair = native.quantize(w, quant_type, dims)
+    if pair is not None:
+        return pair
     require_cuda(w, 'w')
     if w.dtype not in FLOAT_CODES:
         raise ValueError('symmetric_quantize expects float16, bfloat16 or float32, got {}'.format(w.dtype))
@@ -90,6 +93,9 @@ def symmetric_quantize(w: torch.Tensor, quant_type: Union[str, torch.dtype] = 'i
 def symmetric_dequantize(wq: torch.Tensor, scale: torch.Tensor, dims: Union[int, List[int]] = -1) -> torch.Tensor:
     """Returns scale.dtype(wq) * scale, scale broadcast along `dims`
     (python/hidet/graph/ops/quant/symmetric.py:50-61)."""
+    w = native.dequantize(wq, scale, dims)
+    if w is not None:
+        return w
     require_cuda(wq, 'wq')
     require_cuda(scale, 'scale')
     if wq.dtype not in QUANT_CODES:
@@ -118,6 +124,9 @@ def symmetric_dequantize_take(wq: torch.Tensor, scale: torch.Tensor, indices: to
     embedding.py:22-39), without materialising the dequantized table.  wq is int8 / int16 [vocab, dim]
     quantized per row, scale [vocab]; indices are int32 or int64 of any shape; the result has shape
     indices.shape + [dim] and scale's dtype, and equals the rows of the dequantized table bit for bit."""
+    out = native.take(wq, scale, indices)
+    if out is not None:
+        return out
     require_cuda(wq, 'wq')
     require_cuda(scale, 'scale')
     require_cuda(indices, 'indices')

@@ -5,11 +5,11 @@ libhidet_b200q.so.
 """
 from __future__ import annotations
 
-from typing import Dict, Tuple
+from typing import Dict, Optional, Tuple
 
 import torch
 
-from . import ffi
+from . import ffi, native
 
 FLOAT_CODES = {torch.float16: ffi.F16, torch.bfloat16: ffi.BF16, torch.float32: ffi.F32}
 QUANT_CODES = {torch.int8: ffi.I8, torch.int16: ffi.I16}
@@ -50,10 +50,25 @@ class _Workspaces:
             size = 1 << max(20, (nbytes - 1).bit_length())
             buf = torch.zeros(size, dtype=torch.uint8, device=torch.device('cuda', index))
             self._buffers[key] = buf
+            native.load().set_scratch(*key, buf.data_ptr(), buf.numel())  # for the native host path
         return buf.data_ptr(), buf.numel()
 
     def clear(self) -> None:
         self._buffers.clear()
+        if native._module is not None:
+            native._module.clear_scratch()
+
+    def swap(self, device: torch.device, stream: int, buffer: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+        """Puts `buffer` (None: nothing, a new one is made when it is needed) in the place of a stream's scratch and
+        returns what was there.  A captured graph takes the buffer its launches were recorded with into its own keeping
+        this way: streams come from a small pool, so a later graph or eager call may run on the same one, and must neither
+        share the buffer nor replace it by a larger one while the graph still writes to it."""
+        index = device.index if device.index is not None else torch.cuda.current_device()
+        before = self._buffers.pop((index, stream), None)
+        if buffer is not None:
+            self._buffers[(index, stream)] = buffer
+        native.load().set_scratch(index, stream, buffer.data_ptr() if buffer is not None else 0, buffer.numel() if buffer is not None else 0)
+        return before
 
 
 workspaces = _Workspaces()
