@@ -19,8 +19,7 @@
 //
 // The kernel is launched as a programmatic dependent of the kernel before it in the stream: weight
 // tiles and scales do not depend on that kernel, so they are requested before waiting for it, and the
-// kernel after this one is allowed to start once the main loop is over.  (Letting it start earlier was
-// measured and is slower: its weight requests then queue in front of this kernel's own.)
+// kernel after this one may start as soon as that wait is over.
 //
 // Replaces the generated mma.sync kernel of python/hidet/graph/ops/quant/matmul_f16_i8.py:136-485
 // (f16 accumulation, 64x128 tiles, no split-K by default) for M <= 16, and serves larger M by
@@ -33,21 +32,29 @@
 namespace b200q {
 namespace decode {
 
-constexpr int BN = 128;                      // columns per CTA
 constexpr int BK = 64;                       // k rows per pipeline stage
-constexpr int BM = 16;                       // activation rows per CTA
+constexpr int BN = 128;                      // columns per CTA
 constexpr int STAGES = 4;
 constexpr int CONSUMER_WARPS = 4;            // each owns BN / 4 = 32 columns
 constexpr int THREADS = 32 * (CONSUMER_WARPS + 1);
 constexpr int W_STAGE_BYTES = BK * BN;       // 8192
-constexpr int A_STAGE_BYTES = BM * BK * 2;   // 2048
-constexpr int PIPE_BYTES = STAGES * (W_STAGE_BYTES + A_STAGE_BYTES);
 constexpr int RECV_COLS = 168;               // most columns the slices of a cluster cover together (7 ranks x 24 columns)
-constexpr int RECV_BYTES = BM * RECV_COLS * 4; // partial tiles sent by the CTAs of the cluster: [rank][row][cols_per] fp32
 constexpr int STAGING_ROW = 36;              // floats per row of a warp's 32-column staging block (padded: conflict-free)
-constexpr int SMEM_BYTES = PIPE_BYTES + RECV_BYTES + 1024;  // + alignment slack
-static_assert(CONSUMER_WARPS * BM * STAGING_ROW * 4 <= STAGES * W_STAGE_BYTES, "the staging blocks reuse the weight ring");
-constexpr int kCtasPerSm = 4;                // resident CTAs per SM the plan aims at
+
+// Shared memory of a CTA with MT blocks of eight activation rows.
+template <int MT>
+struct Config {
+    static constexpr int ROWS = 8 * MT;                  // activation rows per CTA
+    static constexpr int A_STAGE_BYTES = ROWS * BK * 2;
+    static constexpr int PIPE_BYTES = STAGES * (W_STAGE_BYTES + A_STAGE_BYTES);
+    static constexpr int RECV_BYTES = ROWS * RECV_COLS * 4;  // partial tiles sent by the CTAs of the cluster: [rank][row][cols_per] fp32
+    // + alignment slack; and at least what keeps a fifth CTA off an SM.  The CTAs of the next launch move in beside this
+    // one's (see the kernel) and fill their rings ahead of it; more of them than the fourth slots hold take the
+    // memory system away from the launch they wait for: (1, 4096, 12288) 10.3 -> 11.1 us, (1, 4096, 32000) 22.1 -> 24.0 us.
+    static constexpr int NEED = PIPE_BYTES + RECV_BYTES + 1024;
+    static constexpr int SMEM_BYTES = NEED < 46 * 1024 + 512 ? 46 * 1024 + 512 : NEED;
+    static_assert(CONSUMER_WARPS * ROWS * STAGING_ROW * 4 <= STAGES * W_STAGE_BYTES, "the staging blocks reuse the weight ring");
+};
 constexpr int64_t kMaxCounters = 65536;      // arrival counters at the head of the workspace
 constexpr int kMaxCluster = 8;               // largest cluster of the plan (8 is the portable limit; the reduction reads up to eight partials)
 
@@ -185,7 +192,7 @@ __device__ __forceinline__ void finish(const OutTargets &o, const Epilogue &ep, 
         col = nn >> 1;
     }
     if (!valid || nn >= n_limit) return;
-    if (ep.residual != nullptr) y += __half2float(__ldg(static_cast<const __half *>(ep.residual) + (size_t)row * ep.ldr + col));
+    if (ep.residual != nullptr) y += __half2float(__ldcg(static_cast<const __half *>(ep.residual) + (size_t)row * ep.ldr + col));  // through L2: this CTA may be older than the kernel that wrote it
     store_out(o, row, col, __float2half_rn(y));
 }
 
@@ -212,6 +219,8 @@ struct Params {
 //     plain matrix loads; everything else is shared.
 template <int MT, bool NK>
 __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
+    using Cfg = Config<MT>;
+    constexpr int ROWS = Cfg::ROWS, A_STAGE_BYTES = Cfg::A_STAGE_BYTES, PIPE_BYTES = Cfg::PIPE_BYTES;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t full_bar[STAGES];
     __shared__ __align__(8) uint64_t empty_bar[STAGES];
@@ -232,14 +241,14 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
     const int t = lane & 3;   // thread in group
     const int n0 = blockIdx.x * BN;
     const int split = blockIdx.y;
-    const int m0 = blockIdx.z * BM;
+    const int m0 = blockIdx.z * ROWS;
     const int total_iters = (p.k_end - p.k_begin + BK - 1) / BK;
     const int it_begin = split * p.iters_per_split;
     int n_iters = total_iters - it_begin;
     if (n_iters > p.iters_per_split) n_iters = p.iters_per_split;
     if (n_iters < 0) n_iters = 0;
     int rows = p.M - m0;
-    if (rows > BM) rows = BM;
+    if (rows > ROWS) rows = ROWS;
     const uint32_t nranks = cluster_nctarank();
     const uint32_t rank = cluster_ctarank();
     const int cols_per = p.cols_per;
@@ -283,7 +292,8 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
     if (warp == CONSUMER_WARPS) {
         // ---------------- producer warp ----------------
         // Lane 0 drives the TMA loads of the weight tiles.  The activation slices (8 MT rows x 64 k of f16 per stage,
-        // 128-byte rows, 16-byte chunk c of row r at chunk c ^ (r & 7), the layout a 128B-swizzled TMA tile would have)
+        // 128-byte rows, 16-byte chunk c of row r at chunk c ^ 2 (r & 3), so that a consumer's 8-byte loads of four rows touch
+        // every bank once)
         // are copied by all 32 lanes with cp.async: they are a few hundred bytes that sit in L2, and on the load/store
         // path they do not wait in the TMA queue behind weight tiles that are still on their way from HBM.
         uint32_t dst_off[2 * MT];
@@ -293,10 +303,16 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
         for (int q = 0; q < 2 * MT; ++q) {
             const int chunk = lane + 32 * q;  // 8 chunks per row
             const int r = chunk >> 3, c = chunk & 7;
-            dst_off[q] = r * 128 + ((c ^ (r & 7)) << 4);
+            dst_off[q] = r * 128 + ((c ^ ((r & 3) << 1)) << 4);
             src_row[q] = m0 + r < p.M ? p.a + (size_t)(m0 + r) * p.lda : nullptr;  // rows beyond M are zero-filled
             kc[q] = 8 * c;
         }
+        auto load_weights = [&](int s, int it, uint64_t policy) {
+            const uint32_t bar = smem_u32(&full_bar[s]);
+            const int k0 = p.k_begin + (it_begin + it) * BK;
+            mbar_expect_tx(bar, W_STAGE_BYTES);
+            tma_load_2d_hint(w_base + s * W_STAGE_BYTES, &map_w, NK ? k0 : n0, NK ? n0 : k0, bar, policy);
+        };
         auto copy_activations = [&](int s, int k0) {
 #pragma unroll
             for (int q = 0; q < 2 * MT; ++q) {
@@ -313,14 +329,17 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
             stream_policy = l2_policy_evict_first();  // the weight is read once
             // The weight does not depend on the kernel before this one in the stream; the activations
             // may.  Ask for the first weight tiles, then wait for that kernel, then ask for activations.
-            for (int it = 0; it < prologue; ++it) {
-                const uint32_t bar = smem_u32(&full_bar[it]);
-                mbar_expect_tx(bar, W_STAGE_BYTES);
-                tma_load_2d_hint(w_base + it * W_STAGE_BYTES, &map_w, NK ? p.k_begin + (it_begin + it) * BK : n0, NK ? n0 : p.k_begin + (it_begin + it) * BK, bar, stream_policy);
-            }
+            for (int it = 0; it < prologue; ++it) load_weights(it, it, stream_policy);
         }
         __syncwarp();
         pdl_wait();
+        // The kernel in front is done; the one behind may move in now: its CTAs fill their rings while this launch streams
+        // the rest of its weight, so that it starts with its first stages in shared memory.  Two launches at a time is as
+        // far ahead as pays: allowed at the very start, its successors pile up and all their rings compete with this one's
+        // (1, 4096, 4096: 4.9 us here, 5.5 at the end of the main loop, 5.9 at the start).  With several row blocks the
+        // launch lives from L2, which the next one's rings would only crowd (19 rows through a 7B-shaped step: 458 us, 451
+        // at the end of the main loop).
+        if (gridDim.z == 1) pdl_launch_dependents();
         for (int it = 0; it < prologue; ++it) copy_activations(it, p.k_begin + (it_begin + it) * BK);
         for (int it = STAGES; it < n_iters; ++it) {
             const int s = it % STAGES;
@@ -329,11 +348,7 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
                 break;
             }
             const int k0 = p.k_begin + (it_begin + it) * BK;
-            if (lane == 0) {
-                const uint32_t bar = smem_u32(&full_bar[s]);
-                mbar_expect_tx(bar, W_STAGE_BYTES);
-                tma_load_2d_hint(w_base + s * W_STAGE_BYTES, &map_w, NK ? k0 : n0, NK ? n0 : k0, bar, stream_policy);
-            }
+            if (lane == 0) load_weights(s, it, stream_policy);
             copy_activations(s, k0);
         }
     } else {
@@ -350,7 +365,7 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
         // Activations: row g (and g + 8, same swizzle phase), k = 16 ks + 4t .. 4t+3: bytes 8 (t & 1) of
         // chunk 2 ks + (t >> 1).
         const uint32_t off_a = g * 128 + 8 * (t & 1);
-        const uint32_t a_chunk = (uint32_t)(t >> 1) ^ (uint32_t)g;  // chunk index is (2 ks) ^ a_chunk: bit 0 of 2 ks is free
+        const uint32_t a_chunk = (uint32_t)(t >> 1) ^ (uint32_t)((g & 3) << 1);  // chunk index is (2 ks) ^ a_chunk: bit 0 of 2 ks is free
         for (int it = 0; it < n_iters; ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1)) {
@@ -399,7 +414,7 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
         }
     }
     __syncwarp();  // the role branches above are lane-divergent; the cluster barrier below wants whole warps
-    pdl_launch_dependents();  // the next kernel may start streaming its weight
+    if (gridDim.z > 1) pdl_launch_dependents();
 
     const bool consumer = warp < CONSUMER_WARPS;
     // This thread's four columns inside the tile: 32 warp + 16 j + 8 h + g.
@@ -447,13 +462,13 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
                         const uint32_t rbar = map_to_rank(smem_u32(&recv_bar), owner);
 #pragma unroll
                         for (int e = 0; e < 2; ++e)
-                            if (e < rows) st_async_f32(remote + (((int)rank * BM + e) * cols_per + col_in) * 4, acc[j][0][2 * h + e], rbar);
+                            if (e < rows) st_async_f32(remote + (((int)rank * ROWS + e) * cols_per + col_in) * 4, acc[j][0][2 * h + e], rbar);
                     }
             }
         } else {
             // More rows: transpose through a staging block in the (now idle) weight ring, then 16-byte remote stores.
             asm volatile("bar.sync 1, %0;" ::"n"(32 * CONSUMER_WARPS) : "memory");  // every consumer warp is done with the ring
-            const uint32_t stage_w = w_base + warp * (BM * STAGING_ROW * 4);
+            const uint32_t stage_w = w_base + warp * (ROWS * STAGING_ROW * 4);
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -468,10 +483,10 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
             const int col = 32 * warp + 4 * v4;
             const uint32_t owner = (uint32_t)(col / cols_per);
             const int col_in = col - (int)owner * cols_per;
-            const uint32_t remote = map_to_rank(recv_base, owner) + (((int)rank * BM) * cols_per + col_in) * 4;
+            const uint32_t remote = map_to_rank(recv_base, owner) + (((int)rank * ROWS) * cols_per + col_in) * 4;
             const uint32_t rbar = map_to_rank(smem_u32(&recv_bar), owner);
 #pragma unroll
-            for (int pass = 0; pass < BM / 4; ++pass) {
+            for (int pass = 0; pass < ROWS / 4; ++pass) {
                 const int r = pass * 4 + rr;
                 if (r < rows) st_async_v4f32(remote + r * cols_per * 4, lds128f(stage_w + (r * STAGING_ROW + 4 * v4) * 4), rbar);
             }
@@ -486,7 +501,7 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
     auto sum_ranks = [&](int r, int cc) {
         float v[8];
 #pragma unroll
-        for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? recv[(jr * BM + r) * cols_per + cc] : 0.0f;
+        for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? recv[(jr * ROWS + r) * cols_per + cc] : 0.0f;
         float sum = v[0];
 #pragma unroll
         for (int jr = 1; jr < 8; ++jr) sum += v[jr];
@@ -542,33 +557,100 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
 
 }  // namespace decode
 
+namespace decode {
+
+// One instantiation of the kernel per layout: up to eight activation rows, and more.
+struct Variant {
+    const void *kn, *nk;
+    int rows, smem;
+};
+template <int MT>
+static Variant make_variant() {
+    return {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true>),
+            Config<MT>::ROWS, Config<MT>::SMEM_BYTES};
+}
+static const Variant kVariants[2] = {make_variant<1>(), make_variant<2>()};
+static const Variant &variant(int64_t M) { return kVariants[M <= 8 ? 0 : 1]; }
+
+static int set_attributes() {
+    static std::atomic<bool> attr_set[64];  // per device, zero-initialised; a repeated set by a racing thread is harmless
+    int dev = 0;
+    B200Q_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        for (const Variant &v : kVariants)
+            for (const void *f : {v.kn, v.nk}) B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
+    return B200Q_OK;
+}
+
+// CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use, because a
+// cluster's CTAs stay within one group of SMs.  Asked of the runtime once per device; without a device, an estimate.
+static int resident_ctas(const Variant &v, int cluster) {
+    static std::atomic<int> known[64][2][kMaxCluster + 1];
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || set_attributes() != B200Q_OK) {
+        cudaGetLastError();
+        return 148 * 4 - 30;
+    }
+    std::atomic<int> &slot = known[dev][&v - kVariants][cluster];
+    int n = slot.load(std::memory_order_relaxed);
+    if (n != 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, (unsigned)cluster, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = v.smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = (unsigned)cluster;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, v.kn, &cfg) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        return 148 * 4 - 30;
+    }
+    n *= cluster;
+    slot.store(n, std::memory_order_relaxed);
+    return n;
+}
+
+}  // namespace decode
+
 // Split plan shared by the workspace query and the launch.
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     using namespace decode;
     DecodePlan pl;
+    const Variant &v = variant(M);
     pl.n_tiles = (int)ceil_div(N, BN);
-    pl.m_tiles = (int)ceil_div(M, BM);
+    pl.m_tiles = (int)ceil_div(M, v.rows);
     const int k_iters = (int)ceil_div(K, BK);
     int sms = sm_count();
     if (sms <= 0) sms = 148;
-    const int64_t target = (int64_t)sms * kCtasPerSm;
     const int64_t tiles = (int64_t)pl.n_tiles * pl.m_tiles;
-    // CTAs per tile that fill the machine once, each with at least eight 64-row steps of work.
-    int64_t splits = tiles > 0 ? target / tiles : 1;
-    const int max_splits = k_iters / 8 > 0 ? k_iters / 8 : 1;
-    if (splits > max_splits) splits = max_splits;
-    if (splits > 64) splits = 64;
-    if (splits < 1) splits = 1;
-    // The splits of a tile form clusters of up to eight CTAs (partials meet in distributed shared
-    // memory); more splits than a cluster holds become several full clusters per tile that meet in the
-    // workspace.
-    int c = (int)(splits < kMaxCluster ? splits : kMaxCluster);
-    int groups = (int)(splits / c);
-    if (groups < 1 || tiles * c > kMaxCounters) groups = 1;
-    // Clusters that meet in the workspace pay three dependent trips through L2 at the end of the launch (publish,
-    // count, read back), about 3 us more than partials that meet in distributed shared memory.  That is worth it only
-    // when one cluster per tile would leave most of the machine idle.
-    if (groups > 1 && tiles * c * 2 >= sms) groups = 1;
+    // Each split has at least four 64-row steps of work, a ring's fill: with eight a narrow problem leaves most of the SMs
+    // idle (a step of a 1024-wide decoder 72 -> 57 us), with two the exchange costs what the shorter loop gives (64 us).
+    int64_t max_splits = k_iters / 4 > 0 ? k_iters / 4 : 1;
+    if (max_splits > 64) max_splits = 64;
+    // The splits of a tile form a cluster of up to eight CTAs (partials meet in distributed shared memory), as large as lets
+    // the whole grid run at once: a few clusters left for a second wave double the time of the launch (96 tiles
+    // in clusters of six are 576 CTAs and fit 148 x 4 slots by number, but not the groups of SMs clusters are confined to:
+    // (1, 4096, 12288) 15.1 us, and 10.3 us in clusters of five).
+    int c = 1;
+    // (With several row blocks the second pass over the weight comes from L2 and a second wave costs little.)
+    while (c < kMaxCluster && c < max_splits && tiles * (c + 1) <= (pl.m_tiles > 1 ? (int64_t)sms * 4 : resident_ctas(v, c + 1))) ++c;
+    // More splits than a cluster holds become several full clusters per tile that meet in the workspace.  They pay three
+    // dependent trips through L2 at the end of the launch (publish, count, read back), about 3 us more than partials
+    // that meet in distributed shared memory.  That is worth it only when one cluster per tile would leave most of the
+    // machine idle.
+    int groups = 1;
+    if (c == kMaxCluster && tiles * c * 2 < sms) {
+        int64_t splits = tiles > 0 ? (int64_t)sms * 4 / tiles : 1;
+        if (splits > max_splits) splits = max_splits;
+        groups = (int)(splits / c);
+        if (groups < 1 || tiles * c > kMaxCounters) groups = 1;
+    }
     pl.cluster = c;
     pl.groups = groups;
     pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
@@ -641,25 +723,14 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     p.cols_per = (int)round_up(ceil_div(BN, pl.cluster), 8);
     p.mode = pl.splits == 1 ? kModeDirect : kModeSplit;
 
-    const bool one_block = M - (int64_t)(pl.m_tiles - 1) * BM <= 8 && pl.m_tiles == 1;
-    auto kernel = weight_nk ? (one_block ? qlinear_decode_kn_kernel<1, true> : qlinear_decode_kn_kernel<2, true>)
-                            : (one_block ? qlinear_decode_kn_kernel<1, false> : qlinear_decode_kn_kernel<2, false>);
-    static std::atomic<bool> attr_set[64];  // per device, zero-initialised; a repeated set by a racing thread is harmless
-    int dev = 0;
-    B200Q_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        const void *all[4] = {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<1, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<2, false>),
-                              reinterpret_cast<const void *>(qlinear_decode_kn_kernel<1, true>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<2, true>)};
-        for (const void *f : all) {
-            B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-            B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        }
-        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
-    }
+    const Variant &v = variant(M);
+    const void *kernel = weight_nk ? v.nk : v.kn;
+    const int rc_attr = set_attributes();
+    if (rc_attr != B200Q_OK) return rc_attr;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)pl.n_tiles, (unsigned)pl.splits, (unsigned)pl.m_tiles);
     cfg.blockDim = dim3(THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.dynamicSmemBytes = v.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
     attrs[0].id = cudaLaunchAttributeClusterDimension;
@@ -670,7 +741,8 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = 2;
-    B200Q_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, p));
+    void *args[2] = {&map_w, &p};
+    B200Q_CUDA_TRY(cudaLaunchKernelExC(&cfg, kernel, args));
     return B200Q_OK;
 }
 
