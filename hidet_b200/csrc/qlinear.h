@@ -79,6 +79,10 @@ int launch_prefill_kn(const void *a, const void *wq, const void *scale, void *c,
 // The same kernel on a weight stored [N, K] (weight_nk = true): 16-byte aligned bases, K % 16 == 0, N % 8 == 0.
 bool prefill_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
 
+// [K, N] weights whose rows are not multiples of 16 bytes: N even, K a multiple of 8, 16-byte aligned bases.
+bool unaligned_supported(const void *a, const void *wq, const void *c, int64_t M, int64_t N, int64_t K);
+int launch_unaligned(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+
 // Which kernel serves M activation rows.  The tensor-memory kernel's tiles span 64 or 256 rows and it
 // streams every weight tile once per row block; the small-M kernel re-streams the weight once per 16
 // rows (from L2 after the first pass).  Up to 32 rows the small-M kernel always wins, up to 64 rows it

@@ -95,6 +95,10 @@ B200Q_API int b200q_qlinear_f16_i8(const void *a, const void *wq, const void *sc
     if (w_layout == B200Q_LAYOUT_NK && decode_nk_supported(a, wq, N, K)) {
         return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, workspace, workspace_bytes, s, nullptr, nullptr, true);
     }
+    // Rows that are not multiples of 16 bytes.  The line is where that kernel's loads stay aligned; on the far side of it
+    // (odd N, K not a multiple of 8, unaligned bases) only the one-thread-per-element kernel is left: (7, 4096, 32002)
+    // 420 us against 32, (1, 512, 514) 51 us against 4.
+    if (w_layout == B200Q_LAYOUT_KN && unaligned_supported(a, wq, c, M, N, K)) return launch_unaligned(a, wq, scale, c, M, N, K, s);
     return launch_generic(a, wq, scale, c, M, N, K, 0, K, w_layout, s);
 }
 

@@ -75,11 +75,28 @@ def test_qlinear_larger_m(m, k, n):
 
 @pytest.mark.parametrize('m,k,n', [(3, 100, 36), (4, 64, 20), (2, 36, 16), (1, 4098, 130)])
 def test_qlinear_unaligned_shapes(m, k, n):
-    # rows that are not 16-byte multiples take the shape-agnostic kernel
+    # rows that are not 16-byte multiples: with K a multiple of 8 the kernel for them, else the shape-agnostic one
     wq, scale = _quantized(k, n, seed=7)
     a = seeded_activation(m, k, seed=8)
     c = hidet_b200.symmetric_quant_matmul(torch.from_numpy(a).cuda(), torch.from_numpy(wq).cuda(), torch.from_numpy(scale).cuda())
     _check(a, wq, scale, c)
+
+
+@pytest.mark.parametrize('m,k,n', [(1, 8, 2), (3, 512, 114), (8, 520, 222), (1, 4096, 1006), (9, 1032, 1004), (16, 4104, 8010), (33, 768, 130), (2, 16384, 112 * 3 + 2)])
+def test_qlinear_rows_of_every_offset(m, k, n):
+    """Rows whose starts go through every (even) offset from a 16-byte boundary, around the edges of the kernel's 112-column
+    tiles, chunks of rows and 8-row blocks; one-hot activations bring back rows of the weight to the bit."""
+    wq, scale = _quantized(k, n, seed=7)
+    a = seeded_activation(m, k, seed=8)
+    wq_gpu, scale_gpu = torch.from_numpy(wq).cuda(), torch.from_numpy(scale).cuda()
+    c = hidet_b200.symmetric_quant_matmul(torch.from_numpy(a).cuda(), wq_gpu, scale_gpu)
+    _check(a, wq, scale, c)
+    rows = np.unique(np.linspace(0, k - 1, 16).astype(np.int64))
+    hot = torch.zeros(len(rows), k, dtype=torch.float16, device='cuda')
+    hot[torch.arange(len(rows)), torch.from_numpy(rows)] = 1.0
+    got = hidet_b200.symmetric_quant_matmul(hot, wq_gpu, scale_gpu)
+    assert torch.equal(got, (wq_gpu[torch.from_numpy(rows).cuda()].float() * scale_gpu.float()).half())
+    assert ffi.func('b200q_check_status')() == ffi.OK
 
 
 @pytest.mark.parametrize('parts', [1, 2, 3, 5, 16])
