@@ -44,6 +44,7 @@ unsigned int *device_status_word();  // device address for the current device (n
 
 constexpr unsigned int kKernelDecode = 1;
 constexpr unsigned int kKernelPrefill = 2;
+constexpr unsigned int kKernelU4 = 3;
 constexpr unsigned int kKernelUnaligned = 4;
 
 // Number of SMs of the current device (cached per device).

@@ -8,7 +8,7 @@
 // The weight is taken in that plain row-major form; the reference's tests first permute it into a layout private to
 // their kernel (preprocess_weight), which has no meaning outside that kernel.
 //
-// The op is bound by streaming q (half a byte per weight) once.  A thread owns eight adjacent columns (one 32-bit
+// Two kernels: on tensor cores for group sizes that are multiples of 16 (further down), and this one for the others.  A thread owns eight adjacent columns (one 32-bit
 // word per k row; a warp reads 128 contiguous bytes per row) and a slice of k.  Inside a group the scale and the zero
 // point of a column are constant, so the inner loop multiplies activations with the bare codes and keeps the sum of
 // the activations beside it; at the end of the group
@@ -17,7 +17,7 @@
 // accumulates the products, tests/cute_kernel/quantized_linear.py:1044-1047: same value up to rounding).  The k slices
 // of a CTA meet in shared memory; the CTAs that split K further write fp32 partial sums to the caller's workspace,
 // and a second kernel adds them in slice order and rounds to f16 once: the same result on every run.
-#include "common.cuh"
+#include "stream_mma.cuh"
 
 namespace b200q {
 namespace u4 {
@@ -148,6 +148,273 @@ __global__ void qlinear_u4_reduce_kernel(const float *partial, __half *c, int64_
     c[i] = __float2half_rn(s);
 }
 
+// ---- group sizes that are multiples of 16: tensor cores, one launch ----
+// Warp-level m16n8k16 MMAs with the bare codes as the 16-row operand (exact in f16) and the activations as the 8-column
+// operand, so that the codes are unpacked once for up to 8 MT activation rows and nothing is multiplied per row outside
+// the tensor core.  A CTA owns 64 W columns; its warps and the CTAs of its cluster each take a contiguous
+// run of 16-row steps.  A lane (g, t) copies W words (8 W columns) of rows 4t .. 4t + 3 of a step, DEPTH steps
+// ahead, into places of shared memory that only it reads, so the main loop has no barrier; the two columns
+// 2j, 2j + 1 of a word are rows g and g + 8 of MMA j, and the activations of the same four k are one 8-byte load.  One more
+// MMA per step with ones as the 16-row operand gives every lane the sums of its activations.  At the end of a group (or of
+// the warp's run; a part of a group is a term like any other)
+//     sum += scale * (group sum - zero * activation sum)
+// goes to the lane's own place in shared memory, where the warps, and then the cluster, are summed in a fixed order.
+// What is left is instructions (the unpacking and the MMAs) and the exchange at the end, not bytes.
+// Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 12.8 us, (8, 4096, 4096) 28.7 ->
+// 6.3, (1, 1024, 1000) 6.8 -> 2.8; (16, 12288, 4096) 127 (a call) -> 15.9, (64, 4096, 11008) 43.
+struct MmaParams {
+    const __half *a;        // [M, K]
+    const uint32_t *q;      // [K, N / 8] words
+    const __half *scale;    // [K / G, N]
+    const __half *zeros;    // [K / G, N] or null
+    __half *c;              // [M, N]
+    unsigned int *status;
+    int M, N, K;
+    int steps_per_group;    // G / 16
+};
+
+constexpr int MMA_WARPS = 4;
+constexpr int MMA_THREADS = 32 * MMA_WARPS;
+
+template <int MT, int W>
+struct MmaConfig {
+    static constexpr int TILES = 4 * W;                                 // 16-row MMAs per step
+    static constexpr int ITEMS = TILES * MT * 32;                       // float4 sums of a CTA
+    static constexpr int RED_BYTES = MMA_WARPS * ITEMS * 16;
+    static constexpr int RING_OFF = RED_BYTES + stream_mma::recv_bytes(ITEMS);
+    static constexpr int CTAS = MT == 4 ? 3 : 4;                        // per SM
+    // Steps in flight.  Short rings are enough, and let the clusters fit better: (1, 4096, 12288) takes 12.7 us with four
+    // CTAs of three steps, 15.5 with four of seven; (16, 12288, 4096) 15.9 with three and 19.3 with eight.
+    static constexpr int DEPTH = 3;
+    static constexpr int SLOT_BYTES = 32 * (16 * W + 8 * MT);           // of one warp and step: [row][lane] words, [row][32 bytes] activations
+    static constexpr int SMEM_BYTES = RING_OFF + MMA_WARPS * DEPTH * SLOT_BYTES;
+    static_assert(CTAS * (SMEM_BYTES + 1024 + 16) <= 228 * 1024, "room for CTAS per SM");
+};
+
+// Codes 0 .. 3 of two rows as f16 pairs (row 0, row 1): x holds the rows' 16-bit pieces.  0x6400 | c is 1024 + c, and with
+// the code four bits up 1024 + 16 c, of which a sixteenth less 64 is c; both exact.  (The bare bits as subnormal numbers take
+// half the instructions, but the tensor core aligns products by the operands' unnormalised exponents and the sums lose bits.)
+__device__ __forceinline__ void unpack_pairs(uint32_t x, uint32_t (&h)[4]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t lo = ((x >> (8 * i)) & 0x000f000fu) | 0x64006400u, hi = ((x >> (8 * i)) & 0x00f000f0u) | 0x64006400u;
+        asm("sub.f16x2 %0, %1, %2;" : "=r"(h[2 * i]) : "r"(lo), "r"(0x64006400u));
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(h[2 * i + 1]) : "r"(hi), "r"(0x2c002c00u), "r"(0xd400d400u));
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(N) : "memory");
+}
+
+// WIDE: W words are loaded together (rows are multiples of 4 W bytes).
+template <int MT, int W, bool WIDE>
+__global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u4_mma_kernel(const MmaParams p) {
+    using Cfg = MmaConfig<MT, W>;
+    constexpr int DEPTH = Cfg::DEPTH, TILES = Cfg::TILES;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t recv_bar;
+    stream_mma::cluster_begin(smem_u32(&recv_bar), Cfg::ITEMS);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int m0 = blockIdx.z * 8 * MT;
+    const int words_per_row = p.N / COLS_PER_THREAD;
+    const int word0 = (blockIdx.x * 8 + g) * W;      // this lane's words
+    const int n_lane = word0 * COLS_PER_THREAD;      // and their first column
+    // this warp's run of 16-row steps
+    const int steps = p.K / 16, workers = (int)cluster_nctarank() * MMA_WARPS, worker = (int)cluster_ctarank() * MMA_WARPS + warp;
+    const int share = steps / workers, extra = steps % workers;
+    const int s_begin = worker * share + min(worker, extra), s_end = s_begin + share + (worker < extra ? 1 : 0);
+
+    // Words beyond the row and rows beyond M repeat the last ones: their columns and rows of the result are not stored.
+    bool in[W];
+    const uint32_t *q_src[4][W];  // the words of the next step to fetch
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+        in[i] = word0 + i < words_per_row;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) q_src[r][i] = p.q + (size_t)(s_begin * 16 + 4 * t + r) * words_per_row + min(word0 + (WIDE ? 0 : i), words_per_row - (WIDE ? W : 1));
+    }
+    // The activations of a step are 32 bytes of each row; half a row per lane, lanes 2 (8 mt + row) and + 1, through L2 (this CTA
+    // may be older than the kernel that wrote them, and so may be what the first-level cache holds).
+    constexpr int A_COPIES = (MT + 1) / 2;
+    const __half *a_src[A_COPIES];
+#pragma unroll
+    for (int i = 0; i < A_COPIES; ++i) a_src[i] = p.a + (size_t)min(m0 + 16 * i + (lane >> 1), p.M - 1) * p.K + s_begin * 16 + 8 * (lane & 1);
+    const uint32_t ring = smem_u32(smem) + Cfg::RING_OFF + (uint32_t)warp * DEPTH * Cfg::SLOT_BYTES + lane * 4 * W;
+    const uint32_t ring_a = smem_u32(smem) + Cfg::RING_OFF + (uint32_t)warp * DEPTH * Cfg::SLOT_BYTES + 4 * W * 4 * 32;
+    const size_t step_words = (size_t)16 * words_per_row;
+    auto fetch_codes = [&](uint32_t slot) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int i = 0; i < (WIDE ? 1 : W); ++i) {
+                cp_async<WIDE ? 4 * W : 4>(ring + slot + r * 32 * 4 * W + 4 * i, q_src[r][i]);
+                q_src[r][i] += step_words;
+            }
+    };
+    auto fetch_activations = [&](uint32_t slot) {
+#pragma unroll
+        for (int i = 0; i < A_COPIES; ++i) {
+            if (MT > 1 || lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_a + slot + (i * 32 + lane) * 16), "l"(a_src[i]) : "memory");
+            a_src[i] += 16;
+        }
+    };
+    auto commit = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };  // one group per step, empty ones past the end included
+    // scales and zero points of this lane's columns in a group
+    uint4 sc[W], zp[W];
+    auto load_group = [&](int group) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const size_t off = (size_t)group * p.N + n_lane + 8 * i;
+            sc[i] = zp[i] = make_uint4(0, 0, 0, 0);
+            if (in[i]) sc[i] = __ldg(reinterpret_cast<const uint4 *>(p.scale + off));
+            if (in[i] && p.zeros != nullptr) zp[i] = __ldg(reinterpret_cast<const uint4 *>(p.zeros + off));
+        }
+    };
+
+    // acc[j][mt]: element (column n_lane + 2 j + h, row 8 mt + 2 t + e) is acc[j][mt][2 h + e]; asum[mt][e]: row 8 mt + 2 t + e
+    float acc[TILES][MT][4], asum[MT][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+            for (int j = 0; j < TILES; ++j) acc[j][mt][0] = acc[j][mt][1] = acc[j][mt][2] = acc[j][mt][3] = 0.0f;
+            asum[mt][0] = asum[mt][1] = asum[mt][2] = asum[mt][3] = 0.0f;
+        }
+    };
+    float4 *red = reinterpret_cast<float4 *>(smem) + warp * Cfg::ITEMS + lane;
+    bool first = true;
+    auto flush = [&]() {
+#pragma unroll
+        for (int j = 0; j < TILES; ++j) {
+            const __half2 s2 = reinterpret_cast<const __half2 *>(&sc[j / 4])[j % 4], z2 = reinterpret_cast<const __half2 *>(&zp[j / 4])[j % 4];
+            const float s0 = __low2float(s2), s1 = __high2float(s2), z0 = __low2float(z2), z1 = __high2float(z2);
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                float4 *dst = red + (j * MT + mt) * 32;
+                float4 v = first ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : *dst;
+                v.x = fmaf(s0, acc[j][mt][0] - z0 * asum[mt][0], v.x);
+                v.y = fmaf(s0, acc[j][mt][1] - z0 * asum[mt][1], v.y);
+                v.z = fmaf(s1, acc[j][mt][2] - z1 * asum[mt][0], v.z);
+                v.w = fmaf(s1, acc[j][mt][3] - z1 * asum[mt][1], v.w);
+                *dst = v;
+            }
+        }
+        first = false;
+    };
+
+    clear();
+    int group = s_begin / p.steps_per_group;
+    int left = (group + 1) * p.steps_per_group - s_begin;  // steps to the end of the group
+    // The codes do not depend on the kernel before this one in the stream, the activations may; the kernel after this one
+    // may move in once the wait is over.
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d)
+        if (s_begin + d < s_end) fetch_codes(d * Cfg::SLOT_BYTES);
+    pdl_wait();
+    pdl_launch_dependents();
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+        if (s_begin + d < s_end) fetch_activations(d * Cfg::SLOT_BYTES);
+        commit();
+    }
+    if (s_begin < s_end) load_group(group);
+    uint32_t slot = 0;
+    for (int step = s_begin; step < s_end; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
+        __syncwarp();  // the activations come from other lanes
+        uint32_t w[4][W];
+        uint2 b[MT];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t src = ring + slot + r * 32 * 4 * W;
+            if (W == 2) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[r][0]), "=r"(w[r][W - 1]) : "r"(src) : "memory");
+            else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[r][0]) : "r"(src) : "memory");
+        }
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(b[mt].x), "=r"(b[mt].y) : "r"(ring_a + slot + (8 * mt + g) * 32 + t * 8) : "memory");
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const uint32_t sel = half == 0 ? 0x5410u : 0x7632u;
+                uint32_t h01[4], h23[4];
+                unpack_pairs(__byte_perm(w[0][i], w[1][i], sel), h01);
+                unpack_pairs(__byte_perm(w[2][i], w[3][i], sel), h23);
+#pragma unroll
+                for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+                        mma_m16n8k16(acc[4 * i + 2 * half + jj][mt], h01[2 * jj], h01[2 * jj + 1], h23[2 * jj], h23[2 * jj + 1], b[mt].x, b[mt].y);
+            }
+        const uint32_t ones = 0x3c003c00u;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) mma_m16n8k16(asum[mt], ones, ones, ones, ones, b[mt].x, b[mt].y);
+        __syncwarp();
+        if (step + DEPTH < s_end) {  // into the place just read
+            fetch_codes(slot);
+            fetch_activations(slot);
+        }
+        commit();
+        slot = slot == (DEPTH - 1) * Cfg::SLOT_BYTES ? 0 : slot + Cfg::SLOT_BYTES;
+        if (--left == 0 || step + 1 == s_end) {
+            flush();
+            if (step + 1 < s_end) {
+                clear();
+                load_group(++group);
+                left = p.steps_per_group;
+            }
+        }
+    }
+    if (first) {  // no steps: this warp's sum is zero
+#pragma unroll
+        for (int j = 0; j < TILES * MT; ++j) red[j * 32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    __syncthreads();
+    auto partial = [&](int i) {
+        const float4 *src = reinterpret_cast<const float4 *>(smem) + i;
+        float4 s = src[0];
+#pragma unroll
+        for (int r = 1; r < MMA_WARPS; ++r) {
+            const float4 v = src[r * Cfg::ITEMS];
+            s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+        }
+        return s;
+    };
+    auto finish = [&](int i, float4 s) {
+        const int ln = i & 31, tile = i >> 5, mt = tile % MT, j = tile / MT;
+        const int n = (blockIdx.x * 8 + (ln >> 2)) * W * COLS_PER_THREAD + 2 * j, m = m0 + 8 * mt + 2 * (ln & 3);
+        if (n >= p.N) return;
+        __half2 *dst = reinterpret_cast<__half2 *>(p.c + (size_t)m * p.N + n);
+        if (m < p.M) *dst = __floats2half2_rn(s.x, s.z);
+        if (m + 1 < p.M) dst[p.N / 2] = __floats2half2_rn(s.y, s.w);
+    };
+    stream_mma::cluster_sum(smem_u32(&recv_bar), smem_u32(smem) + Cfg::RED_BYTES, Cfg::ITEMS, p.status, kKernelU4, partial, finish);
+}
+
+template <int MT, int W, bool WIDE>
+int launch_mma(const MmaParams &p, cudaStream_t stream) {
+    using Cfg = MmaConfig<MT, W>;
+    const void *kernel = reinterpret_cast<const void *>(qlinear_u4_mma_kernel<MT, W, WIDE>);
+    static stream_mma::KnownClusters known;
+    const int rc = stream_mma::allow_smem(kernel, Cfg::SMEM_BYTES, known);
+    if (rc != B200Q_OK) return rc;
+    const int64_t n_tiles = ceil_div(p.N, (int64_t)64 * W), m_tiles = ceil_div(p.M, (int64_t)8 * MT);
+    // every warp should have two steps or more
+    const int cluster = stream_mma::choose_cluster(kernel, MMA_THREADS, Cfg::SMEM_BYTES, n_tiles * m_tiles, p.K / (16 * 2 * MMA_WARPS), known);
+    MmaParams copy = p;
+    void *args[1] = {&copy};
+    return stream_mma::launch("qlinear_u4_mma_kernel", kernel, n_tiles, cluster, m_tiles, MMA_THREADS, Cfg::SMEM_BYTES, stream, args);
+}
+
+// The tensor-core kernel's conditions: steps of 16 rows that never cross a group, and what its loads and stores need.
+bool mma_supported(const void *a, const void *c, int64_t M, int64_t G) {
+    return G % 16 == 0 && M <= (int64_t)65535 * 32 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(c) & 3u) == 0;
+}
+
 // f16 (integral values) -> u4 codes, two per byte; C conversion to int, low four bits kept.
 __global__ void u4_pack_kernel(const __half *w, uint8_t *out, int64_t bytes) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -220,6 +487,26 @@ B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *sca
     if (workspace == nullptr || workspace_bytes < need) {
         return set_error(B200Q_WORKSPACE_TOO_SMALL, "qlinear_f16_u4: workspace of %zu bytes given, %zu needed for M=%lld N=%lld K=%lld", workspace_bytes, need,
                          (long long)M, (long long)N, (long long)K);
+    }
+    if (u4::mma_supported(a, c, M, group_size)) {
+        u4::MmaParams mp;
+        mp.a = static_cast<const __half *>(a);
+        mp.q = static_cast<const uint32_t *>(q);
+        mp.scale = static_cast<const __half *>(scale);
+        mp.zeros = static_cast<const __half *>(zeros);
+        mp.c = static_cast<__half *>(c);
+        mp.status = device_status_word();
+        mp.M = (int)M;
+        mp.N = (int)N;
+        mp.K = (int)K;
+        mp.steps_per_group = (int)(group_size / 16);
+        // Wider column strips while one block of rows is enough (64 contiguous bytes of a row: (1, 4096, 12288) 13 us
+        // against 20 with 32), except where they leave too few CTAs ((1, 12288, 256) 7.0 us wide, 5.7 narrow); narrow ones
+        // beyond, where the accumulators of several row blocks take the registers ((16, 4096, 4096) 12.7 us wide, 9.3 narrow).
+        if (M > 16) return u4::launch_mma<4, 1, true>(mp, s);
+        if (M > 8) return u4::launch_mma<2, 1, true>(mp, s);
+        if (N <= 1024) return u4::launch_mma<1, 1, true>(mp, s);
+        return N % 16 == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0 ? u4::launch_mma<1, 2, true>(mp, s) : u4::launch_mma<1, 2, false>(mp, s);
     }
     u4::Params p;
     p.a = static_cast<const __half *>(a);

@@ -69,6 +69,24 @@ def test_quant_linear_on_real_valued_scales(m, n, k, gsize, with_zp):
     assert np.isfinite(c).all()
 
 
+@pytest.mark.parametrize('m,n,k,gsize', [(1, 8, 16, 16), (2, 136, 96, 48), (8, 72, 4096, 32), (9, 64, 512, 256), (16, 1000, 1536, 512), (17, 40, 64, 32),
+                                         (32, 4096, 128, 128), (40, 264, 12288, 128), (1, 12288, 512, 64), (3, 24, 120, 24)])
+@pytest.mark.parametrize('with_zp', [True, False])
+def test_quant_linear_sums_are_exact_where_they_can_be(m, n, k, gsize, with_zp):
+    """Around the kernel's tiles (64 / 128 columns, 8 / 16 / 32 rows, 16-row steps shared out over warps and clusters; a group size
+    that is not a multiple of 16 takes the other kernel): integers small enough for every sum to be exact."""
+    gen = torch.Generator(device='cuda').manual_seed(m * n + k)
+    a = torch.randint(-2, 3, (m, k), device='cuda', generator=gen).half()
+    codes = torch.randint(0, 16, (k, n), device='cuda', generator=gen).half()
+    scale = torch.randint(1, 3, (k // gsize, n), device='cuda', generator=gen).half() / 64
+    zeros = torch.randint(0, 16, (k // gsize, n), device='cuda', generator=gen).half()
+    c = w4a16_linear('w4a16', k, n, gsize, with_zp=with_zp)(a, cast_f16_to_u4(codes), scale, zeros if with_zp else None)
+    w = codes.double().view(k // gsize, gsize, n) - (zeros.double().view(k // gsize, 1, n) if with_zp else 0.0)
+    want = a.double() @ (w * scale.double().view(k // gsize, 1, n)).view(k, n)
+    assert torch.equal(c, want.half())
+    assert ffi.func('b200q_check_status')() == ffi.OK
+
+
 def test_quant_linear_argument_errors():
     f = ffi.func('b200q_qlinear_f16_u4')
     with pytest.raises(ffi.BackendException, match='multiple of the group size'):
