@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __
             const int out_n = pairs ? p.N >> 1 : p.N;    // width of the result
             const int out_n0 = pairs ? n0 >> 1 : n0;     // first result column of this tile
             const int out_col = pairs ? n >> 1 : n;      // this lane's result column
-            const bool writer = n < p.N && !(pairs && (lane & 1));
+            const bool writer = n < p.N;
             const __half *res = FUSED ? static_cast<const __half *>(p.ep.residual) : nullptr;
             const int m_left = p.M - m0;
             const bool cols_ok = out_n0 + chunk * 8 < out_n && !(pairs && chunk >= 8);  // widths are multiples of 8: eight columns are in or out together
@@ -476,14 +476,27 @@ __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __
                 tmem_ld_32x32(tmem_base + ((uint32_t)(32 * q) << 16) + buf * TM + cb * 32, v);
                 tmem_ld_wait();
                 __half *col = reinterpret_cast<__half *>(staging) + (pairs ? (32 * q + lane) >> 1 : 32 * q + lane);
+                if (pairs) {
+                    // The even lane holds the gate of a pair, the odd one the value it multiplies: of two rows, each
+                    // finishes one.  (With the even lane finishing both, every lane computes every activation and half are thrown
+                    // away: (512, 4096, 22016) 140 us against 134.)
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        float y0 = __uint_as_float(v[j]) * sc, y1 = __uint_as_float(v[j + 1]) * sc;
+                        y0 += bias;
+                        y1 += bias;
+                        const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? y0 : y1, 1);
+                        const float gate = (lane & 1) ? other : y0, up = (lane & 1) ? y1 : other;
+                        float y = gate / (1.0f + __expf(-gate)) * up;
+                        const int row = j + (lane & 1);
+                        if (res != nullptr && n < p.N && cb * 32 + row < m_left) y += __half2float(__ldg(res + (size_t)(m0 + cb * 32 + row) * p.ep.ldr + out_col));
+                        if (n < p.N) col[row * (STAGE_ROW_BYTES / 2)] = __float2half_rn(y);
+                    }
+                } else
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     float y = __uint_as_float(v[j]) * sc;
                     if (FUSED) y += bias;
-                    if (pairs) {
-                        const float up = __shfl_xor_sync(0xffffffffu, y, 1);
-                        y = y / (1.0f + __expf(-y)) * up;
-                    }
                     if (res != nullptr && writer && cb * 32 + j < m_left) y += __half2float(__ldg(res + (size_t)(m0 + cb * 32 + j) * p.ep.ldr + out_col));
                     if (writer) col[j * (STAGE_ROW_BYTES / 2)] = __float2half_rn(y);
                 }
