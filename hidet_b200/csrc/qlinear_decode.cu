@@ -575,8 +575,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     const int64_t tiles = (int64_t)pl.n_tiles * pl.m_tiles;
     // Each split has at least four 64-row steps of work, a ring's fill: with eight a narrow problem leaves most of the SMs
     // idle (a step of a 1024-wide decoder 72 -> 57 us), with two the exchange costs what the shorter loop gives (64 us).
-    int64_t max_splits = k_iters / 4 > 0 ? k_iters / 4 : 1;
-    if (max_splits > 64) max_splits = 64;
+    const int max_splits = k_iters / 4 > 0 ? k_iters / 4 : 1;
     // The splits of a tile form a cluster of up to eight CTAs (partials meet in distributed shared memory), as large as lets
     // the whole grid run at once: a few clusters left for a second wave double the time of the launch (96 tiles
     // in clusters of six are 576 CTAs and fit 148 x 4 slots by number, but not the groups of SMs clusters are confined to:
@@ -587,11 +586,14 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // More splits than a cluster holds become several full clusters per tile that meet in the workspace.  They pay three
     // dependent trips through L2 at the end of the launch (publish, count, read back), about 3 us more than partials
     // that meet in distributed shared memory.  That is worth it only when one cluster per tile would leave most of the
-    // machine idle.
+    // machine idle, and only for splits of eight steps or more: with four, (1, 4096, 1024) takes 5.7 us against 3.8 and
+    // (1, 8192, 1024) 6.5 against 6.3, though (1, 8192, 256) gains, 4.8 against 5.7.  (It is also what the scratch is sized by: with
+    // four the partial sums of (16, 1024, 11008) would not fit the array of b200q_qlinear_f16_i8_static any more.)
     int groups = 1;
     if (c == kMaxCluster && tiles * c * 2 < sms) {
         int64_t splits = tiles > 0 ? (int64_t)sms * 4 / tiles : 1;
-        if (splits > max_splits) splits = max_splits;
+        if (splits > k_iters / 8) splits = k_iters / 8;
+        if (splits > 64) splits = 64;
         groups = (int)(splits / c);
         if (groups < 1 || tiles * c > kMaxCounters) groups = 1;
     }

@@ -268,7 +268,7 @@ B200Q_API size_t b200q_qlinear_static_scratch_bytes(void);
  *     of scratch for it, is computed here without the split: same value, fp32 sums grouped differently);
  *   - a problem whose scratch requirement (b200q_qlinear_workspace_bytes) exceeds the built-in array
  *     is refused with B200Q_WORKSPACE_TOO_SMALL and a message naming both sizes (most shapes need no
- *     scratch; narrow, deep weights with 16 or more activation rows can exceed the array);
+ *     scratch; narrow, deep weights with 8 or more activation rows can exceed the array);
  *   - the first call on a device looks up the array's device address (cudaGetSymbolAddress, with that
  *     device current) and sets kernel attributes: make that first call before any stream capture;
  *   - all calls on a device share the one array: calls that may overlap on the GPU (different

@@ -55,6 +55,15 @@ def test_workspace_query_is_pure():
     assert 0 < small <= big < 64 * 1024 * 1024
 
 
+@pytest.mark.parametrize('m,n,k,need', [(16, 1024, 11008, 393216), (16, 1024, 12288, 458752), (16, 1152, 8192, 409600), (12, 1024, 14336, 409600),
+                                        (8, 1152, 16384, 409600)])
+def test_narrow_deep_weights_fit_the_built_in_scratch(m, n, k, need):
+    # the plan for 148 SMs; b200q_qlinear_f16_i8_static serves what fits its array
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip('another number of SMs, another plan')
+    assert ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, ffi.LAYOUT_KN) == need <= ffi.func('b200q_qlinear_static_scratch_bytes')()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(ffi, '_lib', None)
     monkeypatch.setattr(ffi, '_funcs', {})

@@ -69,6 +69,16 @@ def test_static_entry_point_uses_scratch_on_these_shapes():
     assert 0 < ws(8, 1024, 28672, ffi.LAYOUT_KN) <= limit
 
 
+@pytest.mark.parametrize('m,n,k', [(16, 1024, 11008), (16, 1024, 12288), (16, 1152, 8192), (12, 1024, 14336), (8, 1152, 16384)])
+def test_static_entry_point_serves_narrow_deep_weights(m, n, k):
+    """With splits half as long the partial sums of these would no longer fit the built-in array."""
+    a, wq, scale = _problem(m, n, k, seed=m + n)
+    out = torch.full((m, n), float('nan'), dtype=torch.float16, device='cuda')
+    _static_call(a, wq, scale, out)
+    assert torch.equal(out, hidet_b200.symmetric_quant_matmul(a, wq, scale))
+    assert ffi.func('b200q_check_status')() == ffi.OK
+
+
 def test_static_entry_point_refuses_what_does_not_fit():
     m, n, k = 32, 512, 28672
     assert ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, ffi.LAYOUT_KN) > (512 << 10)
