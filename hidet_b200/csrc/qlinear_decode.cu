@@ -127,7 +127,9 @@ __device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x));
 // applies the activation (the value of the partner column nn ^ 1 sits in lane ^ partner_xor; every lane
 // of the calling warp that is active takes part), adds the residual, rounds once and stores.
 __device__ __forceinline__ void finish(const OutTargets &o, const Epilogue &ep, int row, int nn, int n_limit, bool valid, float y, int partner_xor) {
-    if (valid && ep.bias != nullptr) y += __half2float(__ldg(static_cast<const __half *>(ep.bias) + nn));
+    // Bias and residual come through L2: this CTA may be older than the kernel that wrote them, and so may be what the
+    // first-level cache holds.
+    if (valid && ep.bias != nullptr) y += __half2float(__ldcg(static_cast<const __half *>(ep.bias) + nn));
     int col = nn;
     if (ep.act == kActSiluMul) {
         const float other = __shfl_xor_sync(__activemask(), y, partner_xor);
@@ -136,7 +138,7 @@ __device__ __forceinline__ void finish(const OutTargets &o, const Epilogue &ep, 
         col = nn >> 1;
     }
     if (!valid || nn >= n_limit) return;
-    if (ep.residual != nullptr) y += __half2float(__ldcg(static_cast<const __half *>(ep.residual) + (size_t)row * ep.ldr + col));  // through L2: this CTA may be older than the kernel that wrote it
+    if (ep.residual != nullptr) y += __half2float(__ldcg(static_cast<const __half *>(ep.residual) + (size_t)row * ep.ldr + col));
     store_out(o, row, col, __float2half_rn(y));
 }
 

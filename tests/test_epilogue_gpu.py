@@ -111,3 +111,27 @@ def test_fused_epilogue_argument_checks():
     with pytest.raises(ffi.BackendException, match='unknown activation 7'):
         ffi.func('b200q_qlinear_f16_i8_fused')(a.data_ptr(), wq.data_ptr(), scale.data_ptr(), out.data_ptr(), 4, 32, 64, 0, ctypes.byref(ep), None, 0,
                                               torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize('through,m,k,n', [('bias', 1, 256, 688), ('bias', 1, 1024, 4096), ('residual', 1, 256, 688), ('residual', 8, 1024, 1040),
+                                           ('residual', 12, 2048, 528)])
+def test_sums_accumulated_in_place_over_launches_that_overlap(through, m, k, n):
+    """Each launch starts while the one that writes its bias or residual still runs; the slices of a tile's columns share
+    32-byte sectors.  The same chain through fresh buffers, one launch at a time, has to give the same bits."""
+    wq, scale = hidet_b200.symmetric_quantize(torch.from_numpy(seeded_weight(k, n, seed=k)).cuda(), 'int8', dims=0)
+    a = torch.from_numpy(seeded_activation(24 * m, k, seed=n)).cuda().view(24, m, k)
+
+    def add(x, i, out):
+        more = {'bias': x.view(n)} if through == 'bias' else {'residual': x}
+        return hidet_b200.symmetric_quant_matmul(a[i], wq, scale, out=out, **more)
+
+    want = torch.zeros(m, n, dtype=torch.float16, device='cuda')
+    for i in range(24):
+        want = add(want, i, None)
+        torch.cuda.synchronize()
+    for _ in range(20):
+        x = torch.zeros(m, n, dtype=torch.float16, device='cuda')
+        for i in range(24):
+            add(x, i, x)
+        assert torch.equal(x, want)
+    assert ffi.func('b200q_check_status')() == ffi.OK
