@@ -160,8 +160,8 @@ __global__ void qlinear_u4_reduce_kernel(const float *partial, __half *c, int64_
 //     sum += scale * (group sum - zero * activation sum)
 // goes to the lane's own place in shared memory, where the warps, and then the cluster, are summed in a fixed order.
 // What is left is instructions (the unpacking and the MMAs) and the exchange at the end, not bytes.
-// Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 12.8 us, (8, 4096, 4096) 28.7 ->
-// 6.3, (1, 1024, 1000) 6.8 -> 2.8; (16, 12288, 4096) 127 (a call) -> 15.9, (64, 4096, 11008) 43.
+// Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 13.2 us, (8, 4096, 4096) 28.7 ->
+// 6.6; (16, 12288, 4096) 127 (a call) -> 16.5, (64, 4096, 11008) 43.6.
 struct MmaParams {
     const __half *a;        // [M, K]
     const uint32_t *q;      // [K, N / 8] words
@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
         for (int i = 0; i < W; ++i) {
             const size_t off = (size_t)group * p.N + n_lane + 8 * i;
             sc[i] = zp[i] = make_uint4(0, 0, 0, 0);
-            if (in[i]) sc[i] = __ldg(reinterpret_cast<const uint4 *>(p.scale + off));
-            if (in[i] && p.zeros != nullptr) zp[i] = __ldg(reinterpret_cast<const uint4 *>(p.zeros + off));
+            if (in[i]) sc[i] = __ldcg(reinterpret_cast<const uint4 *>(p.scale + off));
+            if (in[i] && p.zeros != nullptr) zp[i] = __ldcg(reinterpret_cast<const uint4 *>(p.zeros + off));
         }
     };
 
@@ -308,16 +308,23 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
     clear();
     int group = s_begin / p.steps_per_group;
     int left = (group + 1) * p.steps_per_group - s_begin;  // steps to the end of the group
-    // The codes do not depend on the kernel before this one in the stream, the activations may; the kernel after this one
-    // may move in once the wait is over.
+    // Nothing is read before the kernel in front is done, so codes and scales may be its results like the activations; the
+    // first codes are only asked into L2, which is coherent: (1, 4096, 4096) 6.5 us, 7.2 without, and 6.3 with the codes copied
+    // ahead of the wait.  The kernel after this one may move in once the wait is over.
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d)
-        if (s_begin + d < s_end) fetch_codes(d * Cfg::SLOT_BYTES);
+        if (s_begin + d < s_end) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(q_src[r][0] + d * step_words));
+        }
     pdl_wait();
     pdl_launch_dependents();
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) {
-        if (s_begin + d < s_end) fetch_activations(d * Cfg::SLOT_BYTES);
+        if (s_begin + d < s_end) {
+            fetch_codes(d * Cfg::SLOT_BYTES);
+            fetch_activations(d * Cfg::SLOT_BYTES);
+        }
         commit();
     }
     if (s_begin < s_end) load_group(group);
@@ -415,7 +422,8 @@ bool mma_supported(const void *a, const void *c, int64_t M, int64_t G) {
     return G % 16 == 0 && M <= (int64_t)65535 * 32 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(c) & 3u) == 0;
 }
 
-// f16 (integral values) -> u4 codes, two per byte; C conversion to int, low four bits kept.
+// f16 (integral values) -> u4 codes, two per byte; C conversion to int, low four bits kept.  Like every kernel here that
+// writes weights, this one never lets dependents start early (the small-M int8 kernel reads weights ahead of its wait).
 __global__ void u4_pack_kernel(const __half *w, uint8_t *out, int64_t bytes) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= bytes) return;

@@ -62,7 +62,8 @@ __device__ __forceinline__ void to_f16(uint32_t pair, uint32_t &first, uint32_t 
     asm("sub.f16x2 %0, %1, %2;" : "=r"(second) : "r"(e1), "r"(bias));
 }
 
-// Through L2: under programmatic launches this CTA may be older than the kernel that wrote the activations.
+// Through L2: under programmatic launches this CTA may be older than the kernel that wrote the activations.  (The weight,
+// too, is read after that kernel, with coherent loads.)
 __device__ __forceinline__ uint4 load_l2(const void *p) { return __ldcg(static_cast<const uint4 *>(p)); }
 
 template <int MT>
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(THREADS, MT == 1 ? 2 : 1) qlinear_unaligned_ke
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             w[i] = make_uint4(0, 0, 0, 0);
-            if (x_in && j + i < groups) asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "l"(src + i * group_bytes));
+            if (x_in && j + i < groups) asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "l"(src + i * group_bytes));
         }
     };
     // piece q of a chunk: activation row q / CHUNK_ROWS, k = 8 j .. 8 j + 7 for the chunk's j = q % CHUNK_ROWS

@@ -45,6 +45,22 @@ def seeded_activation(m: int, k: int, seed: int = 1, dtype=np.float16) -> np.nda
 
 
 @pytest.fixture(scope='session')
+def nvcc_library(tmp_path_factory):
+    """Compiles a source of tests/cuda and loads it."""
+    import ctypes
+    import subprocess
+
+    from hidet_b200 import build
+
+    def load(source, *flags):
+        out = str(tmp_path_factory.mktemp('cuda') / (source + '.so'))
+        subprocess.check_call([build.find_nvcc(), *build.ARCH_FLAGS, '-O2', *flags, '-Xcompiler', '-fPIC', '-shared', os.path.join(ROOT, 'tests', 'cuda', source), '-o', out])
+        return ctypes.CDLL(out)
+
+    return load
+
+
+@pytest.fixture(scope='session')
 def oracle_lib():
     import oracle
 
