@@ -12,7 +12,7 @@ allocation, no synchronisation; tensor maps travel as kernel parameters).
 """
 from __future__ import annotations
 
-from typing import Any, Callable, List, Optional, Sequence
+from typing import Any, Callable, List, Optional, Sequence, Set
 
 import torch
 
@@ -40,6 +40,7 @@ class CudaGraph:
                     outputs = f_run(self._inputs)
         finally:
             self._scratch = workspaces.swap(device, self._stream.cuda_stream, around)  # kept for the replays
+        self._replayed_on: Set[int] = set()  # streams the scratch is known to be used on
         self._outputs: List[torch.Tensor] = list(outputs) if isinstance(outputs, (list, tuple)) else [outputs]
 
     @property
@@ -65,6 +66,11 @@ class CudaGraph:
         outputs; everything is ordered on `stream` (default: the current stream) and nothing is waited for."""
         stream = stream if stream is not None else torch.cuda.current_stream(self._inputs[0].device)
         self.copy_inputs(inputs, stream)
+        # The scratch belongs to the capture stream.  Once this object is gone its block must not be handed out there before
+        # the replays on other streams are over.
+        if self._scratch is not None and stream.cuda_stream not in self._replayed_on:
+            self._scratch.record_stream(stream)
+            self._replayed_on.add(stream.cuda_stream)
         with torch.cuda.stream(stream):
             self._graph.replay()
         return self._outputs
