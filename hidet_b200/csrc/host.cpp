@@ -266,6 +266,7 @@ PyObject *w4(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         zp = zeros->const_data_ptr();
     }
     const int64_t m = a->size(0);
+    PLAIN_OR_NONE(group % 16 != 0 || (reinterpret_cast<uintptr_t>(a->const_data_ptr()) & 15u) == 0);  // else the general path aligns it
     void *ws;
     size_t ws_bytes;
     PLAIN_OR_NONE(find_scratch(w, lib.w4_workspace_bytes(m, n, k, group), ws, ws_bytes));

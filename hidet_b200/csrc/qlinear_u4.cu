@@ -16,7 +16,8 @@
 // all in fp32 (the codes are exact in fp32; the reference multiplies every weight by its scale in f16 first and
 // accumulates the products, tests/cute_kernel/quantized_linear.py:1044-1047: same value up to rounding).  The k slices
 // of a CTA meet in shared memory; the CTAs that split K further write fp32 partial sums to the caller's workspace,
-// and a second kernel adds them in slice order and rounds to f16 once: the same result on every run.
+// and a second kernel adds them in slice order and rounds to f16 once: the same result on every run.  (Without room for
+// partial sums K is not split.)
 #include "stream_mma.cuh"
 
 namespace b200q {
@@ -36,6 +37,7 @@ struct Params {
     const __half *scale;    // [K / G, N]
     const __half *zeros;    // [K / G, N] or null
     float *partial;         // [splits][M, N] fp32
+    __half *direct;         // [M, N]: the result itself, in place of partial sums (one split), or null
     int M, N, K, G;
     int k_per_split;        // a multiple of G
 };
@@ -133,7 +135,9 @@ __global__ void __launch_bounds__(THREADS) qlinear_u4_partial_kernel(const Param
                 float s = 0.0f;
 #pragma unroll
                 for (int sl = 0; sl < K_SLICES; ++sl) s += red[sl][m][col];
-                out[(size_t)(m0 + m) * p.N + n] = s;
+                const size_t at = (size_t)(m0 + m) * p.N + n;
+                if (p.direct != nullptr) p.direct[at] = __float2half_rn(s);
+                else out[at] = s;
             }
         }
         __syncthreads();
@@ -459,6 +463,13 @@ Plan plan(int64_t M, int64_t N, int64_t K, int64_t G) {
     return pl;
 }
 
+// Scratch a call asks for.  The tensor-core kernel has no use for any: its group sizes are held to what the shared head
+// takes, whatever the problem, and a call without a workspace is refused for every group size alike.
+size_t workspace_bytes(int64_t M, int64_t N, int64_t K, int64_t G) {
+    if (G % 16 == 0) return kReservedHead + 256;
+    return kReservedHead + (size_t)plan(M, N, K, G).splits * M * N * sizeof(float);
+}
+
 }  // namespace u4
 }  // namespace b200q
 
@@ -467,7 +478,7 @@ extern "C" {
 B200Q_API size_t b200q_qlinear_f16_u4_workspace_bytes(int64_t M, int64_t N, int64_t K, int64_t group_size) {
     using namespace b200q;
     if (M <= 0 || N <= 0 || K <= 0 || group_size <= 0) return 0;
-    return u4::kReservedHead + (size_t)u4::plan(M, N, K, group_size).splits * M * N * sizeof(float);
+    return u4::workspace_bytes(M, N, K, group_size);
 }
 
 B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *scale, const void *zeros, void *c, int64_t M, int64_t N, int64_t K,
@@ -490,8 +501,7 @@ B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *sca
     if ((reinterpret_cast<uintptr_t>(q) & 3u) != 0 || (reinterpret_cast<uintptr_t>(scale) & 15u) != 0 || (reinterpret_cast<uintptr_t>(zeros) & 15u) != 0) {
         return set_error(B200Q_UNSUPPORTED, "qlinear_f16_u4: codes need a 4-byte aligned base, scales and zero points 16-byte aligned bases");
     }
-    const u4::Plan pl = u4::plan(M, N, K, group_size);
-    const size_t need = u4::kReservedHead + (size_t)pl.splits * M * N * sizeof(float);
+    const size_t need = u4::workspace_bytes(M, N, K, group_size);
     if (workspace == nullptr || workspace_bytes < need) {
         return set_error(B200Q_WORKSPACE_TOO_SMALL, "qlinear_f16_u4: workspace of %zu bytes given, %zu needed for M=%lld N=%lld K=%lld", workspace_bytes, need,
                          (long long)M, (long long)N, (long long)K);
@@ -516,7 +526,12 @@ B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *sca
         if (N <= 1024) return u4::launch_mma<1, 1, true>(mp, s);
         return N % 16 == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0 ? u4::launch_mma<1, 2, true>(mp, s) : u4::launch_mma<1, 2, false>(mp, s);
     }
+    u4::Plan pl = u4::plan(M, N, K, group_size);
+    // Operands the tensor-core kernel cannot take (an unaligned a or c) with its amount of scratch: one split.
+    const bool direct = workspace_bytes < u4::kReservedHead + (size_t)pl.splits * M * N * sizeof(float);
+    if (direct) pl = {1, (int)K};
     u4::Params p;
+    p.direct = direct ? static_cast<__half *>(c) : nullptr;
     p.a = static_cast<const __half *>(a);
     p.q = static_cast<const uint32_t *>(q);
     p.scale = static_cast<const __half *>(scale);
@@ -537,6 +552,7 @@ B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *sca
         u4::qlinear_u4_partial_kernel<4><<<grid, block, 0, s>>>(p);
     }
     B200Q_CHECK_LAUNCH("qlinear_u4_partial_kernel");
+    if (direct) return B200Q_OK;
     const int64_t mn = M * N;
     u4::qlinear_u4_reduce_kernel<<<(unsigned)ceil_div(mn, 256), 256, 0, s>>>(p.partial, static_cast<__half *>(c), mn, pl.splits);
     B200Q_CHECK_LAUNCH("qlinear_u4_reduce_kernel");

@@ -82,6 +82,8 @@ class FpAIntBGemm:
             require_cuda(zeros, 'zeros')
             zp = zeros.contiguous()
         a, b, scale = a.contiguous(), b.contiguous(), scale.contiguous()
+        if self.group_size % 16 == 0 and a.data_ptr() % 16 != 0:  # the tensor-core kernel copies 16 bytes of a row at a time
+            a = a.clone()
         m = a.shape[0]
         c = torch.empty((m, self.n), dtype=torch.float16, device=a.device)
         with torch.cuda.device(a.device):

@@ -125,8 +125,11 @@ B200Q_API int b200q_embedding_dequantize(const void *table, const void *scale, c
  * b200q_u4_pack / the reference's cast_f16_to_u4 produce it (not the kernel-private layout of its
  * preprocess_weight); scale, zeros f16 [K / G, N] (zeros may be NULL: w = scale * q); c f16 [M, N].
  * K must be a multiple of the group size G, N a multiple of 8.  Sums are fp32, the order of every sum is fixed.
- * The workspace (b200q_qlinear_f16_u4_workspace_bytes) holds fp32 partial sums behind an untouched head of 256 KB
- * (where b200q_qlinear_f16_i8 keeps its counters, so that one workspace can serve both) and needs no initialisation.
+ * Group sizes that are multiples of 16 take a tensor-core kernel (16-byte aligned a, 4-byte aligned c) that needs no
+ * scratch; for the others the workspace holds fp32 partial sums behind an untouched head of 256 KB (where
+ * b200q_qlinear_f16_i8 keeps its counters, so that one workspace can serve both) and needs no initialisation.
+ * b200q_qlinear_f16_u4_workspace_bytes is little more than the head for the former, whatever M, N and K, and a workspace of
+ * that size has to be given all the same; unaligned operands are then served without splitting K, more slowly.
  */
 B200Q_API size_t b200q_qlinear_f16_u4_workspace_bytes(int64_t M, int64_t N, int64_t K, int64_t group_size);
 B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *scale, const void *zeros, void *c, int64_t M, int64_t N,

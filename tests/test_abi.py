@@ -64,6 +64,13 @@ def test_narrow_deep_weights_fit_the_built_in_scratch(m, n, k, need):
     assert ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, ffi.LAYOUT_KN) == need <= ffi.func('b200q_qlinear_static_scratch_bytes')()
 
 
+def test_four_bit_scratch_does_not_grow_where_none_is_used():
+    ws = ffi.func('b200q_qlinear_f16_u4_workspace_bytes')
+    for group in (16, 64, 128, 256):
+        assert 65536 * 4 < ws(1, 4096, 4096, group) == ws(2048, 12288, 12288, group) <= 1 << 20
+    assert ws(64, 4096, 4080, 24) >= 65536 * 4 + 64 * 4096 * 4  # the kernel for these keeps its partial sums there
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(ffi, '_lib', None)
     monkeypatch.setattr(ffi, '_funcs', {})

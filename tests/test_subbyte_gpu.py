@@ -87,6 +87,29 @@ def test_quant_linear_sums_are_exact_where_they_can_be(m, n, k, gsize, with_zp):
     assert ffi.func('b200q_check_status')() == ffi.OK
 
 
+@pytest.mark.parametrize('m,n,k,gsize', [(1, 1000, 512, 128), (5, 264, 768, 32), (33, 72, 512, 256), (3, 24, 120, 24)])
+def test_quant_linear_on_operands_off_their_boundaries(m, n, k, gsize):
+    """An unaligned view of the activations through the host layer, and both operands unaligned through the C entry, with no
+    more scratch than the query asks for and with plenty: sums that are exact in any order."""
+    gen = torch.Generator(device='cuda').manual_seed(m + n + k)
+    a = torch.empty(m * k + 1, dtype=torch.float16, device='cuda')[1:].view(m, k)
+    a.copy_(torch.randint(-2, 3, (m, k), device='cuda', generator=gen))
+    assert a.data_ptr() % 16 == 2
+    codes = torch.randint(0, 16, (k, n), device='cuda', generator=gen).half()
+    scale = torch.randint(1, 3, (k // gsize, n), device='cuda', generator=gen).half() / 64
+    bq = cast_f16_to_u4(codes)
+    want = (a.double() @ (codes.double().view(k // gsize, gsize, n) * scale.double().view(k // gsize, 1, n)).view(k, n)).half()
+    assert torch.equal(w4a16_linear('w4a16', k, n, gsize, with_zp=False)(a, bq, scale), want)
+    need = ffi.func('b200q_qlinear_f16_u4_workspace_bytes')(m, n, k, gsize)
+    for size in (need, need + (1 << 24)):
+        ws = torch.zeros(size, dtype=torch.uint8, device='cuda')
+        out = torch.full((m * n + 1,), float('nan'), dtype=torch.float16, device='cuda')[1:].view(m, n)
+        ffi.func('b200q_qlinear_f16_u4')(a.data_ptr(), bq.data_ptr(), scale.data_ptr(), None, out.data_ptr(), m, n, k, gsize, ws.data_ptr(), size,
+                                         torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(out, want)
+        assert not ws[:65536 * 4].any()
+
+
 def test_quant_linear_argument_errors():
     f = ffi.func('b200q_qlinear_f16_u4')
     with pytest.raises(ffi.BackendException, match='multiple of the group size'):
