@@ -1,4 +1,4 @@
-"""Builds ``libhidet_b200q.so`` in-tree from ``hidet_b200/csrc`` with nvcc for sm_100a.
+"""Builds ``libhidet_b200q.so`` in-tree from ``hidet_b200/csrc`` with nvcc for sm_100a, and the native host path beside it.
 
 The library is prebuilt and loaded with ctypes, the way the reference loads its own compiled
 libraries (python/hidet/ffi/ffi.py:32-69); nothing is compiled at import time.
@@ -14,6 +14,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from typing import Dict, List
 
@@ -24,7 +25,6 @@ LIB_DIR = os.path.join(PKG_DIR, 'lib')
 LIB_NAME = 'libhidet_b200q.so'
 LIB_PATH = os.path.join(LIB_DIR, LIB_NAME)
 HOST_SOURCE = os.path.join(SRC_DIR, 'host.cpp')
-HOST_PATH = os.path.join(LIB_DIR, 'hidet_b200_host.so')
 
 ARCH_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a']
 COMMON_FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xcompiler', '-fvisibility=hidden']
@@ -70,23 +70,26 @@ def _compile(nvcc: str, src: str, verbose: bool) -> str:
 
 def build_host_module(force: bool = False) -> str:
     """The CPython module of csrc/host.cpp: host code only, against torch's headers and libraries.  Returns its path."""
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(
-            os.path.getmtime(HOST_SOURCE), os.path.getmtime(__file__), os.path.getmtime(os.path.join(PKG_DIR, '..', 'include', 'hidet_b200q.h'))):
-        return HOST_PATH
     import torch
 
+    from . import native
+
+    path = native.module_path()
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= max(
+            os.path.getmtime(HOST_SOURCE), os.path.getmtime(__file__), os.path.getmtime(os.path.join(PKG_DIR, '..', 'include', 'hidet_b200q.h'))):
+        return path
     torch_dir = os.path.dirname(os.path.abspath(torch.__file__))
     cuda_dir = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
     include = [os.path.join(torch_dir, 'include'), os.path.join(torch_dir, 'include', 'torch', 'csrc', 'api', 'include'),
                os.path.join(cuda_dir, 'include'), sysconfig.get_paths()['include']]
     os.makedirs(LIB_DIR, exist_ok=True)
     cmd = [os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-fvisibility=hidden',
-           '-D_GLIBCXX_USE_CXX11_ABI={}'.format(int(torch._C._GLIBCXX_USE_CXX11_ABI)), *('-isystem' + d for d in include), HOST_SOURCE, '-o', HOST_PATH,
+           '-D_GLIBCXX_USE_CXX11_ABI={}'.format(int(torch._C._GLIBCXX_USE_CXX11_ABI)), *('-isystem' + d for d in include), HOST_SOURCE, '-o', path,
            '-L' + os.path.join(torch_dir, 'lib'), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch_python']
     res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError('g++ failed for host.cpp:\n{}\n{}'.format(' '.join(cmd), res.stdout))
-    return HOST_PATH
+    return path
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
@@ -105,12 +108,15 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         with ThreadPoolExecutor(max_workers=min(8, len(stale))) as pool:
             list(pool.map(lambda s: _compile(nvcc, s, verbose), stale))
     objs = [os.path.join(OBJ_DIR, s[:-3] + '.o') for s in sources()]
-    build_host_module(force)
     if stale or not os.path.exists(LIB_PATH):
         cmd = [nvcc, *ARCH_FLAGS, '-shared', '-o', LIB_PATH, *objs, '-cudart', 'static']
         res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if res.returncode != 0:
             raise RuntimeError('link failed:\n{}\n{}'.format(' '.join(cmd), res.stdout))
+    try:
+        build_host_module(force)
+    except (ImportError, OSError, RuntimeError) as e:  # the package runs without it, only with slower calls
+        warnings.warn('the native host path was not built: {}'.format(e))
     return LIB_PATH
 
 

@@ -19,7 +19,8 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <vector>
+#include <unordered_map>
+#include <utility>
 
 #include "../../include/hidet_b200q.h"
 
@@ -36,14 +37,15 @@ struct Library {
     decltype(&b200q_qlinear_f16_u4) w4 = nullptr;
 } lib;
 
-// Scratch buffers that the Python side owns and has told us about, by (device, stream).
+// Scratch buffers that the Python side owns and has told us about, by stream and device.
 struct Scratch {
-    int device;
-    uintptr_t stream;
     void *ptr;
     size_t bytes;
 };
-std::vector<Scratch> scratch;  // guarded by the GIL
+struct KeyHash {
+    size_t operator()(const std::pair<uintptr_t, int> &k) const { return std::hash<uintptr_t>()(k.first) * 31 + (size_t)k.second; }
+};
+std::unordered_map<std::pair<uintptr_t, int>, Scratch, KeyHash> scratch;  // guarded by the GIL
 
 #define PLAIN_OR_NONE(cond) \
     do {                    \
@@ -76,14 +78,11 @@ inline bool find_scratch(const Where &w, size_t need, void *&ptr, size_t &bytes)
     ptr = nullptr;
     bytes = 0;
     if (need == 0) return true;
-    for (const Scratch &s : scratch) {
-        if (s.device == w.device && s.stream == reinterpret_cast<uintptr_t>(w.stream)) {
-            ptr = s.ptr;
-            bytes = s.bytes;
-            return bytes >= need;
-        }
-    }
-    return false;
+    const auto it = scratch.find({reinterpret_cast<uintptr_t>(w.stream), w.device});
+    if (it == scratch.end() || it->second.bytes < need) return false;
+    ptr = it->second.ptr;
+    bytes = it->second.bytes;
+    return true;
 }
 inline at::Tensor empty(at::IntArrayRef shape, at::ScalarType type, int device) {
     return at::detail::empty_cuda(shape, type, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), c10::nullopt);
@@ -295,20 +294,17 @@ PyObject *bind(PyObject *, PyObject *args) {
     Py_RETURN_NONE;
 }
 
-// set_scratch(device, stream, address, bytes): the buffer of that stream from now on (it replaces an earlier one)
+// set_scratch(device, stream, address, bytes): the buffer of that stream from now on; 0 bytes: it has none
 PyObject *set_scratch(PyObject *, PyObject *args) {
+    HANDLE_TH_ERRORS
     int device;
     unsigned long long stream, ptr, bytes;
     if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &ptr, &bytes)) return nullptr;
-    const Scratch fresh = {device, (uintptr_t)stream, reinterpret_cast<void *>((uintptr_t)ptr), (size_t)bytes};
-    for (Scratch &s : scratch) {
-        if (s.device == fresh.device && s.stream == fresh.stream) {
-            s = fresh;
-            Py_RETURN_NONE;
-        }
-    }
-    scratch.push_back(fresh);
+    const std::pair<uintptr_t, int> key((uintptr_t)stream, device);
+    if (bytes == 0) scratch.erase(key);
+    else scratch[key] = {reinterpret_cast<void *>((uintptr_t)ptr), (size_t)bytes};
     Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject *clear_scratch(PyObject *, PyObject *) {

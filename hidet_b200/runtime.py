@@ -50,13 +50,12 @@ class _Workspaces:
             size = 1 << max(20, (nbytes - 1).bit_length())
             buf = torch.zeros(size, dtype=torch.uint8, device=torch.device('cuda', index))
             self._buffers[key] = buf
-            native.load().set_scratch(*key, buf.data_ptr(), buf.numel())  # for the native host path
+        native.set_scratch(*key, buf.data_ptr(), buf.numel())  # for the native host path, which may be younger than the buffer
         return buf.data_ptr(), buf.numel()
 
     def clear(self) -> None:
         self._buffers.clear()
-        if native._module is not None:
-            native._module.clear_scratch()
+        native.clear_scratch()
 
     def swap(self, device: torch.device, stream: int, buffer: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
         """Puts `buffer` (None: nothing, a new one is made when it is needed) in the place of a stream's scratch and
@@ -67,7 +66,7 @@ class _Workspaces:
         before = self._buffers.pop((index, stream), None)
         if buffer is not None:
             self._buffers[(index, stream)] = buffer
-        native.load().set_scratch(index, stream, buffer.data_ptr() if buffer is not None else 0, buffer.numel() if buffer is not None else 0)
+        native.set_scratch(index, stream, buffer.data_ptr() if buffer is not None else 0, buffer.numel() if buffer is not None else 0)
         return before
 
 

@@ -283,3 +283,20 @@ def test_push_columns_copies_one_column_range_and_nothing_else():
         assert bool((d[:, :col0] == -3.0).all()) and bool((d[:, col0 + cols:] == -3.0).all())
     with pytest.raises(ffi.BackendException, match='do not fit'):
         ffi.func('b200q_push_columns')(src.data_ptr(), table, 3, rows, cols, ld, ld - cols + 1, torch.cuda.current_stream().cuda_stream)
+
+
+def test_package_runs_without_the_native_host_path(monkeypatch, tmp_path):
+    from hidet_b200 import native
+
+    wq, scale = _quantized(16384, 256, seed=3)
+    a, wq, scale = (torch.from_numpy(x).cuda() for x in (seeded_activation(4, 16384, seed=4), wq, scale))
+    want = hidet_b200.symmetric_quant_matmul(a, wq, scale)
+    monkeypatch.setattr(native, '_module', None)
+    for name in native._FUNCTIONS:
+        monkeypatch.setattr(native, name, native._stand_in(name))
+    monkeypatch.setattr(native, 'LIB_DIR', str(tmp_path))
+    with pytest.warns(UserWarning, match='cannot be loaded'):
+        got = hidet_b200.symmetric_quant_matmul(a, wq, scale)
+    assert torch.equal(got, want)
+    graph = hidet_b200.CudaGraph(lambda: [a.clone()], lambda inputs: [hidet_b200.symmetric_quant_matmul(inputs[0], wq, scale)])
+    assert torch.equal(graph.run([a])[0], want)
