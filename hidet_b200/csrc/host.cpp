@@ -3,7 +3,7 @@
 // At decode sizes a kernel of this library takes 3 to 10 us while the same steps in Python (tensor attribute reads, a
 // device context manager, a stream object, two or three ctypes calls) take about 15 us, so an eager program is bound by
 // them; here they take about 4 us.  Every function answers None for whatever is not the plain case -- CPU tensors,
-// wrong types or shapes, tensors that need a copy first, another current device, scratch that does not exist yet, a
+// wrong types or shapes, tensors that need a copy first, an active dispatch mode, another current device, scratch that does not exist yet, a
 // call that failed -- and the Python function that called it then takes its general path, which checks, copies,
 // allocates and reports errors.  So this file decides nothing: it only makes the plain case short.
 //
@@ -14,6 +14,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -52,10 +53,13 @@ std::unordered_map<std::pair<uintptr_t, int>, Scratch, KeyHash> scratch;  // gua
         if (!(cond)) Py_RETURN_NONE; \
     } while (0)
 
-// A strided CUDA tensor with memory of its own and no Python-level overrides, contiguous: what a kernel can be given.
+// A dispatch mode (fake tensors, tracing, counting) wants to see the operators the Python path runs.
+inline bool watched() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }
+// A strided CUDA tensor with memory of its own (a vmap or grad wrapper has none) and no Python-level overrides,
+// contiguous: what a kernel can be given.
 inline bool plain(const at::Tensor &t) {
-    return t.is_cuda() && t.layout() == at::kStrided && !t.unsafeGetTensorImpl()->is_python_dispatch() && t.is_contiguous() &&
-           !t.is_neg();
+    return t.is_cuda() && t.layout() == at::kStrided && t.has_storage() && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
+           t.is_contiguous() && !t.is_neg();
 }
 inline const at::Tensor *plain_tensor(PyObject *o) {
     if (!THPVariable_Check(o)) return nullptr;
@@ -107,7 +111,7 @@ inline int reduce_dim_of(PyObject *o) {
 // linear(a, weight, scale, weight_layout, out, bias, residual, activation)
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    PLAIN_OR_NONE(n_args == 8 && lib.linear != nullptr);
+    PLAIN_OR_NONE(n_args == 8 && lib.linear != nullptr && !watched());
     const at::Tensor *a = plain_tensor(args[0]), *weight = plain_tensor(args[1]), *scale = plain_tensor(args[2]);
     PLAIN_OR_NONE(a && weight && scale);
     const bool nk = is_text(args[3], "NK");
@@ -176,7 +180,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
 // quantize(w, quant_type, dims) -> (wq, scale)
 PyObject *quantize(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    PLAIN_OR_NONE(n_args == 3 && lib.quantize != nullptr);
+    PLAIN_OR_NONE(n_args == 3 && lib.quantize != nullptr && !watched());
     const at::Tensor *x = plain_tensor(args[0]);
     PLAIN_OR_NONE(x && x->dim() == 2 && float_code(x->scalar_type()) >= 0);
     at::ScalarType q;
@@ -205,7 +209,7 @@ PyObject *quantize(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
 // dequantize(wq, scale, dims)
 PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    PLAIN_OR_NONE(n_args == 3 && lib.dequantize != nullptr);
+    PLAIN_OR_NONE(n_args == 3 && lib.dequantize != nullptr && !watched());
     const at::Tensor *q = plain_tensor(args[0]), *scale = plain_tensor(args[1]);
     PLAIN_OR_NONE(q && scale && q->dim() == 2 && scale->dim() == 1 && q->numel() > 0);
     const int reduce = reduce_dim_of(args[2]);
@@ -225,7 +229,7 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
 // take(wq, scale, indices)
 PyObject *take(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    PLAIN_OR_NONE(n_args == 3 && lib.take != nullptr);
+    PLAIN_OR_NONE(n_args == 3 && lib.take != nullptr && !watched());
     const at::Tensor *q = plain_tensor(args[0]), *scale = plain_tensor(args[1]), *idx = plain_tensor(args[2]);
     PLAIN_OR_NONE(q && scale && idx && q->dim() == 2 && scale->dim() == 1 && scale->size(0) == q->size(0));
     const int fc = float_code(scale->scalar_type()), qc = quant_code(q->scalar_type());
@@ -248,7 +252,7 @@ PyObject *take(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
 // w4(a, codes, scale, zeros or None, k, n, group_size)
 PyObject *w4(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
-    PLAIN_OR_NONE(n_args == 7 && lib.w4 != nullptr);
+    PLAIN_OR_NONE(n_args == 7 && lib.w4 != nullptr && !watched());
     const at::Tensor *a = plain_tensor(args[0]), *q = plain_tensor(args[1]), *scale = plain_tensor(args[2]);
     PLAIN_OR_NONE(a && q && scale && PyLong_CheckExact(args[4]) && PyLong_CheckExact(args[5]) && PyLong_CheckExact(args[6]));
     const int64_t k = PyLong_AsLongLong(args[4]), n = PyLong_AsLongLong(args[5]), group = PyLong_AsLongLong(args[6]);
