@@ -139,3 +139,21 @@ def test_f16_quantize_properties():
     wq_full, sc_full = oracle.symmetric_quantize(w, 'int8', 0)
     wq_part, sc_part = oracle.symmetric_quantize(np.ascontiguousarray(w[:, 32:64]), 'int8', 0)
     assert np.array_equal(wq_full[:, 32:64], wq_part) and np.array_equal(sc_full[32:64], sc_part)
+
+
+def test_half_quotient_is_the_rounded_one_for_every_pair_of_significands():
+    """oracle_hdiv on normal quotients (their value depends on the exponents by a power of two only), and the form the quantize
+    kernels compute, the rounded f32 reciprocal times the dividend: both the quotient rounded once.  The yardstick is integer
+    arithmetic."""
+    lib = oracle.load()
+    a, b = np.meshgrid(np.arange(1024, 2048, dtype=np.int64), np.arange(1024, 2048, dtype=np.int64), indexing='ij')
+    shift = np.where(a >= b, 10, 11)  # the quotient's significand m, 1024 <= m < 2048, is a 2^shift / b
+    m, rest = (a << shift) // b, (a << shift) % b
+    m += (2 * rest > b) | ((2 * rest == b) & (m % 2 == 1))
+    want = (m.astype(np.float64) / 2.0 ** shift).astype(np.float16)
+    assert np.array_equal(want.astype(np.float64), m / 2.0 ** shift)
+    ah, bh = a.astype(np.float16), b.astype(np.float16)
+    kernel = ((np.float32(1.0) / bh.astype(np.float32)) * ah.astype(np.float32)).astype(np.float16)
+    assert np.array_equal(kernel.view(np.uint16), want.view(np.uint16))
+    got = np.array([lib.oracle_hdiv(x, y) for x, y in zip(ah.view(np.uint16).ravel().tolist(), bh.view(np.uint16).ravel().tolist())], dtype=np.uint16)
+    assert np.array_equal(got, want.view(np.uint16).ravel())

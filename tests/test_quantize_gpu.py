@@ -186,3 +186,16 @@ def test_quantize_rejects_bad_arguments():
     wq, scale = hidet_b200.symmetric_quantize(w, 'int8', dims=0)
     with pytest.raises(ValueError):
         hidet_b200.symmetric_dequantize(wq, scale[:4], dims=0)
+
+
+def test_quotient_of_halves_is_cuda_s_for_every_pair(nvcc_library):
+    """The quantize kernels take w / scale as the rounded reciprocal times w; all 2^32 pairs, with the flags they are compiled with."""
+    import ctypes
+
+    from hidet_b200.build import PER_SOURCE_FLAGS
+
+    f = nvcc_library('half_quotient.cu', *PER_SOURCE_FLAGS['quantize.cu']).half_quotient_mismatches
+    f.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    mismatches = torch.zeros(1, dtype=torch.int64, device='cuda')
+    assert f(mismatches.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert mismatches.item() == 0
