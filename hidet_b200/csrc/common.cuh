@@ -50,6 +50,10 @@ constexpr unsigned int kKernelUnaligned = 4;
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// Clusters of `cluster` CTAs (along y) of a kernel that run at once on the current device, asked of the runtime: clusters stay
+// within a group of SMs, so it is less than what the slots add up to.  0 if it cannot be told.
+int resident_clusters(const void *kernel, int threads, int smem, int cluster);
+
 // Encodes a 2-D tiled tensor map.  `inner`/`outer` are the tensor extents in elements, `row_bytes`
 // the stride between consecutive outer indices, box_* the tile extents.  swizzle is a
 // CUtensorMapSwizzle value.  Returns a b200q_status.

@@ -530,8 +530,8 @@ static int set_attributes() {
     return B200Q_OK;
 }
 
-// CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use, because a
-// cluster's CTAs stay within one group of SMs.  Asked of the runtime once per device; without a device, an estimate.
+// CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use.  Looked up once
+// per device; without a device, an estimate.
 static int resident_ctas(const Variant &v, int cluster) {
     static std::atomic<int> known[64][2][kMaxCluster + 1];
     int dev = -1;
@@ -542,21 +542,8 @@ static int resident_ctas(const Variant &v, int cluster) {
     std::atomic<int> &slot = known[dev][&v - kVariants][cluster];
     int n = slot.load(std::memory_order_relaxed);
     if (n != 0) return n;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, (unsigned)cluster, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
-    cfg.dynamicSmemBytes = v.smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = (unsigned)cluster;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, v.kn, &cfg) != cudaSuccess || n <= 0) {
-        cudaGetLastError();
-        return 148 * 4 - 30;
-    }
+    n = resident_clusters(v.kn, THREADS, v.smem, cluster);
+    if (n == 0) return 148 * 4 - 30;
     n *= cluster;
     slot.store(n, std::memory_order_relaxed);
     return n;

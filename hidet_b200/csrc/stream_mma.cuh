@@ -72,8 +72,8 @@ inline int allow_smem(const void *kernel, int smem, KnownClusters &known) {
 }
 
 // The largest cluster along K (at most `limit`) with which the whole grid of `tiles` output tiles still runs at once: a
-// few clusters left for a second wave double the time of a launch.  Clusters stay within a group of SMs, so how many fit is
-// asked of the runtime, once per device, kernel and size.
+// few clusters left for a second wave double the time of a launch.  How many fit is looked up once per device, kernel and
+// size.
 inline int choose_cluster(const void *kernel, int threads, int smem, int64_t tiles, int64_t limit, KnownClusters &known) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
@@ -84,21 +84,8 @@ inline int choose_cluster(const void *kernel, int threads, int smem, int64_t til
     for (int c = 2; c <= MAX_CLUSTER && c <= limit; ++c) {
         int n = known[dev][c].load(std::memory_order_relaxed);
         if (n == 0) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(1, (unsigned)c, 1);
-            cfg.blockDim = dim3((unsigned)threads, 1, 1);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1;
-            attr[0].val.clusterDim.y = (unsigned)c;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-                cudaGetLastError();
-                break;
-            }
+            n = resident_clusters(kernel, threads, smem, c);
+            if (n == 0) break;
             known[dev][c].store(n, std::memory_order_relaxed);
         }
         if (tiles > n) break;
