@@ -228,32 +228,42 @@ def run_config(cfg: DecoderConfig = LLAMA_7B, parity_steps: int = 8, seed: int =
     return out
 
 
+def attribute(kernels):
+    """kernels: (start, end, kind) of every launch.  {kind: time}, time that several launches share counted once, for the one
+    that ends last: a launch that starts early and waits for the one in front of it is given what it takes beyond that one's
+    end.  The times add up to the time in which any kernel ran."""
+    times, latest = {}, float('-inf')
+    for start, end, kind in sorted(kernels):
+        times[kind] = times.get(kind, 0.0) + max(0.0, end - max(start, latest))
+        latest = max(latest, end)
+    return times
+
+
 def kernel_time_of_a_step(step_graph, replays: int = 3):
-    """Device time of the kernels of one decode step by kind, from torch.profiler's kernel records of a few replays of
-    the step's CUDA graph: how much of the step is the quantized-linear path and how much the rest of the decoder
-    (attention, normalisation, rotary embedding and the other element-wise kernels torch launches).  None when the
-    profiler gives no kernel records."""
+    """Device time of one decode step by kind, from torch.profiler's kernel records of a few replays of the step's CUDA
+    graph: how much of the step is the quantized-linear path and how much the rest of the decoder (attention,
+    normalisation, rotary embedding and the other element-wise kernels torch launches).  The launches of the
+    quantized path overlap on purpose, so durations are not added up (see attribute).  None when the profiler gives no
+    kernel records."""
     try:
+        from torch.autograd import DeviceType
         from torch.profiler import ProfilerActivity, profile
 
         with profile(activities=[ProfilerActivity.CUDA]) as prof:
             for _ in range(replays):
                 step_graph.run_async()
             torch.cuda.synchronize()
-        kinds = {'qlinear': 0.0, 'embedding_dequant': 0.0, 'other': 0.0}
-        launches = {'qlinear': 0, 'embedding_dequant': 0, 'other': 0}
-        for row in prof.key_averages():
-            t = float(getattr(row, 'device_time_total', 0.0) or getattr(row, 'cuda_time_total', 0.0) or 0.0)
-            if t <= 0.0:
-                continue
-            kind = 'qlinear' if 'qlinear' in row.key else 'embedding_dequant' if 'embedding_dequant' in row.key else 'other'
-            kinds[kind] += t
-            launches[kind] += int(row.count)
-        total = sum(kinds.values())
-        if total <= 0.0:
+        kernels = []
+        for event in prof.events():
+            if event.device_type == DeviceType.CUDA and event.time_range.end > event.time_range.start:
+                kind = 'qlinear' if 'qlinear' in event.name else 'embedding_dequant' if 'embedding_dequant' in event.name else 'other'
+                kernels.append((event.time_range.start, event.time_range.end, kind))
+        if not kernels:
             return None
+        kinds = dict({'qlinear': 0.0, 'embedding_dequant': 0.0, 'other': 0.0}, **attribute(kernels))
+        total = sum(kinds.values())
         return {'us_per_step': {k: round(v / replays, 1) for k, v in kinds.items()},
-                'launches_per_step': {k: v // replays for k, v in launches.items()},
+                'launches_per_step': {k: sum(1 for x in kernels if x[2] == k) // replays for k in kinds},
                 'share_of_kernel_time_in_the_quantized_path': round((kinds['qlinear'] + kinds['embedding_dequant']) / total, 4)}
     except Exception as e:  # the profiler is optional equipment
         return {'unavailable': '{}: {}'.format(type(e).__name__, e)}

@@ -5,6 +5,8 @@ import subprocess
 import sys
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+if ROOT not in sys.path:
+    sys.path.insert(0, ROOT)
 
 
 def _run(extra_env=None, gpus=1):
@@ -40,3 +42,11 @@ def test_reference_arm_runs_on_rank_zero_only():
     done = _run({'RANK': '1', 'LOCAL_RANK': '1', 'WORLD_SIZE': '2'}, gpus=2)
     assert done.returncode == 0, done.stderr[-2000:]
     assert done.stdout.strip() == ''
+
+
+def test_kernel_time_counts_what_launches_share_once():
+    from bench_decoder import attribute
+
+    # the second launch starts early and waits for the first, the third runs inside the second, the fourth after a gap
+    kernels = [(8.0, 15.0, 'qlinear'), (0.0, 10.0, 'other'), (11.0, 14.0, 'other'), (20.0, 22.0, 'qlinear')]
+    assert attribute(kernels) == {'other': 10.0, 'qlinear': 7.0}
