@@ -1,6 +1,7 @@
 """csrc/host.cpp against the Python paths it shortens: the same results where it serves a call, None for whatever it does not."""
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.utils._python_dispatch import TorchDispatchMode
 
 import hidet_b200
@@ -172,6 +173,9 @@ def test_dispatch_modes_see_what_they_saw():
     assert torch.equal(got, want) and any('empty' in name for name in names.seen)
 
 
-def test_wrapped_tensors_are_refused_as_before():
+def test_fake_results_and_wrapped_tensors_are_refused_as_before():
+    a, (wq, scale) = _a(4, 256), _weight(256, 64)
+    with FakeTensorMode(), pytest.raises(ffi.BackendException, match='null output'):
+        hidet_b200.symmetric_quant_matmul(a, wq, scale)
     with pytest.raises(RuntimeError, match='storage'):
         torch.vmap(lambda w: hidet_b200.symmetric_quantize(w, 'int8', dims=0)[0])(_a(2, 8, 16))
