@@ -577,7 +577,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // that meet in distributed shared memory.  That is worth it only when one cluster per tile would leave most of the
     // machine idle, and only for splits of eight steps or more: with four, (1, 4096, 1024) takes 5.7 us against 3.8 and
     // (1, 8192, 1024) 6.5 against 6.3, though (1, 8192, 256) gains, 4.8 against 5.7.  (It is also what the scratch is sized by: with
-    // four the partial sums of (16, 1024, 11008) would not fit the array of b200q_qlinear_f16_i8_static any more.)
+    // four the partial sums of (16, 11008, 1024) would not fit the array of b200q_qlinear_f16_i8_static any more.)
     int groups = 1;
     if (c == kMaxCluster && tiles * c * 2 < sms) {
         int64_t splits = tiles > 0 ? (int64_t)sms * 4 / tiles : 1;
