@@ -20,6 +20,9 @@
 // the other CTAs' shared memory, and the slice is quantized from shared memory, so the weight
 // crosses HBM once.  max is exact and order-independent, so the result does not depend on the
 // schedule.
+//
+// No kernel of this file lets the launch behind it start early: the small-M quantized linear asks for its weight and scale
+// before it waits for the kernel in front, and is safe behind these only because it starts when they have ended.
 #include <cooperative_groups.h>
 #include <cfloat>
 
