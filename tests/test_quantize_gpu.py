@@ -199,3 +199,52 @@ def test_quotient_of_halves_is_cuda_s_for_every_pair(nvcc_library):
     mismatches = torch.zeros(1, dtype=torch.int64, device='cuda')
     assert f(mismatches.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
     assert mismatches.item() == 0
+
+
+def test_quotient_of_bfloat16_is_cuda_s(nvcc_library):
+    """As above for bfloat16, over every divisor that is taken as its reciprocal."""
+    import ctypes
+
+    from hidet_b200.build import PER_SOURCE_FLAGS
+
+    f = nvcc_library('bf16_quotient.cu', *PER_SOURCE_FLAGS['quantize.cu']).bf16_quotient_mismatches
+    f.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    mismatches = torch.zeros(1, dtype=torch.int64, device='cuda')
+    assert f(mismatches.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert mismatches.item() == 0
+
+
+@pytest.mark.parametrize('rows,cols', [(128, 64), (1100, 72), (37, 4104)])
+def test_quantize_bf16_bits(rows, cols):
+    """bfloat16 with special values: the packed kernels (columns a multiple of eight) give what the element-wise ones (an odd
+    count) do, and the definition in f32 steps where all is finite."""
+    g = torch.Generator().manual_seed(rows)
+    w = torch.randn(rows, cols, generator=g).mul_(0.02).to(torch.bfloat16)
+    finite = w.clone()
+    nan, inf = float('nan'), float('inf')
+    w[:, 0] = nan
+    w[:, 1] = -0.0; w[7, 1] = nan
+    w[:, 2] = -0.0; w[rows - 1, 2] = 0.0
+    w[5, 3] = nan
+    w[3, 4] = inf
+    w[rows - 2, 5] = -inf
+    w[:, 6] = -w[:, 6].abs() - 1e-3
+    w[:, 7] = 3.3895313892515355e38
+    w[:, 8] = 1e-40                     # below the normal numbers
+    w[:, 9] = 1.1754943508222875e-38; w[0, 9] = 5e-39   # the smallest normal number: the scale is below
+    w[:, 10] = 1.5e-36; w[0, 10] = 1e-39  # a scale next to the smallest normal number
+    w[:, 11] = torch.arange(rows) % 255 - 127.0   # exact ties
+    for dims in (0, -1):
+        both = w if dims == 0 else w.t().contiguous()
+        odd = both[:, :-1].contiguous() if dims == 0 else torch.cat([both, both[:, :1]], 1)
+        q, s = hidet_b200.symmetric_quantize(both.cuda(), 'int8', dims=dims)
+        qo, so = hidet_b200.symmetric_quantize(odd.cuda(), 'int8', dims=dims)
+        n = qo.shape[1] if dims == 0 else q.shape[1]
+        assert torch.equal(s[:len(so)].view(torch.int16).cpu(), so.view(torch.int16).cpu())
+        assert torch.equal(q[:, :n].cpu(), qo[:, :n].cpu())
+        q, s = hidet_b200.symmetric_quantize(finite.cuda(), 'int8', dims=dims)
+        want_s = (finite.abs().amax(dim=dims).float() / 127).to(torch.bfloat16)
+        assert torch.equal(s.cpu(), want_s)
+        quotient = (finite.float() / want_s.float().unsqueeze(dims)).to(torch.bfloat16)
+        inside = quotient.float().abs() <= 127   # (a scale rounded down leaves quotients of 127.5: what the conversion makes of 128 is compared above)
+        assert torch.equal(q.cpu()[inside], quotient.float().round().to(torch.int8)[inside])
