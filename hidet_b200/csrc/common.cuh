@@ -46,6 +46,8 @@ constexpr unsigned int kKernelDecode = 1;
 constexpr unsigned int kKernelPrefill = 2;
 constexpr unsigned int kKernelU4 = 3;
 constexpr unsigned int kKernelUnaligned = 4;
+constexpr unsigned int kKernelPair = 5;
+constexpr unsigned int kKernelMid = 6;
 
 // Number of SMs of the current device (cached per device).
 int sm_count();
@@ -121,6 +123,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// The same without blocking.  An answer takes about 200 clocks even where the phase is long over, so a pipeline's loop asks for
+// its next stage while it works on this one.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait on an mbarrier phase.  Returns false if `limit` polls passed without the phase
 // completing; the caller then records the failure and leaves.  Each poll of try_wait already
 // blocks for a hardware-defined interval, so the limit is a time bound of the order of a second.
@@ -162,6 +180,10 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
         " [%0], [%1, {%3, %4}], [%2], %5;"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "l"(policy)
         : "memory");
+}
+// Asks the tile into L2 only.
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap *map, int32_t x, int32_t y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t p;
@@ -238,6 +260,10 @@ __device__ __forceinline__ void st_async_v4f32(uint32_t addr, float4 v, uint32_t
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
                  "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
                  : "memory");
+}
+// One arrival on an mbarrier of a CTA of the cluster (address from map_to_rank).
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
 // Bounded wait on an mbarrier phase that remote CTAs complete (acquire at cluster scope).
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {

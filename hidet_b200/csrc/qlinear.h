@@ -22,6 +22,14 @@ struct OutTargets {
     int multicast = 0;
 };
 
+inline OutTargets one_output(void *c, int64_t columns) {
+    OutTargets t;
+    t.ptr[0] = c;
+    t.count = 1;
+    t.ldc = columns;
+    return t;
+}
+
 // What a kernel does to the scaled fp32 sums y[m, n] before the one rounding to f16:
 //   y += bias[n];  activation (silu_mul: the weight's columns come in pairs (gate_j, up_j) = (2j, 2j + 1), and
 //   z[m, j] = silu(y[m, 2j]) * y[m, 2j + 1] is the result, half as wide);  z += residual[m, j].
@@ -60,7 +68,8 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
 // The same kernel on a weight stored [N, K] (weight_nk = true): needs 16-byte aligned bases and K % 16 == 0.
 bool decode_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
 
-// The tensor-memory kernel for large M: same operand requirements as the small-M kernel.
+// The one-SM tensor-memory kernel for large M, which serves the multicast delivery and says what it cannot take: same operand
+// requirements as the small-M kernel.
 bool prefill_kn_supported(const void *a, const void *wq, int64_t N, int64_t K);
 // How the tensor-memory kernel splits K (narrow problems only) and the scratch that takes: fp32 partial sums
 // [k_splits][M][N] behind an untouched head of kSplitWorkspaceHead bytes (the small-M kernel's counters live there).
@@ -78,6 +87,25 @@ int launch_prefill_kn(const void *a, const void *wq, const void *scale, void *c,
                       int64_t lda = 0, void *workspace = nullptr, size_t workspace_bytes = 0);
 // The same kernel on a weight stored [N, K] (weight_nk = true): 16-byte aligned bases, K % 16 == 0, N % 8 == 0.
 bool prefill_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
+
+// More than a few rows: the kernel on pairs of SMs (tm, a multiple of 32 up to 256, rows per tile) and the mid-M
+// kernel (tm, a multiple of 16 up to 128, rows per tile; K split over a cluster).  Operands as for the kernel above;
+// outputs that 16-byte stores can write, at any number of addresses but not a multicast one; no workspace.
+struct LargePlan {
+    enum Kind { kNone, kMid, kPair };  // kNone: the small-M kernel is the better one
+    Kind kind = kNone;
+    int tm = 0;
+    int cluster = 1;
+};
+LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu);
+bool large_supported(const OutTargets &out, int64_t N, bool silu);
+int launch_large(const LargePlan &plan, const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,
+                 const Epilogue *epilogue, bool weight_nk, int64_t lda = 0);
+int launch_pair(const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,
+                const Epilogue *epilogue, bool weight_nk, int64_t lda, int tm);
+int launch_mid(const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,
+               const Epilogue *epilogue, bool weight_nk, int64_t lda, int tm, int cluster);
+int mid_resident_ctas(int tm, int cluster);  // of the mid-M kernel, in clusters of that size, that run at once
 
 // [K, N] weights whose rows are not multiples of 16 bytes: N even, K a multiple of 8, 16-byte aligned bases.
 bool unaligned_supported(const void *a, const void *wq, const void *c, int64_t M, int64_t N, int64_t K);

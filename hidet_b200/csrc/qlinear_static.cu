@@ -73,7 +73,11 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
         return set_error(B200Q_UNSUPPORTED, "qlinear_f16_i8_static: operands need 16-byte aligned bases and rows (N %% 16 == 0, K %% 8 == 0); "
                                             "got N=%lld K=%lld", (long long)N, (long long)K);
     }
-    if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, c, M, N, K, s);  // needs no scratch at all
+    if (use_prefill_kernel(M, N, K)) {  // needs no scratch at all
+        const LargePlan large = plan_large(M, N, K, false);
+        if (large.kind != LargePlan::kNone && large_supported(one_output(c, N), N, false)) return launch_large(large, a, wq, scale, one_output(c, N), M, N, K, s, nullptr, false);
+        return launch_prefill_kn(a, wq, scale, c, M, N, K, s);
+    }
 
     const DecodePlan plan = plan_decode(M, N, K);
     const size_t need = plan.counter_bytes + plan.partial_bytes;
