@@ -36,7 +36,7 @@ double mid_us(int64_t M, int64_t N, int64_t K, int *tm, int *cluster) {
 }
 
 // A 64-k stage of the kernel on SM pairs by tile height, and what a tile costs on top: next to nothing where two accumulators
-// fit in tensor memory (up to 192 rows), the epilogue where only one does.  (512, 4096, 22016) with SiLU: 121 / 93 / 88 / 111 us
+// fit in tensor memory (up to 192 rows), the epilogue where only one does.  (512, 4096, 22016) with SiLU: 124 / 96 / 88 / 87 us
 // at 96 / 128 / 192 / 256 rows; (2048, 8192, 28672): 889 / 728 / 690 / 638 at 128 / 192 / 224 / 256; (256, 4096, 11008): 38 at
 // 96 to 192 rows, 42 at 224, 26 at 256.
 double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
@@ -49,7 +49,7 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
     double best = 1e30;
     for (const auto &f : forms) {
         const int64_t tiles = ceil_div(N, 256) * ceil_div(M, f.tm);
-        const double tile = f.tm <= 192 ? 0.3 : (silu ? 13.0 : 4.0);
+        const double tile = f.tm <= 192 ? 0.3 : (silu ? 6.0 : 2.5);
         const double us = 4.5 + (double)ceil_div(tiles, sms / 2) * ((double)ceil_div(K, 64) * f.stage + tile);
         if (us < best) {
             best = us;

@@ -8,9 +8,11 @@
 // int8 in and out and TM / 2 rows of activations in and out: 48 KB at TM = 256, for 512 clocks of MMA.  The single-SM form
 // (qlinear_prefill.cu) writes and reads the f16 weight there too and fetches every activation row itself: 112 KB.
 //
-// One persistent CTA per SM, fifteen warps:
-//   warps 0-3   epilogue: tensor memory -> scale, bias, gate / up pairing, residual -> f16, transposed through a staging
-//               buffer (two, taken in turn) by matrix stores, 16-byte stores of whole output rows
+// One persistent CTA per SM, nineteen warps:
+//   warps 0-3, 15-18 epilogue, two groups that take the 32-row blocks of a tile in turn: tensor memory -> scale, bias, gate / up pairing, residual -> f16, transposed through a staging
+//               buffer (two per group, taken in turn) by matrix stores, 16-byte stores of whole output rows.  (One group:
+//               (512, 4096, 22016) with SiLU 109 us for 87 in tiles of 256 rows, (1000, 4096, 4096) with a residual 37.6 for
+//               31.7, (2048, 256, 28672) 58.7 for 45.7.)
 //   warps 4-11  converters, two groups that take stages in turn: int8 tile -> registers by matrix loads (transposing ones for
 //               [K, N] weights) that leave a lane four consecutive k of one column, int8 -> exact f16, tcgen05.st.  The
 //               fragment of the loads is the fragment of the 16x256b store, so nothing is exchanged between lanes.
@@ -34,17 +36,18 @@ namespace pair {
 constexpr int TN = 128;                      // weight columns per CTA; a pair's tile has twice as many
 constexpr int BK = 64;                       // k per stage = four MMAs of K = 16
 constexpr int RAW_BYTES = BK * TN;           // int8 tile of one CTA
-constexpr int RAW_SLOTS = 12;                // 96 KB in flight: (512, 4096, 22016) with SiLU 88 us, 97 with 6
+constexpr int RAW_SLOTS = 10;                // 80 KB in flight
 constexpr int ACT_RING_BYTES = 96 * 1024;    // halves of activation tiles: as many slots as fit, at most MAX_SLOTS
 constexpr int MAX_SLOTS = 12;
 constexpr int MAX_W_SLOTS = 8;               // converted weight tiles in tensor memory, 32 columns each, behind the accumulators
 constexpr int TMEM_COLS = 512;
 constexpr int CONV_WARPS = 8, CONV_GROUPS = 2, GROUP_WARPS = CONV_WARPS / CONV_GROUPS;
 constexpr int CONV_WARP0 = 4, RAW_WARP = 12, ACT_WARP = 13, MMA_WARP = 14;
-constexpr int THREADS = 32 * 15;
+constexpr int EPI_GROUPS = 2, EPI_WARP1 = 15;
+constexpr int THREADS = 32 * 19;
 constexpr int ROW_BYTES = TN * 2 + 16;       // one output row in the staging buffer, padded: matrix stores touch every bank once
 constexpr int STAGING_BYTES = 32 * ROW_BYTES;
-constexpr int SMEM_BYTES = ACT_RING_BYTES + RAW_SLOTS * RAW_BYTES + 2 * STAGING_BYTES + 1024;  // + alignment slack
+constexpr int SMEM_BYTES = ACT_RING_BYTES + RAW_SLOTS * RAW_BYTES + EPI_GROUPS * 2 * STAGING_BYTES + 1024;  // + alignment slack
 
 // A parity wait tells a phase only from its neighbours, so a waiter has to see every phase of its barriers: stage i belongs
 // to converter group i % CONV_GROUPS, and every ring's length is a multiple of CONV_GROUPS, so that a slot stays with one group.
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&acc_full[b]), 1);
-            mbar_init(smem_u32(&acc_empty[b]), 2 * 4);
+            mbar_init(smem_u32(&acc_empty[b]), 2 * 4 * EPI_GROUPS);
         }
         mbar_init(smem_u32(&drain_bar), 1);
         abort_flag = 0;
@@ -265,7 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
             umma::commit_pair_self(smem_u32(&drain_bar));
             if (!mbar_wait(smem_u32(&drain_bar), 0)) report_timeout(p.status, kKernelPair, 8);
         }
-    } else if (warp >= CONV_WARP0) {
+    } else if (warp >= CONV_WARP0 && warp < RAW_WARP) {
         // ---------------- converters ----------------
         const int cw = warp - CONV_WARP0;
         const int group = cw / GROUP_WARPS;   // converts stages group, group + CONV_GROUPS, ...
@@ -318,8 +321,10 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         }
     } else {
         // ---------------- epilogue ----------------
-        const int q = warp;                     // tensor-memory lanes 32 q .. 32 q + 31
-        const int et = threadIdx.x;             // 0 .. 127
+        const int eg = warp >= EPI_WARP1 ? 1 : 0;  // takes blocks eg, eg + EPI_GROUPS, ...
+        const int q = warp & 3;                 // tensor-memory lanes 32 q .. 32 q + 31
+        const int et = 32 * q + lane;           // 0 .. 127
+        auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + eg) : "memory"); };
         const int g = lane >> 2, tq = lane & 3; // fragment coordinates: column g of an 8-column block, rows 2 tq, 2 tq + 1 of an 8-row block
         const bool pairs = FUSED && p.ep.act == kActSiluMul;  // columns (2j, 2j + 1) = (gate, up)
         const __half *res = FUSED ? static_cast<const __half *>(p.ep.residual) : nullptr;
@@ -330,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         const int row_in_pass = et >> row_chunks_log2;
         const int pass_rows = 128 >> row_chunks_log2;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * q) << 16);
-        uint32_t t_iter = 0, block = 0;         // block: 32-row blocks so far, staging buffers in turn
+        uint32_t t_iter = 0, block = 0;         // block: the group's 32-row blocks so far, staging buffers in turn
         for (int u = first; u < units; u += step, ++t_iter) {
             int n0, m0;
             tile_of(p, u, n0, m0);
@@ -353,10 +358,14 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
             const int out_n0 = pairs ? n0 >> 1 : n0;
             const bool cols_ok = out_n0 + chunk * 8 < out_n;  // widths are multiples of 8: eight columns are in or out together
             const size_t out_off = (size_t)m0 * p.out.ldc + p.out.col0 + out_n0 + chunk * 8;
+            if (eg >= blocks) {  // a tile of a single block: nothing for this group
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(map_to_rank(smem_u32(&acc_empty[buf]), 0));
+            }
 #pragma unroll 1
-            for (int cb = 0; cb < blocks; ++cb, ++block) {
-                unsigned char *staging = smem_gen + STAGING_OFF + (block & 1) * STAGING_BYTES;
-                const uint32_t staging_a = smem_base + STAGING_OFF + (block & 1) * STAGING_BYTES;
+            for (int cb = eg; cb < blocks; cb += EPI_GROUPS, ++block) {
+                unsigned char *staging = smem_gen + STAGING_OFF + (2 * eg + (block & 1)) * STAGING_BYTES;
+                const uint32_t staging_a = smem_base + STAGING_OFF + (2 * eg + (block & 1)) * STAGING_BYTES;
                 if (res_vec && res != nullptr) {
                     // the residual's block goes through the staging buffer into the fragments' layout
 #pragma unroll
@@ -366,13 +375,13 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
                         if (m < m_left && cols_ok) val = __ldcg(reinterpret_cast<const uint4 *>(res + (size_t)(m0 + m) * p.ep.ldr + out_n0 + chunk * 8));
                         *reinterpret_cast<uint4 *>(staging + r * ROW_BYTES + chunk * 16) = val;
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    group_sync();
                 }
                 uint32_t v[2][16];
                 umma::ld_16x256b_x4(acc + cb * 32, v[0]);
                 umma::ld_16x256b_x4(acc + (16u << 16) + cb * 32, v[1]);
                 umma::ld_wait();
-                if (cb == blocks - 1) {  // the accumulator is in registers
+                if (cb + EPI_GROUPS >= blocks) {  // the group's part of the accumulator is in registers
                     umma::fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_remote(map_to_rank(smem_u32(&acc_empty[buf]), 0));
@@ -446,7 +455,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
                         umma::stmatrix_x4_trans(place, pk);
                     }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps: block complete; the other buffer is free
+                group_sync();  // the four warps: block complete; the other buffer is free
 #pragma unroll 4
                 for (int r = row_in_pass; r < 32; r += pass_rows) {
                     const int m = cb * 32 + r;
