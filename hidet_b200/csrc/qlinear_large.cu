@@ -8,9 +8,9 @@
 namespace b200q {
 namespace {
 
-// The small-M kernel walks its 16-row blocks over the weight, from L2 after the first: (32, 4096, 4096) 9.1 us, (32, 4096, 12288) 27,
-// (64, 4096, 4096) 14.7, (50, 1024, 1024) 4.7.
-double small_m_us(int64_t M, int64_t N, int64_t K) { return 3.3 + (double)K * N / 3.9e6 * (1.0 + 0.6 * (double)(ceil_div(M, 16) - 1)); }
+// The small-M kernel walks its 16-row blocks over the weight, from L2 after the first: (32, 4096, 4096) 8.8 us, (32, 4096, 12288) 25,
+// (32, 11008, 4096) 17.9, (64, 4096, 4096) 13.5, (64, 2048, 2048) 5.9, (64, 1024, 1024) 3.4.
+double small_m_us(int64_t M, int64_t N, int64_t K) { return 2.6 + (double)K * N / 3.9e6 * (1.0 + 0.55 * (double)(ceil_div(M, 16) - 1)); }
 
 // A 64-k stage of the mid-M kernel takes 0.30 us with one CTA an SM and 0.46 with two, a fifth more at 128 rows than at 64; the launch
 // and its tail 4.2, and each CTA of a cluster makes the exchange longer.  (64, 4096, 4096): 24.7 / 15.2 / 10.9 / 11.5 us in

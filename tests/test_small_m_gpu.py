@@ -1,0 +1,45 @@
+"""The small-M kernel's last step, four columns a thread: counts and addresses that are not multiples of four."""
+import ctypes
+
+import pytest
+import torch
+
+import hidet_b200
+from hidet_b200 import ffi
+from hidet_b200.runtime import workspaces
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, k, n, layout):
+    g = torch.Generator(device='cuda').manual_seed(m + k + n)
+    a = torch.randn(m, k, generator=g, device='cuda').half()
+    wq = torch.randint(-128, 128, (k, n) if layout == 'KN' else (n, k), generator=g, device='cuda', dtype=torch.int8)
+    scale = (torch.rand(n, generator=g, device='cuda') * 1e-3 + 1e-4).half()
+    want = (a.double() @ (wq if layout == 'KN' else wq.t()).double()) * scale.double()
+    return a, wq, scale, want
+
+
+def _close(got, want):
+    # one rounding to f16, half an ulp of the value; the f32 sums in front of it are far closer
+    assert float((got.double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
+
+
+@pytest.mark.parametrize('m', [1, 2, 3, 9, 16])
+@pytest.mark.parametrize('k,n', [(1024, 129), (2048, 258), (4096, 1027), (512, 4095)])
+def test_odd_column_counts(m, k, n):
+    a, wq, scale, want = _operands(m, k, n, 'NK')
+    _close(hidet_b200.symmetric_quant_matmul(a, wq, scale, weight_layout='NK'), want)
+
+
+@pytest.mark.parametrize('m', [1, 7, 16])
+@pytest.mark.parametrize('ldc,col0', [(1293, 7), (1290, 2), (1284, 4)])
+def test_destinations_at_any_element(m, ldc, col0):
+    a, wq, scale, want = _operands(m, 1536, 1280, 'KN')
+    out = torch.full((m, ldc), -7.0, dtype=torch.float16, device='cuda')
+    table = (ctypes.c_void_p * 1)(out.data_ptr())
+    ws_ptr, ws_size = workspaces.get(a.device, ffi.func('b200q_qlinear_workspace_bytes')(m, 1280, 1536, 0))
+    ffi.func('b200q_qlinear_f16_i8_to_peers')(a.data_ptr(), wq.data_ptr(), scale.data_ptr(), table, 1, ldc, col0, m, 1280, 1536, ws_ptr, ws_size,
+                                             torch.cuda.current_stream().cuda_stream)
+    _close(out[:, col0:col0 + 1280], want)
+    assert bool((out[:, :col0] == -7.0).all()) and bool((out[:, col0 + 1280:] == -7.0).all())
