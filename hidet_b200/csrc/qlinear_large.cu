@@ -65,7 +65,7 @@ LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu) {
     LargePlan p;
     if (M <= 16) return p;
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
-    const double mid = M <= 512 ? mid_us(M, N, K, &mid_tm, &mid_cluster) : 1e30;
+    const double mid = M <= 65535 * 128 ? mid_us(M, N, K, &mid_tm, &mid_cluster) : 1e30;  // the grid's limit
     const double pair = M > 32 ? pair_us(M, N, K, silu, &pair_tm) : 1e30;
     const double best = mid < pair ? mid : pair;
     if (!use_prefill_kernel(M, N, K) && best > 0.85 * small_m_us(M, N, K)) return p;

@@ -33,7 +33,7 @@ def _run(m, k, n, layout, bias=False, silu=False, residual=False):
     assert float((got.double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
 
 
-# more than 512 rows: always the kernel on SM pairs; the heights of tiles, their last rows and columns, k that ends inside a
+# the kernel on SM pairs, and the mid-M one where columns are few: the heights of tiles, their last rows and columns, k that ends inside a
 # stage, one stage, fewer stages than ring slots and more, one tile and several per pair
 @pytest.mark.parametrize('m,k,n', [(513, 64, 16), (600, 8, 256), (513, 72, 272), (777, 1000, 528), (1025, 520, 2064), (1500, 2048, 1040), (2048, 1032, 16), (3001, 456, 4112)])
 def test_pair_kernel_edges(m, k, n):
@@ -49,7 +49,7 @@ def test_pair_kernel_epilogues(m, k, n, epilogue):
 
 
 # K in one part and in eight, parts of unequal length, tiles of 16 to 128 rows, two row tiles, the last rows and columns
-@pytest.mark.parametrize('m,k,n', [(65, 64, 16), (66, 128, 272), (80, 464, 272), (100, 1872, 336), (33, 2736, 10800), (129, 1032, 144), (144, 4096, 528), (24, 4096, 12288), (200, 8200, 1040)])
+@pytest.mark.parametrize('m,k,n', [(65, 64, 16), (66, 128, 272), (80, 464, 272), (100, 1872, 336), (33, 2736, 10800), (129, 1032, 144), (144, 4096, 528), (24, 4096, 12288), (200, 8200, 1040), (598, 6256, 352)])
 def test_mid_kernel_edges(m, k, n):
     _run(m, k, n, 'KN')
     if k % 16 == 0:
