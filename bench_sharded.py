@@ -253,7 +253,7 @@ def run_sharded(args) -> int:
             'clocks': clocks.summary(),
             'roofline': {'bound': 'hbm for M <= 16, tensor for M >= 256', 'achieved': value, 'peak': peaks['hbm_gbs'] * world, 'unit': 'GB/s',
                          'frac': value / (peaks['hbm_gbs'] * world), 'traffic': None, 'peak_source': peaks['source'] + ' (burst copy) x n_gpus',
-                         'kernel': 'qlinear_decode_kn_kernel / qlinear_prefill_kn_kernel' + (' + ncclAllGather' if args.gather == 'nccl' else ' (peer stores)')},
+                         'kernel': 'qlinear_decode_kn_kernel / qlinear_mid_kernel / qlinear_pair_kernel / qlinear_prefill_kn_kernel' + (' + ncclAllGather' if args.gather == 'nccl' else ' (peer stores)')},
             'shapes': shapes,
             'e2e': {'value': e2e_value, 'unit': 'GB/s', 'h2d_bytes_per_step': sum(t.numel() * 2 for t in pinned_in.values()),
                     'd2h_bytes_per_step': sum(t.numel() * 2 for t in pinned_out.values()), 'ms_per_step': e2e_ms},
