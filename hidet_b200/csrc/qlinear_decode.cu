@@ -217,8 +217,12 @@ struct Params {
 // NK: the weight is [N, K] with K contiguous (the layout torch.nn.Linear keeps) instead of the reference's
 //     [K, N]: a stage is then 128 weight rows of 64 k-bytes (64-byte swizzle) and the fragments come from
 //     plain matrix loads; everything else is shared.
-template <int MT, bool NK>
-__global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
+// QUAD: the elements that a CTA finishes in the split-K reduction are taken four adjacent columns of a row per thread (more than
+//     four rows; with fewer one element per thread is one round anyway: (4, 9648, 1568) 7.9 us, 8.05 so).
+// Shared memory lets four CTAs share an SM; told so, the compiler spills nothing: a decode step for sixteen sequences 252 -> 242 us,
+// for one 208.8 -> 205.6.
+template <int MT, bool NK, bool QUAD>
+__global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
     using Cfg = Config<MT>;
     constexpr int ROWS = Cfg::ROWS, A_STAGE_BYTES = Cfg::A_STAGE_BYTES, PIPE_BYTES = Cfg::PIPE_BYTES;
     extern __shared__ unsigned char smem_dyn[];
@@ -273,14 +277,17 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
     // then every CTA of the cluster has started and set up its barriers, which remote access requires.
     cluster_arrive_release();
 
-    // The four columns of a row that this thread finishes in the split-K reduction, and their scales.  Like the weight, the
-    // scales do not depend on the kernel before this one, so they are fetched now, far from where they are used.
-    const int quads = cols_per >> 2;  // of one row of this CTA's columns
-    float sc_own[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (p.mode == kModeSplit) {
-        const int cc = ((int)threadIdx.x % quads) * 4;
+    // What this thread finishes in the split-K reduction (one element, or with QUAD four columns of a row), and the scales.  Like
+    // the weight, the scales do not depend on the kernel before this one, so they are fetched now, far from where they are used.
+    constexpr int WIDTH = QUAD ? 4 : 1;
+    const int per_row = cols_per / WIDTH;  // such pieces of one row of this CTA's columns
+    float sc_own[WIDTH];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < WIDTH; ++j) sc_own[j] = 0.0f;
+    if (p.mode == kModeSplit) {
+        const int cc = ((int)threadIdx.x % per_row) * WIDTH;
+#pragma unroll
+        for (int j = 0; j < WIDTH; ++j)
             if (cc < own_cols && n0 + own_first + cc + j < p.N) sc_own[j] = __half2float(__ldg(p.scale + n0 + own_first + cc + j));
     }
 
@@ -498,42 +505,63 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
     if (own_cols > 0) {
         if (!mbar_wait_cluster(smem_u32(&recv_bar), 0)) report_timeout(p.status, kKernelDecode, 4);
     }
-    // Owner: four adjacent columns of one row per thread and round, so that 16 rows of a slice are one round (one element per
-    // thread made four of them, each with its trips to memory: (16, 1408, 1408) with a residual 5.5 -> 3.7 us, (16, 4096, 12288)
-    // 13.3 -> 11.9).  Item i is row i / quads, columns 4 (i % quads) .. + 3; the partials of the (at most eight) ranks are read
-    // together and added in rank order.
+    // Owner: the partials of the (at most eight) ranks are read together and added in rank order.
     const int col_first = n0 + own_first;  // first column this CTA owns
-    auto sum_ranks4 = [&](int r, int cc) {
-        float4 v[8];
-#pragma unroll
-        for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? *reinterpret_cast<const float4 *>(recv + (jr * ROWS + r) * cols_per + cc) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 sum = v[0];
-#pragma unroll
-        for (int jr = 1; jr < 8; ++jr) sum.x += v[jr].x, sum.y += v[jr].y, sum.z += v[jr].z, sum.w += v[jr].w;
-        return sum;
-    };
     if (p.groups == 1) {
-        for (int item = threadIdx.x; item < rows * quads; item += THREADS) {
-            const int r = item / quads;
-            const int cc = (item - r * quads) * 4;
-            const int nn = col_first + cc;
-            if (cc >= own_cols || nn >= p.N) continue;  // own_cols is a multiple of 8
-            float4 y = sum_ranks4(r, cc);
-            if (item < THREADS) {
-                y.x *= sc_own[0], y.y *= sc_own[1], y.z *= sc_own[2], y.w *= sc_own[3];
-            } else {
-                y.x *= __half2float(p.scale[nn]);
-                if (nn + 1 < p.N) y.y *= __half2float(p.scale[nn + 1]);
-                if (nn + 2 < p.N) y.z *= __half2float(p.scale[nn + 2]);
-                if (nn + 3 < p.N) y.w *= __half2float(p.scale[nn + 3]);
-            }
-            if (nn + 3 < p.N) {
-                finish4(p.out, p.ep, m0 + r, nn, y);
-            } else {  // the end of an [N, K] weight's odd column count: no epilogue there
-                const float e[3] = {y.x, y.y, y.z};
+        if constexpr (QUAD) {
+            // Four adjacent columns of one row per thread and round, so that 16 rows of a slice are one round (one element per thread
+            // made four of them, each with its trips to memory: (16, 1408, 1408) with a residual 5.5 -> 3.6 us, (16, 4096,
+            // 12288) 13.3 -> 11.9, (7, 896, 12112) 5.8 -> 4.7).  Item i is row i / per_row, columns 4 (i % per_row) .. + 3.
+            auto sum_ranks4 = [&](int r, int cc) {
+                float4 v[8];
 #pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    if (nn + j < p.N) store_out(p.out, m0 + r, nn + j, __float2half_rn(e[j]));
+                for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? *reinterpret_cast<const float4 *>(recv + (jr * ROWS + r) * cols_per + cc) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                float4 sum = v[0];
+#pragma unroll
+                for (int jr = 1; jr < 8; ++jr) sum.x += v[jr].x, sum.y += v[jr].y, sum.z += v[jr].z, sum.w += v[jr].w;
+                return sum;
+            };
+            for (int item = threadIdx.x; item < rows * per_row; item += THREADS) {
+                const int r = item / per_row;
+                const int cc = (item - r * per_row) * 4;
+                const int nn = col_first + cc;
+                if (cc >= own_cols || nn >= p.N) continue;  // own_cols is a multiple of 8
+                float4 y = sum_ranks4(r, cc);
+                if (item < THREADS) {
+                    y.x *= sc_own[0], y.y *= sc_own[1], y.z *= sc_own[2], y.w *= sc_own[3];
+                } else {
+                    y.x *= __half2float(p.scale[nn]);
+                    if (nn + 1 < p.N) y.y *= __half2float(p.scale[nn + 1]);
+                    if (nn + 2 < p.N) y.z *= __half2float(p.scale[nn + 2]);
+                    if (nn + 3 < p.N) y.w *= __half2float(p.scale[nn + 3]);
+                }
+                if (nn + 3 < p.N) {
+                    finish4(p.out, p.ep, m0 + r, nn, y);
+                } else {  // the end of an [N, K] weight's odd column count: no epilogue there
+                    const float e[3] = {y.x, y.y, y.z};
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        if (nn + j < p.N) store_out(p.out, m0 + r, nn + j, __float2half_rn(e[j]));
+                }
+            }
+        } else {
+            // One element per thread and round; element i is row i / cols_per, column i % cols_per of the slice.
+            auto sum_ranks = [&](int r, int cc) {
+                float v[8];
+#pragma unroll
+                for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? recv[(jr * ROWS + r) * cols_per + cc] : 0.0f;
+                float sum = v[0];
+#pragma unroll
+                for (int jr = 1; jr < 8; ++jr) sum += v[jr];
+                return sum;
+            };
+            for (int idx = threadIdx.x; idx < rows * cols_per; idx += THREADS) {
+                const int r = idx / cols_per;
+                const int cc = idx - r * cols_per;
+                const int nn = col_first + cc;
+                const bool valid = nn < p.N && cc < own_cols;  // N and own_cols are even: the two columns of a pair agree
+                const float sc = idx < THREADS ? sc_own[0] : (valid ? __half2float(p.scale[nn]) : 0.0f);
+                finish(p.out, p.ep, m0 + r, nn, p.N, valid, valid ? sum_ranks(r, cc) * sc : 0.0f, 1);
             }
         }
         return;
@@ -573,7 +601,7 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
         if (valid) {
 #pragma unroll 4
             for (int gr = 0; gr < p.groups; ++gr) v += __ldcg(&p.partial[((size_t)gr * p.M + (m0 + r)) * p.N + nn]);
-            v *= __half2float(p.scale[nn]);
+            v *= !QUAD && idx < THREADS ? sc_own[0] : __half2float(p.scale[nn]);
         }
         finish(p.out, p.ep, m0 + r, nn, p.N, valid, v, 1);
     }
@@ -584,18 +612,19 @@ __global__ void __launch_bounds__(THREADS) qlinear_decode_kn_kernel(const __grid
 
 namespace decode {
 
-// One instantiation of the kernel per layout: up to eight activation rows, and more.
+// One instantiation of the kernel per layout: up to four activation rows, up to eight, and more.
 struct Variant {
     const void *kn, *nk;
     int rows, smem;
 };
-template <int MT>
+template <int MT, bool QUAD>
 static Variant make_variant() {
-    return {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true>),
+    return {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false, QUAD>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD>),
             Config<MT>::ROWS, Config<MT>::SMEM_BYTES};
 }
-static const Variant kVariants[2] = {make_variant<1>(), make_variant<2>()};
-static const Variant &variant(int64_t M) { return kVariants[M <= 8 ? 0 : 1]; }
+constexpr int kVariantCount = 3;
+static const Variant kVariants[kVariantCount] = {make_variant<1, false>(), make_variant<1, true>(), make_variant<2, true>()};
+static const Variant &variant(int64_t M) { return kVariants[M <= 4 ? 0 : (M <= 8 ? 1 : 2)]; }
 
 static int set_attributes() {
     static std::atomic<bool> attr_set[64];  // per device, zero-initialised; a repeated set by a racing thread is harmless
@@ -612,7 +641,7 @@ static int set_attributes() {
 // CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use.  Looked up once
 // per device; without a device, an estimate.
 static int resident_ctas(const Variant &v, int cluster) {
-    static std::atomic<int> known[64][2][kMaxCluster + 1];
+    static std::atomic<int> known[64][kVariantCount][kMaxCluster + 1];
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || set_attributes() != B200Q_OK) {
         cudaGetLastError();
