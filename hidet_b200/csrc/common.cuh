@@ -150,6 +150,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     return false;
 }
 
+// One answer for the 128 threads that meet at named barrier `id`: true where all of them bring true.  A wait that may give up is
+// decided so in front of that barrier: with an answer per warp, one could leave and the others stay at the barrier for good.
+__device__ __forceinline__ bool all_of_128(int id, bool ok) {
+    uint32_t all;
+    __syncwarp();
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %2, 0;\n\t"
+        "bar.red.and.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(all)
+        : "r"(id), "r"((uint32_t)ok)
+        : "memory");
+    return all != 0;
+}
+
 // status[0] collects every wait that ran out (codes or-ed together: one failure starves the other
 // roles, whose waits then run out too); status[1] keeps the first one.
 __device__ __forceinline__ void report_timeout(unsigned int *status, unsigned int kernel, unsigned int site) {

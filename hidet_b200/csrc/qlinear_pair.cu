@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
                     sc[h][e] = n < p.N ? __half2float(__ldcg(p.scale + n)) : 0.0f;
                     bias[h][e] = (FUSED && n < p.N && p.ep.bias != nullptr) ? __half2float(__ldcg(static_cast<const __half *>(p.ep.bias) + n)) : 0.0f;
                 }
-            if (!wait(smem_u32(&acc_full[buf]), acc_use & 1, 10)) break;
+            if (!all_of_128(1 + eg, wait(smem_u32(&acc_full[buf]), acc_use & 1, 10))) break;  // the group stays or leaves as one
             umma::fence_after_sync();
             const int out_n0 = pairs ? n0 >> 1 : n0;
             const bool cols_ok = out_n0 + chunk * 8 < out_n;  // widths are multiples of 8: eight columns are in or out together

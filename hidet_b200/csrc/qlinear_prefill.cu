@@ -356,10 +356,9 @@ __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __
                 const uint32_t use = i / STAGES;
                 // The int8 tile must have landed (on the barrier of this slot that belongs to this group),
                 // and the MMAs that read the f16 slot last time must be done.
-                if (!wait(smem_u32(&raw_full[r][group]), (i / RAW_PERIOD) & 1, 4) || (use >= 1 && !wait(smem_u32(&slot_free[s]), (use - 1) & 1, 4))) {
-                    ok = false;
-                    break;
-                }
+                ok = wait(smem_u32(&raw_full[r][group]), (i / RAW_PERIOD) & 1, 4) && (use < 1 || wait(smem_u32(&slot_free[s]), (use - 1) & 1, 4));
+                ok = __all_sync(0xffffffffu, ok);  // a warp stays or leaves as one: the steps below want all of its lanes
+                if (!ok) break;
                 const uint32_t raw = raw_addr(r), wf = wf_addr(s);
                 if (NK) {
                     uint4 v[BK / CONV_ROWS];
@@ -433,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __
             const int n0 = (otile % p.n_tiles) * TN;
             const int m0 = (otile / p.n_tiles) * TM;
             const uint32_t buf = t_iter & 1, acc_use = t_iter >> 1;
-            if (!wait(smem_u32(&acc_full[buf]), acc_use & 1, 5)) break;
+            if (!all_of_128(1, wait(smem_u32(&acc_full[buf]), acc_use & 1, 5))) break;  // the four warps stay or leave as one
             tc_fence_after_sync();
             const int n = n0 + 32 * q + lane;
             if (p.k_splits > 1) {

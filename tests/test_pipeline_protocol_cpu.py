@@ -1,16 +1,16 @@
-"""The large-M kernel's barrier protocol, model-checked on the host under random schedules (no GPU)."""
+"""The barrier protocols of the tensor-memory kernels, model-checked on the host under random schedules (no GPU)."""
 import dataclasses
 import random
 
 import pytest
 
-from pipeline_model import Pipeline, ProtocolError, config_from_source
+from pipeline_model import Pipeline, ProtocolError, TensorMemoryPipeline, config_from_source, pair_config_from_source
 
 
 @pytest.mark.parametrize('tm', [256, 64])
 def test_kernel_configuration_is_consistent(tm):
     cfg = config_from_source(tm)
-    assert cfg.group_warps * cfg.conv_groups == 8
+    assert cfg.group_warps * cfg.conv_groups == 8 and cfg.epilogue_agrees
     # the (slot, group) pair of stage i is (i % raw_slots, i % conv_groups): it recurs with the least common multiple
     lcm = next(n for n in range(1, 1000) if n % cfg.raw_slots == 0 and n % cfg.conv_groups == 0)
     assert cfg.raw_period == lcm
@@ -65,7 +65,7 @@ def test_a_wait_that_runs_out_ends_every_role_and_the_cta_retires_clean(tm):
                 pipe = Pipeline(cfg, 3, 9, random.Random(seed))
                 pipe.expire = (agent, nth)
                 pipe.run(copy_delay=0.9)
-                runs += 1 if pipe.abort else 0
+                runs += 1 if any(pipe.abort) else 0
     assert runs > 100   # the flag was really raised in most of these schedules
 
 
@@ -81,3 +81,51 @@ def test_model_catches_a_teardown_without_the_drain():
             assert 'retired with' in str(e)
             failures += 1
     assert failures > 0
+
+
+def test_model_catches_an_epilogue_whose_warps_decide_one_by_one():
+    """A wait that gives up in one warp while the accumulator completes for the others: those wait for it at the named barrier
+    of the group for good, in front of a barrier that nothing bounds."""
+    for make in (lambda seed: Pipeline(dataclasses.replace(config_from_source(256), epilogue_agrees=False), 3, 3, random.Random(seed)),
+                 lambda seed: TensorMemoryPipeline(dataclasses.replace(pair_config_from_source(256), epilogue_agrees=False), 3, 3, random.Random(seed))):
+        found = 0
+        for seed in range(400):
+            pipe = make(seed)
+            pipe.expire = (len(pipe.roles()) - 1 - seed % 4, 1 + seed)   # a warp of the (last) epilogue group
+            try:
+                pipe.run(copy_delay=0.5)
+            except ProtocolError as e:
+                assert 'deadlock' in str(e)
+                found += 1
+        assert found > 0
+
+
+@pytest.mark.parametrize('tm', range(32, 257, 32))
+def test_pair_kernel_configuration_is_consistent(tm):
+    cfg = pair_config_from_source(tm)
+    assert cfg.epilogue_agrees
+    # a slot stays with one converter group, so that the group sees every phase of its barriers
+    assert cfg.raw_slots % cfg.conv_groups == cfg.act_slots % cfg.conv_groups == cfg.w_slots % cfg.conv_groups == 0
+    assert cfg.n_acc * tm + 32 * cfg.w_slots <= 512 and cfg.w_slots >= 4 and cfg.act_slots >= 4
+
+
+@pytest.mark.parametrize('tm', [32, 160, 192, 224, 256])
+@pytest.mark.parametrize('tiles,k_blocks', [(1, 1), (1, 13), (3, 8), (5, 3)])
+def test_pair_protocol_holds_under_random_schedules(tm, tiles, k_blocks):
+    for seed in range(10):
+        for delay in (0.2, 0.9, 0.99):
+            TensorMemoryPipeline(pair_config_from_source(tm), tiles, k_blocks, random.Random(seed)).run(copy_delay=delay)
+
+
+@pytest.mark.parametrize('tm', [128, 256])
+def test_a_wait_of_the_pair_kernel_that_runs_out_ends_every_role_of_both_ctas(tm):
+    cfg = pair_config_from_source(tm)
+    runs = 0
+    for seed in range(4):
+        for agent in range(1 + 2 * (2 + 8 + 8)):
+            for nth in (1, 3, 17):
+                pipe = TensorMemoryPipeline(cfg, 3, 5, random.Random(seed))
+                pipe.expire = (agent, nth)
+                pipe.run(copy_delay=0.9)
+                runs += 1 if any(pipe.abort) else 0
+    assert runs > 100
