@@ -16,19 +16,20 @@
  *   - every entry point returns a b200q_status.  On failure a thread-local message is kept and
  *     b200q_get_last_error() returns it and clears it (read-and-clear, like
  *     hidet_get_last_error).  Nothing aborts the process and no kernel traps.
- *   - the kernels of the quantized linears (int8 weights at small M, int8 weights whose rows are not multiples of 16
+ *   - the kernels of the quantized linears (int8 weights at any M, int8 weights whose rows are not multiples of 16
  *     bytes, 4-bit weights) are launched as programmatic dependents of the kernel in front of them in the stream, and let
  *     the kernel behind them start while they run if that is launched the same way.  All operands are read, and outputs
  *     and scratch touched, only after the stream dependency on the kernel in front is honoured, with one exception:
- *     the int8 kernel for small M requests `wq` and `scale` before it ([K, N] rows of 16-byte multiples, and
- *     [N, K]).  There they must be complete when the kernel in front may let its dependents start.  Ordinary kernels
- *     (b200q_symmetric_quantize, the packing kernels and every other kernel of this library but the three named above,
- *     memcpy / memset nodes, anything that does not itself execute griddepcontrol.launch_dependents) let dependents
- *     start only when they have finished, so producing a weight with b200q_symmetric_quantize and using it in the next
- *     call on the same stream is safe.  Not safe: writing `wq` or `scale` of an int8 weight from a kernel that triggers
- *     its dependents early when nothing but kernels of that kind lie between it and the quantized linear that reads
- *     them on the same stream (the three kernels named above are themselves of that kind); put an event or any
- *     ordinary kernel between the two.
+ *     the int8 kernel for small M requests the codes `wq` before it ([K, N] rows of 16-byte multiples, and [N, K]); the
+ *     scales it reads after it.  The codes must be complete when the kernel in front may let its dependents start.
+ *     Ordinary kernels (b200q_symmetric_quantize, the packing kernels and every other kernel of this library but the
+ *     quantized linears, memcpy / memset nodes, anything that does not itself execute
+ *     griddepcontrol.launch_dependents) let dependents start only when they have finished, so producing a weight with
+ *     b200q_symmetric_quantize and using it in the next call on the same stream is safe.  Not safe: writing the codes of
+ *     an int8 weight from a kernel that triggers its dependents early when nothing but kernels of that kind lie between
+ *     it and the quantized linear that reads them on the same stream (the quantized linears are themselves of that
+ *     kind: the f16 result of one of them may be the next one's scales, but its bytes may not be the next one's codes);
+ *     put an event or any ordinary kernel between the two.
  *   - matrices are dense row-major.  "KN" weight layout = [K, N] with N contiguous, the layout of
  *     the reference operator (python/hidet/graph/ops/quant/matmul.py:30-32); "NK" = [N, K] with K
  *     contiguous, the layout torch.nn.Linear stores.

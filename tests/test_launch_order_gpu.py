@@ -1,6 +1,6 @@
-"""Weights that the kernel in front writes, where the quantized linears promise to wait for its end: 4-bit weights and int8
-weights whose rows are not multiples of 16 bytes.  (The small-M int8 kernel asks for its weight earlier by contract, and is
-tested behind this library's own producers only.)"""
+"""Operands that the kernel in front writes, where the quantized linears promise to wait for its end: 4-bit weights, int8
+weights whose rows are not multiples of 16 bytes, and the scales of every weight.  (The small-M int8 kernel asks for the codes
+of its weight earlier by contract, and is tested behind this library's own producers only.)"""
 import ctypes
 
 import pytest
@@ -84,3 +84,30 @@ def test_weights_rewritten_by_this_library_between_calls(m):
         got8.append(hidet_b200.symmetric_quant_matmul(a, wq, scale8))
     for i in range(6):
         assert torch.equal(got4[i], want4[i % 2]) and torch.equal(got8[i], want8[i % 2])
+
+
+# in front: the small-M kernel, the mid-M one and the one on SM pairs, each with SMs to spare, so that the launch behind them starts early
+@pytest.mark.parametrize('rows,k,n', [(8, 4096, 1024), (100, 4096, 1024), (520, 4096, 3072)])
+@pytest.mark.parametrize('m', [1, 6, 16])
+@pytest.mark.parametrize('layout', ['KN', 'NK'])
+def test_scales_may_be_the_result_of_the_linear_in_front(rows, k, n, m, layout):
+    gen = torch.Generator(device='cuda').manual_seed(rows + m)
+    codes = torch.randint(-127, 128, (k, n), device='cuda', generator=gen, dtype=torch.int8)
+    ones = torch.full((n,), 1e-4, device='cuda').half()
+    fronts = [torch.randn(rows, k, device='cuda', generator=gen).half() for _ in range(2)]
+    a = torch.randn(m, 4096, device='cuda', generator=gen).half()
+    wq = torch.randint(-127, 128, (4096, n) if layout == 'KN' else (n, 4096), device='cuda', generator=gen, dtype=torch.int8)
+    buffer = torch.zeros(rows, n, dtype=torch.float16, device='cuda')
+
+    def both(x, between):
+        hidet_b200.symmetric_quant_matmul(x, codes, ones, out=buffer)
+        between()
+        return hidet_b200.symmetric_quant_matmul(a, wq, buffer[rows - 1], weight_layout=layout)
+
+    want = [both(x, torch.cuda.synchronize) for x in fronts]
+    torch.cuda.synchronize()
+    got = [both(fronts[i % 2], lambda: None) for i in range(12)]
+    assert not torch.equal(want[0], want[1])
+    for i, g in enumerate(got):
+        assert torch.equal(g, want[i % 2])
+    assert ffi.func('b200q_check_status')() == ffi.OK
