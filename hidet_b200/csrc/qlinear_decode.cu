@@ -144,7 +144,7 @@ __device__ __forceinline__ void finish(const OutTargets &o, const Epilogue &ep, 
 
 // Four adjacent halves, as one load / store where the address allows it.
 __device__ __forceinline__ void load4(const __half *p, float (&v)[4]) {
-    __half h[4];
+    __align__(8) __half h[4];
     if ((reinterpret_cast<uintptr_t>(p) & 7u) == 0) {
         *reinterpret_cast<uint2 *>(h) = __ldcg(reinterpret_cast<const uint2 *>(p));
     } else {
@@ -180,7 +180,7 @@ __device__ __forceinline__ void finish4(const OutTargets &o, const Epilogue &ep,
 #pragma unroll
         for (int j = 0; j < 4; ++j) y[j] += t[j];
     }
-    __half h[4];
+    __align__(8) __half h[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) h[j] = __float2half_rn(y[j]);
     const size_t off = (size_t)row * o.ldc + o.col0 + nn;

@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(256) qlinear_prefill_reduce_kernel(const float
     }
     if (ep.act == kActSiluMul) {
         // columns (2j, 2j + 1) = (gate, up): four results per thread, result column n / 2 + j
-        __half2 r2[2];
+        __align__(8) __half2 r2[2];
         float z[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(256) qlinear_prefill_reduce_kernel(const float
 #pragma unroll
         for (int c = 0; c < 8; ++c) y[c] += __half2float(rh[c]);
     }
-    __half2 h2[4];
+    __align__(16) __half2 h2[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) h2[c] = __floats2half2_rn(y[2 * c], y[2 * c + 1]);
     const uint4 val = *reinterpret_cast<const uint4 *>(h2);

@@ -25,7 +25,7 @@ def _close(got, want):
     assert float((got.double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
 
 
-@pytest.mark.parametrize('m', [1, 2, 3, 9, 16])
+@pytest.mark.parametrize('m', [1, 2, 3, 5, 6, 7, 8, 9, 16])
 @pytest.mark.parametrize('k,n', [(1024, 129), (2048, 258), (4096, 1027), (512, 4095)])
 def test_odd_column_counts(m, k, n):
     a, wq, scale, want = _operands(m, k, n, 'NK')
@@ -43,3 +43,26 @@ def test_destinations_at_any_element(m, ldc, col0):
                                              torch.cuda.current_stream().cuda_stream)
     _close(out[:, col0:col0 + 1280], want)
     assert bool((out[:, :col0] == -7.0).all()) and bool((out[:, col0 + 1280:] == -7.0).all())
+
+
+# scales, bias and residual at any element, rows of the residual and of the result of any length
+@pytest.mark.parametrize('m', [1, 4, 5, 8, 16])
+@pytest.mark.parametrize('offset,ldr', [(0, 1280), (1, 1283), (2, 1281), (3, 1286), (4, 1284)])
+@pytest.mark.parametrize('k', [256, 1536])   # one CTA a tile; K split
+def test_operands_of_the_epilogue_at_any_element(m, k, offset, ldr):
+    n = 1280
+    a, wq, scale, want = _operands(m, k, n, 'KN')
+
+    def at_offset(t):
+        out = torch.empty(offset + t.numel(), dtype=torch.float16, device='cuda')
+        out[offset:] = t.flatten()
+        return out, out.data_ptr() + 2 * offset
+
+    bias, residual = torch.randn(n, device='cuda').half(), torch.randn(m, ldr, device='cuda').half()
+    keep = [at_offset(t) for t in (scale, bias, residual)]
+    out = torch.empty(m, n, dtype=torch.float16, device='cuda')
+    ws_ptr, ws_size = workspaces.get(a.device, ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, 0))
+    ep = ffi.Epilogue(keep[1][1], keep[2][1], ldr, 0)
+    ffi.func('b200q_qlinear_f16_i8_fused')(a.data_ptr(), wq.data_ptr(), keep[0][1], out.data_ptr(), m, n, k, 0, ctypes.byref(ep), ws_ptr, ws_size,
+                                          torch.cuda.current_stream().cuda_stream)
+    _close(out, want + bias.double() + residual[:, :n].double())
