@@ -557,10 +557,9 @@ __global__ void __launch_bounds__(256) qlinear_prefill_reduce_kernel(const float
         y[0] += v0.x, y[1] += v0.y, y[2] += v0.z, y[3] += v0.w;
         y[4] += v1.x, y[5] += v1.y, y[6] += v1.z, y[7] += v1.w;
     }
-    const uint4 sraw = __ldg(reinterpret_cast<const uint4 *>(scale + n));
-    const __half *sh = reinterpret_cast<const __half *>(&sraw);
+    // the scales may start at any element
 #pragma unroll
-    for (int c = 0; c < 8; ++c) y[c] *= __half2float(sh[c]);
+    for (int c = 0; c < 8; ++c) y[c] *= __half2float(__ldg(scale + n + c));
     if (ep.bias != nullptr) {
         const uint4 braw = __ldg(reinterpret_cast<const uint4 *>(static_cast<const __half *>(ep.bias) + n));
         const __half *bh = reinterpret_cast<const __half *>(&braw);

@@ -61,6 +61,22 @@ def nvcc_library(tmp_path_factory):
 
 
 @pytest.fixture(scope='session')
+def large_kernels(nvcc_library):
+    """tests/cuda/large_kernels.cu with the sources of the kernels that it calls."""
+    import ctypes
+
+    from hidet_b200 import build
+
+    sources = [os.path.join(build.SRC_DIR, name + '.cu') for name in ('qlinear_pair', 'qlinear_mid', 'qlinear_prefill', 'qlinear_large', 'runtime')]
+    lib = nvcc_library('large_kernels.cu', '-std=c++17', '-Xcompiler', '-fvisibility=hidden', '--threads', '0', *sources)
+    p, i, n = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
+    lib.plan.argtypes, lib.plan.restype = [n, n, n, i, p], None
+    lib.launch.argtypes = [i, i, i, p, p, p, p, i, n, n, n, n, n, n, i, p, p, n, i, p]
+    lib.launch_one_sm.argtypes = [p, p, p, p, i, n, n, n, n, n, p, ctypes.c_size_t, p]
+    return lib
+
+
+@pytest.fixture(scope='session')
 def oracle_lib():
     import oracle
 
