@@ -99,6 +99,10 @@ struct LargePlan {
 };
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu);
 bool large_supported(const OutTargets &out, int64_t N, bool silu);
+// True where these kernels serve the call and are better at it than the small-M one; *rc is then the launch's status.  What the
+// small-M kernel refuses for want of scratch stays refused.
+bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
+               bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc);
 int launch_large(const LargePlan &plan, const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,
                  const Epilogue *epilogue, bool weight_nk, int64_t lda = 0);
 int launch_pair(const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,

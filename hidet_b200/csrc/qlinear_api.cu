@@ -52,22 +52,6 @@ int check_qlinear_args(const char *op, const void *a, const void *wq, const void
     return B200Q_OK;
 }
 
-// The kernels for more than a few rows, where they serve the call and are the better ones (`rc` is then the launch's
-// status).  What the small-M kernel refuses for want of a workspace stays refused.
-bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
-               bool weight_nk, int64_t lda, const void *workspace, size_t workspace_bytes, int *rc) {
-    const bool silu = epilogue != nullptr && epilogue->act == kActSiluMul;
-    if (M <= 16 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K)) || !large_supported(c, N, silu)) return false;
-    if (!use_prefill_kernel(M, N, K)) {
-        const DecodePlan dp = plan_decode(M, N, K);
-        if (dp.partial_bytes > 0 && (workspace == nullptr || workspace_bytes < dp.counter_bytes + dp.partial_bytes)) return false;
-    }
-    const LargePlan plan = plan_large(M, N, K, silu);
-    if (plan.kind == LargePlan::kNone) return false;
-    *rc = launch_large(plan, a, wq, scale, c, M, N, K, stream, epilogue, weight_nk, lda);
-    return true;
-}
-
 }  // namespace
 }  // namespace b200q
 
@@ -99,7 +83,7 @@ B200Q_API int b200q_qlinear_f16_i8(const void *a, const void *wq, const void *sc
         B200Q_CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(__half), s));
         return B200Q_OK;
     }
-    if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, w_layout == B200Q_LAYOUT_NK, 0, workspace, workspace_bytes, &rc)) return rc;
+    if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, w_layout == B200Q_LAYOUT_NK, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
     if (w_layout == B200Q_LAYOUT_KN && use_prefill_kernel(M, N, K) && prefill_kn_supported(a, wq, N, K)) {
         return launch_prefill_kn(a, wq, scale, c, M, N, K, s, nullptr, nullptr, false, 0, workspace, workspace_bytes);
     }
@@ -145,7 +129,7 @@ B200Q_API int b200q_qlinear_f16_i8_fused(const void *a, const void *wq, const vo
     ep.ldr = epilogue->ldr;
     ep.act = pairs ? kActSiluMul : kActNone;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (try_large(a, wq, scale, one_output(c, n_out), M, N, K, s, &ep, false, 0, workspace, workspace_bytes, &rc)) return rc;
+    if (try_large(a, wq, scale, one_output(c, n_out), M, N, K, s, &ep, false, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
     if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, c, M, N, K, s, nullptr, &ep, false, 0, workspace, workspace_bytes);
     return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, workspace, workspace_bytes, s, nullptr, &ep);
 }
@@ -173,7 +157,7 @@ B200Q_API int b200q_qlinear_f16_i8_to_peers(const void *a, const void *wq, const
     if (!decode_kn_supported(a, wq, N, K)) {
         return set_error(B200Q_UNSUPPORTED, "qlinear_f16_i8_to_peers: operands need 16-byte aligned bases and rows (N %% 16 == 0, K %% 8 == 0)");
     }
-    if (try_large(a, wq, scale, t, M, N, K, s, nullptr, false, 0, workspace, workspace_bytes, &rc)) return rc;
+    if (try_large(a, wq, scale, t, M, N, K, s, nullptr, false, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
     if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, dst[0], M, N, K, s, &t, nullptr, false, 0, workspace, workspace_bytes);
     return launch_decode_kn(a, wq, scale, dst[0], M, N, K, 0, K, true, workspace, workspace_bytes, s, &t);
 }
@@ -228,7 +212,7 @@ B200Q_API int b200q_qlinear_f16_i8_parts(const void *a, const void *wq, const vo
         const __half *a_part = static_cast<const __half *>(a) + k_begin;
         const int8_t *w_part = static_cast<const int8_t *>(wq) + (size_t)k_begin * N;
         if (fast && use_prefill_kernel(M, N, k_end - k_begin) && prefill_kn_supported(a_part, w_part, N, k_end - k_begin)) {
-            if (!try_large(a_part, w_part, scale, one_output(cp, N), M, N, k_end - k_begin, s, nullptr, false, K, nullptr, 0, &rc))
+            if (!try_large(a_part, w_part, scale, one_output(cp, N), M, N, k_end - k_begin, s, nullptr, false, K, 0, &rc))
                 rc = launch_prefill_kn(a_part, w_part, scale, cp, M, N, k_end - k_begin, s, nullptr, nullptr, false, K);
         } else {
             rc = fast ? launch_decode_kn(a, wq, scale, cp, M, N, K, k_begin, k_end, false, nullptr, 0, s)

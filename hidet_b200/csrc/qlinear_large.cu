@@ -82,6 +82,20 @@ bool large_supported(const OutTargets &out, int64_t N, bool silu) {
     return true;
 }
 
+bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
+               bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc) {
+    const bool silu = epilogue != nullptr && epilogue->act == kActSiluMul;
+    if (M <= 16 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K)) || !large_supported(c, N, silu)) return false;
+    if (!use_prefill_kernel(M, N, K)) {
+        const DecodePlan dp = plan_decode(M, N, K);
+        if (dp.partial_bytes > 0 && scratch_bytes < dp.counter_bytes + dp.partial_bytes) return false;
+    }
+    const LargePlan plan = plan_large(M, N, K, silu);
+    if (plan.kind == LargePlan::kNone) return false;
+    *rc = launch_large(plan, a, wq, scale, c, M, N, K, stream, epilogue, weight_nk, lda);
+    return true;
+}
+
 int launch_large(const LargePlan &plan, const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,
                  const Epilogue *epilogue, bool weight_nk, int64_t lda) {
     if (lda <= 0) lda = K;

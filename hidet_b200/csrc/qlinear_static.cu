@@ -73,11 +73,11 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
         return set_error(B200Q_UNSUPPORTED, "qlinear_f16_i8_static: operands need 16-byte aligned bases and rows (N %% 16 == 0, K %% 8 == 0); "
                                             "got N=%lld K=%lld", (long long)N, (long long)K);
     }
-    if (use_prefill_kernel(M, N, K)) {  // needs no scratch at all
-        const LargePlan large = plan_large(M, N, K, false);
-        if (large.kind != LargePlan::kNone && large_supported(one_output(c, N), N, false)) return launch_large(large, a, wq, scale, one_output(c, N), M, N, K, s, nullptr, false);
-        return launch_prefill_kn(a, wq, scale, c, M, N, K, s);
-    }
+    // The kernels for more rows need no scratch.  They take the calls that b200q_qlinear_f16_i8 gives them, so that both give the
+    // same bits.
+    int rc = B200Q_OK;
+    if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, false, 0, kStaticScratchBytes, &rc)) return rc;
+    if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, c, M, N, K, s);
 
     const DecodePlan plan = plan_decode(M, N, K);
     const size_t need = plan.counter_bytes + plan.partial_bytes;
@@ -89,7 +89,7 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
     }
     void *scratch = nullptr;
     if (need > 0) {
-        int rc = static_scratch(&scratch);
+        rc = static_scratch(&scratch);
         if (rc != B200Q_OK) return rc;
         // The arrival counters must read zero when the kernel starts.  A completed call leaves them
         // zero, but the array is shared by every caller and survives failed calls, so clear the ones

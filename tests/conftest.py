@@ -67,7 +67,7 @@ def large_kernels(nvcc_library):
 
     from hidet_b200 import build
 
-    sources = [os.path.join(build.SRC_DIR, name + '.cu') for name in ('qlinear_pair', 'qlinear_mid', 'qlinear_prefill', 'qlinear_large', 'runtime')]
+    sources = [os.path.join(build.SRC_DIR, name + '.cu') for name in ('qlinear_pair', 'qlinear_mid', 'qlinear_prefill', 'qlinear_large', 'qlinear_decode', 'runtime')]
     lib = nvcc_library('large_kernels.cu', '-std=c++17', '-Xcompiler', '-fvisibility=hidden', '--threads', '0', *sources)
     p, i, n = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
     lib.plan.argtypes, lib.plan.restype = [n, n, n, i, p], None

@@ -51,6 +51,16 @@ def test_static_entry_point_matches_the_regular_one_twice(m, n, k):
     assert ffi.func('b200q_check_status')() == ffi.OK
 
 
+@pytest.mark.parametrize('m,n,k', [(17, 4096, 4096), (32, 9408, 6208), (54, 1872, 10528), (64, 4096, 4096), (64, 12288, 4096), (300, 1024, 4096)])
+def test_static_entry_point_takes_the_regular_one_s_kernel_at_more_rows(m, n, k):
+    """Where the kernels for more rows take over from the small-M one the sums are grouped differently: the same on both sides."""
+    a, wq, scale = _problem(m, n, k, seed=m + n)
+    out = torch.full((m, n), float('nan'), dtype=torch.float16, device='cuda')
+    _static_call(a, wq, scale, out)
+    assert torch.equal(out, hidet_b200.symmetric_quant_matmul(a, wq, scale))
+    assert ffi.func('b200q_check_status')() == ffi.OK
+
+
 def test_static_entry_point_with_an_empty_sum_writes_zeros_like_the_regular_one():
     a = torch.zeros(3, 0, dtype=torch.float16, device='cuda')
     wq = torch.zeros(0, 64, dtype=torch.int8, device='cuda')
