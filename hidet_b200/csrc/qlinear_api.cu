@@ -61,15 +61,15 @@ B200Q_API size_t b200q_qlinear_workspace_bytes(int64_t M, int64_t N, int64_t K, 
     using namespace b200q;
     (void)w_layout;
     if (M <= 0 || N <= 0 || K <= 0) return 0;
+    // Of the kernels behind the entry points that take this workspace the small-M one alone uses it.  It may serve any M: operands
+    // that the kernels for more rows cannot take (alignment is not known here) go to it.
     const DecodePlan pl = plan_decode(M, N, K);
-    size_t need = pl.counter_bytes + pl.partial_bytes;
-    if (use_prefill_kernel(M, N, K)) {
-        // the tensor-memory kernel needs scratch only when it splits K; operands it cannot take (alignment is not
-        // known here) go to the small-M kernel, so its need is covered as well
-        const size_t split = plan_prefill_split(M, N, K).workspace_bytes;
-        if (split > need) need = split;
-    }
-    return need;
+    return pl.counter_bytes + pl.partial_bytes;
+}
+
+B200Q_API size_t b200q_qlinear_multicast_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+    using namespace b200q;
+    return M <= 0 || N <= 0 || K <= 0 ? 0 : plan_prefill_split(M, N, K).workspace_bytes;
 }
 
 B200Q_API int b200q_qlinear_f16_i8(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N,

@@ -193,10 +193,14 @@ class ColumnParallelQuantLinear:
         c0 = self.rank * n_local
         qlinear = ffi.func('b200q_qlinear_f16_i8_to_peers')
         with torch.cuda.device(x.device):
-            ws_bytes = ffi.func('b200q_qlinear_workspace_bytes')(rows, n_local, k, ffi.LAYOUT_KN)
-            ws_ptr, ws_size = workspaces.get(x.device, ws_bytes)
             main = torch.cuda.current_stream(x.device)
-            if multicast_ptr and self.multicast and rows >= self.MULTICAST_MIN_ROWS and self.world >= self.MULTICAST_MIN_WORLD:
+            multicast = multicast_ptr and self.multicast and rows >= self.MULTICAST_MIN_ROWS and self.world >= self.MULTICAST_MIN_WORLD
+            if multicast:
+                ws_bytes = ffi.func('b200q_qlinear_multicast_workspace_bytes')(rows, n_local, k)
+            else:
+                ws_bytes = ffi.func('b200q_qlinear_workspace_bytes')(rows, n_local, k, ffi.LAYOUT_KN)
+            ws_ptr, ws_size = workspaces.get(x.device, ws_bytes)
+            if multicast:
                 # large M: every 16 bytes leave this GPU once and the switch delivers them to all ranks
                 ffi.func('b200q_qlinear_f16_i8_to_multicast')(x.data_ptr(), self.wq.data_ptr(), self.scale.data_ptr(), multicast_ptr, n, c0,
                                                             rows, n_local, k, ws_ptr, ws_size, main.cuda_stream)

@@ -145,7 +145,7 @@ B200Q_API int b200q_u4_pack(const void *w, void *packed, int64_t rows, int64_t c
 B200Q_API int b200q_u4_unpack(const void *packed, void *w, int64_t rows, int64_t cols, void *stream);
 
 /*
- * Bytes of scratch b200q_qlinear_f16_i8 needs for this problem (0 is a valid answer).
+ * Bytes of scratch b200q_qlinear_f16_i8, _fused and _to_peers need for this problem (0 is a valid answer).
  * The scratch must be zero-filled once before its first use; every call leaves it zero-filled in
  * the part that has to be (its tile counters), so the same buffer can serve later calls of any
  * shape whose requirement it covers.  Two calls that may overlap on the GPU need two buffers.
@@ -164,7 +164,8 @@ B200Q_API size_t b200q_qlinear_workspace_bytes(int64_t M, int64_t N, int64_t K, 
  *
  *   wq    : int8, [K, N] if w_layout == B200Q_LAYOUT_KN, [N, K] if B200Q_LAYOUT_NK
  *   scale : f16 [N]
- * Picks the small-M streaming kernel or the large-M tensor-core kernel from M.
+ * Picks the kernel from the sizes: one that streams the weight for few rows, one on pairs of SMs for many, one
+ * that splits K over clusters in between and for narrow weights.
  */
 B200Q_API int b200q_qlinear_f16_i8(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N,
                                    int64_t K, int w_layout, void *workspace, size_t workspace_bytes, void *stream);
@@ -232,9 +233,13 @@ B200Q_API int b200q_qlinear_f16_i8_to_peers(const void *a, const void *wq, const
  * torch symmetric-memory handle), and the large-M kernel's epilogue stores every 16 bytes once with multimem.st;
  * the switch delivers them to every GPU, this one included.  The bytes that leave this GPU are 1 / (ranks - 1) of
  * what b200q_qlinear_f16_i8_to_peers sends.  M >= 33 and operands the large-M kernel accepts, else
- * B200Q_UNSUPPORTED (use b200q_qlinear_f16_i8_to_peers); workspace as for b200q_qlinear_f16_i8.  The caller orders the ranks
+ * B200Q_UNSUPPORTED (use b200q_qlinear_f16_i8_to_peers).  The caller orders the ranks
  * afterwards, as above.  No counterpart in the reference beyond the all-gather op named above.
+ * The workspace is optional: with the bytes that b200q_qlinear_multicast_workspace_bytes answers (0 for most shapes; their
+ * contents do not matter, and a workspace of b200q_qlinear_f16_i8 may serve, whose zero-filled part is left alone) narrow
+ * problems split K over several CTAs per tile; with less they are computed in one part, more slowly.
  */
+B200Q_API size_t b200q_qlinear_multicast_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B200Q_API int b200q_qlinear_f16_i8_to_multicast(const void *a, const void *wq, const void *scale, void *multicast_dst, int64_t ldc,
                                                 int64_t col_offset, int64_t M, int64_t N, int64_t K, void *workspace, size_t workspace_bytes,
                                                 void *stream);

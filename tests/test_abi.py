@@ -64,6 +64,14 @@ def test_narrow_deep_weights_fit_the_built_in_scratch(m, n, k, need):
     assert ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, ffi.LAYOUT_KN) == need <= ffi.func('b200q_qlinear_static_scratch_bytes')()
 
 
+def test_scratch_of_many_rows_is_asked_for_where_it_is_used():
+    ws, multicast = ffi.func('b200q_qlinear_workspace_bytes'), ffi.func('b200q_qlinear_multicast_workspace_bytes')
+    for m, n, k in ((256, 3584, 8192), (300, 1024, 4096), (65, 144, 2048), (2048, 4096, 11008)):
+        assert ws(m, n, k, ffi.LAYOUT_KN) == ws(m, n, k, ffi.LAYOUT_NK) == 0
+    assert multicast(256, 3584, 8192) > 65536 * 4 + 2 * 256 * 3584 * 4 - 1   # K is split there
+    assert multicast(2048, 28672, 8192) == multicast(0, 16, 16) == 0
+
+
 def test_four_bit_scratch_does_not_grow_where_none_is_used():
     ws = ffi.func('b200q_qlinear_f16_u4_workspace_bytes')
     for group in (16, 64, 128, 256):
