@@ -68,10 +68,14 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
 // The same kernel on a weight stored [N, K] (weight_nk = true): needs 16-byte aligned bases and K % 16 == 0.
 bool decode_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
 
-// The one-SM tensor-memory kernel for large M, which serves the multicast delivery and says what it cannot take: same operand
-// requirements as the small-M kernel.
+// The operands that all kernels for more than a few rows take: as the small-M kernel, and for a weight stored [N, K] N % 8 == 0 too.
 bool prefill_kn_supported(const void *a, const void *wq, int64_t N, int64_t K);
-// How the tensor-memory kernel splits K (narrow problems only) and the scratch that takes: fp32 partial sums
+bool prefill_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
+// Their outputs are written with 16-byte stores: B200Q_INVALID_ARGUMENT where those cannot write them.
+int check_large_outputs(const OutTargets &out);
+
+// The one-SM tensor-memory kernel for large M ([K, N] weights), which serves the multicast delivery.
+// How it splits K (narrow problems only) and the scratch that takes: fp32 partial sums
 // [k_splits][M][N] behind an untouched head of kSplitWorkspaceHead bytes (the small-M kernel's counters live there).
 constexpr size_t kSplitWorkspaceHead = (size_t)65536 * 4;
 struct PrefillSplit {
@@ -80,17 +84,13 @@ struct PrefillSplit {
     size_t workspace_bytes = 0;
 };
 PrefillSplit plan_prefill_split(int64_t M, int64_t N, int64_t K);
-// lda: elements between rows of `a` when they are longer than K (a k range of wider activations); 0 = K.
 // workspace: where K may be split (see plan_prefill_split); without it the kernel runs one CTA per output tile.
-int launch_prefill_kn(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K,
-                      cudaStream_t stream, const OutTargets *targets = nullptr, const Epilogue *epilogue = nullptr, bool weight_nk = false,
-                      int64_t lda = 0, void *workspace = nullptr, size_t workspace_bytes = 0);
-// The same kernel on a weight stored [N, K] (weight_nk = true): 16-byte aligned bases, K % 16 == 0, N % 8 == 0.
-bool prefill_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
+int launch_prefill_kn(const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream, void *workspace,
+                      size_t workspace_bytes);
 
 // More than a few rows: the kernel on pairs of SMs (tm, a multiple of 32 up to 256, rows per tile) and the mid-M
 // kernel (tm, a multiple of 16 up to 128, rows per tile; K split over a cluster).  Operands as for the kernel above;
-// outputs that 16-byte stores can write, at any number of addresses but not a multicast one; no workspace.
+// outputs at any number of addresses but not a multicast one; no workspace.
 struct LargePlan {
     enum Kind { kNone, kMid, kPair };  // kNone: the small-M kernel is the better one
     Kind kind = kNone;
@@ -98,9 +98,8 @@ struct LargePlan {
     int cluster = 1;
 };
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu);
-bool large_supported(const OutTargets &out, int64_t N, bool silu);
-// True where these kernels serve the call and are better at it than the small-M one; *rc is then the launch's status.  What the
-// small-M kernel refuses for want of scratch stays refused.
+// True where these kernels serve the call and are better at it than the small-M one, or alone would serve it but for its
+// outputs; *rc is then the launch's status or the refusal.  What the small-M kernel refuses for want of scratch stays refused.
 bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
                bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc);
 int launch_large(const LargePlan &plan, const void *a, const void *wq, const void *scale, const OutTargets &out, int64_t M, int64_t N, int64_t K, cudaStream_t stream,

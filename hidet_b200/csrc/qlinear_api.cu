@@ -84,12 +84,6 @@ B200Q_API int b200q_qlinear_f16_i8(const void *a, const void *wq, const void *sc
         return B200Q_OK;
     }
     if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, w_layout == B200Q_LAYOUT_NK, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
-    if (w_layout == B200Q_LAYOUT_KN && use_prefill_kernel(M, N, K) && prefill_kn_supported(a, wq, N, K)) {
-        return launch_prefill_kn(a, wq, scale, c, M, N, K, s, nullptr, nullptr, false, 0, workspace, workspace_bytes);
-    }
-    if (w_layout == B200Q_LAYOUT_NK && use_prefill_kernel(M, N, K) && prefill_nk_supported(a, wq, N, K)) {
-        return launch_prefill_kn(a, wq, scale, c, M, N, K, s, nullptr, nullptr, true, 0, workspace, workspace_bytes);
-    }
     if (w_layout == B200Q_LAYOUT_KN && decode_kn_supported(a, wq, N, K)) {
         return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, workspace, workspace_bytes, s);
     }
@@ -130,7 +124,6 @@ B200Q_API int b200q_qlinear_f16_i8_fused(const void *a, const void *wq, const vo
     ep.act = pairs ? kActSiluMul : kActNone;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (try_large(a, wq, scale, one_output(c, n_out), M, N, K, s, &ep, false, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
-    if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, c, M, N, K, s, nullptr, &ep, false, 0, workspace, workspace_bytes);
     return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, workspace, workspace_bytes, s, nullptr, &ep);
 }
 
@@ -158,7 +151,6 @@ B200Q_API int b200q_qlinear_f16_i8_to_peers(const void *a, const void *wq, const
         return set_error(B200Q_UNSUPPORTED, "qlinear_f16_i8_to_peers: operands need 16-byte aligned bases and rows (N %% 16 == 0, K %% 8 == 0)");
     }
     if (try_large(a, wq, scale, t, M, N, K, s, nullptr, false, 0, workspace == nullptr ? 0 : workspace_bytes, &rc)) return rc;
-    if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, dst[0], M, N, K, s, &t, nullptr, false, 0, workspace, workspace_bytes);
     return launch_decode_kn(a, wq, scale, dst[0], M, N, K, 0, K, true, workspace, workspace_bytes, s, &t);
 }
 
@@ -183,7 +175,7 @@ B200Q_API int b200q_qlinear_f16_i8_to_multicast(const void *a, const void *wq, c
     t.ldc = ldc;
     t.col0 = col_offset;
     t.multicast = 1;
-    return launch_prefill_kn(a, wq, scale, multicast_dst, M, N, K, static_cast<cudaStream_t>(stream), &t, nullptr, false, 0, workspace, workspace_bytes);
+    return launch_prefill_kn(a, wq, scale, t, M, N, K, static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
 }
 
 B200Q_API int b200q_qlinear_f16_i8_parts(const void *a, const void *wq, const void *scale, void *c, int64_t M,
@@ -211,10 +203,7 @@ B200Q_API int b200q_qlinear_f16_i8_parts(const void *a, const void *wq, const vo
         // of rows that stay K long, weight rows k_begin ..); small M: the streaming kernel on the range.
         const __half *a_part = static_cast<const __half *>(a) + k_begin;
         const int8_t *w_part = static_cast<const int8_t *>(wq) + (size_t)k_begin * N;
-        if (fast && use_prefill_kernel(M, N, k_end - k_begin) && prefill_kn_supported(a_part, w_part, N, k_end - k_begin)) {
-            if (!try_large(a_part, w_part, scale, one_output(cp, N), M, N, k_end - k_begin, s, nullptr, false, K, 0, &rc))
-                rc = launch_prefill_kn(a_part, w_part, scale, cp, M, N, k_end - k_begin, s, nullptr, nullptr, false, K);
-        } else {
+        if (!(fast && use_prefill_kernel(M, N, k_end - k_begin) && try_large(a_part, w_part, scale, one_output(cp, N), M, N, k_end - k_begin, s, nullptr, false, K, 0, &rc))) {
             rc = fast ? launch_decode_kn(a, wq, scale, cp, M, N, K, k_begin, k_end, false, nullptr, 0, s)
                       : launch_generic(a, wq, scale, cp, M, N, K, k_begin, k_end, B200Q_LAYOUT_KN, s);
         }

@@ -75,23 +75,25 @@ LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu) {
     return p;
 }
 
-bool large_supported(const OutTargets &out, int64_t N, bool silu) {
-    if (out.multicast || out.ldc % 8 != 0 || out.col0 % 8 != 0 || N % (silu ? 16 : 8) != 0) return false;
+int check_large_outputs(const OutTargets &out) {
     for (int d = 0; d < out.count; ++d)
-        if ((reinterpret_cast<uintptr_t>(out.ptr[d]) & 15u) != 0) return false;
-    return true;
+        if ((reinterpret_cast<uintptr_t>(out.ptr[d]) & 15u) != 0) return set_error(B200Q_INVALID_ARGUMENT, "qlinear: output %d is not 16-byte aligned", d);
+    if (out.ldc % 8 != 0 || out.col0 % 8 != 0) return set_error(B200Q_INVALID_ARGUMENT, "qlinear: output row length and column offset must be multiples of 8 elements");
+    return B200Q_OK;
 }
 
 bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
                bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc) {
-    const bool silu = epilogue != nullptr && epilogue->act == kActSiluMul;
-    if (M <= 16 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K)) || !large_supported(c, N, silu)) return false;
-    if (!use_prefill_kernel(M, N, K)) {
+    if (M <= 16 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
+    const bool only = use_prefill_kernel(M, N, K);  // the small-M kernel is out of the question
+    if (!only) {
         const DecodePlan dp = plan_decode(M, N, K);
         if (dp.partial_bytes > 0 && scratch_bytes < dp.counter_bytes + dp.partial_bytes) return false;
     }
-    const LargePlan plan = plan_large(M, N, K, silu);
+    const LargePlan plan = plan_large(M, N, K, epilogue != nullptr && epilogue->act == kActSiluMul);
     if (plan.kind == LargePlan::kNone) return false;
+    *rc = check_large_outputs(c);
+    if (*rc != B200Q_OK) return only;  // the small-M kernel stores at any element
     *rc = launch_large(plan, a, wq, scale, c, M, N, K, stream, epilogue, weight_nk, lda);
     return true;
 }

@@ -77,7 +77,6 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
     // same bits.
     int rc = B200Q_OK;
     if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, false, 0, kStaticScratchBytes, &rc)) return rc;
-    if (use_prefill_kernel(M, N, K)) return launch_prefill_kn(a, wq, scale, c, M, N, K, s);
 
     const DecodePlan plan = plan_decode(M, N, K);
     const size_t need = plan.counter_bytes + plan.partial_bytes;

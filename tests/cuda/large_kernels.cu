@@ -40,8 +40,7 @@ EXPORT int launch(int kind, int tm, int cluster, const void *a, const void *wq, 
 // Returns how many parts K was split into, or the negative status.
 EXPORT int launch_one_sm(const void *a, const void *wq, const void *scale, void *const *dst, int count, int64_t ldc, int64_t col0, int64_t M, int64_t N, int64_t K,
                          void *workspace, size_t workspace_bytes, cudaStream_t stream) {
-    const OutTargets t = targets(dst, count, ldc, col0);
-    const int rc = launch_prefill_kn(a, wq, scale, dst[0], M, N, K, stream, &t, nullptr, false, 0, workspace, workspace_bytes);
+    const int rc = launch_prefill_kn(a, wq, scale, targets(dst, count, ldc, col0), M, N, K, stream, workspace, workspace_bytes);
     if (rc != B200Q_OK) return -rc;
     const PrefillSplit split = plan_prefill_split(M, N, K);
     return split.workspace_bytes <= workspace_bytes ? split.k_splits : 1;

@@ -70,3 +70,31 @@ def test_both_kernels_repeat_their_bits():
         first = hidet_b200.symmetric_quant_matmul(a, wq, scale)
         for _ in range(20):
             assert torch.equal(hidet_b200.symmetric_quant_matmul(a, wq, scale), first)
+
+
+@pytest.mark.parametrize('ldc,col0,base', [(1284, 0, 0), (1288, 4, 0), (1288, 0, 1)])
+def test_outputs_that_16_byte_stores_cannot_write(ldc, col0, base):
+    """Refused where only the kernels for many rows serve the call; where the small-M kernel does too, it stores at any element."""
+    import ctypes
+
+    from hidet_b200.runtime import workspaces
+
+    k, n = 512, 1280
+    wq, scale = torch.randint(-128, 128, (k, n), device='cuda', dtype=torch.int8), torch.full((n,), 1e-3, device='cuda').half()
+    f, stream = ffi.func('b200q_qlinear_f16_i8_to_peers'), torch.cuda.current_stream().cuda_stream
+    for m in (20, 64, 65, 300):
+        a = torch.randn(m, k, device='cuda').half()
+        out = torch.full((m * ldc + 8,), -7.0, dtype=torch.float16, device='cuda')
+        table = (ctypes.c_void_p * 1)(out.data_ptr() + 2 * base)
+        ws_ptr, ws_size = workspaces.get(a.device, ffi.func('b200q_qlinear_workspace_bytes')(m, n, k, 0))
+        args = (a.data_ptr(), wq.data_ptr(), scale.data_ptr(), table, 1, ldc, col0, m, n, k, ws_ptr, ws_size, stream)
+        if m > 64:
+            with pytest.raises(ffi.BackendException, match='not 16-byte aligned' if base else 'multiples of 8 elements') as e:
+                f(*args)
+            assert e.value.status == ffi.INVALID_ARGUMENT and bool((out == -7.0).all())
+        else:
+            f(*args)
+            rows = out[base:base + m * ldc].view(m, ldc)
+            want = (a.double() @ wq.double()) * scale.double()
+            assert float((rows[:, col0:col0 + n].double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
+            assert bool((rows[:, :col0] == -7.0).all()) and bool((rows[:, col0 + n:] == -7.0).all())
