@@ -43,7 +43,7 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
     static const struct {
         int tm;
         double stage;
-    } forms[] = {{32, 0.262}, {64, 0.262}, {96, 0.262}, {128, 0.265}, {160, 0.28}, {192, 0.315}, {224, 0.32}, {256, 0.335}};
+    } forms[] = {{64, 0.262}, {96, 0.262}, {128, 0.265}, {160, 0.28}, {192, 0.315}, {224, 0.32}, {256, 0.335}};
     int sms = sm_count();
     if (sms <= 0) sms = 148;
     double best = 1e30;

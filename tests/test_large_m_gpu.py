@@ -1,4 +1,7 @@
-"""The kernels for more than a few rows (SM pairs, mid M) at the edges of their tiles, rings and splits."""
+"""The kernels for more than a few rows (SM pairs, mid M) at the edges of their tiles, rings and splits: first through the public
+entry points, where the sizes decide which kernel runs, then each kernel by name with every tile height and split."""
+import ctypes
+
 import pytest
 import torch
 
@@ -6,6 +9,15 @@ import hidet_b200
 from hidet_b200 import ffi
 
 pytestmark = pytest.mark.gpu
+
+
+MID, PAIR = 1, 2
+
+
+def _plan(large_kernels, m, k, n, silu=False):
+    out = (ctypes.c_int * 3)()
+    large_kernels.plan(m, n, k, silu, out)
+    return out[0]
 
 
 def _run(m, k, n, layout, bias=False, silu=False, residual=False):
@@ -33,24 +45,28 @@ def _run(m, k, n, layout, bias=False, silu=False, residual=False):
     assert float((got.double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
 
 
-# the kernel on SM pairs, and the mid-M one where columns are few: the heights of tiles, their last rows and columns, k that ends inside a
-# stage, one stage, fewer stages than ring slots and more, one tile and several per pair
-@pytest.mark.parametrize('m,k,n', [(513, 64, 16), (600, 8, 256), (513, 72, 272), (777, 1000, 528), (1025, 520, 2064), (1500, 2048, 1040), (2048, 1032, 16), (3001, 456, 4112)])
-def test_pair_kernel_edges(m, k, n):
+# k that ends inside a stage, one stage, fewer stages than ring slots and more, one tile and several per pair of SMs or cluster, the last
+# rows and columns
+@pytest.mark.parametrize('kind,m,k,n', [(MID, 513, 64, 16), (MID, 600, 8, 256), (MID, 513, 72, 272), (MID, 777, 1000, 528), (PAIR, 1025, 520, 2064), (PAIR, 1500, 2048, 1040),
+                                        (MID, 2048, 1032, 16), (PAIR, 3001, 456, 4112), (PAIR, 1000, 4096, 4096)])
+def test_many_rows(large_kernels, kind, m, k, n):
+    assert _plan(large_kernels, m, k, n) == kind
     _run(m, k, n, 'KN')
     if k % 16 == 0:
         _run(m, k, n - 8 if n > 16 else n, 'NK')
 
 
 @pytest.mark.parametrize('epilogue', [dict(bias=True), dict(residual=True), dict(bias=True, residual=True), dict(silu=True), dict(silu=True, bias=True, residual=True)])
-@pytest.mark.parametrize('m,k,n', [(520, 328, 272), (1100, 136, 4112)])
-def test_pair_kernel_epilogues(m, k, n, epilogue):
+@pytest.mark.parametrize('kind,m,k,n', [(MID, 520, 328, 272), (PAIR, 1100, 136, 4112), (PAIR, 1000, 4096, 4096)])
+def test_many_rows_with_an_epilogue(large_kernels, kind, m, k, n, epilogue):
+    assert _plan(large_kernels, m, k, n, 'silu' in epilogue) == kind
     _run(m, k, n, 'KN', **epilogue)
 
 
-# K in one part and in eight, parts of unequal length, tiles of 16 to 128 rows, two row tiles, the last rows and columns
-@pytest.mark.parametrize('m,k,n', [(65, 64, 16), (66, 128, 272), (80, 464, 272), (100, 1872, 336), (33, 2736, 10800), (129, 1032, 144), (144, 4096, 528), (24, 4096, 12288), (200, 8200, 1040), (598, 6256, 352)])
-def test_mid_kernel_edges(m, k, n):
+# K in one part and in eight, parts of unequal length, tiles of 48 to 128 rows, two row tiles, the last rows and columns
+@pytest.mark.parametrize('m,k,n', [(65, 64, 16), (66, 128, 272), (80, 464, 272), (100, 1872, 336), (33, 2736, 10800), (129, 1032, 144), (144, 4096, 528), (200, 8200, 1040), (598, 6256, 352)])
+def test_a_few_hundred_rows(large_kernels, m, k, n):
+    assert _plan(large_kernels, m, k, n) == MID
     _run(m, k, n, 'KN')
     if k % 16 == 0:
         _run(m, k, n - 8 if n > 16 else n, 'NK')
@@ -58,25 +74,115 @@ def test_mid_kernel_edges(m, k, n):
 
 @pytest.mark.parametrize('epilogue', [dict(bias=True), dict(residual=True), dict(silu=True), dict(silu=True, bias=True, residual=True)])
 @pytest.mark.parametrize('m,k,n', [(70, 776, 272), (120, 200, 1296)])
-def test_mid_kernel_epilogues(m, k, n, epilogue):
+def test_a_few_hundred_rows_with_an_epilogue(large_kernels, m, k, n, epilogue):
+    assert _plan(large_kernels, m, k, n, 'silu' in epilogue) == MID
     _run(m, k, n, 'KN', **epilogue)
 
 
-def test_both_kernels_repeat_their_bits():
-    for m, k, n in ((100, 3000, 336), (700, 1000, 528)):
-        a = torch.randn(m, k, device='cuda').half()
-        wq = torch.randint(-128, 128, (k, n), device='cuda', dtype=torch.int8)
-        scale = torch.full((n,), 1e-3, device='cuda').half()
-        first = hidet_b200.symmetric_quant_matmul(a, wq, scale)
-        for _ in range(20):
-            assert torch.equal(hidet_b200.symmetric_quant_matmul(a, wq, scale), first)
+def _by_name(lib, kind, tm, cluster, m, k, n, layout='KN', bias=False, silu=False, residual=None, copies=1, lda=0, repeat=1):
+    """One call of a kernel with its tiles and split given.  residual: what the length of its rows exceeds the result's by, None without.
+    copies > 1: as many destinations, each a column range of wider rows.  lda: the activations are a k range of rows that long."""
+    g = torch.Generator(device='cuda').manual_seed(m * 7 + k + n + tm)
+    wide = torch.randn(m, lda or k, generator=g, device='cuda').half()
+    a = wide[:, 8:8 + k] if lda else wide
+    wq = torch.randint(-128, 128, (k, n) if layout == 'KN' else (n, k), generator=g, device='cuda', dtype=torch.int8)
+    scale = (torch.rand(n, generator=g, device='cuda') * 1e-3 + 1e-4).half()
+    width = n // 2 if silu else n
+    ldc, col0 = (width, 0) if copies == 1 else (width + 40, 24)
+    want = (a.double() @ (wq if layout == 'KN' else wq.t()).double()) * scale.double()
+    b = torch.randn(n, generator=g, device='cuda').half() if bias else None
+    r = torch.randn(m, width + residual, generator=g, device='cuda').half() if residual is not None else None
+    if bias:
+        want += b.double()
+    if silu:
+        want = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+    if r is not None:
+        want += r[:, :width].double()
+    first = None
+    for _ in range(repeat):
+        outs = [torch.full((m, ldc), -7.0, dtype=torch.float16, device='cuda') for _ in range(copies)]
+        table = (ctypes.c_void_p * copies)(*[o.data_ptr() for o in outs])
+        assert lib.launch(kind, tm, cluster, a.data_ptr(), wq.data_ptr(), scale.data_ptr(), table, copies, ldc, col0, m, n, k, lda or k, layout == 'NK',
+                          b.data_ptr() if bias else None, r.data_ptr() if r is not None else None, width + (residual or 0), silu,
+                          torch.cuda.current_stream().cuda_stream) == 0
+        if first is None:
+            first = outs[0]
+            for o in outs:
+                # as above; with SiLU the exponential's error, a few units in the last place of f32, is far below that too
+                assert float((o[:, col0:col0 + width].double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
+                assert bool((o[:, :col0] == -7.0).all()) and bool((o[:, col0 + width:] == -7.0).all())
+        assert torch.equal(outs[0], first)
+    assert lib.b200q_check_status() == 0
+
+
+PAIR_HEIGHTS = [64, 96, 128, 160, 192, 224, 256]   # two accumulators up to 192 rows, one above
+
+
+@pytest.mark.parametrize('layout', ['KN', 'NK'])
+@pytest.mark.parametrize('tm', PAIR_HEIGHTS)
+def test_pair_kernel(large_kernels, tm, layout):
+    odd = 8 if layout == 'KN' else 16
+    # k shorter than a stage, one stage, more stages than any ring holds; a tile of one row, of a whole one and one row, of half of its 32-row
+    # blocks; columns of half a CTA's tile, one CTA's of the pair; more tiles than pairs of SMs
+    for m, k, n in ((1, odd, 16), (tm + 1, 64, 144), (2 * tm + 33, 1024 + odd, 272), (3 * tm - tm // 2, 192 + odd, 528), (5 * tm + 7, 128 + odd, 4112)):
+        _by_name(large_kernels, PAIR, tm, 1, m, k, n if layout == 'KN' else n - 8, layout)
+
+
+@pytest.mark.parametrize('epilogue', [dict(bias=True), dict(residual=0), dict(residual=3), dict(bias=True, residual=8), dict(silu=True), dict(silu=True, bias=True, residual=0),
+                                      dict(silu=True, residual=5)])
+@pytest.mark.parametrize('tm', PAIR_HEIGHTS)
+def test_pair_kernel_epilogues(large_kernels, tm, epilogue):
+    for m, k, n in ((2 * tm + 33, 328, 272), (5 * tm + 7, 136, 4112)):
+        _by_name(large_kernels, PAIR, tm, 1, m, k, n, **epilogue)
+
+
+@pytest.mark.parametrize('tm', [128, 192, 224, 256])
+def test_pair_kernel_destinations_bands_and_bits(large_kernels, tm):
+    _by_name(large_kernels, PAIR, tm, 1, 2 * tm + 33, 520, 1040, copies=3, repeat=3)
+    _by_name(large_kernels, PAIR, tm, 1, 2 * tm + 33, 520, 1040, lda=1048)
+    _by_name(large_kernels, PAIR, tm, 1, 5 * tm + 40, 1000, 4112, repeat=10)
+    # more rows than a band of 48 MB of activations holds, and a last band that is not a whole one
+    k = 8192
+    band = (48 << 20) // (tm * k * 2)
+    _by_name(large_kernels, PAIR, tm, 1, (band + 2) * tm - 9, k, 784, repeat=2)
+
+
+@pytest.mark.parametrize('layout', ['KN', 'NK'])
+@pytest.mark.parametrize('cluster', range(1, 9))
+@pytest.mark.parametrize('tm', [16, 48, 64, 80, 112, 128])
+def test_mid_kernel(large_kernels, tm, cluster, layout):
+    odd = 8 if layout == 'KN' else 16
+    # as many stages as CTAs, shares that differ by one, shares beyond every ring; CTAs that own no part of the result; two row tiles
+    for m, k, n in ((tm, 64 * cluster, 16), (tm - 5, 64 * (2 * cluster + 1) - odd, 272), (tm + 1, 64 * 9 * cluster + odd, 144)):
+        _by_name(large_kernels, MID, tm, cluster, m, k, n if layout == 'KN' else n - 8, layout)
+
+
+@pytest.mark.parametrize('epilogue', [dict(bias=True), dict(residual=0), dict(residual=3), dict(silu=True), dict(silu=True, bias=True, residual=5)])
+@pytest.mark.parametrize('tm,cluster', [(32, 1), (64, 3), (96, 8), (128, 5)])
+def test_mid_kernel_epilogues(large_kernels, tm, cluster, epilogue):
+    _by_name(large_kernels, MID, tm, cluster, 2 * tm - 3, 1096, 336, **epilogue)
+
+
+@pytest.mark.parametrize('tm,cluster', [(64, 8), (112, 4), (128, 1)])
+def test_mid_kernel_destinations_and_bits(large_kernels, tm, cluster):
+    _by_name(large_kernels, MID, tm, cluster, 3 * tm - 3, 1096, 336, copies=3, repeat=10)
+    _by_name(large_kernels, MID, tm, cluster, tm, 1096, 336, lda=1200)
+
+
+@pytest.mark.parametrize('kind,m,k,n', [(MID, 100, 3000, 336), (MID, 700, 1000, 528), (PAIR, 1000, 4096, 4096)])
+def test_results_repeat_their_bits(large_kernels, kind, m, k, n):
+    assert _plan(large_kernels, m, k, n) == kind
+    a = torch.randn(m, k, device='cuda').half()
+    wq = torch.randint(-128, 128, (k, n), device='cuda', dtype=torch.int8)
+    scale = torch.full((n,), 1e-3, device='cuda').half()
+    first = hidet_b200.symmetric_quant_matmul(a, wq, scale)
+    for _ in range(20):
+        assert torch.equal(hidet_b200.symmetric_quant_matmul(a, wq, scale), first)
 
 
 @pytest.mark.parametrize('ldc,col0,base', [(1284, 0, 0), (1288, 4, 0), (1288, 0, 1)])
 def test_outputs_that_16_byte_stores_cannot_write(ldc, col0, base):
     """Refused where only the kernels for many rows serve the call; where the small-M kernel does too, it stores at any element."""
-    import ctypes
-
     from hidet_b200.runtime import workspaces
 
     k, n = 512, 1280
