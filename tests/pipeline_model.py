@@ -411,6 +411,14 @@ def pair_config_from_source(tm: int) -> TensorMemoryConfig:
                               group_warps=k['GROUP_WARPS'], epi_groups=k['EPI_GROUPS'], epilogue_agrees=_epilogue_agrees(text))
 
 
+def mid_config_from_source(tm: int) -> TensorMemoryConfig:
+    """As launch_mid sets the kernel up for tiles of `tm` rows."""
+    k = _constants(open(os.path.join(KERNELS, 'qlinear_mid.cu')).read())
+    act_slots = (k['CTA_SMEM'] - 1024 - k['RAW_SLOTS'] * k['RAW_BYTES']) // (tm * k['BK'] * 2)
+    return TensorMemoryConfig(ctas=1, raw_slots=k['RAW_SLOTS'], act_slots=min(act_slots, k['MAX_SLOTS']), w_slots=k['W_SLOTS'], n_acc=1, conv_groups=k['CONV_GROUPS'],
+                              group_warps=k['GROUP_WARPS'], epi_groups=0)
+
+
 class TensorMemoryPipeline(Scheduler):
     def __init__(self, cfg: TensorMemoryConfig, tiles: int, k_blocks: int, rng: random.Random):
         super().__init__(rng, cfg.ctas)
@@ -450,6 +458,8 @@ class TensorMemoryPipeline(Scheduler):
             yield from role
         except Aborted:
             pass
+        if self.cfg.epi_groups == 0:
+            yield ('drain', lambda: self.acc_full[0][0].phases_done > 0)   # all MMAs issued have completed
         yield self.exit.come()[1]
 
     def producer(self, cta: int, what: str):
@@ -506,7 +516,7 @@ class TensorMemoryPipeline(Scheduler):
             pass
         if self.cfg.epi_groups == 0:
             self.commits.append(self.acc_full[0][0].arrive)
-        if self.cfg.drain_on_exit:
+        elif self.cfg.drain_on_exit:
             yield ('drain', lambda: not self.commits)
 
     def _mma_loop(self):

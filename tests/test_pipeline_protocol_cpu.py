@@ -4,7 +4,7 @@ import random
 
 import pytest
 
-from pipeline_model import Pipeline, ProtocolError, TensorMemoryPipeline, config_from_source, pair_config_from_source
+from pipeline_model import Pipeline, ProtocolError, TensorMemoryPipeline, config_from_source, mid_config_from_source, pair_config_from_source
 
 
 @pytest.mark.parametrize('tm', [256, 64])
@@ -129,3 +129,42 @@ def test_a_wait_of_the_pair_kernel_that_runs_out_ends_every_role_of_both_ctas(tm
                 pipe.run(copy_delay=0.9)
                 runs += 1 if any(pipe.abort) else 0
     assert runs > 100
+
+
+@pytest.mark.parametrize('tm', [16, 64, 80, 112, 128])
+@pytest.mark.parametrize('k_blocks', [1, 2, 5, 13, 40])
+def test_mid_protocol_holds_under_random_schedules(tm, k_blocks):
+    cfg = mid_config_from_source(tm)
+    assert cfg.raw_slots % cfg.conv_groups == cfg.w_slots % cfg.conv_groups == 0 and cfg.act_slots >= 3
+    for seed in range(10):
+        for delay in (0.2, 0.9, 0.99):
+            TensorMemoryPipeline(cfg, 1, k_blocks, random.Random(seed)).run(copy_delay=delay)
+
+
+def test_a_wait_of_the_mid_kernel_that_runs_out_ends_every_role():
+    cfg = mid_config_from_source(128)
+    runs = 0
+    for seed in range(8):
+        for agent in range(1 + 2 + 8):
+            for nth in (1, 3, 17):
+                pipe = TensorMemoryPipeline(cfg, 1, 15, random.Random(seed))
+                pipe.expire = (agent, nth)
+                pipe.run(copy_delay=0.9)
+                runs += 1 if any(pipe.abort) else 0
+    assert runs > 100
+
+
+@pytest.mark.parametrize('cfg,expire', [(dataclasses.replace(pair_config_from_source(256), raw_slots=5), None),
+                                        (dataclasses.replace(mid_config_from_source(128), drain_on_exit=False), (0, 2))])
+def test_model_catches_a_ring_whose_slots_change_groups_and_a_teardown_without_the_drain(cfg, expire):
+    """An odd ring of int8 tiles takes a slot from one converter group to the other, which skips phases of its barrier; a teardown that does
+    not wait leaves copies in flight when the last role is gone (the MMA thread gives up early)."""
+    found = 0
+    for seed in range(40):
+        pipe = TensorMemoryPipeline(cfg, 1 if cfg.ctas == 1 else 3, 16, random.Random(seed))
+        pipe.expire = expire
+        try:
+            pipe.run(copy_delay=0.95)
+        except ProtocolError:
+            found += 1
+    assert found > 0
