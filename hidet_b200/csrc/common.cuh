@@ -73,12 +73,6 @@ inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-__device__ __forceinline__ uint32_t lane_id() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%laneid;" : "=r"(r));
-    return r;
-}
-
 // One lane of the (fully converged) warp.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
@@ -222,19 +216,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// ---- int8 -> f16 ----
-// Four signed bytes packed in `v` -> (b0, b2) in lo and (b1, b3) in hi as exact f16 values.
-// 0x6400 | u is the f16 number 1024 + u for u in [0, 256); with u = b ^ 0x80 = b + 128 the
-// subtraction of 1152 leaves b exactly.
-__device__ __forceinline__ void cvt_s8x4_to_f16x4(uint32_t v, uint32_t &lo, uint32_t &hi) {
-    const uint32_t magic = 0x64806480u;           // per half: 0x6400 | 0x80 folds the sign flip in
-    const uint32_t bias = 0x64806480u;            // f16x2 (1152, 1152)
-    uint32_t l = (v & 0x00ff00ffu) ^ magic;
-    uint32_t h = ((v >> 8) & 0x00ff00ffu) ^ magic;
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(l), "r"(bias));
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(h), "r"(bias));
-}
-
 // ---- warp-level tensor-core MMA ----
 // D[16 x 8] += A[16 x 16] * B[16 x 8]: A row-major (the kernels here: 16 weight columns x 16 k), B column-major
 // (16 k x 8 activation rows).
@@ -275,7 +256,11 @@ __device__ __forceinline__ void st_async_v4f32(uint32_t addr, float4 v, uint32_t
                  "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
                  : "memory");
 }
-// One arrival on an mbarrier of a CTA of the cluster (address from map_to_rank).
+// One arrival on an mbarrier of a CTA of the cluster (address from map_to_rank).  The default release is at CTA scope: it publishes
+// nothing that this thread stored in shared or global memory to the other CTA.  It is for a signal that carries no such stores,
+// only that something is over: a phase of a barrier of this CTA whose copies have landed in its shared memory, accesses to tensor
+// memory that tcgen05.wait and tcgen05.fence::before_thread_sync stand behind.  (With .release.cluster an arrival takes 350 clocks
+// for 141, and the kernel on SM pairs, whose converters arrive once a stage, 1.6 to 2 times as long.)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "qlinear.h"
+#include "umma.cuh"
 
 namespace b200q {
 namespace decode {
@@ -62,37 +63,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
-}
-
-// Two 16 x 16 byte tiles, transposed on the way to registers.  Lanes 0-15 give the addresses of the 16
-// rows (16 bytes each) of the first tile, lanes 16-31 those of the second.  With a tile stored as
-// [k][column], lane (g = lane / 4, t = lane % 4) receives, for tile i, in r[2i] the bytes
-// (k = 4t .. 4t+3, column g) and in r[2i+1] the bytes (k = 4t .. 4t+3, column g + 8): four consecutive
-// k of one column per register, the packing an MMA operand wants.
-__device__ __forceinline__ void ldmatrix_x2_trans_b8(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-
-// Four signed bytes (b0 .. b3) -> f16 pairs (b0, b1) and (b2, b3), exactly.  b ^ 0x80 = b + 128 as an
-// unsigned byte u; the half with bits 0x6400 | u is 1024 + u; subtracting 1152 leaves b.
-__device__ __forceinline__ void cvt_s8x4_to_f16_pairs(uint32_t v, uint32_t &p01, uint32_t &p23) {
-    const uint32_t u = v ^ 0x80808080u;
-    const uint32_t e01 = __byte_perm(u, 0x64646464u, 0x4140);  // u0 0x64 u1 0x64
-    const uint32_t e23 = __byte_perm(u, 0x64646464u, 0x4342);  // u2 0x64 u3 0x64
-    const uint32_t bias = 0x64806480u;                          // f16x2 (1152, 1152)
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(p01) : "r"(e01), "r"(bias));
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(p23) : "r"(e23), "r"(bias));
-}
-
-// Four 8 x 16 byte tiles as they lie.  Lanes 8i .. 8i+7 give the addresses of the rows of tile i; lane
-// (g = lane / 4, t = lane % 4) receives in r[i] the bytes 4t .. 4t+3 of row g of tile i.  With a weight
-// stored as [column][k] that is again four consecutive k of one column per register.
-__device__ __forceinline__ void ldmatrix_x4_b16(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
 }
 
 __device__ __forceinline__ float4 lds128f(uint32_t addr) {
@@ -395,7 +365,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             uint2 b[4][MT];
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-                if (!NK) ldmatrix_x2_trans_b8(q[ks], wb + ks * 2048);
+                if (!NK) umma::ldmatrix_x2_trans_b8(q[ks], wb + ks * 2048);
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt) b[ks][mt] = lds64(ab + mt * 1024 + (((2 * ks) ^ a_chunk) << 4));
             }
@@ -406,7 +376,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
                     for (int kh = 0; kh < 2; ++kh) {
                         const uint32_t row = nk_row + 16 * j;
                         uint32_t r[4];
-                        ldmatrix_x4_b16(r, w_base + s * W_STAGE_BYTES + row * 64 + (((2 * kh + nk_chunk) ^ ((row >> 1) & 3)) << 4));
+                        umma::ldmatrix_x4(r, w_base + s * W_STAGE_BYTES + row * 64 + (((2 * kh + nk_chunk) ^ ((row >> 1) & 3)) << 4));
                         q[2 * kh][2 * j] = r[0];
                         q[2 * kh][2 * j + 1] = r[1];
                         q[2 * kh + 1][2 * j] = r[2];
@@ -422,8 +392,8 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
                     // tile j: MMA rows g / g + 8 are columns 32 warp + 16 j + g / + 8 + g;
                     // k slots (2t, 2t+1) and (2t+8, 2t+9) carry k = 4t, 4t+1 and 4t+2, 4t+3
                     uint32_t a0, a1, a2, a3;
-                    cvt_s8x4_to_f16_pairs(q[ks][2 * j], a0, a2);
-                    cvt_s8x4_to_f16_pairs(q[ks][2 * j + 1], a1, a3);
+                    umma::cvt_s8x4_to_f16_pairs(q[ks][2 * j], a0, a2);
+                    umma::cvt_s8x4_to_f16_pairs(q[ks][2 * j + 1], a1, a3);
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt) mma_m16n8k16(acc[j][mt], a0, a1, a2, a3, b[ks][mt].x, b[ks][mt].y);
                 }

@@ -57,26 +57,6 @@ static int smem_of(int tm, int cluster) {
     return (rings > exchange ? rings : exchange) + 1024;
 }
 
-constexpr uint32_t kFastPolls = 4096;
-__device__ __noinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, unsigned int site, int *abort_flag, unsigned int *status) {
-    for (uint32_t round = 0; round < kSpinLimit / 1024u; ++round) {
-        if (mbar_wait(bar, parity, 1024u)) return true;
-        if (*reinterpret_cast<volatile int *>(abort_flag) != 0) return false;
-    }
-    report_timeout(status, kKernelMid, site);
-    atomicExch(abort_flag, 1);
-    return false;
-}
-
-// A position in a ring of `n` slots, with the parity of the slot's phase.
-struct Ring {
-    uint32_t slot = 0, phase = 0;
-    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {
-        slot += by;
-        if (slot >= n) slot -= n, phase ^= 1u;
-    }
-};
-
 template <bool FUSED, bool NK>
 __global__ void __launch_bounds__(THREADS, 2)
     qlinear_mid_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const Params p) {
@@ -137,14 +117,14 @@ __global__ void __launch_bounds__(THREADS, 2)
     pdl_wait();  // every role: none of the bounded waits below runs against the kernel in front
 
     auto wait = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
-        bool ok = mbar_wait(bar, parity, kFastPolls);
+        bool ok = mbar_wait(bar, parity, umma::kFastPolls);
         if (__all_sync(0xffffffffu, ok)) return true;
-        if (!ok) ok = wait_or_abort(bar, parity, site, &abort_flag, p.status);
+        if (!ok) ok = umma::wait_or_abort<kKernelMid>(bar, parity, site, &abort_flag, p.status);
         return __all_sync(0xffffffffu, ok);
     };
 
     auto wait_one = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {  // one thread's
-        return mbar_wait(bar, parity, kFastPolls) || wait_or_abort(bar, parity, site, &abort_flag, p.status);
+        return mbar_wait(bar, parity, umma::kFastPolls) || umma::wait_or_abort<kKernelMid>(bar, parity, site, &abort_flag, p.status);
     };
 
     if (warp == RAW_WARP) {
@@ -153,7 +133,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         pdl_launch_dependents();  // tensor memory is allocated: a kernel that moves in cannot take it away from this one
         if (lane == 0) tma_prefetch_desc(&map_w);
         uint32_t i = 0;
-        Ring r;
+        umma::Ring r;
         for (; i < n_it; ++i, r.advance(1, raw_slots)) {
             if (i >= raw_slots && !wait(smem_u32(&raw_empty[r.slot]), r.phase ^ 1u, 1)) break;
             if (elect_one()) {
@@ -176,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         if (lane == 0) tma_prefetch_desc(&map_a);
         const uint64_t keep = l2_policy_evict_last();
         uint32_t i = 0;
-        Ring r;
+        umma::Ring r;
         for (; i < n_it; ++i, r.advance(1, act_slots)) {
             if (i >= act_slots && !wait(smem_u32(&act_empty[r.slot]), r.phase ^ 1u, 2)) break;
             if (elect_one()) {
@@ -197,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         // outside 47.  The barriers of the next stage are asked while this one's MMAs are on their way.
         if (elect_one()) {
             const uint32_t idesc = umma::instr_desc_f16(TN, p.tm);
-            Ring a, w;
+            umma::Ring a, w;
             bool act_ok = false, w_ok = false;
             for (uint32_t i = 0; i < n_it; ++i) {
                 if (!act_ok && !wait_one(smem_u32(&act_full[a.slot]), a.phase, 3)) break;
@@ -226,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         const uint32_t kn_off = (uint32_t)(lane & 15) * 128u + (((uint32_t)(2 * q + (lane >> 4)) ^ (uint32_t)(lane & 7)) << 4);
         const uint32_t nk_row = (uint32_t)(32 * q + lane);
         const uint32_t nk_off = nk_row * 64u, nk_sw = (nk_row >> 1) & 3u;
-        Ring r, w;
+        umma::Ring r, w;
         r.slot = group, w.slot = group;
         bool raw_ok = false;
         for (uint32_t i = group; i < n_it; i += CONV_GROUPS, w.advance(CONV_GROUPS, W_SLOTS)) {

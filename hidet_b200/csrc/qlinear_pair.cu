@@ -19,7 +19,8 @@
 //   warp 12     TMA producer of the int8 tiles
 //   warp 13     TMA producer of the activation tiles
 //   warp 14     MMA issuer (first CTA of the pair only): one thread for the whole loop, one barrier a stage: each CTA's converters
-//               tell it that their weight tile is in tensor memory and that their CTA's activations have landed
+//               tell it that their weight tile is in tensor memory and that their CTA's activations have landed (arrivals on
+//               the first CTA's barriers that carry no stores with them: see mbar_arrive_remote)
 //
 // Every wait is bounded, as in qlinear_prefill.cu: a wait that runs out records where and raises a CTA-wide flag, all roles
 // leave, the producers wait for the copies they armed, the MMA thread for what it issued, and the two CTAs meet at a cluster
@@ -77,28 +78,6 @@ __device__ __forceinline__ void tile_of(const Params &p, int u, int &n0, int &m0
     const int n = r / rows;
     n0 = n * 2 * TN;
     m0 = (b * p.band + (r - n * rows)) * p.tm;
-}
-
-// A position in a ring of `n` slots, with the parity of the slot's phase.
-struct Ring {
-    uint32_t slot = 0, phase = 0;
-    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {
-        slot += by;
-        if (slot >= n) slot -= n, phase ^= 1u;
-    }
-};
-
-constexpr uint32_t kFastPolls = 4096;
-// The rest of a bounded wait: polls on, looking at the CTA's abort flag between runs of polls; when its own limit runs out it
-// records the site and raises the flag for the other roles of the CTA.
-__device__ __noinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, unsigned int site, int *abort_flag, unsigned int *status) {
-    for (uint32_t round = 0; round < kSpinLimit / 1024u; ++round) {
-        if (mbar_wait(bar, parity, 1024u)) return true;
-        if (*reinterpret_cast<volatile int *>(abort_flag) != 0) return false;
-    }
-    report_timeout(status, kKernelPair, site);
-    atomicExch(abort_flag, 1);
-    return false;
 }
 
 // NK: the weight is [N, K] with K contiguous.
@@ -164,13 +143,13 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
 
     // Bounded wait of a whole warp (true in all lanes or false in all lanes) / of one thread.
     auto wait = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
-        bool ok = mbar_wait(bar, parity, kFastPolls);
+        bool ok = mbar_wait(bar, parity, umma::kFastPolls);
         if (__all_sync(0xffffffffu, ok)) return true;
-        if (!ok) ok = wait_or_abort(bar, parity, site, &abort_flag, p.status);
+        if (!ok) ok = umma::wait_or_abort<kKernelPair>(bar, parity, site, &abort_flag, p.status);
         return __all_sync(0xffffffffu, ok);
     };
     auto wait_one = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
-        return mbar_wait(bar, parity, kFastPolls) || wait_or_abort(bar, parity, site, &abort_flag, p.status);
+        return mbar_wait(bar, parity, umma::kFastPolls) || umma::wait_or_abort<kKernelPair>(bar, parity, site, &abort_flag, p.status);
     };
 
     if (warp == RAW_WARP) {
@@ -179,7 +158,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         if (lane == 0) {
             tma_prefetch_desc(&map_w);
             uint32_t i = 0;
-            Ring r;
+            umma::Ring r;
             bool ok = true;
             for (int u = first; u < units && ok; u += step) {
                 int n, m0;
@@ -209,7 +188,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
             tma_prefetch_desc(&map_a);
             const uint64_t keep = l2_policy_evict_last();  // every column tile reads them again
             uint32_t i = 0;
-            Ring r;
+            umma::Ring r;
             bool ok = true;
             for (int u = first; u < units && ok; u += step) {
                 int n0, m;
@@ -238,7 +217,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         if (rank == 0 && elect_one()) {
             const uint32_t idesc = umma::instr_desc_f16(2 * TN, p.tm);
             uint32_t t_iter = 0;
-            Ring ra, rw;
+            umma::Ring ra, rw;
             bool ok = true, here = false;
             for (int u = first; u < units && ok; u += step, ++t_iter) {
                 const uint32_t buf = n_acc == 2 ? (t_iter & 1) : 0, acc_use = n_acc == 2 ? (t_iter >> 1) : t_iter;
@@ -283,7 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         const uint32_t nk_off = nk_row * 64u, nk_sw = (nk_row >> 1) & 3u;
         const int my_units = units > first ? (units - first + step - 1) / step : 0;
         const uint32_t stages = (uint32_t)my_units * (uint32_t)p.k_blocks;
-        Ring rr, ra, rw;
+        umma::Ring rr, ra, rw;
         rr.slot = ra.slot = rw.slot = (uint32_t)group;
         bool raw_ok = false;
         for (uint32_t i = group; i < stages; i += CONV_GROUPS, ra.advance(CONV_GROUPS, act_slots), rw.advance(CONV_GROUPS, w_slots)) {
@@ -317,6 +296,9 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
             umma::fence_before_sync();
             if (!__all_sync(0xffffffffu, t_act) && !wait(smem_u32(&act_full[ra.slot]), ra.phase, 9)) break;
             __syncwarp();
+            // What the MMA reads behind this arrival is the weight in this CTA's tensor memory, stored (st_wait) and fenced above, and the
+            // activations that the copy engine put into this CTA's shared memory, complete before the phase that was waited for: no
+            // store of this warp is among it, so the arrival needs no wider scope.
             if (lane == 0) mbar_arrive_remote(ready0 + 8 * rw.slot);
         }
     } else {

@@ -113,19 +113,6 @@ struct Params {
     float *partial;
 };
 
-constexpr uint32_t kFastPolls = 4096;
-// The rest of a bounded wait: polls on, looking at the CTA's abort flag between runs of polls; when its own
-// limit runs out it records the site and raises the flag for the other roles.
-__device__ __noinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, unsigned int site, int *abort_flag, unsigned int *status) {
-    for (uint32_t round = 0; round < kSpinLimit / 1024u; ++round) {
-        if (mbar_wait(bar, parity, 1024u)) return true;
-        if (*reinterpret_cast<volatile int *>(abort_flag) != 0) return false;
-    }
-    report_timeout(status, kKernelPrefill, site);
-    atomicExch(abort_flag, 1);
-    return false;
-}
-
 template <int TM>
 __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                         const __grid_constant__ CUtensorMap map_a,
@@ -192,12 +179,9 @@ __global__ void __launch_bounds__(THREADS, 1) qlinear_prefill_kn_kernel(const __
     umma::fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
     // Bounded wait that also ends when another role has given up; the role whose own limit runs out reports it.
-    // The first polls are the plain inlined loop; everything else lives in a function of its own, so that the
-    // code around the hot loops stays what it is without the flag (with the flag test inlined at every wait the
-    // kernel lost a tenth of its speed, although the test never ran).
     auto wait = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
-        if (mbar_wait(bar, parity, kFastPolls)) return true;
-        return wait_or_abort(bar, parity, site, &abort_flag, p.status);
+        if (mbar_wait(bar, parity, umma::kFastPolls)) return true;
+        return umma::wait_or_abort<kKernelPrefill>(bar, parity, site, &abort_flag, p.status);
     };
 
     if (warp == PRODUCER_WARP) {

@@ -129,5 +129,31 @@ __device__ __forceinline__ void cvt_s8x4_to_f16_pairs(uint32_t v, uint32_t &p01,
     asm("sub.f16x2 %0, %1, %2;" : "=r"(p23) : "r"(e23), "r"(bias));
 }
 
+// ---- what the kernels' pipelines share ----
+// A position in a ring of `n` slots, with the parity of the slot's phase.
+struct Ring {
+    uint32_t slot = 0, phase = 0;
+    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {
+        slot += by;
+        if (slot >= n) slot -= n, phase ^= 1u;
+    }
+};
+
+// A bounded wait is this many plain polls, inline, and then `wait_or_abort`: the code around the hot loops stays what it is without
+// the flag (with the flag tested at every wait the one-SM kernel lost a tenth of its speed, although the test never ran).
+constexpr uint32_t kFastPolls = 4096;
+// Polls on, looking at the CTA's abort flag between runs of polls; when its own limit runs out it records the site and raises
+// the flag for the other roles of the CTA.
+template <unsigned int KERNEL>
+__device__ __noinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, unsigned int site, int *abort_flag, unsigned int *status) {
+    for (uint32_t round = 0; round < kSpinLimit / 1024u; ++round) {
+        if (mbar_wait(bar, parity, 1024u)) return true;
+        if (*reinterpret_cast<volatile int *>(abort_flag) != 0) return false;
+    }
+    report_timeout(status, KERNEL, site);
+    atomicExch(abort_flag, 1);
+    return false;
+}
+
 }  // namespace umma
 }  // namespace b200q
