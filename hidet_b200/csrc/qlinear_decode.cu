@@ -189,8 +189,8 @@ struct Params {
 //     plain matrix loads; everything else is shared.
 // QUAD: the elements that a CTA finishes in the split-K reduction are taken four adjacent columns of a row per thread (more than
 //     four rows; with fewer one element per thread is one round anyway: (4, 9648, 1568) 7.9 us, 8.05 so).
-// Shared memory lets four CTAs share an SM; told so, the compiler spills nothing: a decode step for sixteen sequences 252 -> 242 us,
-// for one 208.8 -> 205.6.
+// Shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
+// bytes in one form): a decode step at 7B widths for one sequence 216 -> 209 us, for sixteen 256 -> 252.
 template <int MT, bool NK, bool QUAD>
 __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
     using Cfg = Config<MT>;
@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t full_bar[STAGES];
     __shared__ __align__(8) uint64_t empty_bar[STAGES];
-    __shared__ __align__(8) uint64_t recv_bar;  // the partial tiles of this CTA's columns have landed
+    __shared__ __align__(8) uint64_t recv_bar;  // the partial tiles of this CTA's columns have landed, and their scales
+    __shared__ __align__(8) unsigned short own_scales[BN];  // f16 bits
     __shared__ unsigned int is_last;
 
     // 128B-swizzled TMA tiles need 1024-byte aligned bases.
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             mbar_init(smem_u32(&full_bar[s]), 1 + 32);  // the weight tile (TMA bytes) and the producer warp's 32 lanes, each when its activation copies have landed
             mbar_init(smem_u32(&empty_bar[s]), CONSUMER_WARPS);
         }
-        mbar_init(smem_u32(&recv_bar), 1);
+        mbar_init(smem_u32(&recv_bar), 1 + 1);  // the expected bytes, and the producer warp with the scales
         mbar_fence_init();
         // Bytes the cluster will send here: every rank, `rows` rows of this CTA's columns.
         if (p.mode == kModeSplit && own_cols > 0) mbar_expect_tx(smem_u32(&recv_bar), nranks * (uint32_t)rows * (uint32_t)own_cols * 4u);
@@ -247,24 +248,14 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
     // then every CTA of the cluster has started and set up its barriers, which remote access requires.
     cluster_arrive_release();
 
-    // What this thread finishes in the split-K reduction (one element, or with QUAD four columns of a row), and its scales
-    // (without a split: those of its four columns of the tile).  They may be a result of the kernel in front, so they are asked for
-    // when that one is done, through L2, far from where they are used, and stay as they come until then: converted on the
-    // spot, the warps would wait for them in front of the main loop ((4, 4096, 1024) 4.4 us for 3.9).
-    constexpr int WIDTH = QUAD ? 4 : 1;
-    const int per_row = cols_per / WIDTH;  // such pieces of one row of this CTA's columns
-    const bool direct = p.mode == kModeDirect;
-    const int own_cc = direct ? 32 * warp + g : own_first + ((int)threadIdx.x % per_row) * WIDTH;  // the first of them in the tile
-    const int own_step = direct ? 8 : 1;
-    const bool owner = direct ? warp < CONSUMER_WARPS : (int)threadIdx.x < rows * per_row;
-    const int own_end = owner ? min(direct ? own_cc + 25 : min(own_cc + WIDTH, own_first + own_cols), p.N - n0) : 0;
-    const unsigned short *own_scales = reinterpret_cast<const unsigned short *>(p.scale) + n0 + own_cc;
-    unsigned short sc_bits[4];
-    auto load_scales = [&]() {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) sc_bits[j] = own_cc + j * own_step < own_end ? __ldcg(own_scales + j * own_step) : (unsigned short)0;
-    };
-    auto own_scale = [&](int j) { return __half2float(__ushort_as_half(sc_bits[j])); };
+    // The scales may be a result of the kernel in front: they are asked for when that one is done, through L2, far from where they are
+    // used, by the producer warp for the columns that this CTA sums (in shared memory at the end of its loop; by every thread for itself a
+    // decode step takes 209.0 us for 207.6), without a split by every consumer for its own four.  They stay as they come until
+    // they are used: a conversion where they are loaded waits for them in front of the main loop ((4, 4096, 1024) 4.4 us
+    // for 3.9 to 4.1).
+    const unsigned short *scale_bits = reinterpret_cast<const unsigned short *>(p.scale) + n0;
+    unsigned short sc_bits[4] = {0, 0, 0, 0};
+    auto scale_of = [&](int cc) { return __half2float(__ushort_as_half(own_scales[cc])); };
 
     // acc[j][mt][.]: 16 x 8 tile j of this warp's 32 columns, activation rows 8 * mt ... 8 * mt + 7.
     // Element (column 16 j + 8 h + g, row 8 mt + 2t + e) is acc[j][mt][2h + e].
@@ -326,7 +317,13 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
         // at the end of the main loop).
         if (gridDim.z == 1) pdl_launch_dependents();
         for (int it = 0; it < prologue; ++it) copy_activations(it, p.k_begin + (it_begin + it) * BK);
-        load_scales();
+        if (p.mode == kModeSplit) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int cc = 4 * lane + j;
+                if (cc < own_cols && n0 + own_first + cc < p.N) sc_bits[j] = __ldcg(scale_bits + own_first + cc);
+            }
+        }
         for (int it = STAGES; it < n_iters; ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(smem_u32(&empty_bar[s]), ((it / STAGES) - 1) & 1)) {
@@ -337,10 +334,21 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             if (lane == 0) load_weights(s, it, stream_policy);
             copy_activations(s, k0);
         }
+        if (p.mode == kModeSplit) {
+            *reinterpret_cast<uint2 *>(own_scales + 4 * lane) = make_uint2(sc_bits[0] | (uint32_t)sc_bits[1] << 16, sc_bits[2] | (uint32_t)sc_bits[3] << 16);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&recv_bar));
+        }
     } else {
         // ---------------- consumers ----------------
         pdl_wait();
-        load_scales();
+        if (p.mode == kModeDirect) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // i = 2 j + h, see below
+                const int cc = 32 * warp + 8 * i + g;
+                if (n0 + cc < p.N) sc_bits[i] = __ldcg(scale_bits + cc);
+            }
+        }
         // Weights: one transposing matrix load per 16 k-rows brings this warp's 32 columns (16-byte
         // chunks 2 warp and 2 warp + 1 of each row).  Lane l addresses row (l & 15) of chunk
         // 2 warp + (l >> 4); under the 128B swizzle chunk c of row r sits at chunk c ^ (r & 7).
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int nn = n0 + col_base + 16 * j + 8 * h;
-                    const float sc = own_scale(2 * j + h);
+                    const float sc = __half2float(__ushort_as_half(sc_bits[2 * j + h]));
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -489,6 +497,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             // Four adjacent columns of one row per thread and round, so that 16 rows of a slice are one round (one element per thread
             // made four of them, each with its trips to memory: (16, 1408, 1408) with a residual 5.5 -> 3.6 us, (16, 4096,
             // 12288) 13.3 -> 11.9, (7, 896, 12112) 5.8 -> 4.7).  Item i is row i / per_row, columns 4 (i % per_row) .. + 3.
+            const int per_row = cols_per / 4;
             auto sum_ranks4 = [&](int r, int cc) {
                 float4 v[8];
 #pragma unroll
@@ -504,14 +513,9 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
                 const int nn = col_first + cc;
                 if (cc >= own_cols || nn >= p.N) continue;  // own_cols is a multiple of 8
                 float4 y = sum_ranks4(r, cc);
-                if (item < THREADS) {
-                    y.x *= own_scale(0), y.y *= own_scale(1), y.z *= own_scale(2), y.w *= own_scale(3);
-                } else {
-                    y.x *= __half2float(__ldcg(p.scale + nn));
-                    if (nn + 1 < p.N) y.y *= __half2float(__ldcg(p.scale + nn + 1));
-                    if (nn + 2 < p.N) y.z *= __half2float(__ldcg(p.scale + nn + 2));
-                    if (nn + 3 < p.N) y.w *= __half2float(__ldcg(p.scale + nn + 3));
-                }
+                const uint2 sc4 = *reinterpret_cast<const uint2 *>(own_scales + cc);
+                const float2 sc01 = __half22float2(*reinterpret_cast<const __half2 *>(&sc4.x)), sc23 = __half22float2(*reinterpret_cast<const __half2 *>(&sc4.y));
+                y.x *= sc01.x, y.y *= sc01.y, y.z *= sc23.x, y.w *= sc23.y;
                 if (nn + 3 < p.N) {
                     finish4(p.out, p.ep, m0 + r, nn, y);
                 } else {  // the end of an [N, K] weight's odd column count: no epilogue there
@@ -537,8 +541,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
                 const int cc = idx - r * cols_per;
                 const int nn = col_first + cc;
                 const bool valid = nn < p.N && cc < own_cols;  // N and own_cols are even: the two columns of a pair agree
-                const float sc = idx < THREADS ? own_scale(0) : (valid ? __half2float(__ldcg(p.scale + nn)) : 0.0f);
-                finish(p.out, p.ep, m0 + r, nn, p.N, valid, valid ? sum_ranks(r, cc) * sc : 0.0f, 1);
+                finish(p.out, p.ep, m0 + r, nn, p.N, valid, valid ? sum_ranks(r, cc) * scale_of(cc) : 0.0f, 1);
             }
         }
         return;
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
         if (valid) {
 #pragma unroll 4
             for (int gr = 0; gr < p.groups; ++gr) v += __ldcg(&p.partial[((size_t)gr * p.M + (m0 + r)) * p.N + nn]);
-            v *= !QUAD && idx < THREADS ? own_scale(0) : __half2float(__ldcg(p.scale + nn));
+            v *= scale_of(cc);
         }
         finish(p.out, p.ep, m0 + r, nn, p.N, valid, v, 1);
     }
