@@ -114,10 +114,10 @@ int mid_resident_ctas(int tm, int cluster);  // of the mid-M kernel, in clusters
 bool unaligned_supported(const void *a, const void *wq, const void *c, int64_t M, int64_t N, int64_t K);
 int launch_unaligned(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 
-// Which kernel serves M activation rows.  The tensor-memory kernel's tiles span 64 or 256 rows and it
-// streams every weight tile once per row block; the small-M kernel re-streams the weight once per 16
-// rows (from L2 after the first pass).  Up to 32 rows the small-M kernel always wins, up to 64 rows it
-// still wins on weights of a few tens of MB.
+// Where the small-M kernel, which re-streams the weight once per 16 rows (from L2 after the first pass), is out of the question: the
+// kernels for more rows then refuse what they cannot take.  (The line was drawn against the one-SM kernel, up to 64 rows by the size of
+// the weight; below it plan_large compares estimates.  By those the small-M kernel would still be ahead of it in
+// corners, (128, 1024, 1024) and (100, 4096, 1024) among them, which are not timed.)
 constexpr int64_t kPrefillMinM = 33;
 inline bool use_prefill_kernel(int64_t M, int64_t N, int64_t K) {
     if (M < kPrefillMinM) return false;

@@ -219,21 +219,21 @@ B200Q_API int b200q_qlinear_f16_i8_parts(const void *a, const void *wq, const vo
  * python/hidet/graph/ops/distributed.py:63-97 (whose result is rank-major and needs a reshuffle).
  * The caller orders the ranks afterwards (a barrier between "all kernels done" and "outputs read").
  * `dst` is a host array.  KN layout; workspace as for b200q_qlinear_f16_i8 with the same M, N, K.
- * Both kernels store to every destination from their epilogue, tile by tile, so the delivery overlaps
- * the rest of the product; ldc and col_offset must be multiples of 8 and the destinations 16-byte aligned
- * when the large-M kernel serves the call.
+ * All kernels store to every destination from their epilogue, tile by tile, so the delivery overlaps
+ * the rest of the product; with more than 64 rows (33 where K * N is above 24 Mi) ldc and col_offset must be
+ * multiples of 8 and the destinations 16-byte aligned.
  */
 B200Q_API int b200q_qlinear_f16_i8_to_peers(const void *a, const void *wq, const void *scale, void *const *dst, int n_dst,
                                             int64_t ldc, int64_t col_offset, int64_t M, int64_t N, int64_t K, void *workspace,
                                             size_t workspace_bytes, void *stream);
 
 /*
- * The same for large M through an NVLink multicast address: `multicast_dst` maps the [M, ldc] output buffers of all
+ * The same for many rows through an NVLink multicast address: `multicast_dst` maps the [M, ldc] output buffers of all
  * ranks of the group at once (a multicast object over symmetric allocations, e.g. the multicast pointer of a
- * torch symmetric-memory handle), and the large-M kernel's epilogue stores every 16 bytes once with multimem.st;
+ * torch symmetric-memory handle), and the kernel's epilogue stores every 16 bytes once with multimem.st;
  * the switch delivers them to every GPU, this one included.  The bytes that leave this GPU are 1 / (ranks - 1) of
- * what b200q_qlinear_f16_i8_to_peers sends.  M >= 33 and operands the large-M kernel accepts, else
- * B200Q_UNSUPPORTED (use b200q_qlinear_f16_i8_to_peers).  The caller orders the ranks
+ * what b200q_qlinear_f16_i8_to_peers sends.  The row counts just named and
+ * 16-byte aligned operands, else B200Q_UNSUPPORTED (use b200q_qlinear_f16_i8_to_peers).  The caller orders the ranks
  * afterwards, as above.  No counterpart in the reference beyond the all-gather op named above.
  * The workspace is optional: with the bytes that b200q_qlinear_multicast_workspace_bytes answers (0 for most shapes; their
  * contents do not matter, and a workspace of b200q_qlinear_f16_i8 may serve, whose zero-filled part is left alone) narrow

@@ -154,8 +154,8 @@ def test_explicit_k_parts_at_a_large_m(parts):
 
 def test_quantize_then_linear_inside_one_captured_graph():
     """The linear requests its weight tiles before it waits for the kernel in front of it (programmatic
-    dependent launch).  That is only sound because no kernel of this library lets its dependents start
-    before it has finished writing: a weight quantized by the launch directly in front must be seen whole."""
+    dependent launch).  That is only sound because the kernels that write weights let their dependents start
+    when they have finished: a weight quantized by the launch directly in front must be seen whole."""
     k, n, m = 4096, 4096, 4
     gen = torch.Generator(device='cuda').manual_seed(5)
     ws = [(torch.randn(k, n, generator=gen, device='cuda', dtype=torch.float32) * 0.02).half() for _ in range(3)]
