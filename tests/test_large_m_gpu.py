@@ -11,7 +11,7 @@ from hidet_b200 import ffi
 pytestmark = pytest.mark.gpu
 
 
-MID, PAIR = 1, 2
+SMALL, MID, PAIR = 0, 1, 2
 
 
 def _plan(large_kernels, m, k, n, silu=False):
@@ -48,7 +48,7 @@ def _run(m, k, n, layout, bias=False, silu=False, residual=False):
 # k that ends inside a stage, one stage, fewer stages than ring slots and more, one tile and several per pair of SMs or cluster, the last
 # rows and columns
 @pytest.mark.parametrize('kind,m,k,n', [(MID, 513, 64, 16), (MID, 600, 8, 256), (MID, 513, 72, 272), (MID, 777, 1000, 528), (PAIR, 1025, 520, 2064), (PAIR, 1500, 2048, 1040),
-                                        (MID, 2048, 1032, 16), (PAIR, 3001, 456, 4112), (PAIR, 1000, 4096, 4096)])
+                                        (MID, 2048, 1032, 16), (PAIR, 3001, 456, 4112), (PAIR, 1000, 4096, 4096), (SMALL, 24, 4096, 12288)])
 def test_many_rows(large_kernels, kind, m, k, n):
     assert _plan(large_kernels, m, k, n) == kind
     _run(m, k, n, 'KN')
