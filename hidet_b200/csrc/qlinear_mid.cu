@@ -8,7 +8,7 @@
 //
 // Warps: converters in two groups that take stages in turn, then do the reduction and the epilogue; a TMA producer of the int8
 // tiles; a TMA producer of the activation tiles; the MMA issuer.
-// Nothing is read before the kernel in front is done, the weight included.  Every wait is bounded (see qlinear_prefill.cu).
+// Nothing is read before the kernel in front is done, the weight included; the first tiles are asked into L2 meanwhile.  Every wait is bounded (see qlinear_prefill.cu).
 #include <atomic>
 
 #include "common.cuh"
@@ -114,6 +114,14 @@ __global__ void __launch_bounds__(THREADS, 2)
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    // A ring's fill of the weight, into L2 only, while the kernel in front ends: (64, 4096, 11008) 16.2 -> 15.8 us, [N, K] 16.8 -> 16.1,
+    // (64, 2304, 6912) 10.6 -> 10.3.
+    if (warp == RAW_WARP && lane == 0) {
+        for (uint32_t i = 0; i < n_it && i < raw_slots; ++i) {
+            const int k0 = (kb_begin + (int)i) * BK;
+            tma_prefetch_2d(&map_w, NK ? k0 : n0, NK ? n0 : k0);
+        }
+    }
     pdl_wait();  // every role: none of the bounded waits below runs against the kernel in front
 
     auto wait = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
