@@ -46,6 +46,7 @@ struct Epilogue {
 
 // How the small-M kernel splits a problem over CTAs, and the scratch that split needs.
 struct DecodePlan {
+    int variant = 0;           // which form of the kernel: rows per pass
     int n_tiles = 0;
     int m_tiles = 0;
     int splits = 1;            // CTAs along K per output tile
@@ -53,7 +54,8 @@ struct DecodePlan {
     int groups = 1;            // clusters per tile; > 1: the clusters meet in the workspace
     int iters_per_split = 0;   // 64-row k steps each of them takes
     size_t counter_bytes = 0;  // head of the workspace: one arrival counter per output tile
-    size_t partial_bytes = 0;  // then [groups][M][N] fp32 partial sums (0 when groups == 1)
+    size_t partial_bytes = 0;  // then [groups][M][N] fp32 partial sums.  Both are asked of the caller where clusters of the portable size
+                               // would meet in the workspace, also where larger ones (groups == 1) do without
 };
 
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K);

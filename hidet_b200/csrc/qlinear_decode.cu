@@ -7,9 +7,9 @@
 // fetches its slice with transposing matrix loads (four consecutive k of one column per register),
 // turns the bytes into exact f16 pairs in registers and feeds warp-level m16n8k16 tensor-core MMAs
 // with fp32 accumulators; the weight is the MMA's 16-row operand and the activations its 8-column operand, so up to 8 activation rows
-// cost one MMA per 16 x 16 weight block and up to 16 rows two (rows beyond M are zero-filled).
+// cost one MMA per 16 x 16 weight block, up to 16 rows two (rows beyond M are zero-filled).
 //
-// K is split across CTAs to fill the machine.  Up to 8 splits of one output tile form a thread-block
+// K is split across CTAs to fill the machine.  Up to 16 splits of one output tile form a thread-block
 // cluster: every CTA sends its partial tile into the shared memory of the CTA that owns those columns
 // with asynchronous remote stores that count bytes on an mbarrier of the owner (no cluster barrier
 // round trip); the owner waits for the byte count, adds the partials in rank order, applies the
@@ -39,13 +39,14 @@ constexpr int STAGES = 4;
 constexpr int CONSUMER_WARPS = 4;            // each owns BN / 4 = 32 columns
 constexpr int THREADS = 32 * (CONSUMER_WARPS + 1);
 constexpr int W_STAGE_BYTES = BK * BN;       // 8192
-constexpr int RECV_COLS = 168;               // most columns the slices of a cluster cover together (7 ranks x 24 columns)
+constexpr int RECV_COLS = 168;               // most columns the slices of a cluster cover together (7 ranks x 24 columns, 14 x 12)
 constexpr int STAGING_ROW = 36;              // floats per row of a warp's 32-column staging block (padded: conflict-free)
 
 // Shared memory of a CTA with MT blocks of eight activation rows.
 template <int MT>
 struct Config {
     static constexpr int ROWS = 8 * MT;                  // activation rows per CTA
+    static constexpr int CTAS = 4;                       // that share an SM
     static constexpr int A_STAGE_BYTES = ROWS * BK * 2;
     static constexpr int PIPE_BYTES = STAGES * (W_STAGE_BYTES + A_STAGE_BYTES);
     static constexpr int RECV_BYTES = ROWS * RECV_COLS * 4;  // partial tiles sent by the CTAs of the cluster: [rank][row][cols_per] fp32
@@ -57,7 +58,8 @@ struct Config {
     static_assert(CONSUMER_WARPS * ROWS * STAGING_ROW * 4 <= STAGES * W_STAGE_BYTES, "the staging blocks reuse the weight ring");
 };
 constexpr int64_t kMaxCounters = 65536;      // arrival counters at the head of the workspace
-constexpr int kMaxCluster = 8;               // largest cluster of the plan (8 is the portable limit; the reduction reads up to eight partials)
+constexpr int kPortableCluster = 8;          // what every device runs; beyond it the occupancy query has the last word
+constexpr int kMaxCluster = 16;              // largest cluster of the plan, which leaves out 15 (slices of 12 columns would cover 180)
 
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
@@ -179,7 +181,7 @@ struct Params {
     int k_begin, k_end;       // the k range this launch sums over (k_end is also the tensor maps' K extent)
     int iters_per_split;      // BK-sized k steps per split
     int groups;               // clusters per output tile (splits = groups * cluster size)
-    int cols_per;             // columns of a tile each CTA of the cluster owns in the reduction (a multiple of 8)
+    int cols_per;             // columns of a tile each CTA of the cluster owns in the reduction (a multiple of 4)
     int mode;                 // kModeDirect or kModeSplit
 };
 
@@ -189,12 +191,14 @@ struct Params {
 //     plain matrix loads; everything else is shared.
 // QUAD: the elements that a CTA finishes in the split-K reduction are taken four adjacent columns of a row per thread (more than
 //     four rows; with fewer one element per thread is one round anyway: (4, 9648, 1568) 7.9 us, 8.05 so).
+// WIDE: clusters beyond the portable size (the eight partials that a smaller one sums at once stay one piece of code without a loop:
+//     (16, 4096, 12288) 12.0 us, 12.4 with it).
 // Shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
 // bytes in one form): a decode step at 7B widths for one sequence 216 -> 209 us, for sixteen 256 -> 252.
-template <int MT, bool NK, bool QUAD>
-__global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
+template <int MT, bool NK, bool QUAD, bool WIDE>
+__global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
     using Cfg = Config<MT>;
-    constexpr int ROWS = Cfg::ROWS, A_STAGE_BYTES = Cfg::A_STAGE_BYTES, PIPE_BYTES = Cfg::PIPE_BYTES;
+    constexpr int ROWS = Cfg::ROWS, A_STAGE_BYTES = Cfg::A_STAGE_BYTES, PIPE_BYTES = Cfg::PIPE_BYTES, MAX_RANKS = WIDE ? kMaxCluster : kPortableCluster;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t full_bar[STAGES];
     __shared__ __align__(8) uint64_t empty_bar[STAGES];
@@ -490,8 +494,21 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
     if (own_cols > 0) {
         if (!mbar_wait_cluster(smem_u32(&recv_bar), 0)) report_timeout(p.status, kKernelDecode, 4);
     }
-    // Owner: the partials of the (at most eight) ranks are read together and added in rank order.
+    // Owner: the partials of the ranks are read eight together and added in rank order.
     const int col_first = n0 + own_first;  // first column this CTA owns
+    auto sum_ranks = [&](int r, int cc) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int first = 0; first < MAX_RANKS; first += 8) {
+            float v[8];
+#pragma unroll
+            for (int jr = 0; jr < 8; ++jr) v[jr] = first + jr < (int)nranks ? recv[((first + jr) * ROWS + r) * cols_per + cc] : 0.0f;
+            if (first == 0) sum = v[0];
+#pragma unroll
+            for (int jr = first == 0 ? 1 : 0; jr < 8; ++jr) sum += v[jr];
+        }
+        return sum;
+    };
     if (p.groups == 1) {
         if constexpr (QUAD) {
             // Four adjacent columns of one row per thread and round, so that 16 rows of a slice are one round (one element per thread
@@ -499,19 +516,24 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             // 12288) 13.3 -> 11.9, (7, 896, 12112) 5.8 -> 4.7).  Item i is row i / per_row, columns 4 (i % per_row) .. + 3.
             const int per_row = cols_per / 4;
             auto sum_ranks4 = [&](int r, int cc) {
-                float4 v[8];
+                float4 sum;
 #pragma unroll
-                for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? *reinterpret_cast<const float4 *>(recv + (jr * ROWS + r) * cols_per + cc) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                float4 sum = v[0];
+                for (int first = 0; first < MAX_RANKS; first += 8) {
+                    float4 v[8];
 #pragma unroll
-                for (int jr = 1; jr < 8; ++jr) sum.x += v[jr].x, sum.y += v[jr].y, sum.z += v[jr].z, sum.w += v[jr].w;
+                    for (int jr = 0; jr < 8; ++jr)
+                        v[jr] = first + jr < (int)nranks ? *reinterpret_cast<const float4 *>(recv + ((first + jr) * ROWS + r) * cols_per + cc) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (first == 0) sum = v[0];
+#pragma unroll
+                    for (int jr = first == 0 ? 1 : 0; jr < 8; ++jr) sum.x += v[jr].x, sum.y += v[jr].y, sum.z += v[jr].z, sum.w += v[jr].w;
+                }
                 return sum;
             };
             for (int item = threadIdx.x; item < rows * per_row; item += THREADS) {
                 const int r = item / per_row;
                 const int cc = (item - r * per_row) * 4;
                 const int nn = col_first + cc;
-                if (cc >= own_cols || nn >= p.N) continue;  // own_cols is a multiple of 8
+                if (cc >= own_cols || nn >= p.N) continue;  // own_cols is a multiple of 4
                 float4 y = sum_ranks4(r, cc);
                 const uint2 sc4 = *reinterpret_cast<const uint2 *>(own_scales + cc);
                 const float2 sc01 = __half22float2(*reinterpret_cast<const __half2 *>(&sc4.x)), sc23 = __half22float2(*reinterpret_cast<const __half2 *>(&sc4.y));
@@ -527,15 +549,6 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
             }
         } else {
             // One element per thread and round; element i is row i / cols_per, column i % cols_per of the slice.
-            auto sum_ranks = [&](int r, int cc) {
-                float v[8];
-#pragma unroll
-                for (int jr = 0; jr < 8; ++jr) v[jr] = jr < (int)nranks ? recv[(jr * ROWS + r) * cols_per + cc] : 0.0f;
-                float sum = v[0];
-#pragma unroll
-                for (int jr = 1; jr < 8; ++jr) sum += v[jr];
-                return sum;
-            };
             for (int idx = threadIdx.x; idx < rows * cols_per; idx += THREADS) {
                 const int r = idx / cols_per;
                 const int cc = idx - r * cols_per;
@@ -555,12 +568,7 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
         const int r = idx / cols_per;
         const int cc = idx - r * cols_per;
         const int nn = col_first + cc;
-        if (nn < p.N && cc < own_cols) {
-            float sum = recv[r * cols_per + cc];
-#pragma unroll
-            for (int jr = 1; jr < 8; ++jr) sum += jr < (int)nranks ? recv[(jr * ROWS + r) * cols_per + cc] : 0.0f;
-            __stcg(&p.partial[((size_t)group * p.M + (m0 + r)) * p.N + nn], sum);
-        }
+        if (nn < p.N && cc < own_cols) __stcg(&p.partial[((size_t)group * p.M + (m0 + r)) * p.N + nn], sum_ranks(r, cc));
     }
     __threadfence();
     __syncthreads();
@@ -592,46 +600,50 @@ __global__ void __launch_bounds__(THREADS, 4) qlinear_decode_kn_kernel(const __g
 
 namespace decode {
 
-// One instantiation of the kernel per layout: up to four activation rows, up to eight, and more.
+// Instantiations by rows: up to four, eight and sixteen; of each, by layout and for clusters beyond the portable size.
 struct Variant {
-    const void *kn, *nk;
-    int rows, smem;
+    const void *kernel[2][2];  // [weight_nk][cluster > kPortableCluster]
+    int rows, smem, ctas;
 };
 template <int MT, bool QUAD>
 static Variant make_variant() {
-    return {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false, QUAD>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD>),
-            Config<MT>::ROWS, Config<MT>::SMEM_BYTES};
+    return {{{reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false, QUAD, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, false, QUAD, true>)},
+             {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD, true>)}},
+            Config<MT>::ROWS, Config<MT>::SMEM_BYTES, Config<MT>::CTAS};
 }
 constexpr int kVariantCount = 3;
 static const Variant kVariants[kVariantCount] = {make_variant<1, false>(), make_variant<1, true>(), make_variant<2, true>()};
-static const Variant &variant(int64_t M) { return kVariants[M <= 4 ? 0 : (M <= 8 ? 1 : 2)]; }
-
 static int set_attributes() {
     static std::atomic<bool> attr_set[64];  // per device, zero-initialised; a repeated set by a racing thread is harmless
     int dev = 0;
     B200Q_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
         for (const Variant &v : kVariants)
-            for (const void *f : {v.kn, v.nk}) B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+            for (int i = 0; i < 4; ++i) {
+                const void *f = v.kernel[i >> 1][i & 1];
+                B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+                if (i & 1) B200Q_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            }
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
     return B200Q_OK;
 }
 
 // CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use.  Looked up once
-// per device; without a device, an estimate.
+// per device; without a device, an estimate (none of clusters that not every device runs: the plan does without them).
 static int resident_ctas(const Variant &v, int cluster) {
     static std::atomic<int> known[64][kVariantCount][kMaxCluster + 1];
+    const int estimate = cluster <= kPortableCluster ? (148 - 8) * v.ctas : 0;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || set_attributes() != B200Q_OK) {
         cudaGetLastError();
-        return 148 * 4 - 30;
+        return estimate;
     }
     std::atomic<int> &slot = known[dev][&v - kVariants][cluster];
     int n = slot.load(std::memory_order_relaxed);
     if (n != 0) return n;
-    n = resident_clusters(v.kn, THREADS, v.smem, cluster);
-    if (n == 0) return 148 * 4 - 30;
+    n = resident_clusters(v.kernel[0][cluster > kPortableCluster], THREADS, v.smem, cluster);
+    if (n == 0) return estimate;
     n *= cluster;
     slot.store(n, std::memory_order_relaxed);
     return n;
@@ -643,23 +655,30 @@ static int resident_ctas(const Variant &v, int cluster) {
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     using namespace decode;
     DecodePlan pl;
-    const Variant &v = variant(M);
     pl.n_tiles = (int)ceil_div(N, BN);
-    pl.m_tiles = (int)ceil_div(M, v.rows);
     const int k_iters = (int)ceil_div(K, BK);
     int sms = sm_count();
     if (sms <= 0) sms = 148;
+    // What every device can run: blocks of up to 16 rows, clusters of up to eight CTAs.  The scratch that callers are asked for is this
+    // plan's, whether the one below it that is launched needs any or not.
+    const Variant &v = kVariants[M <= 4 ? 0 : (M <= 8 ? 1 : 2)];
+    pl.variant = (int)(&v - kVariants);
+    pl.m_tiles = (int)ceil_div(M, v.rows);
     const int64_t tiles = (int64_t)pl.n_tiles * pl.m_tiles;
     // Each split has at least four 64-row steps of work, a ring's fill: with eight a narrow problem leaves most of the SMs
-    // idle (a step of a 1024-wide decoder 72 -> 57 us), with two the exchange costs what the shorter loop gives (64 us).
-    const int max_splits = k_iters / 4 > 0 ? k_iters / 4 : 1;
+    // idle (a step of a 1024-wide decoder 72 -> 57 us), with two the exchange costs what the shorter loop gives (64 us).  Only where
+    // that leaves fewer than four splits are two steps enough, for the last phase's sake: one CTA alone finishes 16 rows of 128
+    // columns in several rounds ((16, 256, 688) 4.2 -> 3.0 us, (1, 256, 688) 2.75 -> 2.15, (16, 640, 2048) 3.8 -> 2.8), and where the grid has
+    // the room ((16, 512, 16384) 4.5 -> 4.8).
+    int max_splits = k_iters >= 4 ? k_iters / 4 : 1;
+    if (max_splits < 4 && k_iters >= 4) max_splits = k_iters < 8 ? (tiles * 4 <= 2 * sms ? k_iters / 2 : 2) : (tiles * 4 <= 2 * sms ? 4 : max_splits);
     // The splits of a tile form a cluster of up to eight CTAs (partials meet in distributed shared memory), as large as lets
     // the whole grid run at once: a few clusters left for a second wave double the time of the launch (96 tiles
     // in clusters of six are 576 CTAs and fit 148 x 4 slots by number, but not the groups of SMs clusters are confined to:
     // (1, 4096, 12288) 15.1 us, and 10.3 us in clusters of five).
     int c = 1;
     // (With several row blocks the second pass over the weight comes from L2 and a second wave costs little.)
-    while (c < kMaxCluster && c < max_splits && tiles * (c + 1) <= (pl.m_tiles > 1 ? (int64_t)sms * 4 : resident_ctas(v, c + 1))) ++c;
+    while (c < kPortableCluster && c < max_splits && tiles * (c + 1) <= (pl.m_tiles > 1 ? (int64_t)sms * v.ctas : resident_ctas(v, c + 1))) ++c;
     // More splits than a cluster holds become several full clusters per tile that meet in the workspace.  They pay three
     // dependent trips through L2 at the end of the launch (publish, count, read back), about 3 us more than partials
     // that meet in distributed shared memory.  That is worth it only when one cluster per tile would leave most of the
@@ -667,21 +686,35 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // (1, 8192, 1024) 6.5 against 6.3, though (1, 8192, 256) gains, 4.8 against 5.7.  (It is also what the scratch is sized by: with
     // four the partial sums of (16, 11008, 1024) would not fit the array of b200q_qlinear_f16_i8_static any more.)
     int groups = 1;
-    if (c == kMaxCluster && tiles * c * 2 < sms) {
+    if (c == kPortableCluster && tiles * c * 2 < sms) {
         int64_t splits = tiles > 0 ? (int64_t)sms * 4 / tiles : 1;
         if (splits > k_iters / 8) splits = k_iters / 8;
         if (splits > 64) splits = 64;
         groups = (int)(splits / c);
         if (groups < 1 || tiles * c > kMaxCounters) groups = 1;
     }
-    pl.cluster = c;
-    pl.groups = groups;
-    pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
-    pl.iters_per_split = (int)ceil_div(k_iters, pl.splits);
     // The counter region has one fixed size, so that counters never land on bytes an earlier call of
     // another shape used for partial sums: the region stays all-zero between calls.
     pl.counter_bytes = groups > 1 ? (size_t)kMaxCounters * 4 : 0;
     pl.partial_bytes = groups > 1 ? (size_t)groups * M * N * 4 : 0;
+    // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
+    // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
+    // takes as long as its chain of waits and loads, not as its bytes ((1, 11008, 4096), 256 CTAs of 22 steps, 11.4 us; 448 of 13, 10.1;
+    // (16, 11008, 4096) 12.9 -> 12.0).  Short runs in many parts lose more in the exchange, which grows with the rows: (1, 4096, 4096) 5.0 -> 5.8
+    // in sixteen parts of four steps, (16, 5376, 2304) 6.1 -> 6.4.
+    if (pl.m_tiles == 1 && c == kPortableCluster && k_iters >= 48) {
+        const int portable = pl.n_tiles * c;
+        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * c;
+        for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
+            if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[pl.variant], wide)) continue;
+            c = wide, groups = 1;
+            break;
+        }
+    }
+    pl.cluster = c;
+    pl.groups = groups;
+    pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
+    pl.iters_per_split = (int)ceil_div(k_iters, pl.splits);
     return pl;
 }
 
@@ -735,7 +768,7 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     }
     if (epilogue != nullptr) p.ep = *epilogue;
     p.counters = static_cast<unsigned int *>(workspace);
-    p.partial = pl.partial_bytes > 0 ? reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + pl.counter_bytes) : nullptr;
+    p.partial = pl.groups > 1 ? reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + pl.counter_bytes) : nullptr;
     p.status = device_status_word();
     p.M = (int)M;
     p.N = (int)N;
@@ -743,11 +776,11 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     p.k_end = (int)k_end;
     p.iters_per_split = pl.iters_per_split;
     p.groups = pl.groups;
-    p.cols_per = (int)round_up(ceil_div(BN, pl.cluster), 8);
+    p.cols_per = (int)round_up(ceil_div(BN, pl.cluster), pl.cluster <= kPortableCluster ? 8 : 4);
     p.mode = pl.splits == 1 ? kModeDirect : kModeSplit;
 
-    const Variant &v = variant(M);
-    const void *kernel = weight_nk ? v.nk : v.kn;
+    const Variant &v = kVariants[pl.variant];
+    const void *kernel = v.kernel[weight_nk][pl.cluster > kPortableCluster];
     const int rc_attr = set_attributes();
     if (rc_attr != B200Q_OK) return rc_attr;
     cudaLaunchConfig_t cfg = {};

@@ -71,6 +71,7 @@ def large_kernels(nvcc_library):
     lib = nvcc_library('large_kernels.cu', '-std=c++17', '-Xcompiler', '-fvisibility=hidden', '--threads', '0', *sources)
     p, i, n = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
     lib.plan.argtypes, lib.plan.restype = [n, n, n, i, p], None
+    lib.small_plan.argtypes, lib.small_plan.restype = [n, n, n, p], None
     lib.launch.argtypes = [i, i, i, p, p, p, p, i, n, n, n, n, n, n, i, p, p, n, i, p]
     lib.launch_one_sm.argtypes = [p, p, p, p, i, n, n, n, n, n, p, ctypes.c_size_t, p]
     return lib

@@ -22,6 +22,12 @@ EXPORT void plan(int64_t M, int64_t N, int64_t K, int silu, int *out) {
     out[0] = p.kind, out[1] = p.tm, out[2] = p.cluster;
 }
 
+// out: rows per pass of the small-M kernel's plan, CTAs per cluster, clusters per tile
+EXPORT void small_plan(int64_t M, int64_t N, int64_t K, int *out) {
+    const DecodePlan p = plan_decode(M, N, K);
+    out[0] = (int)((M + p.m_tiles - 1) / p.m_tiles), out[1] = p.cluster, out[2] = p.groups;
+}
+
 EXPORT int launch(int kind, int tm, int cluster, const void *a, const void *wq, const void *scale, void *const *dst, int count, int64_t ldc, int64_t col0, int64_t M, int64_t N,
                   int64_t K, int64_t lda, int nk, const void *bias, const void *residual, int64_t ldr, int silu, cudaStream_t stream) {
     LargePlan p;

@@ -1,4 +1,4 @@
-"""The small-M kernel's last step, four columns a thread: counts and addresses that are not multiples of four."""
+"""The small-M kernel: its last step (four columns a thread, counts and addresses that are not multiples of four) and its splits."""
 import ctypes
 
 import pytest
@@ -66,3 +66,30 @@ def test_operands_of_the_epilogue_at_any_element(m, k, offset, ldr):
     ffi.func('b200q_qlinear_f16_i8_fused')(a.data_ptr(), wq.data_ptr(), keep[0][1], out.data_ptr(), m, n, k, 0, ctypes.byref(ep), ws_ptr, ws_size,
                                           torch.cuda.current_stream().cuda_stream)
     _close(out, want + bias.double() + residual[:, :n].double())
+
+
+def _plan(large_kernels, m, k, n):
+    out = (ctypes.c_int * 3)()
+    large_kernels.small_plan(m, n, k, out)
+    return tuple(out)
+
+
+# clusters beyond eight CTAs: nine to sixteen with slices of every width, splits that get fewer steps than others or none, a last step that is
+# cut short, tiles that are; short K in two to four splits
+@pytest.mark.parametrize('m', [1, 2, 3, 8, 9, 16, 17, 24])
+@pytest.mark.parametrize('k,n', [(3072, 16), (3080, 272), (4096, 1024), (4104, 16), (11008, 4096), (11024, 3328), (12288, 4592), (16376, 512), (9000, 5120)])
+def test_wide_clusters(large_kernels, m, k, n):
+    assert _plan(large_kernels, m, k, n)[1] > 8 or m > 16 or (m > 8 and n > 1536)
+    a, wq, scale, want = _operands(m, k, n, 'KN')
+    _close(hidet_b200.symmetric_quant_matmul(a, wq, scale), want)
+    if k % 16 == 0:
+        a, wq, scale, want = _operands(m, k, n + 1, 'NK')
+        _close(hidet_b200.symmetric_quant_matmul(a, wq, scale, weight_layout='NK'), want)
+
+
+@pytest.mark.parametrize('m', [1, 4, 7, 16])
+@pytest.mark.parametrize('k,n,splits', [(192, 272, 1), (200, 272, 2), (256, 688, 2), (328, 2048, 3), (512, 16, 4), (1016, 1040, 4), (256, 12288, 2), (512, 16384, 2)])
+def test_short_splits(large_kernels, m, k, n, splits):
+    assert _plan(large_kernels, m, k, n)[1] == splits
+    a, wq, scale, want = _operands(m, k, n, 'KN')
+    _close(hidet_b200.symmetric_quant_matmul(a, wq, scale), want)
