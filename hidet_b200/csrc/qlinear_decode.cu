@@ -7,7 +7,7 @@
 // fetches its slice with transposing matrix loads (four consecutive k of one column per register),
 // turns the bytes into exact f16 pairs in registers and feeds warp-level m16n8k16 tensor-core MMAs
 // with fp32 accumulators; the weight is the MMA's 16-row operand and the activations its 8-column operand, so up to 8 activation rows
-// cost one MMA per 16 x 16 weight block, up to 16 rows two (rows beyond M are zero-filled).
+// cost one MMA per 16 x 16 weight block, up to 16 rows two and up to 24 three (rows beyond M are zero-filled).
 //
 // K is split across CTAs to fill the machine.  Up to 16 splits of one output tile form a thread-block
 // cluster: every CTA sends its partial tile into the shared memory of the CTA that owns those columns
@@ -46,7 +46,7 @@ constexpr int STAGING_ROW = 36;              // floats per row of a warp's 32-co
 template <int MT>
 struct Config {
     static constexpr int ROWS = 8 * MT;                  // activation rows per CTA
-    static constexpr int CTAS = 4;                       // that share an SM
+    static constexpr int CTAS = MT <= 2 ? 4 : 3;         // that share an SM
     static constexpr int A_STAGE_BYTES = ROWS * BK * 2;
     static constexpr int PIPE_BYTES = STAGES * (W_STAGE_BYTES + A_STAGE_BYTES);
     static constexpr int RECV_BYTES = ROWS * RECV_COLS * 4;  // partial tiles sent by the CTAs of the cluster: [rank][row][cols_per] fp32
@@ -193,12 +193,15 @@ struct Params {
 //     four rows; with fewer one element per thread is one round anyway: (4, 9648, 1568) 7.9 us, 8.05 so).
 // WIDE: clusters beyond the portable size (the eight partials that a smaller one sums at once stay one piece of code without a loop:
 //     (16, 4096, 12288) 12.0 us, 12.4 with it).
-// Shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
+// With 24 rows three CTAs share an SM, and the weight is not asked for ahead of the kernel in front but only fetched into L2 (EARLY): these
+// calls were mostly served by a kernel that waits, and their codes may be that kernel's results ((24, 4096, 4096) 7.6 us with, 8.1 without).
+// Otherwise shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
 // bytes in one form): a decode step at 7B widths for one sequence 216 -> 209 us, for sixteen 256 -> 252.
 template <int MT, bool NK, bool QUAD, bool WIDE>
 __global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
     using Cfg = Config<MT>;
     constexpr int ROWS = Cfg::ROWS, A_STAGE_BYTES = Cfg::A_STAGE_BYTES, PIPE_BYTES = Cfg::PIPE_BYTES, MAX_RANKS = WIDE ? kMaxCluster : kPortableCluster;
+    constexpr bool EARLY = MT <= 2;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t full_bar[STAGES];
     __shared__ __align__(8) uint64_t empty_bar[STAGES];
@@ -309,10 +312,17 @@ __global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_k
             stream_policy = l2_policy_evict_first();  // the weight is read once
             // The weight does not depend on the kernel before this one in the stream; the activations
             // may.  Ask for the first weight tiles, then wait for that kernel, then ask for activations.
-            for (int it = 0; it < prologue; ++it) load_weights(it, it, stream_policy);
+            for (int it = 0; it < prologue; ++it) {
+                if (EARLY) load_weights(it, it, stream_policy);
+                else tma_prefetch_2d(&map_w, NK ? p.k_begin + (it_begin + it) * BK : n0, NK ? n0 : p.k_begin + (it_begin + it) * BK);
+            }
         }
         __syncwarp();
         pdl_wait();
+        if (!EARLY && lane == 0) {
+            for (int it = 0; it < prologue; ++it) load_weights(it, it, stream_policy);
+        }
+        __syncwarp();
         // The kernel in front is done; the one behind may move in now: its CTAs fill their rings while this launch streams
         // the rest of its weight, so that it starts with its first stages in shared memory.  Two launches at a time is as
         // far ahead as pays: allowed at the very start, its successors pile up and all their rings compete with this one's
@@ -600,7 +610,7 @@ __global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_k
 
 namespace decode {
 
-// Instantiations by rows: up to four, eight and sixteen; of each, by layout and for clusters beyond the portable size.
+// Instantiations by rows: up to four, eight, sixteen and twenty-four; of each, by layout and for clusters beyond the portable size.
 struct Variant {
     const void *kernel[2][2];  // [weight_nk][cluster > kPortableCluster]
     int rows, smem, ctas;
@@ -611,8 +621,8 @@ static Variant make_variant() {
              {reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD, false>), reinterpret_cast<const void *>(qlinear_decode_kn_kernel<MT, true, QUAD, true>)}},
             Config<MT>::ROWS, Config<MT>::SMEM_BYTES, Config<MT>::CTAS};
 }
-constexpr int kVariantCount = 3;
-static const Variant kVariants[kVariantCount] = {make_variant<1, false>(), make_variant<1, true>(), make_variant<2, true>()};
+constexpr int kVariantCount = 4;
+static const Variant kVariants[kVariantCount] = {make_variant<1, false>(), make_variant<1, true>(), make_variant<2, true>(), make_variant<3, true>()};
 static int set_attributes() {
     static std::atomic<bool> attr_set[64];  // per device, zero-initialised; a repeated set by a racing thread is harmless
     int dev = 0;
@@ -697,6 +707,17 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // another shape used for partial sums: the region stays all-zero between calls.
     pl.counter_bytes = groups > 1 ? (size_t)kMaxCounters * 4 : 0;
     pl.partial_bytes = groups > 1 ? (size_t)groups * M * N * 4 : 0;
+    // Up to 24 rows in one pass where the weight is more than what L2 delivers again for nothing: (24, 4096, 4096) 8.5 -> 8.2 us, (24, 4096, 12288)
+    // 23.0 -> 14.5, (17, 2304, 6912) 8.3 -> 7.3 against two passes of 16 rows; below the line the passes run side by side ((24, 2048, 2048)
+    // 4.0 us, 4.4 in one).  A form for 32 rows was no better than two passes or the mid-M kernel ((32, 4096, 4096) 8.8 and 8.5 us, (32, 4096,
+    // 12288) 16.1 and 17.7): the warp-level MMAs of four row blocks take longer than the stream.
+    if (M > 16 && M <= 24 && N * K >= (int64_t)6 * 1024 * 1024) {
+        const Variant &one = kVariants[3];
+        int wide = 1;
+        while (wide < kPortableCluster && wide < max_splits && pl.n_tiles * (wide + 1) <= resident_ctas(one, wide + 1)) ++wide;
+        pl.variant = 3, pl.m_tiles = 1;
+        c = wide, groups = 1;
+    }
     // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
     // takes as long as its chain of waits and loads, not as its bytes ((1, 11008, 4096), 256 CTAs of 22 steps, 11.4 us; 448 of 13, 10.1;

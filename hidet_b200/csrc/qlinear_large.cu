@@ -1,7 +1,8 @@
 // Which kernel serves a quantized linear of more than a few rows, and with what tiles.
 //
 // The choice is by estimated time, in microseconds; the constants are measured (B200, graph replay of weights that exceed L2) and
-// stand beside what they describe.  The small-M kernel stays for what it does better: up to 16 rows always.
+// stand beside what they describe.  The small-M kernel stays for what it does better: up to 24 rows always (24 rows, small-M against the
+// better of the others: (4096, 12288) 14.5 and 17.5 us, (4096, 22016) 24.8 and 29.8, (11008, 4096) 15.0 and 17.5, (1024, 1024) 3.1 and 5.2).
 #include "common.cuh"
 #include "qlinear.h"
 
@@ -63,12 +64,14 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
 
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu) {
     LargePlan p;
-    if (M <= 16) return p;
+    if (M <= 24) return p;
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
     const double mid = M <= 65535 * 128 ? mid_us(M, N, K, &mid_tm, &mid_cluster) : 1e30;  // the grid's limit
     const double pair = M > 32 ? pair_us(M, N, K, silu, &pair_tm) : 1e30;
     const double best = mid < pair ? mid : pair;
-    if (!use_prefill_kernel(M, N, K) && best > 0.85 * small_m_us(M, N, K)) return p;
+    // The estimates are within a tenth of each other's error, so nearly as good is good enough (a sixth was asked for before, and
+    // (32, 4096, 12288) took 23.4 us for 17.7, (32, 4096, 22016) 36.0 for 29.8, (48, 4096, 4096) 13.6 for 9.9).
+    if (!use_prefill_kernel(M, N, K) && best > 0.95 * small_m_us(M, N, K)) return p;
     p.kind = mid < pair ? LargePlan::kMid : LargePlan::kPair;
     p.tm = mid < pair ? mid_tm : pair_tm;
     p.cluster = mid_cluster;
@@ -84,7 +87,7 @@ int check_large_outputs(const OutTargets &out) {
 
 bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
                bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc) {
-    if (M <= 16 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
+    if (M <= 24 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
     const bool only = use_prefill_kernel(M, N, K);  // the small-M kernel is out of the question
     if (!only) {
         const DecodePlan dp = plan_decode(M, N, K);

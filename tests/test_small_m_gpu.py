@@ -93,3 +93,15 @@ def test_short_splits(large_kernels, m, k, n, splits):
     assert _plan(large_kernels, m, k, n)[1] == splits
     a, wq, scale, want = _operands(m, k, n, 'KN')
     _close(hidet_b200.symmetric_quant_matmul(a, wq, scale), want)
+
+
+@pytest.mark.parametrize('m', [17, 20, 23, 24, 25])
+@pytest.mark.parametrize('k,n', [(4096, 1536), (1000, 6304), (2048, 3072), (6264, 1024), (520, 16400)])
+def test_rows_up_to_24_in_one_pass(large_kernels, m, k, n):
+    if k * n >= 6 * 1024 * 1024:
+        assert (_plan(large_kernels, m, k, n)[0] == m) == (m <= 24)
+    a, wq, scale, want = _operands(m, k, n, 'KN')
+    _close(hidet_b200.symmetric_quant_matmul(a, wq, scale), want)
+    gate = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+    residual = torch.randn(m, n // 2, device='cuda').half()
+    _close(hidet_b200.symmetric_quant_matmul(a, wq, scale, activation='silu_mul', residual=residual), gate + residual.double())
