@@ -163,10 +163,12 @@ __global__ void qlinear_u4_reduce_kernel(const float *partial, __half *c, int64_
 // the warp's run; a part of a group is a term like any other)
 //     sum += scale * (group sum - zero * activation sum)
 // goes to the lane's own place in shared memory, where the warps, and then the cluster, are summed in a fixed order.
-// What is left is not bytes: at (1, 4096, 12288) the schedulers issue in 10 300 of 25 000 clocks (mostly unpacking), and four warps each,
-// in chains of short dependent steps, do not hide the latency between; then the exchange at the end.
-// Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 13.2 us, (8, 4096, 4096) 28.7 ->
-// 6.6; (16, 12288, 4096) 127 (a call) -> 16.5, (64, 4096, 11008) 43.6.
+// What is left is not bytes: at (1, 4096, 12288) the schedulers issue in 10 300 of 25 000 clocks (mostly unpacking; an eighth fewer since the
+// constants are kept in registers), and four warps each, in chains of short dependent steps, do not hide the latency between; then the
+// exchange at the end.  (Built like the small-M int8 kernel, with a TMA producer and transposing matrix loads of bytes, it takes
+// 11.2 us there for 11.6, 6.4 for 6.0 at (1, 4096, 4096), and 16.3 for 11.7 where rows are not multiples of 16 bytes.)
+// Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 11.6 us, (8, 4096, 4096) 28.7 ->
+// 6.1; (16, 12288, 4096) 127 (a call) -> 16.0, (64, 4096, 11008) 42.
 struct MmaParams {
     const __half *a;        // [M, K]
     const uint32_t *q;      // [K, N / 8] words
@@ -187,7 +189,7 @@ struct MmaConfig {
     static constexpr int ITEMS = TILES * MT * 32;                       // float4 sums of a CTA
     static constexpr int RED_BYTES = MMA_WARPS * ITEMS * 16;
     static constexpr int RING_OFF = RED_BYTES + stream_mma::recv_bytes(ITEMS);
-    static constexpr int CTAS = MT == 4 ? 3 : 4;                        // per SM
+    static constexpr int CTAS = MT * MT * W > 4 ? 3 : 4;                // per SM
     // Steps in flight.  Short rings are enough, and let the clusters fit better (measured while codes were copied ahead of the
     // wait, 0.4 us less than now): (1, 4096, 12288) takes 12.7 us with four
     // CTAs of three steps, 15.5 with four of seven; (16, 12288, 4096) 15.9 with three and 19.3 with eight.
@@ -200,12 +202,27 @@ struct MmaConfig {
 // Codes 0 .. 3 of two rows as f16 pairs (row 0, row 1): x holds the rows' 16-bit pieces.  0x6400 | c is 1024 + c, and with
 // the code four bits up 1024 + 16 c, of which a sixteenth less 64 is c; both exact.  (The bare bits as subnormal numbers take
 // half the instructions, but the tensor core aligns products by the operands' unnormalised exponents and the sums lose bits.)
-__device__ __forceinline__ void unpack_pairs(uint32_t x, uint32_t (&h)[4]) {
+// The constants are kept in registers, where the compiler cannot see them: a logical operation takes one immediate, so that
+// with two constants in place (x & mask) | bias becomes two operations: 65 instructions for four words, 50 so; (1, 4096, 12288)
+// 13.3 -> 12.3 us, (8, 4096, 4096) 6.6 -> 6.1.
+struct UnpackConstants {
+    uint32_t lower, upper, bias, sixteenth, minus64;
+    __device__ __forceinline__ UnpackConstants() {
+        asm volatile("mov.b32 %0, 0x000f000f;" : "=r"(lower));
+        asm volatile("mov.b32 %0, 0x00f000f0;" : "=r"(upper));
+        asm volatile("mov.b32 %0, 0x64006400;" : "=r"(bias));
+        asm volatile("mov.b32 %0, 0x2c002c00;" : "=r"(sixteenth));
+        asm volatile("mov.b32 %0, 0xd400d400;" : "=r"(minus64));
+    }
+};
+__device__ __forceinline__ void unpack_pairs(uint32_t x, uint32_t (&h)[4], const UnpackConstants &k) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const uint32_t lo = ((x >> (8 * i)) & 0x000f000fu) | 0x64006400u, hi = ((x >> (8 * i)) & 0x00f000f0u) | 0x64006400u;
-        asm("sub.f16x2 %0, %1, %2;" : "=r"(h[2 * i]) : "r"(lo), "r"(0x64006400u));
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(h[2 * i + 1]) : "r"(hi), "r"(0x2c002c00u), "r"(0xd400d400u));
+        uint32_t lo, hi;  // (x & mask) | bias
+        asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(lo) : "r"(x >> (8 * i)), "r"(k.lower), "r"(k.bias));
+        asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(hi) : "r"(x >> (8 * i)), "r"(k.upper), "r"(k.bias));
+        asm("sub.f16x2 %0, %1, %2;" : "=r"(h[2 * i]) : "r"(lo), "r"(k.bias));
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(h[2 * i + 1]) : "r"(hi), "r"(k.sixteenth), "r"(k.minus64));
     }
 }
 
@@ -233,7 +250,7 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
     const int share = steps / workers, extra = steps % workers;
     const int s_begin = worker * share + min(worker, extra), s_end = s_begin + share + (worker < extra ? 1 : 0);
 
-    // Words beyond the row and rows beyond M repeat the last ones: their columns and rows of the result are not stored.
+    // Words beyond the row repeat the last ones: their columns of the result are not stored.  Rows beyond M are zeros.
     bool in[W];
     const uint32_t *q_src[4][W];  // the words of the next step to fetch
 #pragma unroll
@@ -246,8 +263,14 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
     // may be older than the kernel that wrote them, and so may be what the first-level cache holds).
     constexpr int A_COPIES = (MT + 1) / 2;
     const __half *a_src[A_COPIES];
+    int a_size[A_COPIES];  // bytes to copy, the rest of the 16 is zeros (rows beyond M used to repeat the last one, whose lines every CTA then asked
+                           // for many times over: (24, 4096, 12288) 33 -> 22 us, (9, 4096, 4096) 9.9 -> 7.5, (1, 4096, 12288) 12.3 -> 11.6)
 #pragma unroll
-    for (int i = 0; i < A_COPIES; ++i) a_src[i] = p.a + (size_t)min(m0 + 16 * i + (lane >> 1), p.M - 1) * p.K + s_begin * 16 + 8 * (lane & 1);
+    for (int i = 0; i < A_COPIES; ++i) {
+        const int row = m0 + 16 * i + (lane >> 1);
+        a_size[i] = row < p.M ? 16 : 0;
+        a_src[i] = p.a + (size_t)min(row, p.M - 1) * p.K + s_begin * 16 + 8 * (lane & 1);
+    }
     const uint32_t ring = smem_u32(smem) + Cfg::RING_OFF + (uint32_t)warp * DEPTH * Cfg::SLOT_BYTES + lane * 4 * W;
     const uint32_t ring_a = smem_u32(smem) + Cfg::RING_OFF + (uint32_t)warp * DEPTH * Cfg::SLOT_BYTES + 4 * W * 4 * 32;
     const size_t step_words = (size_t)16 * words_per_row;
@@ -263,7 +286,7 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
     auto fetch_activations = [&](uint32_t slot) {
 #pragma unroll
         for (int i = 0; i < A_COPIES; ++i) {
-            if (MT > 1 || lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_a + slot + (i * 32 + lane) * 16), "l"(a_src[i]) : "memory");
+            if (MT > 1 || lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring_a + slot + (i * 32 + lane) * 16), "l"(a_src[i]), "r"(a_size[i]) : "memory");
             a_src[i] += 16;
         }
     };
@@ -311,6 +334,10 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
         first = false;
     };
 
+    const UnpackConstants constants;
+    uint32_t ones[4];  // a register each, as above: otherwise the four are put in place again for every MMA
+#pragma unroll
+    for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, 0x3c003c00;" : "=r"(ones[i]));
     clear();
     int group = s_begin / p.steps_per_group;
     int left = (group + 1) * p.steps_per_group - s_begin;  // steps to the end of the group
@@ -355,17 +382,16 @@ __global__ void __launch_bounds__(MMA_THREADS, MmaConfig<MT, W>::CTAS) qlinear_u
             for (int half = 0; half < 2; ++half) {
                 const uint32_t sel = half == 0 ? 0x5410u : 0x7632u;
                 uint32_t h01[4], h23[4];
-                unpack_pairs(__byte_perm(w[0][i], w[1][i], sel), h01);
-                unpack_pairs(__byte_perm(w[2][i], w[3][i], sel), h23);
+                unpack_pairs(__byte_perm(w[0][i], w[1][i], sel), h01, constants);
+                unpack_pairs(__byte_perm(w[2][i], w[3][i], sel), h23, constants);
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj)
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
                         mma_m16n8k16(acc[4 * i + 2 * half + jj][mt], h01[2 * jj], h01[2 * jj + 1], h23[2 * jj], h23[2 * jj + 1], b[mt].x, b[mt].y);
             }
-        const uint32_t ones = 0x3c003c00u;
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) mma_m16n8k16(asum[mt], ones, ones, ones, ones, b[mt].x, b[mt].y);
+        for (int mt = 0; mt < MT; ++mt) mma_m16n8k16(asum[mt], ones[0], ones[1], ones[2], ones[3], b[mt].x, b[mt].y);
         __syncwarp();
         if (step + DEPTH < s_end) {  // into the place just read
             fetch_codes(slot);
@@ -521,12 +547,15 @@ B200Q_API int b200q_qlinear_f16_u4(const void *a, const void *q, const void *sca
         mp.K = (int)K;
         mp.steps_per_group = (int)(group_size / 16);
         // Wider column strips while one block of rows is enough (64 contiguous bytes of a row: (1, 4096, 12288) 13 us
-        // against 20 with 32), except where they leave too few CTAs ((1, 12288, 256) 7.0 us wide, 5.7 narrow); narrow ones
-        // beyond, where the accumulators of several row blocks take the registers ((16, 4096, 4096) 12.7 us wide, 9.3 narrow).
+        // against 20 with 32), except where they leave too few CTAs ((1, 12288, 256) 7.0 us wide, 5.7 narrow).  With two blocks they
+        // take a CTA off the SM for the accumulators' registers: wide where columns abound and K is long enough ((16, 4096, 12288) 19.6 -> 13.3,
+        // (9, 4096, 8192) 12.4 -> 10.6, (16, 2432, 7040) 8.7 -> 7.8; (16, 1024, 8192) 5.8 -> 6.2, (16, 4096, 4096) 8.1 -> 8.3,
+        // (16, 12288, 4096) 16.1 -> 17.4); narrow with four, where two CTAs an SM are left ((24, 4096, 12288) 22.2 and 24.3).
+        const bool whole = N % 16 == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;  // rows of 8-byte pieces
         if (M > 16) return u4::launch_mma<4, 1, true>(mp, s);
-        if (M > 8) return u4::launch_mma<2, 1, true>(mp, s);
+        if (M > 8) return N >= 6144 && K >= 2048 && whole ? u4::launch_mma<2, 2, true>(mp, s) : u4::launch_mma<2, 1, true>(mp, s);
         if (N <= 1024) return u4::launch_mma<1, 1, true>(mp, s);
-        return N % 16 == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0 ? u4::launch_mma<1, 2, true>(mp, s) : u4::launch_mma<1, 2, false>(mp, s);
+        return whole ? u4::launch_mma<1, 2, true>(mp, s) : u4::launch_mma<1, 2, false>(mp, s);
     }
     u4::Plan pl = u4::plan(M, N, K, group_size);
     // Operands the tensor-core kernel cannot take (an unaligned a or c) with its amount of scratch: one split.

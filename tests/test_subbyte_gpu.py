@@ -110,6 +110,21 @@ def test_quant_linear_on_operands_off_their_boundaries(m, n, k, gsize):
         assert not ws[:65536 * 4].any()
 
 
+# rows short of a block of 8, 16 and 32 (the copies of the others bring zeros), column strips of both widths, their last columns, short last groups
+@pytest.mark.parametrize('m', [2, 7, 9, 15, 16, 17, 31])
+@pytest.mark.parametrize('k,n,gsize', [(2048, 6144, 128), (2064, 6160, 48), (2080, 6152, 32), (2048, 6136, 64), (512, 6144, 64), (1024, 200, 256)])
+def test_quant_linear_rows_short_of_a_block(m, n, k, gsize):
+    gen = torch.Generator(device='cuda').manual_seed(m + n + k)
+    a = torch.randint(-2, 3, (m, k), device='cuda', generator=gen).half()
+    codes = torch.randint(0, 16, (k, n), device='cuda', generator=gen).half()
+    scale = torch.randint(1, 3, (k // gsize, n), device='cuda', generator=gen).half() / 64
+    zeros = torch.randint(0, 16, (k // gsize, n), device='cuda', generator=gen).half()
+    w = (codes.double().view(k // gsize, gsize, n) - zeros.double().view(k // gsize, 1, n)) * scale.double().view(k // gsize, 1, n)
+    got = w4a16_linear('w4a16', k, n, gsize)(a, cast_f16_to_u4(codes), scale, zeros)
+    assert torch.equal(got, (a.double() @ w.view(k, n)).half())  # sums that are exact in any order
+    assert ffi.func('b200q_check_status')() == ffi.OK
+
+
 def test_quant_linear_argument_errors():
     f = ffi.func('b200q_qlinear_f16_u4')
     with pytest.raises(ffi.BackendException, match='multiple of the group size'):
