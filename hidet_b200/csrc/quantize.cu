@@ -681,6 +681,8 @@ __global__ void __launch_bounds__(kThreads) embedding_dequant_kernel(const Q *__
 
 // Largest dynamic shared memory a quantize_cols CTA may ask for (the static arrays need a little).
 constexpr size_t kMaxTileBytes = 200 * 1024;
+// What it may ask for by default: 48 KB with the static arrays, a few KB of them.
+constexpr size_t kDefaultTileBytes = 40 * 1024;
 
 // Threads across a panel row when a thread moves a 16-byte vector: 4 make a panel of 64 bytes per row (32 f16
 // columns), so that a [4096, 4096] weight gives 1024 CTAs of 32 KB, several to an SM and more than one wave.
@@ -705,7 +707,7 @@ int launch_quantize_cols(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols
         tile_bytes = 0;
     }
     auto kernel = quantize_cols_kernel<T, Q, VEC, TX>;
-    if (tile_bytes > 48 * 1024) {
+    if (tile_bytes > kDefaultTileBytes) {
         B200Q_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxTileBytes));
     }
     cudaLaunchConfig_t cfg = {};

@@ -248,3 +248,18 @@ def test_quantize_bf16_bits(rows, cols):
         quotient = (finite.float() / want_s.float().unsqueeze(dims)).to(torch.bfloat16)
         inside = quotient.float().abs() <= 127   # (a scale rounded down leaves quotients of 127.5: what the conversion makes of 128 is compared above)
         assert torch.equal(q.cpu()[inside], quotient.float().round().to(torch.int8)[inside])
+
+
+def test_slices_that_fill_the_default_shared_memory():
+    """Slices of a panel between 47 and 48 KB, with the static arrays above what a launch gets unasked: in a process of its own, where no
+    larger slice has asked for more."""
+    import os
+    import subprocess
+    import sys
+
+    code = ("import torch, hidet_b200\n"
+            "w = torch.randn(6144, 64, device='cuda').half()\n"
+            "wq, scale = hidet_b200.symmetric_quantize(w, 'int8', dims=0)\n"
+            "rows = [hidet_b200.symmetric_quantize(w.t().contiguous(), 'int8', dims=-1)]\n"
+            "assert torch.equal(wq, rows[0][0].t()) and torch.equal(scale, rows[0][1])\n")
+    subprocess.run([sys.executable, '-c', code], check=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
