@@ -539,14 +539,14 @@ __global__ void __launch_bounds__(kThreads) quantize_rows_kernel(const T *w, Q *
     }
 }
 
-// A warp per row, for rows of at most kWarpRowBytes: the row is brought into the warp's part of shared memory by
+// A warp per row, for rows of at most half of kRowCtaBytes: the row is brought into the warp's part of shared memory by
 // asynchronous 16-byte copies, all in flight at once, and both phases read it from there.  A lane reads back only
 // what it copied itself and the warps of a CTA share nothing, so there is no barrier; the reduction is one round
 // of warp shuffles instead of a CTA's.  grid = ceil(rows / W) CTAs of W <= kRowWarps warps (fewer for long rows, so
 // that a CTA's rows stay near kRowCtaBytes and several CTAs fit an SM).
 constexpr int kRowWarps = 4;
-constexpr size_t kWarpRowBytes = 48 * 1024;
-constexpr size_t kRowCtaBytes = 48 * 1024;
+constexpr size_t kRowCtaBytes = 48 * 1024 - 64;  // the kernels keep a few bytes statically
+constexpr size_t kLongRowBytes = 96 * 1024;       // two CTAs an SM
 
 template <typename T, typename Q, int VEC>
 __global__ void __launch_bounds__(kRowWarps * 32) quantize_rows_warp_kernel(const T *w, Q *wq,
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) quantize_rows_warp_kernel(cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
     if (row >= rows) return;
-    const int nvec = (int)(cols / VEC);       // cols % VEC == 0, and a row is at most kWarpRowBytes
+    const int nvec = (int)(cols / VEC);       // cols % VEC == 0, and a row is at most kRowCtaBytes
     T *mine = reinterpret_cast<T *>(smem_raw) + (size_t)warp * cols;
     const T *src = w + row * cols;
     Q *dst = wq + row * cols;
@@ -585,6 +585,95 @@ __global__ void __launch_bounds__(kRowWarps * 32) quantize_rows_warp_kernel(cons
         Vec<Q, VEC> q;
         QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(load_vec<T, VEC>(mine + (size_t)i * VEC), &s, q);
         store_vec<Q, VEC>(dst + (size_t)i * VEC, q);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// widths that are not multiples of a vector
+// ---------------------------------------------------------------------------------------------
+// A matrix without gaps between its rows is one run of elements, and runs are read and written in aligned vectors wherever the rows
+// begin.  A vector at the end of a row holds elements of the next one, which each kernel leaves out in its own way.  Element by element,
+// two bytes a load: 4147 x 8242 f16 per row 55.4 us, 31.8 so; 2024 x 3302 19.1 and 7.3; 2945 x 4447 restored with a scale per row 31.6 and
+// 11.7.  (Per column such a form, panels of seven vectors read as eight, gains nothing: 2024 x 3302 16.3 us for 14.5, 4147 x 8242 61.9 for 65.8.)
+
+// The bytes of a 16-byte piece that lie inside an array of `total` elements.
+template <typename T, int VEC>
+__device__ __forceinline__ int bytes_inside(int64_t first, int64_t total) {
+    const int64_t left = total - first;
+    return left >= VEC ? 16 : (left > 0 ? (int)(left * (int64_t)sizeof(T)) : 0);
+}
+__device__ __forceinline__ void copy_async_part(uint32_t dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ T nan_of();
+template <>
+__device__ __forceinline__ __half nan_of<__half>() { return __ushort_as_half(0x7fff); }
+template <>
+__device__ __forceinline__ __nv_bfloat16 nan_of<__nv_bfloat16>() { return __ushort_as_bfloat16(0x7fff); }
+template <>
+__device__ __forceinline__ float nan_of<float>() { return __uint_as_float(0x7fffffffu); }
+
+// quantize_rows_warp_kernel for any row length: a warp, or for long rows a CTA (LONG), copies the vectors that its row touches.  In the
+// first and the last one the neighbours' elements are NaN for the maximum, which skips it, and are not written.
+template <typename T, typename Q, int VEC, bool LONG>
+__global__ void __launch_bounds__(kRowWarps * 32) quantize_rows_flat_kernel(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols, int row_bytes) {
+    using A = Arith<T>;
+    constexpr int STEP = LONG ? kRowWarps * 32 : 32;  // threads per row
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ T part[kRowWarps];
+    pdl_wait();
+    const int of_cta = threadIdx.x / STEP, lane = threadIdx.x % STEP;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x / STEP) + of_cta;
+    if (row >= rows) return;
+    const int64_t begin = row * cols, first = begin / VEC * VEC;
+    const int head = (int)(begin - first), stop = head + (int)cols;  // the row's elements, counted from `first`
+    const int nvec = (stop + VEC - 1) / VEC;
+    T *mine = reinterpret_cast<T *>(smem_raw + (size_t)of_cta * row_bytes);
+    const uint32_t base = smem_u32(mine);
+    for (int i = lane; i < nvec; i += STEP) copy_async_part(base + i * 16, w + first + i * VEC, bytes_inside<T, VEC>(first + i * VEC, rows * cols));
+    copy_async_wait_all();
+    AbsMaxVec<T, VEC> acc;
+    acc.init();
+#pragma unroll 4
+    for (int i = lane; i < nvec; i += STEP) {
+        Vec<T, VEC> x = load_vec<T, VEC>(mine + i * VEC);
+        if (i == 0 || i == nvec - 1) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e)
+                if (i * VEC + e < head || i * VEC + e >= stop) x.v[e] = nan_of<T>();
+        }
+        acc.add(x);
+    }
+    T each[VEC];
+    acc.template finish<32>(each);
+    T m = A::lowest();
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) m = A::max_(m, each[e]);
+    m = warp_max<T>(m);
+    if (LONG) {
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+        __syncthreads();
+        m = A::lowest();
+#pragma unroll
+        for (int i = 0; i < kRowWarps; ++i) m = A::max_(m, part[i]);
+    }
+    const T s_val = A::div_(m, A::qmax(QMax<Q>::value));
+    if (lane == 0) scale[row] = s_val;
+    const typename A::Divisor s = A::prepare(s_val);
+    Q *dst = wq + first;
+#pragma unroll 4
+    for (int i = lane; i < nvec; i += STEP) {
+        const Vec<T, VEC> x = load_vec<T, VEC>(mine + i * VEC);
+        Vec<Q, VEC> q;
+        QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(x, &s, q);
+        if (i * VEC >= head && (i + 1) * VEC <= stop) {
+            store_vec<Q, VEC>(dst + i * VEC, q);
+        } else {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e)
+                if (i * VEC + e >= head && i * VEC + e < stop) dst[i * VEC + e] = q.v[e];
+        }
     }
 }
 
@@ -660,6 +749,52 @@ __global__ void __launch_bounds__(kThreads) dequantize_kernel(const Q *wq, const
                 Vec<T, VEC> out;
                 DequantVec<T, Q, VEC>::template run<false>(load_l2<Q, VEC>(src + i * sweep), &s, out);
                 store_vec<T, VEC>(dst + i * sweep, out);
+            }
+        }
+    }
+}
+
+// The same for any width of at least VEC: VEC rows together are whole vectors, so a thread takes the same vector of every group of
+// VEC rows; it holds elements of one row or of two, at the same columns in each group.  grid = (vectors of a group, groups / kDqGroups)
+// The scales of the columns go through shared memory: fetched by each thread for itself, two bytes at a time, they ask the same few lines of L2
+// too often (895 x 327 6.7 us, 4.1 element by element).
+constexpr int kDqGroups = 4;                      // per thread and trip
+template <typename T, typename Q, int VEC>
+__global__ void __launch_bounds__(kThreads) dequantize_flat_kernel(const Q *wq, const T *scale, T *w, int64_t rows, int64_t cols, int reduce_dim) {
+    __shared__ __align__(16) T col_scale[kThreads * VEC];
+    pdl_wait();
+    const int64_t v0 = (int64_t)blockIdx.x * kThreads, v = v0 + threadIdx.x;
+    if (reduce_dim == 0) {
+        const unsigned int width = (unsigned int)cols, c0 = (unsigned int)(v0 * VEC % cols);  // the launcher keeps cols below 2^31
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            const unsigned int at = threadIdx.x + i * kThreads;
+            col_scale[at] = load_l2<T, 1>(scale + (c0 + at) % width).v[0];
+        }
+        __syncthreads();
+    }
+    if (v >= cols) return;                        // a group is VEC * cols elements
+    const int64_t row = v * VEC / cols, col = v * VEC - row * cols;
+    const int here = cols - col < VEC ? (int)(cols - col) : VEC;  // elements in the first of the two rows
+    const int64_t total = rows * cols, groups = (rows + VEC - 1) / VEC;
+    Vec<T, VEC> s;
+    if (reduce_dim == 0) s = load_vec<T, VEC>(col_scale + threadIdx.x * VEC);
+    for (int64_t g0 = (int64_t)blockIdx.y * kDqGroups; g0 < groups; g0 += (int64_t)gridDim.y * kDqGroups) {
+#pragma unroll
+        for (int i = 0; i < kDqGroups; ++i) {
+            const int64_t r = (g0 + i) * VEC + row, at = ((g0 + i) * cols + v) * VEC;
+            if (r >= rows) break;
+            if (reduce_dim != 0) {
+                const T s0 = load_l2<T, 1>(scale + r).v[0], s1 = here < VEC && r + 1 < rows ? load_l2<T, 1>(scale + r + 1).v[0] : s0;
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) s.v[e] = e < here ? s0 : s1;
+            }
+            Vec<T, VEC> out;
+            if (at + VEC <= total) {
+                DequantVec<T, Q, VEC>::template run<true>(load_l2<Q, VEC>(wq + at), s.v, out);
+                store_vec<T, VEC>(w + at, out);
+            } else {                              // the end of the matrix
+                for (int e = 0; at + e < total; ++e) w[at + e] = Arith<T>::template dequant<Q>(load_l2<Q, 1>(wq + at + e).v[0], s.v[e]);
             }
         }
     }
@@ -758,15 +893,29 @@ int launch_quantize_cols(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols
     return launch_dependent("quantize_cols_kernel", kernel, dim3((unsigned)cluster, (unsigned)panels, 1), kThreads, tile_bytes, cluster, stream, w, wq, scale, rows, cols, rows_per_cta, cache);
 }
 
+// VEC: elements per vector where bases are aligned (16 bytes of w), else 1.
 template <typename T, typename Q, int VEC>
 int launch_quantize_rows(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols, cudaStream_t stream) {
     if (rows > 2147483647LL) return set_error(B200Q_UNSUPPORTED, "symmetric_quantize: %lld rows exceed the grid limit", (long long)rows);
-    if (VEC > 1 && (size_t)cols * sizeof(T) <= kWarpRowBytes) {
-        const size_t row_bytes = (size_t)cols * sizeof(T);
+    if constexpr (VEC > 1) {
+        const bool whole = cols % VEC == 0;   // rows are whole vectors
+        const size_t row_bytes = whole ? (size_t)cols * sizeof(T) : (size_t)(ceil_div(cols, VEC) + 1) * 16;
         int warps = (int)(kRowCtaBytes / row_bytes);
         warps = warps < 1 ? 1 : (warps > kRowWarps ? kRowWarps : warps);
-        const size_t smem = warps * row_bytes;  // at most kRowCtaBytes, the default limit for dynamic shared memory
-        return launch_dependent("quantize_rows_warp_kernel", quantize_rows_warp_kernel<T, Q, VEC>, dim3((unsigned)ceil_div(rows, warps)), warps * 32, smem, 1, stream, w, wq, scale, rows, cols);
+        const size_t smem = warps * row_bytes;  // at most kRowCtaBytes, with a few static bytes the default limit for shared memory
+        const dim3 grid((unsigned)ceil_div(rows, warps));
+        // A row of more than half of a CTA's share has the whole CTA (a warp has few loads in flight for it, and few warps fit an SM): 4096 x 12280
+        // f32 85 -> 63 us, 4147 x 8242 f32 53 -> 34, 4096 x 12288 f16 39 -> 28, 674 x 6912 f32 12.2 -> 7.6.
+        if (row_bytes > kRowCtaBytes / 2 && row_bytes <= kLongRowBytes) {
+            auto kernel = quantize_rows_flat_kernel<T, Q, VEC, true>;
+            if (row_bytes > kRowCtaBytes) B200Q_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongRowBytes));
+            return launch_dependent("quantize_rows_flat_kernel", kernel, dim3((unsigned)rows), kRowWarps * 32, row_bytes, 1, stream, w, wq, scale, rows, cols, (int)row_bytes);
+        }
+        if (row_bytes <= kRowCtaBytes) {
+            if (whole) return launch_dependent("quantize_rows_warp_kernel", quantize_rows_warp_kernel<T, Q, VEC>, grid, warps * 32, smem, 1, stream, w, wq, scale, rows, cols);
+            return launch_dependent("quantize_rows_flat_kernel", quantize_rows_flat_kernel<T, Q, VEC, false>, grid, warps * 32, smem, 1, stream, w, wq, scale, rows, cols, (int)row_bytes);
+        }
+        if (!whole) return launch_quantize_rows<T, Q, 1>(w, wq, scale, rows, cols, stream);
     }
     const int64_t nvec = cols / VEC;
     int threads = (int)round_up(nvec < 32 ? 32 : nvec, 32);
@@ -780,13 +929,12 @@ int quantize_typed(const void *w_, void *wq_, void *scale_, int64_t rows, int64_
     Q *wq = static_cast<Q *>(wq_);
     T *scale = static_cast<T *>(scale_);
     constexpr int VEC = 16 / sizeof(T);
-    const bool vec_ok = (cols % VEC == 0) && aligned(w, 16) && aligned(wq, VEC * sizeof(Q));
+    const bool bases_ok = aligned(w, 16) && aligned(wq, VEC * sizeof(Q));
     if (reduce_dim == 0) {
-        return vec_ok ? launch_quantize_cols<T, Q, VEC, kPanelThreads>(w, wq, scale, rows, cols, stream)
-                      : launch_quantize_cols<T, Q, 1, 32>(w, wq, scale, rows, cols, stream);
+        return bases_ok && cols % VEC == 0 ? launch_quantize_cols<T, Q, VEC, kPanelThreads>(w, wq, scale, rows, cols, stream)
+                                           : launch_quantize_cols<T, Q, 1, 32>(w, wq, scale, rows, cols, stream);
     }
-    return vec_ok ? launch_quantize_rows<T, Q, VEC>(w, wq, scale, rows, cols, stream)
-                  : launch_quantize_rows<T, Q, 1>(w, wq, scale, rows, cols, stream);
+    return bases_ok && cols >= VEC ? launch_quantize_rows<T, Q, VEC>(w, wq, scale, rows, cols, stream) : launch_quantize_rows<T, Q, 1>(w, wq, scale, rows, cols, stream);
 }
 
 template <typename T, typename Q>
@@ -798,6 +946,11 @@ int dequantize_typed(const void *wq_, const void *scale_, void *w_, int64_t rows
     constexpr int VEC = 16 / sizeof(T);  // 16-byte scale / output vectors; input vector is VEC * sizeof(Q)
     const bool vec_ok = (cols % VEC == 0) && aligned(w, 16) && aligned(wq, VEC * sizeof(Q)) && aligned(scale, 16);
     if (rows == 0 || cols == 0) return B200Q_OK;
+    if (cols % VEC != 0 && cols >= VEC && aligned(w, 16) && aligned(wq, VEC * sizeof(Q)) && cols <= 2147483647LL - kThreads * VEC) {
+        const int64_t groups = ceil_div(ceil_div(rows, VEC), kDqGroups);
+        return launch_dependent("dequantize_flat_kernel", dequantize_flat_kernel<T, Q, VEC>, dim3((unsigned)ceil_div(cols, kThreads), (unsigned)(groups < kDqGridY ? groups : kDqGridY)), kThreads, 0, 1,
+                                stream, wq, scale, w, rows, cols, reduce_dim);
+    }
     const int64_t row_blocks = ceil_div(rows, kDqRows);
     const int64_t col_blocks = ceil_div(vec_ok ? cols / VEC : cols, kDqVecs);
     if (row_blocks > kDqGridY * kDqGridY || col_blocks > 65535) {

@@ -250,6 +250,35 @@ def test_quantize_bf16_bits(rows, cols):
         assert torch.equal(q.cpu()[inside], quotient.float().round().to(torch.int8)[inside])
 
 
+def _bits(t):
+    return t if t.dtype in (torch.int8, torch.int16) else t.view(torch.int16 if t.element_size() == 2 else torch.int32)
+
+
+# Widths that are not whole vectors against the same matrix with its rows filled up, which the kernels for whole vectors take (and the oracle
+# pins): with NaN, which the maximum skips.  Rows that begin everywhere inside a vector, rows shorter than a panel and longer than what a warp
+# keeps, fewer rows than a group, a last vector that would reach past the matrix, slices that do not fit shared memory.
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('quant_type', ['int8', 'int16'])
+@pytest.mark.parametrize('rows,cols', [(1, 9), (7, 9), (3, 57), (64, 63), (513, 113), (2001, 1027), (4099, 62), (260, 517), (19, 24581), (26111, 58)])
+def test_widths_that_are_not_whole_vectors(rows, cols, quant_type, dtype):
+    g = torch.Generator(device='cuda').manual_seed(rows + cols)
+    wide = torch.full((rows, (cols + 15) // 8 * 8), float('nan'), device='cuda', dtype=dtype)
+    wide[:, :cols] = torch.randn(rows, cols, device='cuda', generator=g).mul_(0.02).to(dtype)
+    wide[0, 0], wide[rows - 1, cols - 1], wide[rows // 2, cols // 2] = float('nan'), float('inf'), -0.0
+    wide[rows // 3, :cols] = -0.0
+    wide[:, 4] = -wide[:, 4].abs()
+    w = wide[:, :cols].contiguous()
+    for dims in (0, -1):
+        wq, scale = hidet_b200.symmetric_quantize(w, quant_type, dims=dims)
+        wq_w, scale_w = hidet_b200.symmetric_quantize(wide, quant_type, dims=dims)
+        assert torch.equal(_bits(scale), _bits(scale_w)[:cols] if dims == 0 else _bits(scale_w))
+        assert torch.equal(wq, wq_w[:, :cols])
+        scale = torch.rand(scale.shape, device='cuda', generator=g).to(dtype)
+        scale_w = scale if dims == -1 else torch.cat([scale, scale.new_ones(wide.shape[1] - cols)])
+        back = hidet_b200.symmetric_dequantize(wq, scale, dims=dims)
+        assert torch.equal(_bits(back), _bits(hidet_b200.symmetric_dequantize(wq_w, scale_w, dims=dims)[:, :cols].contiguous()))
+
+
 def test_slices_that_fill_the_default_shared_memory():
     """Slices of a panel between 47 and 48 KB, with the static arrays above what a launch gets unasked: in a process of its own, where no
     larger slice has asked for more."""
