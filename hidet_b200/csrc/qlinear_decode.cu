@@ -93,8 +93,6 @@ __device__ __forceinline__ void store_out(const OutTargets &o, int row, int col,
     for (int i = 0; i < o.count; ++i) static_cast<__half *>(o.ptr[i])[off] = v;
 }
 
-__device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
-
 // The end of every path: y is the scaled fp32 sum of column nn (in range or not), row `row`.  Adds the bias,
 // applies the activation (the value of the partner column nn ^ 1 sits in lane ^ partner_xor; every lane
 // of the calling warp that is active takes part), adds the residual, rounds once and stores.

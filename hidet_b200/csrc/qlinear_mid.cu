@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 2)
                 for (int i = 0; i < 2; ++i) {
                     const float other = __shfl_xor_sync(0xffffffffu, odd ? y[0][i] : y[1][i], 4);
                     const float gate = odd ? other : y[0][i], up = odd ? y[1][i] : other;
-                    z[i] = gate / (1.0f + __expf(-gate)) * up;
+                    z[i] = silu(gate) * up;
                     const int oc = out_n0 + 8 * cw + (odd ? 4 : 0) + (g >> 1), m = m0 + mb + i;
                     if (res != nullptr && oc < out_n && m < p.M) z[i] += __half2float(__ldcg(res + (size_t)m * p.ep.ldr + oc));
                 }

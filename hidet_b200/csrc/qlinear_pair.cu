@@ -375,26 +375,38 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
                     const bool odd = g & 1;
 #pragma unroll
                     for (int j = 0; j < 4; j += 2) {
-                        uint32_t pk[4];  // [row block j, j + 1][column block h]
+                        // Eight results side by side, and no branch between them: one after the other, with the residual's test in each, a
+                        // block of 32 rows took 1.45 us for 0.9.
+                        float z[2][2][2];  // [row block j, j + 1][column block h][row]
 #pragma unroll
                         for (int jj = 0; jj < 2; ++jj)
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                float z[2];
+                            for (int h = 0; h < 2; ++h)
 #pragma unroll
                                 for (int i = 0; i < 2; ++i) {
                                     float y0 = __uint_as_float(v[h][4 * (j + jj) + i]) * sc[h][0], y1 = __uint_as_float(v[h][4 * (j + jj) + 2 + i]) * sc[h][1];
                                     y0 += bias[h][0];
                                     y1 += bias[h][1];
                                     const float other = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 4);
-                                    const float gate = odd ? other : y0, up = odd ? y1 : other;
-                                    z[i] = gate / (1.0f + __expf(-gate)) * up;
-                                    if (res != nullptr) {
-                                        const int oc = out_n0 + 16 * q + 8 * h + (odd ? 4 : 0) + (g >> 1), m = cb * 32 + 8 * (j + jj) + 2 * tq + i;
-                                        if (oc < out_n && m < m_left) z[i] += __half2float(__ldcg(res + (size_t)(m0 + m) * p.ep.ldr + oc));
-                                    }
+                                    z[jj][h][i] = silu(odd ? other : y0) * (odd ? y1 : other);
                                 }
-                                const __half2 z2 = __floats2half2_rn(z[0], z[1]);
+                        if (res != nullptr) {
+#pragma unroll
+                            for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) {
+                                        const int oc = out_n0 + 16 * q + 8 * h + (odd ? 4 : 0) + (g >> 1), m = cb * 32 + 8 * (j + jj) + 2 * tq + i;
+                                        if (oc < out_n && m < m_left) z[jj][h][i] += __half2float(__ldcg(res + (size_t)(m0 + m) * p.ep.ldr + oc));
+                                    }
+                        }
+                        uint32_t pk[4];
+#pragma unroll
+                        for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const __half2 z2 = __floats2half2_rn(z[jj][h][0], z[jj][h][1]);
                                 pk[2 * jj + h] = *reinterpret_cast<const uint32_t *>(&z2);
                             }
                         // result column g / 2 (even g) or 4 + g / 2 (odd g) of each 8: stored in the order of g, put right on the way out

@@ -135,3 +135,27 @@ def test_sums_accumulated_in_place_over_launches_that_overlap(through, m, k, n):
             add(x, i, x)
         assert torch.equal(x, want)
     assert ffi.func('b200q_check_status')() == ffi.OK
+
+
+# gates at the ends of every range of the quotient: zeros, where exp(-g) vanishes against 1 and where 1 does against it, where it overflows,
+# infinities and NaN; one size per kernel (small M, mid M, SM pairs)
+@pytest.mark.parametrize('m', [1, 9, 60, 1100])
+def test_gates_of_every_magnitude(m):
+    gates = torch.tensor([0.0, -0.0, 6e-8, -6e-8, 1e-3, -1e-3, 0.5, -0.5, 1.0, -1.0, 9.0, -9.0, 17.0, -17.0, 87.0, -87.0, 87.5, -87.5, 88.5, -88.5, 89.0, -89.0, 104.0,
+                          -104.0, 6e4, -6e4, float('inf'), float('-inf'), float('nan')])
+    k, n = 256, 512
+    bias = torch.zeros(n)
+    bias[0::2] = gates.repeat(n // 2 // len(gates) + 1)[:n // 2]
+    bias[1::2] = torch.tensor([1.0, -3.0, 0.25, 1000.0, float('inf')]).repeat(n // 10 + 1)[:n // 2]
+    bias = bias.half().cuda()
+    wq, scale = torch.zeros(k, n, dtype=torch.int8, device='cuda'), torch.ones(n, dtype=torch.float16, device='cuda')
+    got = hidet_b200.symmetric_quant_matmul(torch.ones(m, k, dtype=torch.float16, device='cuda'), wq, scale, bias=bias, activation='silu_mul')
+    g, u = bias[0::2].double(), bias[1::2].double()
+    want = (g / (1.0 + torch.exp(-g)) * u).half().expand(m, -1)   # -inf / inf is a NaN, in 64 bits as in 32
+    got, want = got[:, ~((g < -88.7) & u.isinf())], want[:, ~((g < -88.7) & u.isinf())]   # exp overflows in 32 bits there: 0 x inf, which is -inf in 64
+    assert torch.equal(got.isnan(), want.isnan())
+    finite = want.isfinite()
+    assert torch.equal(got[~finite & ~want.isnan()], want[~finite & ~want.isnan()])
+    # f32 in front of one rounding to f16: half an ulp of the value, or of the smallest number; exp's own error grows with |g| and is 2^-20 of it at 104
+    err = (got.double() - want.double()).abs()[finite]
+    assert bool((err <= 2.0 ** -10 * want.double().abs()[finite] + 2.0 ** -24).all())
