@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(THREADS, 2)
             tma_prefetch_2d(&map_w, NK ? k0 : n0, NK ? n0 : k0);
         }
     }
+    if (warp == ACT_WARP && lane == 0) tma_prefetch_desc(&map_a);
     pdl_wait();  // every role: none of the bounded waits below runs against the kernel in front
 
     auto wait = [&](uint32_t bar, uint32_t parity, unsigned int site) -> bool {
@@ -139,7 +140,6 @@ __global__ void __launch_bounds__(THREADS, 2)
         // ---------------- TMA producer: int8 weight tiles ----------------
         const uint64_t once = l2_policy_evict_first();
         pdl_launch_dependents();  // tensor memory is allocated: a kernel that moves in cannot take it away from this one
-        if (lane == 0) tma_prefetch_desc(&map_w);
         uint32_t i = 0;
         umma::Ring r;
         for (; i < n_it; ++i, r.advance(1, raw_slots)) {
@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(THREADS, 2)
         }
     } else if (warp == ACT_WARP) {
         // ---------------- TMA producer: activation tiles ----------------
-        if (lane == 0) tma_prefetch_desc(&map_a);
         const uint64_t keep = l2_policy_evict_last();
         uint32_t i = 0;
         umma::Ring r;
@@ -250,6 +249,17 @@ __global__ void __launch_bounds__(THREADS, 2)
 
     // ---------------- the main loop is over in this CTA, then in all of them: the rings are free ----------------
     __syncwarp();
+    // What the end needs from memory is asked for now, so that it is there when the sums are, and converted then: a conversion waits.
+    const int cw = warp & 7;  // this warp: columns 16 cw + 8 e + g of the tile
+    unsigned short sc_bits[2] = {0, 0}, bias_bits[2] = {0, 0};
+    if (warp < CONV_WARPS) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = n0 + 16 * cw + 8 * e + g;
+            if (n < p.N) sc_bits[e] = __ldcg(reinterpret_cast<const unsigned short *>(p.scale) + n);
+            if (FUSED && n < p.N && p.ep.bias != nullptr) bias_bits[e] = __ldcg(static_cast<const unsigned short *>(p.ep.bias) + n);
+        }
+    }
     if (!mbar_wait(smem_u32(&acc_full), 0)) report_timeout(p.status, kKernelMid, 8);
     __syncthreads();  // the producers' copies have landed
     umma::fence_after_sync();
@@ -261,76 +271,101 @@ __global__ void __launch_bounds__(THREADS, 2)
         // (lane (g, t): rows 2t, 2t + 1 of column g, then of column g + 8, of 16 columns); the owner adds the ranks' blocks
         // in rank order and finishes.
         const int q = warp & 3;
-        for (int b = warp >> 2; b < blocks; b += CONV_WARPS / 4) {
-            const int owner = b % ranks, slot = b / ranks;
-            const uint32_t dst = map_to_rank(smem_base, owner) + (uint32_t)((slot * ranks + rank) * BLOCK_BYTES) + (uint32_t)(2 * q * 32 + lane) * 16u;
-            const uint32_t bar = map_to_rank(smem_u32(&recv_bar), owner);
-            uint32_t v[2][4];
-            umma::ld_16x256b_x1(tmem_base + ((uint32_t)(32 * q) << 16) + 8 * b, v[0]);
-            umma::ld_16x256b_x1(tmem_base + ((uint32_t)(32 * q + 16) << 16) + 8 * b, v[1]);
+        // Two blocks are loaded together: one at a time, each waits for its own way out of tensor memory ((128, 4096, 4096) 12.6 us, 12.0 with
+        // this and two of the last phase's blocks side by side, (64, 4096, 12288) 20.6 and 20.0; four of either are more code and no faster).
+        constexpr int TOGETHER = 2, STEP = CONV_WARPS / 4;
+        for (int b0 = warp >> 2; b0 < blocks; b0 += TOGETHER * STEP) {
+            uint32_t v[TOGETHER][2][4];
+#pragma unroll
+            for (int i = 0; i < TOGETHER; ++i) {
+                if (b0 + i * STEP < blocks) {
+                    umma::ld_16x256b_x1(tmem_base + ((uint32_t)(32 * q) << 16) + 8 * (b0 + i * STEP), v[i][0]);
+                    umma::ld_16x256b_x1(tmem_base + ((uint32_t)(32 * q + 16) << 16) + 8 * (b0 + i * STEP), v[i][1]);
+                }
+            }
             umma::ld_wait();
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                st_async_v4f32(dst + h * 512, make_float4(__uint_as_float(v[h][0]), __uint_as_float(v[h][1]), __uint_as_float(v[h][2]), __uint_as_float(v[h][3])), bar);
+            for (int i = 0; i < TOGETHER; ++i) {
+                const int b = b0 + i * STEP;
+                if (b >= blocks) break;
+                const int owner = b % ranks, slot = b / ranks;
+                const uint32_t dst = map_to_rank(smem_base, owner) + (uint32_t)((slot * ranks + rank) * BLOCK_BYTES) + (uint32_t)(2 * q * 32 + lane) * 16u;
+                const uint32_t bar = map_to_rank(smem_u32(&recv_bar), owner);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    st_async_v4f32(dst + h * 512, make_float4(__uint_as_float(v[i][h][0]), __uint_as_float(v[i][h][1]), __uint_as_float(v[i][h][2]), __uint_as_float(v[i][h][3])), bar);
+            }
         }
         umma::fence_before_sync();
         if (own_blocks > 0 && !mbar_wait_cluster(smem_u32(&recv_bar), 0)) report_timeout(p.status, kKernelMid, 10);
         const bool pairs = FUSED && p.ep.act == kActSiluMul;
         const __half *res = FUSED ? static_cast<const __half *>(p.ep.residual) : nullptr;
         const int out_n = pairs ? p.N >> 1 : p.N, out_n0 = pairs ? n0 >> 1 : n0;
-        const int cw = warp & 7;  // this warp: columns 16 cw + 8 e + g of the tile, every CONV_WARPS / 8th block
-        float sc[2], bias[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int n = n0 + 16 * cw + 8 * e + g;
-            sc[e] = n < p.N ? __half2float(__ldcg(p.scale + n)) : 0.0f;
-            bias[e] = (FUSED && n < p.N && p.ep.bias != nullptr) ? __half2float(__ldcg(static_cast<const __half *>(p.ep.bias) + n)) : 0.0f;
-        }
+        const float sc[2] = {__half2float(__ushort_as_half(sc_bits[0])), __half2float(__ushort_as_half(sc_bits[1]))};
+        const float bias[2] = {__half2float(__ushort_as_half(bias_bits[0])), __half2float(__ushort_as_half(bias_bits[1]))};
         const uint32_t staging = smem_base + (uint32_t)(own_blocks * ranks) * BLOCK_BYTES;
         unsigned char *staging_gen = smem_gen + own_blocks * ranks * BLOCK_BYTES;
-        for (int slot = warp >> 3; slot < own_blocks; slot += CONV_WARPS / 8) {
-            const float4 *src = reinterpret_cast<const float4 *>(smem_gen + (size_t)slot * ranks * BLOCK_BYTES) + cw * 32 + lane;
-            float4 s = src[0];
-            for (int r = 1; r < ranks; ++r) {
-                const float4 x = src[r * (BLOCK_BYTES / 16)];
-                s.x += x.x, s.y += x.y, s.z += x.z, s.w += x.w;
+        // SLOTS blocks side by side: their residuals are on their way together, and the sums of one fill the waits of another.
+        static_assert(CONV_WARPS == 8, "a warp finishes its columns of every block");
+        constexpr int SLOTS = 2;
+        const bool odd = g & 1;
+        for (int slot0 = 0; slot0 < own_blocks; slot0 += SLOTS) {
+            float r[SLOTS][2][2];  // [column half][row], or [row] in the first half with pairs
+            if (FUSED && res != nullptr) {
+#pragma unroll
+                for (int i = 0; i < SLOTS; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int n = pairs ? out_n0 + 8 * cw + (odd ? 4 : 0) + (g >> 1) : n0 + 16 * cw + 8 * e + g, m = m0 + ((slot0 + i) * ranks + rank) * 8 + 2 * tq + k;
+                            r[i][e][k] = 0.0f;
+                            if (n < out_n && m < p.M && slot0 + i < own_blocks && !(pairs && e == 1)) r[i][e][k] = __half2float(__ldcg(res + (size_t)m * p.ep.ldr + n));
+                        }
             }
-            float y[2][2] = {{s.x * sc[0], s.y * sc[0]}, {s.z * sc[1], s.w * sc[1]}};  // [column half][row]
-            const int mb = (slot * ranks + rank) * 8 + 2 * tq;                          // this lane's first row in the tile
-            if (FUSED) {
+            float4 sum[SLOTS];
 #pragma unroll
-                for (int e = 0; e < 2; ++e) y[e][0] += bias[e], y[e][1] += bias[e];
-            }
-            const uint32_t row = staging + (uint32_t)(slot * 8 + (lane & 7)) * ROW_BYTES;
-            if (pairs) {
-                // Lanes with even g hold gates, the lanes with g + 1 what they multiply; of the two 8-column halves each lane of
-                // such a pair finishes one, for its two rows.
-                const bool odd = g & 1;
-                float z[2];
+            for (int i = 0; i < SLOTS; ++i)
+                if (slot0 + i < own_blocks) sum[i] = reinterpret_cast<const float4 *>(smem_gen + (size_t)(slot0 + i) * ranks * BLOCK_BYTES)[cw * 32 + lane];
+            for (int k = 1; k < ranks; ++k) {
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float other = __shfl_xor_sync(0xffffffffu, odd ? y[0][i] : y[1][i], 4);
-                    const float gate = odd ? other : y[0][i], up = odd ? y[1][i] : other;
-                    z[i] = silu(gate) * up;
-                    const int oc = out_n0 + 8 * cw + (odd ? 4 : 0) + (g >> 1), m = m0 + mb + i;
-                    if (res != nullptr && oc < out_n && m < p.M) z[i] += __half2float(__ldcg(res + (size_t)m * p.ep.ldr + oc));
-                }
-                const __half2 z2 = __floats2half2_rn(z[0], z[1]);
-                umma::stmatrix_x1_trans(row + 16 * cw, *reinterpret_cast<const uint32_t *>(&z2));
-            } else {
-                uint32_t pk[2];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (FUSED && res != nullptr) {
-                        const int n = n0 + 16 * cw + 8 * e + g;
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (n < p.N && m0 + mb + i < p.M) y[e][i] += __half2float(__ldcg(res + (size_t)(m0 + mb + i) * p.ep.ldr + n));
+                for (int i = 0; i < SLOTS; ++i)
+                    if (slot0 + i < own_blocks) {
+                        const float4 x = reinterpret_cast<const float4 *>(smem_gen + ((size_t)(slot0 + i) * ranks + k) * BLOCK_BYTES)[cw * 32 + lane];
+                        sum[i].x += x.x, sum[i].y += x.y, sum[i].z += x.z, sum[i].w += x.w;
                     }
-                    const __half2 y2 = __floats2half2_rn(y[e][0], y[e][1]);
-                    pk[e] = *reinterpret_cast<const uint32_t *>(&y2);
+            }
+#pragma unroll
+            for (int i = 0; i < SLOTS; ++i) {
+                if (slot0 + i >= own_blocks) break;
+                float y[2][2] = {{sum[i].x * sc[0], sum[i].y * sc[0]}, {sum[i].z * sc[1], sum[i].w * sc[1]}};  // [column half][row]
+                if (FUSED) {
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) y[e][0] += bias[e], y[e][1] += bias[e];
                 }
-                umma::stmatrix_x2_trans(row + (16 * cw + 8 * ((lane >> 3) & 1)) * 2, pk);
+                const uint32_t row = staging + (uint32_t)((slot0 + i) * 8 + (lane & 7)) * ROW_BYTES;
+                if (pairs) {
+                    // Lanes with even g hold gates, the lanes with g + 1 what they multiply; of the two 8-column halves each lane of
+                    // such a pair finishes one, for its two rows.
+                    float z[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? y[0][k] : y[1][k], 4);
+                        z[k] = silu(odd ? other : y[0][k]) * (odd ? y[1][k] : other);
+                        if (res != nullptr) z[k] += r[i][0][k];
+                    }
+                    const __half2 z2 = __floats2half2_rn(z[0], z[1]);
+                    umma::stmatrix_x1_trans(row + 16 * cw, *reinterpret_cast<const uint32_t *>(&z2));
+                } else {
+                    uint32_t pk[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (FUSED && res != nullptr) y[e][0] += r[i][e][0], y[e][1] += r[i][e][1];
+                        const __half2 y2 = __floats2half2_rn(y[e][0], y[e][1]);
+                        pk[e] = *reinterpret_cast<const uint32_t *>(&y2);
+                    }
+                    umma::stmatrix_x2_trans(row + (16 * cw + 8 * ((lane >> 3) & 1)) * 2, pk);
+                }
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(CONV_THREADS) : "memory");

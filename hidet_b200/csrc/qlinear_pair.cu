@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
     cluster_wait_acquire();  // both CTAs' barriers are set up and both have their tensor memory
     umma::fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    if (lane == 0 && (warp == RAW_WARP || warp == ACT_WARP)) tma_prefetch_desc(warp == RAW_WARP ? &map_w : &map_a);
     pdl_wait();  // every role: none of the bounded waits below runs against the kernel in front
 
     // Bounded wait of a whole warp (true in all lanes or false in all lanes) / of one thread.
@@ -156,7 +157,6 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
         // ---------------- TMA producer: int8 weight tiles ----------------
         pdl_launch_dependents();  // tensor memory is allocated: a kernel that is placed as this one's CTAs leave cannot take it away
         if (lane == 0) {
-            tma_prefetch_desc(&map_w);
             uint32_t i = 0;
             umma::Ring r;
             bool ok = true;
@@ -185,7 +185,6 @@ __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
     } else if (warp == ACT_WARP) {
         // ---------------- TMA producer: this CTA's half of the activation tiles ----------------
         if (lane == 0) {
-            tma_prefetch_desc(&map_a);
             const uint64_t keep = l2_policy_evict_last();  // every column tile reads them again
             uint32_t i = 0;
             umma::Ring r;
