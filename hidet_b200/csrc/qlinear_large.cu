@@ -1,8 +1,10 @@
 // Which kernel serves a quantized linear of more than a few rows, and with what tiles.
 //
 // The choice is by estimated time, in microseconds; the constants are measured (B200, graph replay of weights that exceed L2) and
-// stand beside what they describe.  The small-M kernel stays for what it does better: up to 24 rows always (24 rows, small-M against the
-// better of the others: (4096, 12288) 14.5 and 17.5 us, (4096, 22016) 24.8 and 29.8, (11008, 4096) 15.0 and 17.5, (1024, 1024) 3.1 and 5.2).
+// stand beside what they describe.  Over 580 drawn sizes of 25 to 2048 rows it is 1.1 % behind the best kernel, tile and cluster that were
+// timed for each (10 % with estimates that left the epilogue out and took the SMs for evenly filled).  The small-M kernel stays for what it
+// does better: up to 24 rows always (24 rows, small-M against the better of the others: (4096, 12288) 14.5 and 17.5 us,
+// (4096, 22016) 24.8 and 29.8, (11008, 4096) 15.0 and 17.5, (1024, 1024) 3.1 and 5.2).
 #include "common.cuh"
 #include "qlinear.h"
 
@@ -13,21 +15,27 @@ namespace {
 // (32, 11008, 4096) 17.9, (64, 4096, 4096) 13.5, (64, 2048, 2048) 5.9, (64, 1024, 1024) 3.4.
 double small_m_us(int64_t M, int64_t N, int64_t K) { return 2.6 + (double)K * N / 3.9e6 * (1.0 + 0.55 * (double)(ceil_div(M, 16) - 1)); }
 
-// A 64-k stage of the mid-M kernel takes 0.30 us with one CTA an SM and 0.46 with two, a fifth more at 128 rows than at 64; the launch
-// and its tail 4.2, and each CTA of a cluster makes the exchange longer.  (64, 4096, 4096): 24.7 / 15.2 / 10.9 / 11.5 us in
-// clusters of 1 / 2 / 4 / 8; (64, 4096, 11008) 20.2 in clusters of 2, 16.6 of 3; (64, 11008, 4096) 18.2 of 4, 15.1 of 8.
-double mid_us(int64_t M, int64_t N, int64_t K, int *tm, int *cluster) {
-    const int64_t m_tiles = ceil_div(M, 128), n_tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
-    const int64_t tiles = m_tiles * n_tiles;
+// The mid-M kernel: a launch 2.9, each CTA of a cluster 0.12, and per tile what grows with its rows (loads of the accumulator, the exchange, the
+// way out) 0.021 each, a block of eight rows that a CTA finishes 0.07 (with SiLU 0.26), and a 64-k stage: 0.32 with one CTA an SM, with two
+// 0.27 to 0.41 and more with the rows (what two CTAs take from shared memory), and 2 to fill two rings.  How many CTAs get an SM of their
+// own depends on the cluster: of 1 and 2 all of them, of 3 to 6 nine tenths, of 7 and 8 fifteen clusters (the jump is there at every size that
+// was tried).  Estimate and time: (128, 4096, 4096) in clusters of 4 11.5 and 12.0 us, (59, 3792, 2928) in 5 8.8 and 9.1, in 6 10.5 and 11.0,
+// (43, 9536, 13264) in 2 35.0 and 35.2, (249, 3376, 1744) in 4 10.8 and 11.6, (96, 2048, 19200) in 1 20.3 and 19.9.
+double mid_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm, int *cluster) {
+    const int64_t m_tiles = ceil_div(M, 128), tiles = m_tiles * ceil_div(N, 128), k_blocks = ceil_div(K, 64);
     *tm = (int)round_up(ceil_div(M, m_tiles), 16);
     int sms = sm_count();
     if (sms <= 0) sms = 148;
     double best = 1e30;
     for (int c = 1; c <= 8 && (c == 1 || k_blocks >= 2 * c); ++c) {
-        const int64_t resident = mid_resident_ctas(*tm, c), ctas = tiles * c;
+        const int64_t ctas = tiles * c, alone = c <= 2 ? sms : (c <= 6 ? sms * 9 / 10 : c * (sms / 10 + 1));
+        if (c > 1 && ctas > 2 * sms) break;
+        const int64_t resident = c == 1 || ctas * 5 <= sms * 8 ? 2 * sms : mid_resident_ctas(*tm, c);  // asked only where it may be short
         if (c > 1 && ctas > resident) break;  // a few clusters left for a second wave double the time
-        const double stage = (ctas <= sms ? 0.30 : 0.46) * (*tm > 64 ? 1.0 + 0.2 * (*tm - 64) / 64.0 : 1.0);
-        const double us = 4.2 + 0.3 * c + (double)ceil_div(ctas, resident) * (double)ceil_div(k_blocks, c) * stage;
+        const double shared = ctas >= 2 * sms ? 1.0 : (double)(ctas - sms) / sms;  // of the SMs: how many have two
+        const double stage = ctas <= alone ? 0.32 : 0.27 + 0.0012 * *tm + 0.135 * shared;
+        const double tile = (ctas <= alone ? 0.0 : 2.0) + 0.021 * *tm + (silu ? 0.26 : 0.07) * (double)ceil_div(*tm / 8, c) + (double)ceil_div(k_blocks, c) * stage;
+        const double us = 2.9 + 0.12 * c + (double)ceil_div(ctas, resident) * tile;
         if (us < best) {
             best = us;
             *cluster = c;
@@ -36,22 +44,28 @@ double mid_us(int64_t M, int64_t N, int64_t K, int *tm, int *cluster) {
     return best;
 }
 
-// A 64-k stage of the kernel on SM pairs by tile height, and what a tile costs on top: next to nothing where two accumulators
-// fit in tensor memory (up to 192 rows), the epilogue where only one does.  (512, 4096, 22016) with SiLU: 124 / 96 / 88 / 87 us
-// at 96 / 128 / 192 / 256 rows; (2048, 8192, 28672): 889 / 728 / 690 / 638 at 128 / 192 / 224 / 256; (256, 4096, 11008): 38 at
-// 96 to 192 rows, 42 at 224, 26 at 256.
+// The kernel on SM pairs: a 64-k stage by tile height, for the only wave and for one of several, and the epilogue by rows.  Where two accumulators
+// fit in tensor memory (up to 192 rows) the epilogue runs beside the next tile, which for short K it outlasts; where one does it comes on top.
+// Estimate and time: (512, 4096, 22016) with SiLU 82 and 77 us at 256 rows, (1900, 368, 19264) 33.5 and 36.0 at 192, 35.3 and 38.9 at 160,
+// (2048, 256, 8192) 16.9 and 16.6 at 192, 18.4 and 18.3 at 128, (1024, 320, 16384) 18.7 and 19.3 at 128, (1337, 464, 3008) 7.9 and 9.0 at 224.
 double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
     static const struct {
         int tm;
-        double stage;
-    } forms[] = {{64, 0.262}, {96, 0.262}, {128, 0.265}, {160, 0.28}, {192, 0.315}, {224, 0.32}, {256, 0.335}};
+        double one, more;
+    } forms[] = {{64, 0.29, 0.267}, {96, 0.285, 0.27}, {128, 0.28, 0.267}, {160, 0.26, 0.27}, {192, 0.262, 0.285}, {224, 0.284, 0.305}, {256, 0.32, 0.33}};
     int sms = sm_count();
     if (sms <= 0) sms = 148;
     double best = 1e30;
     for (const auto &f : forms) {
-        const int64_t tiles = ceil_div(N, 256) * ceil_div(M, f.tm);
-        const double tile = f.tm <= 192 ? 0.3 : (silu ? 6.0 : 2.5);
-        const double us = 4.5 + (double)ceil_div(tiles, sms / 2) * ((double)ceil_div(K, 64) * f.stage + tile);
+        const int64_t waves = ceil_div(ceil_div(N, 256) * ceil_div(M, f.tm), sms / 2);
+        const double rows = waves == 1 && M < f.tm ? (double)M : f.tm, loop = (double)ceil_div(K, 64) * (waves == 1 ? f.one : f.more);
+        double us;
+        if (f.tm <= 192) {
+            const double epilogue = (silu ? 0.023 : 0.0085) * rows, next = loop + 0.65 > epilogue + 1.05 ? loop + 0.65 : epilogue + 1.05;
+            us = 3.55 + loop + 0.9 * epilogue + (double)(waves - 1) * next;
+        } else {
+            us = 3.5 + (double)waves * (loop + (silu ? 0.02 : 0.0095) * rows);
+        }
         if (us < best) {
             best = us;
             *tm = f.tm;
@@ -66,8 +80,13 @@ LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu) {
     LargePlan p;
     if (M <= 24) return p;
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
-    const double mid = M <= 65535 * 128 ? mid_us(M, N, K, &mid_tm, &mid_cluster) : 1e30;  // the grid's limit
-    const double pair = M > 32 ? pair_us(M, N, K, silu, &pair_tm) : 1e30;
+    const bool mid_takes = M <= (int64_t)65535 * 128;  // the grid's limit
+    const double mid = mid_takes ? mid_us(M, N, K, silu, &mid_tm, &mid_cluster) : 1e30;
+    // What was measured of the kernel on SM pairs ends at K = 256 and at columns that fill one tile and a sliver of another: below, the mid-M
+    // kernel stays as long as its tiles run at once.
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    const bool pair_too = !mid_takes || (K >= 256 && N >= 288) || ceil_div(M, 128) * ceil_div(N, 128) > sms;
+    const double pair = M > 32 && pair_too ? pair_us(M, N, K, silu, &pair_tm) : 1e30;
     const double best = mid < pair ? mid : pair;
     // The estimates are within a tenth of each other's error, so nearly as good is good enough (a sixth was asked for before, and
     // (32, 4096, 12288) took 23.4 us for 17.7, (32, 4096, 22016) 36.0 for 29.8, (48, 4096, 4096) 13.6 for 9.9).
