@@ -719,11 +719,11 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
     // takes as long as its chain of waits and loads, not as its bytes ((1, 11008, 4096), 256 CTAs of 22 steps, 11.4 us; 448 of 13, 10.1;
-    // (16, 11008, 4096) 12.9 -> 12.0).  Short runs in many parts lose more in the exchange, which grows with the rows: (1, 4096, 4096) 5.0 -> 5.8
+    // (16, 11008, 4096) 12.9 -> 12.0, (1, 16384, 5120) 19.1 -> 16.1; not with three CTAs an SM, (7, 10080, 7088) 14.5 -> 16.8).  Short runs in many parts lose more in the exchange, which grows with the rows: (1, 4096, 4096) 5.0 -> 5.8
     // in sixteen parts of four steps, (16, 5376, 2304) 6.1 -> 6.4.
     if (pl.m_tiles == 1 && c == kPortableCluster && k_iters >= 48) {
         const int portable = pl.n_tiles * c;
-        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * c;
+        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * c && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
             if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[pl.variant], wide)) continue;
             c = wide, groups = 1;
