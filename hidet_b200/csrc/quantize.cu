@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(kThreads) dequantize_flat_kernel(const Q *wq, 
     pdl_wait();
     const int64_t v0 = (int64_t)blockIdx.x * kThreads, v = v0 + threadIdx.x;
     if (reduce_dim == 0) {
-        const unsigned int width = (unsigned int)cols, c0 = (unsigned int)(v0 * VEC % cols);  // the launcher keeps cols below 2^31
+        const unsigned int width = (unsigned int)cols, c0 = (unsigned int)(v0 * VEC % cols);  // the launcher keeps cols below 2^22
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
             const unsigned int at = threadIdx.x + i * kThreads;
@@ -946,15 +946,15 @@ int dequantize_typed(const void *wq_, const void *scale_, void *w_, int64_t rows
     constexpr int VEC = 16 / sizeof(T);  // 16-byte scale / output vectors; input vector is VEC * sizeof(Q)
     const bool vec_ok = (cols % VEC == 0) && aligned(w, 16) && aligned(wq, VEC * sizeof(Q)) && aligned(scale, 16);
     if (rows == 0 || cols == 0) return B200Q_OK;
-    if (cols % VEC != 0 && cols >= VEC && aligned(w, 16) && aligned(wq, VEC * sizeof(Q)) && cols <= 2147483647LL - kThreads * VEC) {
-        const int64_t groups = ceil_div(ceil_div(rows, VEC), kDqGroups);
-        return launch_dependent("dequantize_flat_kernel", dequantize_flat_kernel<T, Q, VEC>, dim3((unsigned)ceil_div(cols, kThreads), (unsigned)(groups < kDqGridY ? groups : kDqGridY)), kThreads, 0, 1,
-                                stream, wq, scale, w, rows, cols, reduce_dim);
-    }
     const int64_t row_blocks = ceil_div(rows, kDqRows);
     const int64_t col_blocks = ceil_div(vec_ok ? cols / VEC : cols, kDqVecs);
     if (row_blocks > kDqGridY * kDqGridY || col_blocks > 65535) {
         return set_error(B200Q_UNSUPPORTED, "symmetric_dequantize: [%lld, %lld] exceeds the grid limit", (long long)rows, (long long)cols);
+    }
+    if (cols % VEC != 0 && cols >= VEC && aligned(w, 16) && aligned(wq, VEC * sizeof(Q))) {
+        const int64_t groups = ceil_div(ceil_div(rows, VEC), kDqGroups);
+        return launch_dependent("dequantize_flat_kernel", dequantize_flat_kernel<T, Q, VEC>, dim3((unsigned)ceil_div(cols, kThreads), (unsigned)(groups < kDqGridY ? groups : kDqGridY)), kThreads, 0, 1,
+                                stream, wq, scale, w, rows, cols, reduce_dim);
     }
     const dim3 grid((unsigned)col_blocks, (unsigned)(row_blocks < kDqGridY ? row_blocks : kDqGridY), (unsigned)ceil_div(row_blocks, kDqGridY));
     auto kernel = vec_ok ? dequantize_kernel<T, Q, VEC> : dequantize_kernel<T, Q, 1>;
