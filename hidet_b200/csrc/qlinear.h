@@ -99,7 +99,7 @@ struct LargePlan {
     int tm = 0;
     int cluster = 1;
 };
-LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu);
+LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk = false);
 // True where these kernels serve the call and are better at it than the small-M one, or alone would serve it but for its
 // outputs; *rc is then the launch's status or the refusal.  What the small-M kernel refuses for want of scratch stays refused.
 bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,

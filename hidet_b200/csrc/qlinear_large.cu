@@ -21,7 +21,10 @@ double small_m_us(int64_t M, int64_t N, int64_t K) { return 2.6 + (double)K * N 
 // own depends on the cluster: of 1 and 2 all of them, of 3 to 6 nine tenths, of 7 and 8 fifteen clusters (the jump is there at every size that
 // was tried).  Estimate and time: (128, 4096, 4096) in clusters of 4 11.5 and 12.0 us, (59, 3792, 2928) in 5 8.8 and 9.1, in 6 10.5 and 11.0,
 // (43, 9536, 13264) in 2 35.0 and 35.2, (249, 3376, 1744) in 4 10.8 and 11.6, (96, 2048, 19200) in 1 20.3 and 19.9.
-double mid_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm, int *cluster) {
+// Rows of the weight that are not whole 32-byte sectors cost a sector more a row of a tile: with two CTAs an SM a stage is then 1.25 times as
+// long for [N, K], whose tile rows are two sectors ((121, 3728, 20272) 43.1 us, (121, 5680, 28432) 69.1; on SM pairs 37.1 and 53.7), and 1.1
+// times for [K, N] where no other row of tiles reads them again (38.7 and 59.8; 36.2 and 52.2).
+double mid_us(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk, int *tm, int *cluster) {
     const int64_t m_tiles = ceil_div(M, 128), tiles = m_tiles * ceil_div(N, 128), k_blocks = ceil_div(K, 64);
     *tm = (int)round_up(ceil_div(M, m_tiles), 16);
     int sms = sm_count();
@@ -33,7 +36,8 @@ double mid_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm, int *cluster)
         const int64_t resident = c == 1 || ctas * 5 <= sms * 8 ? 2 * sms : mid_resident_ctas(*tm, c);  // asked only where it may be short
         if (c > 1 && ctas > resident) break;  // a few clusters left for a second wave double the time
         const double shared = ctas >= 2 * sms ? 1.0 : (double)(ctas - sms) / sms;  // of the SMs: how many have two
-        const double stage = ctas <= alone ? 0.32 : 0.27 + 0.0012 * *tm + 0.135 * shared;
+        const double slow = (weight_nk ? K : N) % 32 == 0 ? 1.0 : (weight_nk ? 1.25 : (m_tiles == 1 ? 1.1 : 1.0));
+        const double stage = ctas <= alone ? 0.32 : slow * (0.27 + 0.0012 * *tm + 0.135 * shared);
         const double tile = (ctas <= alone ? 0.0 : 2.0) + 0.021 * *tm + (silu ? 0.26 : 0.07) * (double)ceil_div(*tm / 8, c) + (double)ceil_div(k_blocks, c) * stage;
         const double us = 2.9 + 0.12 * c + (double)ceil_div(ctas, resident) * tile;
         if (us < best) {
@@ -76,12 +80,12 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
 
 }  // namespace
 
-LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu) {
+LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk) {
     LargePlan p;
     if (M <= 24) return p;
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
     const bool mid_takes = M <= (int64_t)65535 * 128;  // the grid's limit
-    const double mid = mid_takes ? mid_us(M, N, K, silu, &mid_tm, &mid_cluster) : 1e30;
+    const double mid = mid_takes ? mid_us(M, N, K, silu, weight_nk, &mid_tm, &mid_cluster) : 1e30;
     // What was measured of the kernel on SM pairs ends at K = 256 and at columns that fill one tile and a sliver of another: below, the mid-M
     // kernel stays as long as its tiles run at once.
     const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -112,7 +116,7 @@ bool try_large(const void *a, const void *wq, const void *scale, const OutTarget
         const DecodePlan dp = plan_decode(M, N, K);
         if (dp.partial_bytes > 0 && scratch_bytes < dp.counter_bytes + dp.partial_bytes) return false;
     }
-    const LargePlan plan = plan_large(M, N, K, epilogue != nullptr && epilogue->act == kActSiluMul);
+    const LargePlan plan = plan_large(M, N, K, epilogue != nullptr && epilogue->act == kActSiluMul, weight_nk);
     if (plan.kind == LargePlan::kNone) return false;
     *rc = check_large_outputs(c);
     if (*rc != B200Q_OK) return only;  // the small-M kernel stores at any element
