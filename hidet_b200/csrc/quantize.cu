@@ -127,7 +127,10 @@ struct QMax<int16_t> {
     static constexpr int value = 32767;
 };
 
-// N elements of T moved as one naturally aligned vector.
+// N elements of T moved as one naturally aligned vector.  Operands are read with ordinary loads, behind the wait that makes the results of
+// the kernel in front visible, and not through pointers that promise no aliasing: those would let the compiler take the path for data that is
+// constant while a kernel runs, which under programmatic launches it is not.  So the compiler cannot move a load over a store either,
+// and where a thread handles several vectors their loads stand together in front of the stores.
 template <typename T, int N>
 struct alignas(sizeof(T) * N) Vec {
     T v[N];
@@ -136,21 +139,6 @@ struct alignas(sizeof(T) * N) Vec {
 template <typename T, int N>
 __device__ __forceinline__ Vec<T, N> load_vec(const T *p) {
     return *reinterpret_cast<const Vec<T, N> *>(p);
-}
-// The same through L2: under programmatic launches a CTA may be older than the kernel that wrote what it reads, and so may be what the
-// first-level cache holds.
-template <int BYTES>
-struct RawVec;
-template <> struct RawVec<1> { typedef unsigned char Type; };
-template <> struct RawVec<2> { typedef unsigned short Type; };
-template <> struct RawVec<4> { typedef unsigned int Type; };
-template <> struct RawVec<8> { typedef uint2 Type; };
-template <> struct RawVec<16> { typedef uint4 Type; };
-template <typename T, int N>
-__device__ __forceinline__ Vec<T, N> load_l2(const T *p) {
-    typedef typename RawVec<sizeof(T) * N>::Type Raw;
-    const Raw raw = __ldcg(reinterpret_cast<const Raw *>(p));
-    return *reinterpret_cast<const Vec<T, N> *>(&raw);
 }
 template <typename T, int N>
 __device__ __forceinline__ void store_vec(T *p, const Vec<T, N> &x) {
@@ -407,7 +395,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
             T *t = tile + ty * PW + tx * VEC;
 #pragma unroll 4
             for (int r = ty; r < nrows; r += TY, src += sweep, t += TY * PW) {
-                Vec<T, VEC> x = load_l2<T, VEC>(src);
+                Vec<T, VEC> x = load_vec<T, VEC>(src);
                 if (cache) store_vec<T, VEC>(t, x);
                 acc.add(x);
             }
@@ -453,13 +441,29 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
         for (int i = 0; i < VEC; ++i) s[i] = div_s[tx * VEC + i];
         const T *src = w + (row0 + ty) * cols + col;
         Q *dst = wq + (row0 + ty) * cols + col;
-        const T *t = tile + ty * PW + tx * VEC;
+        if (cache) {
+            const T *t = tile + ty * PW + tx * VEC;
 #pragma unroll 4
-        for (int r = ty; r < nrows; r += TY, src += sweep, dst += sweep, t += TY * PW) {
-            Vec<T, VEC> x = cache ? load_vec<T, VEC>(t) : load_l2<T, VEC>(src);
-            Vec<Q, VEC> q;
-            QuantVec<T, Q, VEC, typename A::Divisor>::template run<true>(x, s, q);
-            store_vec<Q, VEC>(dst, q);
+            for (int r = ty; r < nrows; r += TY, dst += sweep, t += TY * PW) {
+                Vec<Q, VEC> q;
+                QuantVec<T, Q, VEC, typename A::Divisor>::template run<true>(load_vec<T, VEC>(t), s, q);
+                store_vec<Q, VEC>(dst, q);
+            }
+        } else {
+            constexpr int BATCH = 4;
+            for (int left = nrows - ty; left > 0; left -= BATCH * TY, src += BATCH * sweep, dst += BATCH * sweep) {
+                Vec<T, VEC> x[BATCH];
+#pragma unroll
+                for (int i = 0; i < BATCH; ++i)
+                    if (i * TY < left) x[i] = load_vec<T, VEC>(src + i * sweep);
+#pragma unroll
+                for (int i = 0; i < BATCH; ++i) {
+                    if (i * TY >= left) break;
+                    Vec<Q, VEC> q;
+                    QuantVec<T, Q, VEC, typename A::Divisor>::template run<true>(x[i], s, q);
+                    store_vec<Q, VEC>(dst + i * sweep, q);
+                }
+            }
         }
     }
 }
@@ -498,11 +502,11 @@ __global__ void __launch_bounds__(kThreads) quantize_rows_kernel(const T *w, Q *
     for (int j = 0; j < REG_CHUNKS; ++j) {
         const int64_t i = threadIdx.x + j * stride;
         if (i < nvec) {
-            keep[j] = load_l2<T, VEC>(src + i * VEC);
+            keep[j] = load_vec<T, VEC>(src + i * VEC);
             acc.add(keep[j]);
         }
     }
-    for (int64_t i = threadIdx.x + REG_CHUNKS * stride; i < nvec; i += stride) acc.add(load_l2<T, VEC>(src + i * VEC));
+    for (int64_t i = threadIdx.x + REG_CHUNKS * stride; i < nvec; i += stride) acc.add(load_vec<T, VEC>(src + i * VEC));
     T each[VEC];
     acc.template finish<32>(each);
     T m = A::lowest();
@@ -531,11 +535,19 @@ __global__ void __launch_bounds__(kThreads) quantize_rows_kernel(const T *w, Q *
             store_vec<Q, VEC>(dst + i * VEC, q);
         }
     }
-    for (int64_t i = threadIdx.x + REG_CHUNKS * stride; i < nvec; i += stride) {
-        Vec<T, VEC> x = load_l2<T, VEC>(src + i * VEC);
-        Vec<Q, VEC> q;
-        QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(x, &s, q);
-        store_vec<Q, VEC>(dst + i * VEC, q);
+    constexpr int BATCH = 4;
+    for (int64_t i = threadIdx.x + REG_CHUNKS * stride; i < nvec; i += BATCH * stride) {
+        Vec<T, VEC> x[BATCH];
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j)
+            if (i + j * stride < nvec) x[j] = load_vec<T, VEC>(src + (i + j * stride) * VEC);
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+            if (i + j * stride >= nvec) break;
+            Vec<Q, VEC> q;
+            QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(x[j], &s, q);
+            store_vec<Q, VEC>(dst + (i + j * stride) * VEC, q);
+        }
     }
 }
 
@@ -731,25 +743,30 @@ __global__ void __launch_bounds__(kThreads) dequantize_kernel(const Q *wq, const
     const Q *src = wq + r0 * cols + c;
     T *dst = w + r0 * cols + c;
     const int64_t sweep = (int64_t)kDqSweep * cols;
-    if (reduce_dim == 0) {
-        const Vec<T, VEC> s = load_l2<T, VEC>(scale + c);
+    constexpr int EACH = kDqRows / kDqSweep;
+    Vec<Q, VEC> q[EACH];
+    Vec<T, VEC> out;
 #pragma unroll
-        for (int i = 0; i < kDqRows / kDqSweep; ++i) {
-            if (r0 + i * kDqSweep < rows) {
-                Vec<T, VEC> out;
-                DequantVec<T, Q, VEC>::template run<true>(load_l2<Q, VEC>(src + i * sweep), s.v, out);
-                store_vec<T, VEC>(dst + i * sweep, out);
-            }
+    for (int i = 0; i < EACH; ++i)
+        if (r0 + i * kDqSweep < rows) q[i] = load_vec<Q, VEC>(src + i * sweep);
+    if (reduce_dim == 0) {
+        const Vec<T, VEC> s = load_vec<T, VEC>(scale + c);
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            if (r0 + i * kDqSweep >= rows) break;
+            DequantVec<T, Q, VEC>::template run<true>(q[i], s.v, out);
+            store_vec<T, VEC>(dst + i * sweep, out);
         }
     } else {
+        T s[EACH];
 #pragma unroll
-        for (int i = 0; i < kDqRows / kDqSweep; ++i) {
-            if (r0 + i * kDqSweep < rows) {
-                const T s = load_l2<T, 1>(scale + r0 + i * kDqSweep).v[0];
-                Vec<T, VEC> out;
-                DequantVec<T, Q, VEC>::template run<false>(load_l2<Q, VEC>(src + i * sweep), &s, out);
-                store_vec<T, VEC>(dst + i * sweep, out);
-            }
+        for (int i = 0; i < EACH; ++i)
+            if (r0 + i * kDqSweep < rows) s[i] = scale[r0 + i * kDqSweep];
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            if (r0 + i * kDqSweep >= rows) break;
+            DequantVec<T, Q, VEC>::template run<false>(q[i], &s[i], out);
+            store_vec<T, VEC>(dst + i * sweep, out);
         }
     }
 }
@@ -769,7 +786,7 @@ __global__ void __launch_bounds__(kThreads) dequantize_flat_kernel(const Q *wq, 
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
             const unsigned int at = threadIdx.x + i * kThreads;
-            col_scale[at] = load_l2<T, 1>(scale + (c0 + at) % width).v[0];
+            col_scale[at] = scale[(c0 + at) % width];
         }
         __syncthreads();
     }
@@ -780,21 +797,32 @@ __global__ void __launch_bounds__(kThreads) dequantize_flat_kernel(const Q *wq, 
     Vec<T, VEC> s;
     if (reduce_dim == 0) s = load_vec<T, VEC>(col_scale + threadIdx.x * VEC);
     for (int64_t g0 = (int64_t)blockIdx.y * kDqGroups; g0 < groups; g0 += (int64_t)gridDim.y * kDqGroups) {
+        const int64_t r0 = g0 * VEC + row, at0 = (g0 * cols + v) * VEC, step = VEC * cols;
+        Vec<Q, VEC> q[kDqGroups];
+        T first[kDqGroups], second[kDqGroups];
 #pragma unroll
         for (int i = 0; i < kDqGroups; ++i) {
-            const int64_t r = (g0 + i) * VEC + row, at = ((g0 + i) * cols + v) * VEC;
-            if (r >= rows) break;
-            if (reduce_dim != 0) {
-                const T s0 = load_l2<T, 1>(scale + r).v[0], s1 = here < VEC && r + 1 < rows ? load_l2<T, 1>(scale + r + 1).v[0] : s0;
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) s.v[e] = e < here ? s0 : s1;
+            const int64_t r = r0 + i * VEC;
+            if (r < rows && at0 + i * step + VEC <= total) q[i] = load_vec<Q, VEC>(wq + at0 + i * step);
+            if (reduce_dim != 0 && r < rows) {
+                first[i] = scale[r];
+                second[i] = here < VEC && r + 1 < rows ? scale[r + 1] : first[i];
             }
-            Vec<T, VEC> out;
+        }
+#pragma unroll
+        for (int i = 0; i < kDqGroups; ++i) {
+            const int64_t at = at0 + i * step;
+            if (r0 + i * VEC >= rows) break;
+            if (reduce_dim != 0) {
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) s.v[e] = e < here ? first[i] : second[i];
+            }
             if (at + VEC <= total) {
-                DequantVec<T, Q, VEC>::template run<true>(load_l2<Q, VEC>(wq + at), s.v, out);
+                Vec<T, VEC> out;
+                DequantVec<T, Q, VEC>::template run<true>(q[i], s.v, out);
                 store_vec<T, VEC>(w + at, out);
             } else {                              // the end of the matrix
-                for (int e = 0; at + e < total; ++e) w[at + e] = Arith<T>::template dequant<Q>(load_l2<Q, 1>(wq + at + e).v[0], s.v[e]);
+                for (int e = 0; at + e < total; ++e) w[at + e] = Arith<T>::template dequant<Q>(wq[at + e], s.v[e]);
             }
         }
     }
@@ -818,20 +846,37 @@ __global__ void __launch_bounds__(kThreads) embedding_dequant_kernel(const Q *ta
     const int64_t c = ((int64_t)blockIdx.y * kDqVecs + (threadIdx.x % kDqVecs)) * VEC;
     if (c >= dim) return;                         // dim % VEC == 0 whenever VEC > 1
     const int64_t r0 = (int64_t)blockIdx.x * kEmbRows + threadIdx.x / kDqVecs;
+    constexpr int EACH = kEmbRows / kDqSweep;
+    int64_t row[EACH];                            // -1: outside the table
+    T s[EACH];
+    Vec<Q, VEC> q[EACH];
 #pragma unroll
-    for (int i = 0; i < kEmbRows / kDqSweep; ++i) {
+    for (int i = 0; i < EACH; ++i) {
+        const int64_t r = r0 + i * kDqSweep;
+        row[i] = r < n_idx ? (int64_t)idx[r] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        if (r0 + i * kDqSweep >= n_idx) break;
+        if (row[i] < 0) row[i] += vocab;
+        if (row[i] < 0 || row[i] >= vocab) {
+            row[i] = -1;
+        } else {
+            s[i] = scale[row[i]];
+            q[i] = load_vec<Q, VEC>(table + row[i] * dim + c);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
         const int64_t r = r0 + i * kDqSweep;
         if (r >= n_idx) break;
-        int64_t row = (int64_t)load_l2<I, 1>(idx + r).v[0];
-        if (row < 0) row += vocab;
         Vec<T, VEC> o;
-        if (row < 0 || row >= vocab) {
+        if (row[i] < 0) {
 #pragma unroll
             for (int e = 0; e < VEC; ++e) o.v[e] = (T)0.0f;
             if (c == 0 && status != nullptr) atomicOr(status, 0x40000000u);
         } else {
-            const T s = load_l2<T, 1>(scale + row).v[0];
-            DequantVec<T, Q, VEC>::template run<false>(load_l2<Q, VEC>(table + row * dim + c), &s, o);
+            DequantVec<T, Q, VEC>::template run<false>(q[i], &s[i], o);
         }
         store_vec<T, VEC>(out + r * dim + c, o);
     }
