@@ -78,6 +78,21 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
     return best;
 }
 
+// The kernels for more rows wait for the kernel in front before they read anything; the small-M kernel asks for its codes earlier.  A call that once
+// waited goes on waiting, since its codes may be the result of that kernel: true for all calls of more than 24 rows that the first estimates of
+// this rule gave to the kernels for more rows (and, by the roundings below, for 630 of 84 000 drawn ones of 25 to 64 rows that they did not).
+// It is no slower there either: (64, 1536, 6144) 8.4 us, 11.8 in the small-M kernel, (60, 256, 28672) with SiLU 8.3 and 13.4, (51, 1680, 5776) 9.0 and 9.8.
+bool codes_may_be_late(int64_t M, int64_t N, int64_t K) {
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    const int64_t tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
+    double best = M > 32 ? 4.5 + (double)ceil_div(ceil_div(N, 256), sms / 2) * ((double)k_blocks * 0.262 + 0.3) : 1e30;
+    for (int c = 1; c <= 8 && (c == 1 || (k_blocks >= 2 * c && tiles * c <= 2 * sms)); ++c) {
+        const double us = 4.2 + 0.3 * c + (double)ceil_div(tiles * c, 2 * sms) * (double)ceil_div(k_blocks, c) * (tiles * c <= sms ? 0.30 : 0.46);
+        if (us < best) best = us;
+    }
+    return best <= 0.85 * small_m_us(M, N, K);
+}
+
 }  // namespace
 
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk) {
@@ -94,7 +109,7 @@ LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk)
     const double best = mid < pair ? mid : pair;
     // The estimates are within a tenth of each other's error, so nearly as good is good enough (a sixth was asked for before, and
     // (32, 4096, 12288) took 23.4 us for 17.7, (32, 4096, 22016) 36.0 for 29.8, (48, 4096, 4096) 13.6 for 9.9).
-    if (!use_prefill_kernel(M, N, K) && best > 0.95 * small_m_us(M, N, K)) return p;
+    if (!use_prefill_kernel(M, N, K) && best > 0.95 * small_m_us(M, N, K) && !codes_may_be_late(M, N, K)) return p;
     p.kind = mid < pair ? LargePlan::kMid : LargePlan::kPair;
     p.tm = mid < pair ? mid_tm : pair_tm;
     p.cluster = mid_cluster;

@@ -212,3 +212,14 @@ def test_quantize_and_dequantize_may_read_the_result_of_the_linear_in_front(rows
     for i in range(12):
         assert torch.equal(all_three(fronts[i % 2], lambda: None), want[i % 2])
     assert ffi.func('b200q_check_status')() == ffi.OK
+
+
+# calls beyond 24 rows that the small-M kernel would serve as fast
+@pytest.mark.parametrize('m,k,n', [(56, 1536, 6144), (64, 1536, 6144), (51, 1680, 5776), (49, 1536, 6144)])
+@pytest.mark.parametrize('layout', ['KN', 'NK'])
+def test_weights_beyond_24_rows_may_be_the_result_of_a_kernel_that_triggers_early(late_copy, m, k, n, layout):
+    gen = torch.Generator(device='cuda').manual_seed(m)
+    a = torch.randn(m, k, device='cuda', generator=gen).half()
+    weights = [(torch.randint(-127, 128, (k, n) if layout == 'KN' else (n, k), device='cuda', generator=gen, dtype=torch.int8),
+                torch.rand(n, device='cuda', generator=gen).mul_(1e-2).half()) for _ in range(2)]
+    _check(late_copy, weights, lambda wq, scale: hidet_b200.symmetric_quant_matmul(a, wq, scale, weight_layout=layout))
