@@ -220,11 +220,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// silu(g) = g / (1 + exp(-g)) for an epilogue: the quotient from an approximate reciprocal, corrected once by its remainder, which leaves no
-// more than the last rounding.  (The exact division tests its operands and calls a subroutine for those out of range, a zero among them:
-// columns and rows that only fill up a tile are zeros.  A 32-row block of the kernel on SM pairs took 1.3 us with it, 3.6 where a tile has
-// such columns.)  d is a quarter of the divisor, which keeps its reciprocal a normal number for every finite exp(-g).  Where the
-// remainder is zero (g may be -0) or, for an infinity, a NaN, the first quotient is the answer.
+// silu(g) = g / (1 + exp(-g)) for an epilogue: a quotient from an approximate reciprocal, corrected once by its remainder in fused multiply-adds
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  Before its
+// last rounding the corrected quotient is off by about 2^-44 of its value, so that it differs from the division's only where that lies on a rounding
+// boundary, by one ulp: 2 of 350 million gates of 1e-38 to 88; largest and mean error against 64 bits are the division's (tests/test_silu_gpu.py).
+// For gates of at most 2^125 in magnitude (sums of f16 times int8 end near 2^70); beyond, g * r may overflow.
+// It has no branch: with the division a 32-row block of the kernel on SM pairs took 1.3 us, 3.6 where columns that only fill up the
+// tile make its gates zeros, and 0.9 with this.
+// d is a quarter of the divisor, which keeps its reciprocal a normal number for every finite exp(-g).  Where the remainder is zero (g may be
+// -0) or, for an infinity, a NaN, the first quotient is the answer.
 __device__ __forceinline__ float silu(float g) {
     const float d = fmaf(0.25f, __expf(-g), 0.25f);
     float r;
