@@ -57,6 +57,7 @@ struct Config {
     static constexpr int SMEM_BYTES = NEED < 46 * 1024 + 512 ? 46 * 1024 + 512 : NEED;
     static_assert(CONSUMER_WARPS * ROWS * STAGING_ROW * 4 <= STAGES * W_STAGE_BYTES, "the staging blocks reuse the weight ring");
 };
+constexpr int64_t kOnePassCodes = 6 * 1024 * 1024;  // codes of a weight from which on 17 to 24 rows are one pass (see the plan)
 constexpr int64_t kMaxCounters = 65536;      // arrival counters at the head of the workspace
 constexpr int kPortableCluster = 8;          // what every device runs; beyond it the occupancy query has the last word
 constexpr int kMaxCluster = 16;              // largest cluster of the plan, which leaves out 15 (slices of 12 columns would cover 180)
@@ -181,6 +182,7 @@ struct Params {
     int groups;               // clusters per output tile (splits = groups * cluster size)
     int cols_per;             // columns of a tile each CTA of the cluster owns in the reduction (a multiple of 4)
     int mode;                 // kModeDirect or kModeSplit
+    bool late;                // the weight may be a result of the kernel in front (with two row blocks; three always take it so)
 };
 
 // MT: 8-row blocks of activations per CTA (1: up to 8 rows, 2: up to 16).
@@ -191,9 +193,9 @@ struct Params {
 //     four rows; with fewer one element per thread is one round anyway: (4, 9648, 1568) 7.9 us, 8.05 so).
 // WIDE: clusters beyond the portable size (the eight partials that a smaller one sums at once stay one piece of code without a loop:
 //     (16, 4096, 12288) 12.0 us, 12.4 with it).
-// With 24 rows three CTAs share an SM, and the weight is not asked for ahead of the kernel in front but only fetched into L2 (EARLY): these
-// calls were mostly served by a kernel that waits, and their codes may be that kernel's results ((24, 4096, 4096) 7.6 us with, 8.1 without).
-// Otherwise shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
+// With 17 to 24 rows on weights of kOnePassCodes and more, the weight is not asked for ahead of the kernel in front: these calls were mostly served
+// by a kernel that waits, and their codes may be that kernel's results.  In one pass (EARLY false) it is fetched into L2 meanwhile ((24, 4096, 4096) 7.6 us
+// with, 8.1 without), and three CTAs share an SM.  Otherwise shared memory lets four CTAs share an SM; told so, the compiler takes up to 72 registers where it stopped at 56 (and spilled four
 // bytes in one form): a decode step at 7B widths for one sequence 216 -> 209 us, for sixteen 256 -> 252.
 template <int MT, bool NK, bool QUAD, bool WIDE>
 __global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
@@ -310,6 +312,7 @@ __global__ void __launch_bounds__(THREADS, Config<MT>::CTAS) qlinear_decode_kn_k
             stream_policy = l2_policy_evict_first();  // the weight is read once
             // The weight does not depend on the kernel before this one in the stream; the activations
             // may.  Ask for the first weight tiles, then wait for that kernel, then ask for activations.
+            if (MT == 2 && p.late) pdl_wait();
             for (int it = 0; it < prologue; ++it) {
                 if (EARLY) load_weights(it, it, stream_policy);
                 else tma_prefetch_2d(&map_w, NK ? p.k_begin + (it_begin + it) * BK : n0, NK ? n0 : p.k_begin + (it_begin + it) * BK);
@@ -709,26 +712,34 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // 23.0 -> 14.5, (17, 2304, 6912) 8.3 -> 7.3 against two passes of 16 rows; below the line the passes run side by side ((24, 2048, 2048)
     // 4.0 us, 4.4 in one).  A form for 32 rows was no better than two passes or the mid-M kernel ((32, 4096, 4096) 8.8 and 8.5 us, (32, 4096,
     // 12288) 16.1 and 17.7): the warp-level MMAs of four row blocks take longer than the stream.
-    if (M > 16 && M <= 24 && N * K >= (int64_t)6 * 1024 * 1024) {
-        const Variant &one = kVariants[3];
-        int wide = 1;
-        while (wide < kPortableCluster && wide < max_splits && pl.n_tiles * (wide + 1) <= resident_ctas(one, wide + 1)) ++wide;
-        pl.variant = 3, pl.m_tiles = 1;
-        c = wide, groups = 1;
+    int variant = pl.variant, m_tiles = pl.m_tiles, one = c;  // of the plan with one cluster a tile, of `one` CTAs
+    if (M > 16 && M <= 24 && N * K >= kOnePassCodes) {
+        variant = 3, m_tiles = 1, one = 1;
+        while (one < kPortableCluster && one < max_splits && pl.n_tiles * (one + 1) <= resident_ctas(kVariants[variant], one + 1)) ++one;
     }
     // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
     // takes as long as its chain of waits and loads, not as its bytes ((1, 11008, 4096), 256 CTAs of 22 steps, 11.4 us; 448 of 13, 10.1;
     // (16, 11008, 4096) 12.9 -> 12.0, (1, 16384, 5120) 19.1 -> 16.1; not with three CTAs an SM, (7, 10080, 7088) 14.5 -> 16.8).  Short runs in many parts lose more in the exchange, which grows with the rows: (1, 4096, 4096) 5.0 -> 5.8
     // in sixteen parts of four steps, (16, 5376, 2304) 6.1 -> 6.4.
-    if (pl.m_tiles == 1 && c == kPortableCluster && k_iters >= 48) {
-        const int portable = pl.n_tiles * c;
-        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * c && portable * 4 <= sms * 9;
+    if (m_tiles == 1 && one == kPortableCluster && k_iters >= 48) {
+        const int portable = pl.n_tiles * one;
+        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
-            if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[pl.variant], wide)) continue;
-            c = wide, groups = 1;
+            if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[variant], wide)) continue;
+            one = wide;
             break;
         }
+    }
+    // Several clusters a tile stay where one would leave each CTA so many more steps (0.24 to 0.3 us each) that the three trips through L2 cost less;
+    // what goes through L2 grows with the tiles and the rows.  Over 378 sizes of K 16384 to 65536 and N 16 to 1536 within 0.7 % of the better
+    // one: (1, 65536, 128) 8.4 us in eight clusters a tile, 17.2 in one; (16, 32768, 256) 8.7 and 10.8, (24, 65536, 512) 17.6 and 22.3;
+    // but (8, 16384, 512) 6.4 and 6.0, (16, 24576, 768) 11.7 and 9.2, (24, 24576, 512) 11.7 and 10.0.
+    const double extra = 8.0 + 1.4 * (double)tiles + (M <= 8 ? 0.0 : (M <= 16 ? 0.8 * (double)(M - 9) : 2.0));
+    const bool other = one > c || m_tiles != pl.m_tiles;
+    if (other && (groups == 1 || (double)(ceil_div(k_iters, one) - ceil_div(k_iters, c * groups)) <= extra)) {
+        pl.variant = variant, pl.m_tiles = m_tiles;
+        c = one, groups = 1;
     }
     pl.cluster = c;
     pl.groups = groups;
@@ -797,6 +808,7 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     p.groups = pl.groups;
     p.cols_per = (int)round_up(ceil_div(BN, pl.cluster), pl.cluster <= kPortableCluster ? 8 : 4);
     p.mode = pl.splits == 1 ? kModeDirect : kModeSplit;
+    p.late = M > 16 && M <= 24 && N * (k_end - k_begin) >= kOnePassCodes;
 
     const Variant &v = kVariants[pl.variant];
     const void *kernel = v.kernel[weight_nk][pl.cluster > kPortableCluster];
