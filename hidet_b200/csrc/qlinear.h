@@ -53,11 +53,14 @@ struct DecodePlan {
     int cluster = 1;           // of them, this many form a thread-block cluster that needs no workspace
     int groups = 1;            // clusters per tile; > 1: the clusters meet in the workspace
     int iters_per_split = 0;   // 64-row k steps each of them takes
+    int most_splits = 1;       // as many as K has work for
     size_t counter_bytes = 0;  // head of the workspace: one arrival counter per output tile
     size_t partial_bytes = 0;  // then [groups][M][N] fp32 partial sums.  Both are asked of the caller where clusters of the portable size
                                // would meet in the workspace, also where larger ones (groups == 1) do without
 };
 
+// Codes of a weight from which on 17 to 24 rows are one pass.
+constexpr int64_t kOnePassCodes = 6 * 1024 * 1024;
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K);
 
 // True when the TMA-based [K, N] kernel can take these operands (16-byte aligned bases and rows).

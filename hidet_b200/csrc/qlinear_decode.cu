@@ -57,7 +57,6 @@ struct Config {
     static constexpr int SMEM_BYTES = NEED < 46 * 1024 + 512 ? 46 * 1024 + 512 : NEED;
     static_assert(CONSUMER_WARPS * ROWS * STAGING_ROW * 4 <= STAGES * W_STAGE_BYTES, "the staging blocks reuse the weight ring");
 };
-constexpr int64_t kOnePassCodes = 6 * 1024 * 1024;  // codes of a weight from which on 17 to 24 rows are one pass (see the plan)
 constexpr int64_t kMaxCounters = 65536;      // arrival counters at the head of the workspace
 constexpr int kPortableCluster = 8;          // what every device runs; beyond it the occupancy query has the last word
 constexpr int kMaxCluster = 16;              // largest cluster of the plan, which leaves out 15 (slices of 12 columns would cover 180)
@@ -721,10 +720,10 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
     // takes as long as its chain of waits and loads, not as its bytes ((1, 11008, 4096), 256 CTAs of 22 steps, 11.4 us; 448 of 13, 10.1;
     // (16, 11008, 4096) 12.9 -> 12.0, (1, 16384, 5120) 19.1 -> 16.1; not with three CTAs an SM, (7, 10080, 7088) 14.5 -> 16.8).  Short runs in many parts lose more in the exchange, which grows with the rows: (1, 4096, 4096) 5.0 -> 5.8
-    // in sixteen parts of four steps, (16, 5376, 2304) 6.1 -> 6.4.
+    // in sixteen parts of four steps, (16, 5376, 2304) 6.1 -> 6.4, (24, 4608, 1536) 5.3 -> 6.1 ((24, 5120, 1280) 5.6 -> 5.1).
     if (m_tiles == 1 && one == kPortableCluster && k_iters >= 48) {
         const int portable = pl.n_tiles * one;
-        const bool narrow = M <= 8 ? portable <= sms : portable * 3 <= sms * 2, deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
+        const bool narrow = M <= 8 ? portable <= sms : (M <= 16 ? portable * 3 <= sms * 2 : portable * 11 <= sms * 6), deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
             if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[variant], wide)) continue;
             one = wide;
@@ -743,6 +742,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     }
     pl.cluster = c;
     pl.groups = groups;
+    pl.most_splits = max_splits;
     pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
     pl.iters_per_split = (int)ceil_div(k_iters, pl.splits);
     return pl;

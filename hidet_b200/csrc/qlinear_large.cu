@@ -3,8 +3,7 @@
 // The choice is by estimated time, in microseconds; the constants are measured (B200, graph replay of weights that exceed L2) and
 // stand beside what they describe.  Over 580 drawn sizes of 25 to 2048 rows it is 1.1 % behind the best kernel, tile and cluster that were
 // timed for each (10 % with estimates that left the epilogue out and took the SMs for evenly filled).  The small-M kernel stays for what it
-// does better: up to 24 rows always (24 rows, small-M against the better of the others: (4096, 12288) 14.5 and 17.5 us,
-// (4096, 22016) 24.8 and 29.8, (11008, 4096) 15.0 and 17.5, (1024, 1024) 3.1 and 5.2).
+// does better: up to 16 rows always, and up to 24 where one pass fills the SMs (see mid_instead_of_one_pass).
 #include "common.cuh"
 #include "qlinear.h"
 
@@ -93,14 +92,34 @@ bool codes_may_be_late(int64_t M, int64_t N, int64_t K) {
     return best <= 0.85 * small_m_us(M, N, K);
 }
 
+// 17 to 24 rows, which the small-M kernel takes in one pass: the mid-M kernel where that pass leaves the SMs thinly filled.  Its CTAs need about 0.62 us
+// a 64-k step whether two or three share an SM, so time is its steps, and the mid-M kernel with as many CTAs is faster.  24 rows, one pass and mid M:
+//   at most two CTAs an SM although K has work for more splits: (4096, 32000) 42.4 and 29.4 us, (8192, 28672) 76.8 and 53.0, (2048, 18432) 14.0
+//     and 11.3; otherwise one pass is ahead, (4096, 12288) 13.8 and 16.6, (4096, 26624) 24.5 and 28.8, (1024, 8192) 6.1 and 6.6;
+//   a second wave that is not full, in two of the mid-M kernel: (4096, 57344) 63.5 and 57.1, (4096, 65536) 65.3 and 59.1; (4096, 50000) 45.3 and 54.7,
+//     (1760, 76368) 37.9 and 43.2;
+//   long K, over at least two thirds as many CTAs: (28672, 4096) 31.1 and 27.4, (14336, 16384) 50.4 and 46.8; (28672, 12288) 73.2 and 88.7 with half.
+bool mid_instead_of_one_pass(int64_t K, const DecodePlan &one, int mid_cluster) {
+    const int64_t sms = sm_count() > 0 ? sm_count() : 148, ctas = (int64_t)one.n_tiles * one.splits, mid_ctas = (int64_t)one.n_tiles * mid_cluster;
+    const bool thin = one.splits < 8 && one.splits < one.most_splits && ctas <= 2 * sms;
+    const bool second_wave = one.n_tiles > 3 * sms && one.n_tiles <= 4 * sms && K >= 512;
+    const bool deep = K >= 12288 && mid_ctas <= 2 * sms && 3 * mid_ctas >= 2 * ctas;
+    return thin || second_wave || deep;
+}
+
 }  // namespace
 
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk) {
     LargePlan p;
-    if (M <= 24) return p;
+    if (M <= 16 || (M <= 24 && N * K < kOnePassCodes)) return p;
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
     const bool mid_takes = M <= (int64_t)65535 * 128;  // the grid's limit
     const double mid = mid_takes ? mid_us(M, N, K, silu, weight_nk, &mid_tm, &mid_cluster) : 1e30;
+    if (M <= 24) {
+        const DecodePlan one = plan_decode(M, N, K);
+        if (one.m_tiles == 1 && mid_instead_of_one_pass(K, one, mid_cluster)) p.kind = LargePlan::kMid, p.tm = mid_tm, p.cluster = mid_cluster;
+        return p;
+    }
     // What was measured of the kernel on SM pairs ends at K = 256 and at columns that fill one tile and a sliver of another: below, the mid-M
     // kernel stays as long as its tiles run at once.
     const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -125,7 +144,7 @@ int check_large_outputs(const OutTargets &out) {
 
 bool try_large(const void *a, const void *wq, const void *scale, const OutTargets &c, int64_t M, int64_t N, int64_t K, cudaStream_t stream, const Epilogue *epilogue,
                bool weight_nk, int64_t lda, size_t scratch_bytes, int *rc) {
-    if (M <= 24 || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
+    if (M <= 16 || (M <= 24 && N * K < kOnePassCodes) || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
     const bool only = use_prefill_kernel(M, N, K);  // the small-M kernel is out of the question
     if (!only) {
         const DecodePlan dp = plan_decode(M, N, K);

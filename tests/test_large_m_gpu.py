@@ -204,3 +204,14 @@ def test_outputs_that_16_byte_stores_cannot_write(ldc, col0, base):
             want = (a.double() @ wq.double()) * scale.double()
             assert float((rows[:, col0:col0 + n].double() - want).abs().max()) <= 2.0 ** -11 * 1.01 * float(want.abs().max())
             assert bool((rows[:, :col0] == -7.0).all()) and bool((rows[:, col0 + n:] == -7.0).all())
+
+
+# 17 to 24 rows: where one pass of the small-M kernel fills the SMs thinly, in a second wave that is not full, and with long K; and beside those lines
+@pytest.mark.parametrize('kind,m,k,n', [(MID, 20, 1024, 32000), (MID, 17, 256, 28688), (MID, 24, 2056, 18432), (MID, 24, 512, 57344), (MID, 18, 520, 65552), (MID, 24, 14336, 4096),
+                                        (SMALL, 24, 1024, 12288), (SMALL, 24, 512, 26624), (SMALL, 17, 512, 43008), (SMALL, 24, 1024, 8192), (SMALL, 20, 128, 96000), (SMALL, 24, 14336, 1024)])
+def test_17_to_24_rows(large_kernels, kind, m, k, n):
+    assert _plan(large_kernels, m, k, n) == kind
+    _run(m, k, n, 'KN')
+    _run(m, k, n, 'KN', bias=True, silu=True, residual=True)
+    if k % 16 == 0:
+        _run(m, k, n - 8, 'NK')
