@@ -62,6 +62,7 @@ struct DecodePlan {
 // Codes of a weight from which on 17 to 24 rows are one pass.
 constexpr int64_t kOnePassCodes = 6 * 1024 * 1024;
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K);
+DecodePlan plan_decode_portable(int64_t M, int64_t N, int64_t K);  // the same scratch, for less
 
 // True when the TMA-based [K, N] kernel can take these operands (16-byte aligned bases and rows).
 bool decode_kn_supported(const void *a, const void *wq, int64_t N, int64_t K);

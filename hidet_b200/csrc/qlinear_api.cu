@@ -63,7 +63,7 @@ B200Q_API size_t b200q_qlinear_workspace_bytes(int64_t M, int64_t N, int64_t K, 
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     // Of the kernels behind the entry points that take this workspace the small-M one alone uses it.  It may serve any M: operands
     // that the kernels for more rows cannot take (alignment is not known here) go to it.
-    const DecodePlan pl = plan_decode(M, N, K);
+    const DecodePlan pl = plan_decode_portable(M, N, K);
     return pl.counter_bytes + pl.partial_bytes;
 }
 

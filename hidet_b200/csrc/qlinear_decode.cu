@@ -639,19 +639,27 @@ static int set_attributes() {
     return B200Q_OK;
 }
 
+// The current device, asked once a plan: a plan looks at up to fifteen cluster sizes, and a call makes several plans.  -1: none.
+static int current_device() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) return dev;
+    cudaGetLastError();
+    return -1;
+}
+
 // CTAs of a variant that run at once in clusters of `cluster`: four per SM less what the clusters cannot use.  Looked up once
 // per device; without a device, an estimate (none of clusters that not every device runs: the plan does without them).
-static int resident_ctas(const Variant &v, int cluster) {
+static int resident_ctas(int dev, const Variant &v, int cluster) {
     static std::atomic<int> known[64][kVariantCount][kMaxCluster + 1];
     const int estimate = cluster <= kPortableCluster ? (148 - 8) * v.ctas : 0;
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || set_attributes() != B200Q_OK) {
-        cudaGetLastError();
-        return estimate;
-    }
+    if (dev < 0) return estimate;
     std::atomic<int> &slot = known[dev][&v - kVariants][cluster];
     int n = slot.load(std::memory_order_relaxed);
     if (n != 0) return n;
+    if (set_attributes() != B200Q_OK) {
+        cudaGetLastError();
+        return estimate;
+    }
     n = resident_clusters(v.kernel[0][cluster > kPortableCluster], THREADS, v.smem, cluster);
     if (n == 0) return estimate;
     n *= cluster;
@@ -661,16 +669,16 @@ static int resident_ctas(const Variant &v, int cluster) {
 
 }  // namespace decode
 
-// Split plan shared by the workspace query and the launch.
-DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
+// The plan that every device can run: blocks of up to 16 rows, clusters of up to eight CTAs.  The scratch that callers are asked for is this
+// plan's, whether the one that is launched needs any or not.
+DecodePlan plan_decode_portable(int64_t M, int64_t N, int64_t K) {
     using namespace decode;
     DecodePlan pl;
     pl.n_tiles = (int)ceil_div(N, BN);
     const int k_iters = (int)ceil_div(K, BK);
     int sms = sm_count();
     if (sms <= 0) sms = 148;
-    // What every device can run: blocks of up to 16 rows, clusters of up to eight CTAs.  The scratch that callers are asked for is this
-    // plan's, whether the one below it that is launched needs any or not.
+    const int dev = current_device();
     const Variant &v = kVariants[M <= 4 ? 0 : (M <= 8 ? 1 : 2)];
     pl.variant = (int)(&v - kVariants);
     pl.m_tiles = (int)ceil_div(M, v.rows);
@@ -688,7 +696,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // (1, 4096, 12288) 15.1 us, and 10.3 us in clusters of five).
     int c = 1;
     // (With several row blocks the second pass over the weight comes from L2 and a second wave costs little.)
-    while (c < kPortableCluster && c < max_splits && tiles * (c + 1) <= (pl.m_tiles > 1 ? (int64_t)sms * v.ctas : resident_ctas(v, c + 1))) ++c;
+    while (c < kPortableCluster && c < max_splits && tiles * (c + 1) <= (pl.m_tiles > 1 ? (int64_t)sms * v.ctas : resident_ctas(dev, v, c + 1))) ++c;
     // More splits than a cluster holds become several full clusters per tile that meet in the workspace.  They pay three
     // dependent trips through L2 at the end of the launch (publish, count, read back), about 3 us more than partials
     // that meet in distributed shared memory.  That is worth it only when one cluster per tile would leave most of the
@@ -707,6 +715,22 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // another shape used for partial sums: the region stays all-zero between calls.
     pl.counter_bytes = groups > 1 ? (size_t)kMaxCounters * 4 : 0;
     pl.partial_bytes = groups > 1 ? (size_t)groups * M * N * 4 : 0;
+    pl.cluster = c;
+    pl.groups = groups;
+    pl.most_splits = max_splits;
+    pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
+    pl.iters_per_split = (int)ceil_div(k_iters, pl.splits);
+    return pl;
+}
+
+// The plan that is launched.
+DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
+    using namespace decode;
+    DecodePlan pl = plan_decode_portable(M, N, K);
+    const int k_iters = (int)ceil_div(K, BK), c = pl.cluster, groups = pl.groups;
+    int sms = sm_count();
+    if (sms <= 0) sms = 148;
+    const int dev = current_device();
     // Up to 24 rows in one pass where the weight is more than what L2 delivers again for nothing: (24, 4096, 4096) 8.5 -> 8.2 us, (24, 4096, 12288)
     // 23.0 -> 14.5, (17, 2304, 6912) 8.3 -> 7.3 against two passes of 16 rows; below the line the passes run side by side ((24, 2048, 2048)
     // 4.0 us, 4.4 in one).  A form for 32 rows was no better than two passes or the mid-M kernel ((32, 4096, 4096) 8.8 and 8.5 us, (32, 4096,
@@ -714,7 +738,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     int variant = pl.variant, m_tiles = pl.m_tiles, one = c;  // of the plan with one cluster a tile, of `one` CTAs
     if (M > 16 && M <= 24 && N * K >= kOnePassCodes) {
         variant = 3, m_tiles = 1, one = 1;
-        while (one < kPortableCluster && one < max_splits && pl.n_tiles * (one + 1) <= resident_ctas(kVariants[variant], one + 1)) ++one;
+        while (one < kPortableCluster && one < pl.most_splits && pl.n_tiles * (one + 1) <= resident_ctas(dev, kVariants[variant], one + 1)) ++one;
     }
     // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
@@ -725,7 +749,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
         const int portable = pl.n_tiles * one;
         const bool narrow = M <= 8 ? portable <= sms : (M <= 16 ? portable * 3 <= sms * 2 : portable * 11 <= sms * 6), deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
-            if (wide == 15 || pl.n_tiles * wide > resident_ctas(kVariants[variant], wide)) continue;
+            if (wide == 15 || pl.n_tiles * wide > resident_ctas(dev, kVariants[variant], wide)) continue;
             one = wide;
             break;
         }
@@ -734,17 +758,13 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // what goes through L2 grows with the tiles and the rows.  Over 378 sizes of K 16384 to 65536 and N 16 to 1536 within 0.7 % of the better
     // one: (1, 65536, 128) 8.4 us in eight clusters a tile, 17.2 in one; (16, 32768, 256) 8.7 and 10.8, (24, 65536, 512) 17.6 and 22.3;
     // but (8, 16384, 512) 6.4 and 6.0, (16, 24576, 768) 11.7 and 9.2, (24, 24576, 512) 11.7 and 10.0.
-    const double extra = 8.0 + 1.4 * (double)tiles + (M <= 8 ? 0.0 : (M <= 16 ? 0.8 * (double)(M - 9) : 2.0));
+    const double extra = 8.0 + 1.4 * (double)pl.n_tiles * pl.m_tiles + (M <= 8 ? 0.0 : (M <= 16 ? 0.8 * (double)(M - 9) : 2.0));
     const bool other = one > c || m_tiles != pl.m_tiles;
     if (other && (groups == 1 || (double)(ceil_div(k_iters, one) - ceil_div(k_iters, c * groups)) <= extra)) {
         pl.variant = variant, pl.m_tiles = m_tiles;
-        c = one, groups = 1;
+        pl.cluster = pl.splits = one, pl.groups = 1;
+        pl.iters_per_split = (int)ceil_div(k_iters, one);
     }
-    pl.cluster = c;
-    pl.groups = groups;
-    pl.most_splits = max_splits;
-    pl.splits = c * groups;  // the grid holds whole clusters; a split may get fewer steps than others, or none
-    pl.iters_per_split = (int)ceil_div(k_iters, pl.splits);
     return pl;
 }
 

@@ -3,7 +3,7 @@
 // The choice is by estimated time, in microseconds; the constants are measured (B200, graph replay of weights that exceed L2) and
 // stand beside what they describe.  Over 580 drawn sizes of 25 to 2048 rows it is 1.1 % behind the best kernel, tile and cluster that were
 // timed for each (10 % with estimates that left the epilogue out and took the SMs for evenly filled).  The small-M kernel stays for what it
-// does better: up to 16 rows always, and up to 24 where one pass fills the SMs (see mid_instead_of_one_pass).
+// does better: up to 16 rows always, and up to 24 where one pass fills the SMs (see one_pass_or_mid).
 #include "common.cuh"
 #include "qlinear.h"
 
@@ -82,6 +82,8 @@ double pair_us(int64_t M, int64_t N, int64_t K, bool silu, int *tm) {
 // this rule gave to the kernels for more rows (and, by the roundings below, for 630 of 84 000 drawn ones of 25 to 64 rows that they did not).
 // It is no slower there either: (64, 1536, 6144) 8.4 us, 11.8 in the small-M kernel, (60, 256, 28672) with SiLU 8.3 and 13.4, (51, 1680, 5776) 9.0 and 9.8.
 bool codes_may_be_late(int64_t M, int64_t N, int64_t K) {
+    const double enough = 0.85 * small_m_us(M, N, K);
+    if (enough < 4.8) return false;  // the least that any size takes below
     const int sms = sm_count() > 0 ? sm_count() : 148;
     const int64_t tiles = ceil_div(N, 128), k_blocks = ceil_div(K, 64);
     double best = M > 32 ? 4.5 + (double)ceil_div(ceil_div(N, 256), sms / 2) * ((double)k_blocks * 0.262 + 0.3) : 1e30;
@@ -89,7 +91,7 @@ bool codes_may_be_late(int64_t M, int64_t N, int64_t K) {
         const double us = 4.2 + 0.3 * c + (double)ceil_div(tiles * c, 2 * sms) * (double)ceil_div(k_blocks, c) * (tiles * c <= sms ? 0.30 : 0.46);
         if (us < best) best = us;
     }
-    return best <= 0.85 * small_m_us(M, N, K);
+    return best <= enough;
 }
 
 // 17 to 24 rows, which the small-M kernel takes in one pass: the mid-M kernel where that pass leaves the SMs thinly filled.  Its CTAs need about 0.62 us
@@ -99,12 +101,19 @@ bool codes_may_be_late(int64_t M, int64_t N, int64_t K) {
 //   a second wave that is not full, in two of the mid-M kernel: (4096, 57344) 63.5 and 57.1, (4096, 65536) 65.3 and 59.1; (4096, 50000) 45.3 and 54.7,
 //     (1760, 76368) 37.9 and 43.2;
 //   long K, over at least two thirds as many CTAs: (28672, 4096) 31.1 and 27.4, (14336, 16384) 50.4 and 46.8; (28672, 12288) 73.2 and 88.7 with half.
-bool mid_instead_of_one_pass(int64_t K, const DecodePlan &one, int mid_cluster) {
-    const int64_t sms = sm_count() > 0 ? sm_count() : 148, ctas = (int64_t)one.n_tiles * one.splits, mid_ctas = (int64_t)one.n_tiles * mid_cluster;
+LargePlan one_pass_or_mid(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk) {
+    LargePlan p;
+    const DecodePlan one = plan_decode(M, N, K);
+    const int64_t sms = sm_count() > 0 ? sm_count() : 148, ctas = (int64_t)one.n_tiles * one.splits;
     const bool thin = one.splits < 8 && one.splits < one.most_splits && ctas <= 2 * sms;
     const bool second_wave = one.n_tiles > 3 * sms && one.n_tiles <= 4 * sms && K >= 512;
+    if (one.m_tiles != 1 || !(thin || second_wave || K >= 12288)) return p;
+    int tm = 0, cluster = 1;
+    mid_us(M, N, K, silu, weight_nk, &tm, &cluster);
+    const int64_t mid_ctas = (int64_t)one.n_tiles * cluster;
     const bool deep = K >= 12288 && mid_ctas <= 2 * sms && 3 * mid_ctas >= 2 * ctas;
-    return thin || second_wave || deep;
+    if (thin || second_wave || deep) p.kind = LargePlan::kMid, p.tm = tm, p.cluster = cluster;
+    return p;
 }
 
 }  // namespace
@@ -112,14 +121,10 @@ bool mid_instead_of_one_pass(int64_t K, const DecodePlan &one, int mid_cluster) 
 LargePlan plan_large(int64_t M, int64_t N, int64_t K, bool silu, bool weight_nk) {
     LargePlan p;
     if (M <= 16 || (M <= 24 && N * K < kOnePassCodes)) return p;
+    if (M <= 24) return one_pass_or_mid(M, N, K, silu, weight_nk);
     int mid_tm = 0, mid_cluster = 1, pair_tm = 0;
     const bool mid_takes = M <= (int64_t)65535 * 128;  // the grid's limit
     const double mid = mid_takes ? mid_us(M, N, K, silu, weight_nk, &mid_tm, &mid_cluster) : 1e30;
-    if (M <= 24) {
-        const DecodePlan one = plan_decode(M, N, K);
-        if (one.m_tiles == 1 && mid_instead_of_one_pass(K, one, mid_cluster)) p.kind = LargePlan::kMid, p.tm = mid_tm, p.cluster = mid_cluster;
-        return p;
-    }
     // What was measured of the kernel on SM pairs ends at K = 256 and at columns that fill one tile and a sliver of another: below, the mid-M
     // kernel stays as long as its tiles run at once.
     const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -147,7 +152,7 @@ bool try_large(const void *a, const void *wq, const void *scale, const OutTarget
     if (M <= 16 || (M <= 24 && N * K < kOnePassCodes) || !(weight_nk ? prefill_nk_supported(a, wq, N, K) : prefill_kn_supported(a, wq, N, K))) return false;
     const bool only = use_prefill_kernel(M, N, K);  // the small-M kernel is out of the question
     if (!only) {
-        const DecodePlan dp = plan_decode(M, N, K);
+        const DecodePlan dp = plan_decode_portable(M, N, K);
         if (dp.partial_bytes > 0 && scratch_bytes < dp.counter_bytes + dp.partial_bytes) return false;
     }
     const LargePlan plan = plan_large(M, N, K, epilogue != nullptr && epilogue->act == kActSiluMul, weight_nk);

@@ -92,9 +92,10 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
         if (rc != B200Q_OK) return rc;
         // The arrival counters must read zero when the kernel starts.  A completed call leaves them
         // zero, but the array is shared by every caller and survives failed calls, so clear the ones
-        // this problem uses (one per output tile and cluster rank) here.
+        // this problem uses (one per output tile and cluster rank) here; none with one cluster a tile, which asks
+        // for the scratch of the portable plan without using it.
         const size_t used = (size_t)plan.n_tiles * plan.m_tiles * plan.cluster * sizeof(unsigned int);
-        B200Q_CUDA_TRY(cudaMemsetAsync(scratch, 0, used < plan.counter_bytes ? used : plan.counter_bytes, s));
+        if (plan.groups > 1) B200Q_CUDA_TRY(cudaMemsetAsync(scratch, 0, used < plan.counter_bytes ? used : plan.counter_bytes, s));
     }
     return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, scratch, need, s);
 }
