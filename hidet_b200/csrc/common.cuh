@@ -55,6 +55,8 @@ int sm_count();
 // Clusters of `cluster` CTAs (along y) of a kernel that run at once on the current device, asked of the runtime: clusters stay
 // within a group of SMs, so it is less than what the slots add up to.  0 if it cannot be told.
 int resident_clusters(const void *kernel, int threads, int smem, int cluster);
+// True where the stream has only some of the device's SMs (a green context's): launches there may not hold what the device holds.
+bool part_of_device(cudaStream_t stream);
 
 // Encodes a 2-D tiled tensor map.  `inner`/`outer` are the tensor extents in elements, `row_bytes`
 // the stride between consecutive outer indices, box_* the tile extents.  swizzle is a

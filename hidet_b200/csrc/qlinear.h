@@ -63,6 +63,7 @@ struct DecodePlan {
 constexpr int64_t kOnePassCodes = 6 * 1024 * 1024;
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K);
 DecodePlan plan_decode_portable(int64_t M, int64_t N, int64_t K);  // the same scratch, for less
+DecodePlan plan_decode_on(cudaStream_t stream, int64_t M, int64_t N, int64_t K);  // the one that is launched on a stream
 
 // True when the TMA-based [K, N] kernel can take these operands (16-byte aligned bases and rows).
 bool decode_kn_supported(const void *a, const void *wq, int64_t N, int64_t K);

@@ -723,7 +723,7 @@ DecodePlan plan_decode_portable(int64_t M, int64_t N, int64_t K) {
     return pl;
 }
 
-// The plan that is launched.
+// The plan where all SMs are at hand.
 DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     using namespace decode;
     DecodePlan pl = plan_decode_portable(M, N, K);
@@ -768,6 +768,12 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     return pl;
 }
 
+// Clusters beyond the portable size are taken by what the device holds; a part of its SMs may hold none of them, and the launch would fail.
+DecodePlan plan_decode_on(cudaStream_t stream, int64_t M, int64_t N, int64_t K) {
+    const DecodePlan pl = plan_decode(M, N, K);
+    return pl.cluster > decode::kPortableCluster && part_of_device(stream) ? plan_decode_portable(M, N, K) : pl;
+}
+
 bool decode_kn_supported(const void *a, const void *wq, int64_t N, int64_t K) {
     return (N % 16 == 0) && (K % 8 == 0) && ((reinterpret_cast<uintptr_t>(a) & 15u) == 0) &&
            ((reinterpret_cast<uintptr_t>(wq) & 15u) == 0);
@@ -782,7 +788,7 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
                      int64_t k_begin, int64_t k_end, bool allow_split, void *workspace, size_t workspace_bytes,
                      cudaStream_t stream, const OutTargets *targets, const Epilogue *epilogue, bool weight_nk) {
     using namespace decode;
-    DecodePlan pl = plan_decode(M, N, k_end - k_begin);
+    DecodePlan pl = plan_decode_on(stream, M, N, k_end - k_begin);
     if (!allow_split) {
         pl.iters_per_split = (int)ceil_div(k_end - k_begin, BK);
         pl.splits = 1;

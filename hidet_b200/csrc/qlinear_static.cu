@@ -78,7 +78,7 @@ B200Q_API int b200q_qlinear_f16_i8_static(const void *a, const void *wq, const v
     int rc = B200Q_OK;
     if (try_large(a, wq, scale, one_output(c, N), M, N, K, s, nullptr, false, 0, kStaticScratchBytes, &rc)) return rc;
 
-    const DecodePlan plan = plan_decode(M, N, K);
+    const DecodePlan plan = plan_decode_on(s, M, N, K);
     const size_t need = plan.counter_bytes + plan.partial_bytes;
     if (need > kStaticScratchBytes) {
         return set_error(B200Q_WORKSPACE_TOO_SMALL,

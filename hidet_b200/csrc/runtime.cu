@@ -101,6 +101,19 @@ int resident_clusters(const void *kernel, int threads, int smem, int cluster) {
     return n;
 }
 
+bool part_of_device(cudaStream_t stream) {
+    typedef CUresult (*GetGreenCtxFn)(CUstream, CUgreenCtx *);
+    static GetGreenCtxFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, []() {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuStreamGetGreenCtx", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess) fn = reinterpret_cast<GetGreenCtxFn>(p);
+    });
+    CUgreenCtx green = nullptr;
+    return fn != nullptr && fn(stream, &green) == CUDA_SUCCESS && green != nullptr;
+}
+
 int make_tensor_map_2d(CUtensorMap *map, CUtensorMapDataType dtype, const void *base, uint64_t inner, uint64_t outer,
                        uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle,
                        CUtensorMapL2promotion promo) {

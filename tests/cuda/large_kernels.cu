@@ -28,6 +28,12 @@ EXPORT void small_plan(int64_t M, int64_t N, int64_t K, int *out) {
     out[0] = (int)((M + p.m_tiles - 1) / p.m_tiles), out[1] = p.cluster, out[2] = p.groups;
 }
 
+// The same for a launch on a stream.
+EXPORT void small_plan_on(cudaStream_t stream, int64_t M, int64_t N, int64_t K, int *out) {
+    const DecodePlan p = plan_decode_on(stream, M, N, K);
+    out[0] = (int)((M + p.m_tiles - 1) / p.m_tiles), out[1] = p.cluster, out[2] = p.groups;
+}
+
 EXPORT int launch(int kind, int tm, int cluster, const void *a, const void *wq, const void *scale, void *const *dst, int count, int64_t ldc, int64_t col0, int64_t M, int64_t N,
                   int64_t K, int64_t lda, int nk, const void *bias, const void *residual, int64_t ldr, int silu, cudaStream_t stream) {
     LargePlan p;
