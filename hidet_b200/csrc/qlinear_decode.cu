@@ -728,6 +728,8 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     using namespace decode;
     DecodePlan pl = plan_decode_portable(M, N, K);
     const int k_iters = (int)ceil_div(K, BK), c = pl.cluster, groups = pl.groups;
+    const bool one_pass = M > 16 && M <= 24 && N * K >= kOnePassCodes;
+    if (!one_pass && (pl.m_tiles > 1 || c < kPortableCluster || k_iters < 48)) return pl;
     int sms = sm_count();
     if (sms <= 0) sms = 148;
     const int dev = current_device();
@@ -736,7 +738,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // 4.0 us, 4.4 in one).  A form for 32 rows was no better than two passes or the mid-M kernel ((32, 4096, 4096) 8.8 and 8.5 us, (32, 4096,
     // 12288) 16.1 and 17.7): the warp-level MMAs of four row blocks take longer than the stream.
     int variant = pl.variant, m_tiles = pl.m_tiles, one = c;  // of the plan with one cluster a tile, of `one` CTAs
-    if (M > 16 && M <= 24 && N * K >= kOnePassCodes) {
+    if (one_pass) {
         variant = 3, m_tiles = 1, one = 1;
         while (one < kPortableCluster && one < pl.most_splits && pl.n_tiles * (one + 1) <= resident_ctas(dev, kVariants[variant], one + 1)) ++one;
     }
