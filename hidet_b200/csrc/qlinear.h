@@ -71,7 +71,8 @@ bool decode_kn_supported(const void *a, const void *wq, int64_t N, int64_t K);
 // c[M, N] = scale * (a[:, k_begin:k_end] x wq[k_begin:k_end, :]).  K is the row length of `a`.
 int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K,
                      int64_t k_begin, int64_t k_end, bool allow_split, void *workspace, size_t workspace_bytes,
-                     cudaStream_t stream, const OutTargets *targets = nullptr, const Epilogue *epilogue = nullptr, bool weight_nk = false);
+                     cudaStream_t stream, const OutTargets *targets = nullptr, const Epilogue *epilogue = nullptr, bool weight_nk = false,
+                     const DecodePlan *plan = nullptr);  // plan: instead of the one that plan_decode_on makes
 // The same kernel on a weight stored [N, K] (weight_nk = true): needs 16-byte aligned bases and K % 16 == 0.
 bool decode_nk_supported(const void *a, const void *wq, int64_t N, int64_t K);
 

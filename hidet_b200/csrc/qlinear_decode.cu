@@ -39,7 +39,7 @@ constexpr int STAGES = 4;
 constexpr int CONSUMER_WARPS = 4;            // each owns BN / 4 = 32 columns
 constexpr int THREADS = 32 * (CONSUMER_WARPS + 1);
 constexpr int W_STAGE_BYTES = BK * BN;       // 8192
-constexpr int RECV_COLS = 168;               // most columns the slices of a cluster cover together (7 ranks x 24 columns, 14 x 12)
+constexpr int RECV_COLS = 168;               // most columns the slices of a cluster cover together (7 ranks x 24 columns, 14 x 12; see slices_fit)
 constexpr int STAGING_ROW = 36;              // floats per row of a warp's 32-column staging block (padded: conflict-free)
 
 // Shared memory of a CTA with MT blocks of eight activation rows.
@@ -59,7 +59,17 @@ struct Config {
 };
 constexpr int64_t kMaxCounters = 65536;      // arrival counters at the head of the workspace
 constexpr int kPortableCluster = 8;          // what every device runs; beyond it the occupancy query has the last word
-constexpr int kMaxCluster = 16;              // largest cluster of the plan, which leaves out 15 (slices of 12 columns would cover 180)
+constexpr int kMaxCluster = 16;              // largest cluster of the plan
+// Columns of a tile that each CTA of a cluster owns, and whether a rank's slices from all of them have their place in the receive buffer (not
+// those of 15 CTAs, 12 columns each).
+constexpr int slice_cols(int cluster) {
+    const int step = cluster <= kPortableCluster ? 8 : 4;
+    return ((BN + cluster - 1) / cluster + step - 1) / step * step;
+}
+constexpr bool slices_fit(int cluster) { return slice_cols(cluster) * cluster <= RECV_COLS; }
+constexpr bool all_slices_fit(int cluster) { return cluster == 0 || (slices_fit(cluster) && all_slices_fit(cluster - 1)); }
+static_assert(all_slices_fit(kPortableCluster), "clusters up to the portable size are launched unasked");
+static_assert(slices_fit(kMaxCluster), "the largest cluster of the plan");
 
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
@@ -751,7 +761,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
         const int portable = pl.n_tiles * one;
         const bool narrow = M <= 8 ? portable <= sms : (M <= 16 ? portable * 3 <= sms * 2 : portable * 11 <= sms * 6), deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
-            if (wide == 15 || pl.n_tiles * wide > resident_ctas(dev, kVariants[variant], wide)) continue;
+            if (!slices_fit(wide) || pl.n_tiles * wide > resident_ctas(dev, kVariants[variant], wide)) continue;
             one = wide;
             break;
         }
@@ -788,9 +798,10 @@ bool decode_nk_supported(const void *a, const void *wq, int64_t N, int64_t K) {
 
 int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K,
                      int64_t k_begin, int64_t k_end, bool allow_split, void *workspace, size_t workspace_bytes,
-                     cudaStream_t stream, const OutTargets *targets, const Epilogue *epilogue, bool weight_nk) {
+                     cudaStream_t stream, const OutTargets *targets, const Epilogue *epilogue, bool weight_nk, const DecodePlan *plan) {
     using namespace decode;
-    DecodePlan pl = plan_decode_on(stream, M, N, k_end - k_begin);
+    DecodePlan pl = plan != nullptr ? *plan : plan_decode_on(stream, M, N, k_end - k_begin);
+    if (pl.cluster > kMaxCluster || !slices_fit(pl.cluster)) return set_error(B200Q_INVALID_ARGUMENT, "qlinear: no clusters of %d CTAs", pl.cluster);
     if (!allow_split) {
         pl.iters_per_split = (int)ceil_div(k_end - k_begin, BK);
         pl.splits = 1;
@@ -834,7 +845,7 @@ int launch_decode_kn(const void *a, const void *wq, const void *scale, void *c, 
     p.k_end = (int)k_end;
     p.iters_per_split = pl.iters_per_split;
     p.groups = pl.groups;
-    p.cols_per = (int)round_up(ceil_div(BN, pl.cluster), pl.cluster <= kPortableCluster ? 8 : 4);
+    p.cols_per = slice_cols(pl.cluster);
     p.mode = pl.splits == 1 ? kModeDirect : kModeSplit;
     p.late = M > 16 && M <= 24 && N * (k_end - k_begin) >= kOnePassCodes;
 

@@ -34,6 +34,24 @@ EXPORT void small_plan_on(cudaStream_t stream, int64_t M, int64_t N, int64_t K, 
     out[0] = (int)((M + p.m_tiles - 1) / p.m_tiles), out[1] = p.cluster, out[2] = p.groups;
 }
 
+// The small-M kernel in its form for up to 4, 8, 16 or 24 rows a pass (0 to 3) with one cluster of that many CTAs a tile.
+EXPORT int launch_small(int form, int cluster, const void *a, const void *wq, const void *scale, void *c, int64_t M, int64_t N, int64_t K, int nk, const void *bias,
+                        const void *residual, int silu, cudaStream_t stream) {
+    static const int rows[] = {4, 8, 16, 24};
+    DecodePlan p;
+    p.variant = form;
+    p.n_tiles = (int)((N + 127) / 128);
+    p.m_tiles = (int)((M + rows[form] - 1) / rows[form]);
+    p.cluster = p.splits = cluster;
+    p.iters_per_split = (int)(((K + 63) / 64 + cluster - 1) / cluster);
+    Epilogue ep;
+    ep.bias = bias;
+    ep.residual = residual;
+    ep.ldr = silu ? N / 2 : N;
+    ep.act = silu ? kActSiluMul : kActNone;
+    return launch_decode_kn(a, wq, scale, c, M, N, K, 0, K, true, nullptr, 0, stream, nullptr, &ep, nk != 0, &p);
+}
+
 EXPORT int launch(int kind, int tm, int cluster, const void *a, const void *wq, const void *scale, void *const *dst, int count, int64_t ldc, int64_t col0, int64_t M, int64_t N,
                   int64_t K, int64_t lda, int nk, const void *bias, const void *residual, int64_t ldr, int silu, cudaStream_t stream) {
     LargePlan p;

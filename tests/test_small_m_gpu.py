@@ -105,3 +105,38 @@ def test_rows_up_to_24_in_one_pass(large_kernels, m, k, n):
     gate = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
     residual = torch.randn(m, n // 2, device='cuda').half()
     _close(hidet_b200.symmetric_quant_matmul(a, wq, scale, activation='silu_mul', residual=residual), gate + residual.double())
+
+
+# every form in every cluster size that the plan may take, by name: slices of every width, ranks that own no columns, splits that get fewer steps
+# than others or none, rows short of the form's, the last columns
+@pytest.mark.parametrize('cluster', [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16])
+@pytest.mark.parametrize('form,rows', [(0, [1, 2, 4]), (1, [3, 5, 8]), (2, [9, 16, 31]), (3, [17, 20, 24])])
+def test_every_cluster(large_kernels, cluster, form, rows):
+    p, i, n = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
+    launch = large_kernels.launch_small
+    launch.argtypes = [i, i, p, p, p, p, n, n, n, i, p, p, i, p]
+    stream = torch.cuda.current_stream().cuda_stream
+    for m in rows:
+        for k, cols, layout in ((3080, 272, 'KN'), (512, 16, 'KN'), (1040, 391, 'NK')):
+            a, wq, scale, want = _operands(m, k, cols, layout)
+            out = torch.full((m, cols), -7.0, dtype=torch.float16, device='cuda')
+            assert launch(form, cluster, a.data_ptr(), wq.data_ptr(), scale.data_ptr(), out.data_ptr(), m, cols, k, layout == 'NK', None, None, 0, stream) == 0
+            _close(out, want)
+            if cols % 2 == 0:
+                bias, residual = torch.randn(cols, device='cuda').half(), torch.randn(m, cols // 2, device='cuda').half()
+                out = torch.full((m, cols // 2), -7.0, dtype=torch.float16, device='cuda')
+                assert launch(form, cluster, a.data_ptr(), wq.data_ptr(), scale.data_ptr(), out.data_ptr(), m, cols, k, 0, bias.data_ptr(), residual.data_ptr(), 1, stream) == 0
+                y = want + bias.double()
+                _close(out, torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2] + residual.double())
+    assert large_kernels.b200q_check_status() == 0
+
+
+def test_no_clusters_of_fifteen(large_kernels):
+    """Slices of twelve columns from fifteen CTAs would not fit where they are received."""
+    p, i, n = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
+    launch = large_kernels.launch_small
+    launch.argtypes = [i, i, p, p, p, p, n, n, n, i, p, p, i, p]
+    a, wq, scale, _ = _operands(4, 3072, 256, 'KN')
+    out = torch.empty(4, 256, dtype=torch.float16, device='cuda')
+    for cluster in (15, 17):
+        assert launch(0, cluster, a.data_ptr(), wq.data_ptr(), scale.data_ptr(), out.data_ptr(), 4, 256, 3072, 0, None, None, 0, torch.cuda.current_stream().cuda_stream) == ffi.INVALID_ARGUMENT
