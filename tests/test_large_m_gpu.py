@@ -215,3 +215,32 @@ def test_17_to_24_rows(large_kernels, kind, m, k, n):
     _run(m, k, n, 'KN', bias=True, silu=True, residual=True)
     if k % 16 == 0:
         _run(m, k, n - 8, 'NK')
+
+
+# gates at the ends of every range of the epilogue's quotient, in each kernel by name: zeros, where exp(-g) vanishes against 1 and where 1 does
+# against it, where it overflows, infinities and NaN
+@pytest.mark.parametrize('kind,tm,cluster', [(MID, 48, 1), (MID, 128, 3), (PAIR, 96, 1), (PAIR, 256, 1)])
+def test_gates_of_every_magnitude(large_kernels, kind, tm, cluster):
+    gates = torch.tensor([0.0, -0.0, 6e-8, -6e-8, 1e-3, -1e-3, 0.5, -0.5, 1.0, -1.0, 9.0, -9.0, 17.0, -17.0, 87.0, -87.0, 88.5, -88.5, 89.0, -89.0, 104.0, -104.0, 6e4, -6e4,
+                          float('inf'), float('-inf'), float('nan')])
+    m, k, n = tm + 5, 256, 528
+    bias = torch.zeros(n)
+    bias[0::2] = gates.repeat(n // 2 // len(gates) + 1)[:n // 2]
+    bias[1::2] = torch.tensor([1.0, -3.0, 0.25, 1000.0, float('inf')]).repeat(n // 10 + 1)[:n // 2]
+    bias = bias.half().cuda()
+    a, wq, scale = torch.ones(m, k, dtype=torch.float16, device='cuda'), torch.zeros(k, n, dtype=torch.int8, device='cuda'), torch.ones(n, dtype=torch.float16, device='cuda')
+    got = torch.full((m, n // 2), -7.0, dtype=torch.float16, device='cuda')
+    table = (ctypes.c_void_p * 1)(got.data_ptr())
+    assert large_kernels.launch(kind, tm, cluster, a.data_ptr(), wq.data_ptr(), scale.data_ptr(), table, 1, n // 2, 0, m, n, k, k, 0, bias.data_ptr(), None, 0, 1,
+                                torch.cuda.current_stream().cuda_stream) == 0
+    g, u = bias[0::2].double(), bias[1::2].double()
+    want = (g / (1.0 + torch.exp(-g)) * u).half().expand(m, -1)
+    keep = ~((g < -88.7) & u.isinf())   # exp overflows in 32 bits there: 0 x inf, which is -inf in 64
+    got, want = got[:, keep], want[:, keep]
+    assert torch.equal(got.isnan(), want.isnan())
+    finite = want.isfinite()
+    assert torch.equal(got[~finite & ~want.isnan()], want[~finite & ~want.isnan()])
+    # f32 in front of one rounding to f16: an ulp of the value at most, or of the smallest number; exp's own error is 2^-20 of it at 104
+    err = (got.double() - want.double()).abs()[finite]
+    assert bool((err <= 2.0 ** -10 * want.double().abs()[finite] + 2.0 ** -24).all())
+    assert large_kernels.b200q_check_status() == 0
