@@ -344,14 +344,17 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 // grid = (cluster_size, panels); the CTAs of one cluster share blockIdx.y (a panel of PW = TX*VEC
 // columns) and split the rows.  TX threads lie across a panel row, kThreads / TX rows make a sweep.
-// cache != 0: the CTA's rows of the panel are kept in dynamic shared memory between the two phases
+// CACHE: the CTA's rows of the panel are kept in dynamic shared memory between the two phases
 // (with VEC > 1 they are brought there by asynchronous 16-byte copies, all in flight at once, and the
-// absmax is taken from shared memory); cache == 0: phase 2 reads them again from global memory.
+// absmax is taken from shared memory); without, phase 2 reads them again from global memory.
 // Each thread reads back only what it copied itself, so the copies need no barrier.
-template <typename T, typename Q, int VEC, int TX>
-__global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *wq,
+// Two kernels, since the one without holds a batch of vectors in registers: with both in one, four CTAs shared an SM for five and
+// 1353 x 2432 f16 took 7.3 us for 5.6.  The one without gains from registers (one CTA asked for an SM, 100000 x 512 f32 129 us -> 106); element by
+// element it is CTAs that count (eight an SM, 1000 x 40001 f32 per row 96 -> 73).
+template <typename T, typename Q, int VEC, int TX, bool CACHE>
+__global__ void __launch_bounds__(kThreads, VEC == 1 ? 8 : (CACHE ? 0 : 1)) quantize_cols_kernel(const T *w, Q *wq,
                                                                  T *scale, int64_t rows, int64_t cols,
-                                                                 int64_t rows_per_cta, int cache) {
+                                                                 int64_t rows_per_cta) {
     constexpr int TY = kThreads / TX;          // rows per sweep
     constexpr int PW = TX * VEC;               // panel width in elements
     constexpr int WARPS = kThreads / 32;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
     acc.init();
     if (col_ok) {
         const T *src = w + (row0 + ty) * cols + col;
-        if (ASYNC && cache) {
+        if (ASYNC && CACHE) {
             uint32_t dst = smem_u32(tile) + (uint32_t)((ty * PW + tx * VEC) * sizeof(T));
             for (int r = ty; r < nrows; r += TY, src += sweep, dst += (uint32_t)(TY * PW * sizeof(T))) copy_async_16(dst, src);
             copy_async_wait_all();
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
 #pragma unroll 4
             for (int r = ty; r < nrows; r += TY, src += sweep, t += TY * PW) {
                 Vec<T, VEC> x = load_vec<T, VEC>(src);
-                if (cache) store_vec<T, VEC>(t, x);
+                if (CACHE) store_vec<T, VEC>(t, x);
                 acc.add(x);
             }
         }
@@ -441,7 +444,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
         for (int i = 0; i < VEC; ++i) s[i] = div_s[tx * VEC + i];
         const T *src = w + (row0 + ty) * cols + col;
         Q *dst = wq + (row0 + ty) * cols + col;
-        if (cache) {
+        if (CACHE) {
             const T *t = tile + ty * PW + tx * VEC;
 #pragma unroll 4
             for (int r = ty; r < nrows; r += TY, dst += sweep, t += TY * PW) {
@@ -451,18 +454,22 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const T *w, Q *
             }
         } else {
             constexpr int BATCH = 4;
-            for (int left = nrows - ty; left > 0; left -= BATCH * TY, src += BATCH * sweep, dst += BATCH * sweep) {
+            int left = nrows - ty;
+            for (; left > (BATCH - 1) * TY; left -= BATCH * TY, src += BATCH * sweep, dst += BATCH * sweep) {
                 Vec<T, VEC> x[BATCH];
 #pragma unroll
-                for (int i = 0; i < BATCH; ++i)
-                    if (i * TY < left) x[i] = load_vec<T, VEC>(src + i * sweep);
+                for (int i = 0; i < BATCH; ++i) x[i] = load_vec<T, VEC>(src + i * sweep);
 #pragma unroll
                 for (int i = 0; i < BATCH; ++i) {
-                    if (i * TY >= left) break;
                     Vec<Q, VEC> q;
                     QuantVec<T, Q, VEC, typename A::Divisor>::template run<true>(x[i], s, q);
                     store_vec<Q, VEC>(dst + i * sweep, q);
                 }
+            }
+            for (; left > 0; left -= TY, src += sweep, dst += sweep) {
+                Vec<Q, VEC> q;
+                QuantVec<T, Q, VEC, typename A::Divisor>::template run<true>(load_vec<T, VEC>(src), s, q);
+                store_vec<Q, VEC>(dst, q);
             }
         }
     }
@@ -482,7 +489,7 @@ __device__ __forceinline__ T warp_max(T a) {
 // REG_CHUNKS: vectors of the row each thread keeps in registers between the two phases; rows longer
 // than blockDim * VEC * REG_CHUNKS read the remainder again (it is in L1/L2 by then).
 template <typename T, typename Q, int VEC, int REG_CHUNKS>
-__global__ void __launch_bounds__(kThreads) quantize_rows_kernel(const T *w, Q *wq,
+__global__ void __launch_bounds__(kThreads, VEC == 1 ? 8 : 0) quantize_rows_kernel(const T *w, Q *wq,
                                                                  T *scale, int64_t rows, int64_t cols) {
     using A = Arith<T>;
     __shared__ T warp_part[kThreads / 32];
@@ -536,18 +543,22 @@ __global__ void __launch_bounds__(kThreads) quantize_rows_kernel(const T *w, Q *
         }
     }
     constexpr int BATCH = 4;
-    for (int64_t i = threadIdx.x + REG_CHUNKS * stride; i < nvec; i += BATCH * stride) {
+    int64_t i = threadIdx.x + REG_CHUNKS * stride;
+    for (; i + (BATCH - 1) * stride < nvec; i += BATCH * stride) {
         Vec<T, VEC> x[BATCH];
 #pragma unroll
-        for (int j = 0; j < BATCH; ++j)
-            if (i + j * stride < nvec) x[j] = load_vec<T, VEC>(src + (i + j * stride) * VEC);
+        for (int j = 0; j < BATCH; ++j) x[j] = load_vec<T, VEC>(src + (i + j * stride) * VEC);
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
-            if (i + j * stride >= nvec) break;
             Vec<Q, VEC> q;
             QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(x[j], &s, q);
             store_vec<Q, VEC>(dst + (i + j * stride) * VEC, q);
         }
+    }
+    for (; i < nvec; i += stride) {
+        Vec<Q, VEC> q;
+        QuantVec<T, Q, VEC, typename A::Divisor>::template run<false>(load_vec<T, VEC>(src + i * VEC), &s, q);
+        store_vec<Q, VEC>(dst + i * VEC, q);
     }
 }
 
@@ -925,17 +936,22 @@ int launch_quantize_cols(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols
     int cluster = kMaxCluster;
     while (cluster > 1 && ceil_div(rows, cluster) < TY) cluster >>= 1;
     const int64_t rows_per_cta = ceil_div(rows, cluster);
-    size_t tile_bytes = (size_t)rows_per_cta * PW * sizeof(T);
-    int cache = 1;
-    if (tile_bytes > kMaxTileBytes) {
-        cache = 0;
-        tile_bytes = 0;
-    }
-    auto kernel = quantize_cols_kernel<T, Q, VEC, TX>;
+    const size_t tile_bytes = (size_t)rows_per_cta * PW * sizeof(T);
+    const dim3 grid((unsigned)cluster, (unsigned)panels, 1);
+    if (tile_bytes > kMaxTileBytes) return launch_dependent("quantize_cols_kernel", quantize_cols_kernel<T, Q, VEC, TX, false>, grid, kThreads, 0, cluster, stream, w, wq, scale, rows, cols, rows_per_cta);
+    auto kernel = quantize_cols_kernel<T, Q, VEC, TX, true>;
     if (tile_bytes > kDefaultTileBytes) {
         B200Q_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxTileBytes));
     }
-    return launch_dependent("quantize_cols_kernel", kernel, dim3((unsigned)cluster, (unsigned)panels, 1), kThreads, tile_bytes, cluster, stream, w, wq, scale, rows, cols, rows_per_cta, cache);
+    // Slices of about 32 KB leave six CTAs an SM.  Five are better where the sixth would empty the second wave but for a sliver (4096 x 4096 f16
+    // 15.0 us with six, 14.3 with five), not where it is well filled or there are more (3800 x 5000 18.0 and 18.9, 4096 x 4096 f32 23.8 and 25.4,
+    // 4096 x 14336 f16 39.1 and 39.5).
+    size_t ask = tile_bytes;
+    if (VEC > 1 && tile_bytes > 28 * 1024 && tile_bytes < 37 * 1024) {
+        const int64_t wave = 6 * (int64_t)sm_count(), ctas = cluster * panels;
+        if (wave > 0 && ctas > wave && ctas < 2 * wave && ctas % wave * 3 < wave) ask = 37 * 1024;
+    }
+    return launch_dependent("quantize_cols_kernel", kernel, grid, kThreads, ask, cluster, stream, w, wq, scale, rows, cols, rows_per_cta);
 }
 
 // VEC: elements per vector where bases are aligned (16 bytes of w), else 1.
