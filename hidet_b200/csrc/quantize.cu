@@ -488,8 +488,9 @@ __device__ __forceinline__ T warp_max(T a) {
 
 // REG_CHUNKS: vectors of the row each thread keeps in registers between the two phases; rows longer
 // than blockDim * VEC * REG_CHUNKS read the remainder again (it is in L1/L2 by then).
+// Four or five CTAs an SM (600 x 24576 f32 24 us with four, 19 with five), eight of the element-wise form.
 template <typename T, typename Q, int VEC, int REG_CHUNKS>
-__global__ void __launch_bounds__(kThreads, VEC == 1 ? 8 : 0) quantize_rows_kernel(const T *w, Q *wq,
+__global__ void __launch_bounds__(kThreads, VEC == 1 ? 8 : (sizeof(T) == 4 ? 5 : 4)) quantize_rows_kernel(const T *w, Q *wq,
                                                                  T *scale, int64_t rows, int64_t cols) {
     using A = Arith<T>;
     __shared__ T warp_part[kThreads / 32];
@@ -965,17 +966,22 @@ int launch_quantize_rows(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols
         warps = warps < 1 ? 1 : (warps > kRowWarps ? kRowWarps : warps);
         const size_t smem = warps * row_bytes;  // at most kRowCtaBytes, with a few static bytes the default limit for shared memory
         const dim3 grid((unsigned)ceil_div(rows, warps));
-        // A row of more than half of a CTA's share has the whole CTA (a warp has few loads in flight for it, and few warps fit an SM): 4096 x 12280
-        // f32 85 -> 63 us, 4147 x 8242 f32 53 -> 34, 4096 x 12288 f16 39 -> 28, 674 x 6912 f32 12.2 -> 7.6.
-        if (row_bytes > kRowCtaBytes / 2 && row_bytes <= kLongRowBytes) {
+        // A row of more than half of a CTA's share has the whole CTA (a warp has few loads in flight for it, and few warps fit an SM): 4147 x 8242
+        // f32 53 -> 34 us, 4096 x 12288 f16 39 -> 28, 674 x 6912 f32 12.2 -> 7.6.  Whole rows beyond that share are faster in the kernel below,
+        // which keeps the SMs full (2000 x 20480 f32 61 us so, 45 there; 300 x 40960 f16 21 and 15), odd ones only beyond kLongRowBytes.
+        // f32 rows that leave no SM more than one of them or two stay (64 x 24576 8.1 us so, 10.1 there; 1 x 12652 4.5 and 3.6).
+        const int sms = sm_count() > 0 ? sm_count() : 148;
+        const bool few = sizeof(T) == 4 && rows * 4 > sms && rows * 2 <= 3 * (int64_t)sms;
+        if (row_bytes > kRowCtaBytes / 2 && row_bytes <= (whole && !few ? kRowCtaBytes : kLongRowBytes)) {
             auto kernel = quantize_rows_flat_kernel<T, Q, VEC, true>;
             if (row_bytes > kRowCtaBytes) B200Q_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongRowBytes));
             return launch_dependent("quantize_rows_flat_kernel", kernel, dim3((unsigned)rows), kRowWarps * 32, row_bytes, 1, stream, w, wq, scale, rows, cols, (int)row_bytes);
         }
-        if (row_bytes <= kRowCtaBytes) {
-            if (whole) return launch_dependent("quantize_rows_warp_kernel", quantize_rows_warp_kernel<T, Q, VEC>, grid, warps * 32, smem, 1, stream, w, wq, scale, rows, cols);
+        if (whole && row_bytes <= kRowCtaBytes) return launch_dependent("quantize_rows_warp_kernel", quantize_rows_warp_kernel<T, Q, VEC>, grid, warps * 32, smem, 1, stream, w, wq, scale, rows, cols);
+        // A warp a row needs rows to fill the SMs with, short ones more of them; with fewer, a CTA a row element by element is faster (256 x 513 f16
+        // 1.7 us, 1.9 a warp a row, 256 x 4097 f32 3.7 and 5.2, 7 x 8466 bf16 6.0 and 7.9; but 1000 x 257 f16 2.4 and 1.9, 4000 x 33 2.6 and 2.2).
+        if (!whole && row_bytes <= kRowCtaBytes && (rows >= 8 * (int64_t)sms || (rows >= 4 * (int64_t)sms && row_bytes >= 512)))
             return launch_dependent("quantize_rows_flat_kernel", quantize_rows_flat_kernel<T, Q, VEC, false>, grid, warps * 32, smem, 1, stream, w, wq, scale, rows, cols, (int)row_bytes);
-        }
         if (!whole) return launch_quantize_rows<T, Q, 1>(w, wq, scale, rows, cols, stream);
     }
     const int64_t nvec = cols / VEC;
