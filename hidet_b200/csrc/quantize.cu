@@ -140,6 +140,21 @@ template <typename T, int N>
 __device__ __forceinline__ Vec<T, N> load_vec(const T *p) {
     return *reinterpret_cast<const Vec<T, N> *>(p);
 }
+// The same past the first-level cache, for what is read once by threads that have little else to do (codes of a narrow matrix restored per row:
+// 100000 x 8 f16 9.1 us through it, 5.8 past it).  Volatile: where several are to be in flight they stand together.
+template <int BYTES>
+struct RawVec;
+template <> struct RawVec<1> { typedef unsigned char Type; };
+template <> struct RawVec<2> { typedef unsigned short Type; };
+template <> struct RawVec<4> { typedef unsigned int Type; };
+template <> struct RawVec<8> { typedef uint2 Type; };
+template <> struct RawVec<16> { typedef uint4 Type; };
+template <typename T, int N>
+__device__ __forceinline__ Vec<T, N> load_l2(const T *p) {
+    typedef typename RawVec<sizeof(T) * N>::Type Raw;
+    const Raw raw = __ldcg(reinterpret_cast<const Raw *>(p));
+    return *reinterpret_cast<const Vec<T, N> *>(&raw);
+}
 template <typename T, int N>
 __device__ __forceinline__ void store_vec(T *p, const Vec<T, N> &x) {
     *reinterpret_cast<Vec<T, N> *>(p) = x;
@@ -755,36 +770,37 @@ __global__ void __launch_bounds__(kThreads) dequantize_kernel(const Q *wq, const
     const Q *src = wq + r0 * cols + c;
     T *dst = w + r0 * cols + c;
     const int64_t sweep = (int64_t)kDqSweep * cols;
-    constexpr int EACH = kDqRows / kDqSweep;
-    Vec<Q, VEC> q[EACH];
-    Vec<T, VEC> out;
-#pragma unroll
-    for (int i = 0; i < EACH; ++i)
-        if (r0 + i * kDqSweep < rows) q[i] = load_vec<Q, VEC>(src + i * sweep);
+    static_assert(kDqRows == 2 * kDqSweep, "two rows a thread");
+    if (r0 >= rows) return;
+    if (r0 + kDqSweep >= rows) {                  // one row: a way of its own is shorter for the smallest matrices (5 x 256 1.0 -> 0.8 us)
+        Vec<T, VEC> o;
+        if (reduce_dim == 0) {
+            DequantVec<T, Q, VEC>::template run<true>(load_l2<Q, VEC>(src), load_vec<T, VEC>(scale + c).v, o);
+        } else {
+            const T s = scale[r0];
+            DequantVec<T, Q, VEC>::template run<false>(load_l2<Q, VEC>(src), &s, o);
+        }
+        store_vec<T, VEC>(dst, o);
+        return;
+    }
+    const Vec<Q, VEC> q0 = load_l2<Q, VEC>(src), q1 = load_l2<Q, VEC>(src + sweep);
+    Vec<T, VEC> o0, o1;
     if (reduce_dim == 0) {
         const Vec<T, VEC> s = load_vec<T, VEC>(scale + c);
-#pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-            if (r0 + i * kDqSweep >= rows) break;
-            DequantVec<T, Q, VEC>::template run<true>(q[i], s.v, out);
-            store_vec<T, VEC>(dst + i * sweep, out);
-        }
+        DequantVec<T, Q, VEC>::template run<true>(q0, s.v, o0);
+        DequantVec<T, Q, VEC>::template run<true>(q1, s.v, o1);
     } else {
-        T s[EACH];
-#pragma unroll
-        for (int i = 0; i < EACH; ++i)
-            if (r0 + i * kDqSweep < rows) s[i] = scale[r0 + i * kDqSweep];
-#pragma unroll
-        for (int i = 0; i < EACH; ++i) {
-            if (r0 + i * kDqSweep >= rows) break;
-            DequantVec<T, Q, VEC>::template run<false>(q[i], &s[i], out);
-            store_vec<T, VEC>(dst + i * sweep, out);
-        }
+        const T s0 = scale[r0], s1 = scale[r0 + kDqSweep];
+        DequantVec<T, Q, VEC>::template run<false>(q0, &s0, o0);
+        DequantVec<T, Q, VEC>::template run<false>(q1, &s1, o1);
     }
+    store_vec<T, VEC>(dst, o0);
+    store_vec<T, VEC>(dst + sweep, o1);
 }
 
 // The same for any width of at least VEC: VEC rows together are whole vectors, so a thread takes the same vector of every group of
 // VEC rows; it holds elements of one row or of two, at the same columns in each group.  grid = (vectors of a group, groups / kDqGroups)
+// One vector at a time: all four in front of the stores take registers, and CTAs hide more (4000 x 20001 f16 70 us so, 54 one by one, bf16 102 and 55).
 // The scales of the columns go through shared memory: fetched by each thread for itself, two bytes at a time, they ask the same few lines of L2
 // too often (895 x 327 6.7 us, 4.1 element by element).
 constexpr int kDqGroups = 4;                      // per thread and trip
@@ -809,29 +825,18 @@ __global__ void __launch_bounds__(kThreads) dequantize_flat_kernel(const Q *wq, 
     Vec<T, VEC> s;
     if (reduce_dim == 0) s = load_vec<T, VEC>(col_scale + threadIdx.x * VEC);
     for (int64_t g0 = (int64_t)blockIdx.y * kDqGroups; g0 < groups; g0 += (int64_t)gridDim.y * kDqGroups) {
-        const int64_t r0 = g0 * VEC + row, at0 = (g0 * cols + v) * VEC, step = VEC * cols;
-        Vec<Q, VEC> q[kDqGroups];
-        T first[kDqGroups], second[kDqGroups];
 #pragma unroll
         for (int i = 0; i < kDqGroups; ++i) {
-            const int64_t r = r0 + i * VEC;
-            if (r < rows && at0 + i * step + VEC <= total) q[i] = load_vec<Q, VEC>(wq + at0 + i * step);
-            if (reduce_dim != 0 && r < rows) {
-                first[i] = scale[r];
-                second[i] = here < VEC && r + 1 < rows ? scale[r + 1] : first[i];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kDqGroups; ++i) {
-            const int64_t at = at0 + i * step;
-            if (r0 + i * VEC >= rows) break;
+            const int64_t r = (g0 + i) * VEC + row, at = ((g0 + i) * cols + v) * VEC;
+            if (r >= rows) break;
             if (reduce_dim != 0) {
+                const T s0 = scale[r], s1 = here < VEC && r + 1 < rows ? scale[r + 1] : s0;
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) s.v[e] = e < here ? first[i] : second[i];
+                for (int e = 0; e < VEC; ++e) s.v[e] = e < here ? s0 : s1;
             }
+            Vec<T, VEC> out;
             if (at + VEC <= total) {
-                Vec<T, VEC> out;
-                DequantVec<T, Q, VEC>::template run<true>(q[i], s.v, out);
+                DequantVec<T, Q, VEC>::template run<true>(load_vec<Q, VEC>(wq + at), s.v, out);
                 store_vec<T, VEC>(w + at, out);
             } else {                              // the end of the matrix
                 for (int e = 0; at + e < total; ++e) w[at + e] = Arith<T>::template dequant<Q>(wq[at + e], s.v[e]);
@@ -1018,7 +1023,11 @@ int dequantize_typed(const void *wq_, const void *scale_, void *w_, int64_t rows
     if (row_blocks > kDqGridY * kDqGridY || col_blocks > 65535) {
         return set_error(B200Q_UNSUPPORTED, "symmetric_dequantize: [%lld, %lld] exceeds the grid limit", (long long)rows, (long long)cols);
     }
-    if (cols % VEC != 0 && cols >= VEC && aligned(w, 16) && aligned(wq, VEC * sizeof(Q))) {
+    // Vectors for widths that are not whole ones from 3 Mi elements and 96 columns on (48 with 16 Mi elements).  Below, element by element is faster: in
+    // vectors a thread finds its rows by divisions and walks thirty-two of them, and a CTA covers 256 vectors of a row group that has `cols` (256 x 257
+    // f16 1.0 us, 2.6 in vectors; 60000 x 9 2.9 and 6.2; 1000 x 2049 4.2 and 5.0; 1000 x 4097 8.4 and 6.3; 60000 x 129 16 and 11; 400000 x 63 42 and 29).
+    const int64_t enough = (cols >= 96 ? 3 : 16) * (int64_t)1024 * 1024;
+    if (cols % VEC != 0 && cols >= 48 && rows >= enough / cols && aligned(w, 16) && aligned(wq, VEC * sizeof(Q))) {
         const int64_t groups = ceil_div(ceil_div(rows, VEC), kDqGroups);
         return launch_dependent("dequantize_flat_kernel", dequantize_flat_kernel<T, Q, VEC>, dim3((unsigned)ceil_div(cols, kThreads), (unsigned)(groups < kDqGridY ? groups : kDqGridY)), kThreads, 0, 1,
                                 stream, wq, scale, w, rows, cols, reduce_dim);

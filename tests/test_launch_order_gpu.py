@@ -223,3 +223,16 @@ def test_weights_beyond_24_rows_may_be_the_result_of_a_kernel_that_triggers_earl
     weights = [(torch.randint(-127, 128, (k, n) if layout == 'KN' else (n, k), device='cuda', generator=gen, dtype=torch.int8),
                 torch.rand(n, device='cuda', generator=gen).mul_(1e-2).half()) for _ in range(2)]
     _check(late_copy, weights, lambda wq, scale: hidet_b200.symmetric_quant_matmul(a, wq, scale, weight_layout=layout))
+
+
+# the kernels that take odd widths in aligned vectors, which they do from more elements on than the shapes above have
+@pytest.mark.parametrize('dims', [0, -1])
+@pytest.mark.parametrize('dtype,quant', [(torch.float16, torch.int8), (torch.float32, torch.int16)])
+def test_odd_widths_in_vectors_may_be_the_result_of_a_kernel_that_triggers_early(late_copy, dims, dtype, quant):
+    rows, cols = 3072, 1026 + (dtype == torch.float16)   # 1026 is not a multiple of four
+    gen = torch.Generator(device='cuda').manual_seed(cols)
+    weights = [(torch.randn(rows, cols, device='cuda', generator=gen).to(dtype),) for _ in range(2)]
+    _check(late_copy, weights, lambda w: _bytes(*hidet_b200.symmetric_quantize(w, 'int8', dims=dims)))
+    codes = [(torch.randint(-127, 128, (rows, cols), device='cuda', generator=gen).to(quant), torch.rand(cols // 4 * 4 + 4 if dims == 0 else rows, device='cuda', generator=gen).to(dtype))
+             for _ in range(2)]
+    _check(late_copy, codes, lambda q, s: _bytes(hidet_b200.symmetric_dequantize(q, s[:cols if dims == 0 else rows], dims=dims)))

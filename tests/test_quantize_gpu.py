@@ -292,3 +292,25 @@ def test_slices_that_fill_the_default_shared_memory():
             "rows = [hidet_b200.symmetric_quantize(w.t().contiguous(), 'int8', dims=-1)]\n"
             "assert torch.equal(wq, rows[0][0].t()) and torch.equal(scale, rows[0][1])\n")
     subprocess.run([sys.executable, '-c', code], check=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+
+# sizes beyond the lines from which on odd widths go in aligned vectors: restored from 3 Mi elements (96 columns) and 16 Mi (48), quantized per row
+# from four rows an SM (512 bytes) and eight; below and above each
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('quant_type', ['int8', 'int16'])
+@pytest.mark.parametrize('rows,cols', [(3063, 1027), (3062, 1027), (32769, 97), (33150, 95), (6, 600001), (350003, 49), (342393, 49), (593, 301), (591, 301), (1185, 9), (1183, 9), (2003, 12001)])
+def test_widths_in_vectors_and_element_by_element(rows, cols, quant_type, dtype):
+    g = torch.Generator(device='cuda').manual_seed(rows + cols)
+    wide = torch.full((rows, (cols + 15) // 8 * 8), float('nan'), device='cuda', dtype=dtype)
+    wide[:, :cols] = torch.randn(rows, cols, device='cuda', generator=g).mul_(0.02).to(dtype)
+    wide[0, 0], wide[rows - 1, cols - 1], wide[rows // 2, cols // 2] = float('nan'), float('inf'), -0.0
+    w = wide[:, :cols].contiguous()
+    for dims in (0, -1):
+        wq, scale = hidet_b200.symmetric_quantize(w, quant_type, dims=dims)
+        wq_w, scale_w = hidet_b200.symmetric_quantize(wide, quant_type, dims=dims)
+        assert torch.equal(_bits(scale), _bits(scale_w)[:cols] if dims == 0 else _bits(scale_w))
+        assert torch.equal(wq, wq_w[:, :cols])
+        scale = torch.rand(scale.shape, device='cuda', generator=g).to(dtype)
+        scale_w = scale if dims == -1 else torch.cat([scale, scale.new_ones(wide.shape[1] - cols)])
+        back = hidet_b200.symmetric_dequantize(wq, scale, dims=dims)
+        assert torch.equal(_bits(back), _bits(hidet_b200.symmetric_dequantize(wq_w, scale_w, dims=dims)[:, :cols].contiguous()))
