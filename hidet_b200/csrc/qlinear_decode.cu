@@ -697,9 +697,11 @@ DecodePlan plan_decode_portable(int64_t M, int64_t N, int64_t K) {
     // idle (a step of a 1024-wide decoder 72 -> 57 us), with two the exchange costs what the shorter loop gives (64 us).  Only where
     // that leaves fewer than four splits are two steps enough, for the last phase's sake: one CTA alone finishes 16 rows of 128
     // columns in several rounds ((16, 256, 688) 4.2 -> 3.0 us, (1, 256, 688) 2.75 -> 2.15, (16, 640, 2048) 3.8 -> 2.8), and where the grid has
-    // the room ((16, 512, 16384) 4.5 -> 4.8).
+    // the room: four splits up to four ninths as many tiles as SMs ((1, 512, 8192) 2.7 -> 2.6, (1, 512, 9472) 2.8 -> 3.1, (16, 512, 16384) 4.5 -> 4.8), two
+    // of fewer than eight steps up to as many ((1, 384, 18688) 3.5 -> 2.9, (1, 384, 28160) 3.7 -> 4.0; with more than eight rows half as many again).
     int max_splits = k_iters >= 4 ? k_iters / 4 : 1;
-    if (max_splits < 4 && k_iters >= 4) max_splits = k_iters < 8 ? (tiles * 4 <= 2 * sms ? k_iters / 2 : 2) : (tiles * 4 <= 2 * sms ? 4 : max_splits);
+    if (k_iters >= 4 && k_iters < 8) max_splits = tiles * 4 <= 2 * sms ? k_iters / 2 : (M > 16 || tiles <= (M <= 8 ? sms : sms * 3 / 2) ? 2 : 1);
+    else if (max_splits < 4 && k_iters >= 8 && (M > 16 ? tiles * 4 <= 2 * sms : tiles * 9 <= 4 * sms)) max_splits = 4;
     // The splits of a tile form a cluster of up to eight CTAs (partials meet in distributed shared memory), as large as lets
     // the whole grid run at once: a few clusters left for a second wave double the time of the launch (96 tiles
     // in clusters of six are 576 CTAs and fit 148 x 4 slots by number, but not the groups of SMs clusters are confined to:
@@ -748,9 +750,15 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
     // 4.0 us, 4.4 in one).  A form for 32 rows was no better than two passes or the mid-M kernel ((32, 4096, 4096) 8.8 and 8.5 us, (32, 4096,
     // 12288) 16.1 and 17.7): the warp-level MMAs of four row blocks take longer than the stream.
     int variant = pl.variant, m_tiles = pl.m_tiles, one = c;  // of the plan with one cluster a tile, of `one` CTAs
+    // With three CTAs an SM, of clusters that are not of one, two or a multiple of four the last few that the query allows wait for CTAs of the launch
+    // behind that have moved in ((24, 4096, 17408), 408 CTAs, 17.4 us; 414 19.6, 420 23.3, 426 24.9; (24, 8192, 8704), 408, 17.1 and with 426 22.1).
+    auto full = [&](int cluster) {
+        const int n = resident_ctas(dev, kVariants[variant], cluster), most = sms * 69 / 25;
+        return variant == 3 && cluster > 2 && cluster % 4 != 0 && n > most ? most : n;
+    };
     if (one_pass) {
         variant = 3, m_tiles = 1, one = 1;
-        while (one < kPortableCluster && one < pl.most_splits && pl.n_tiles * (one + 1) <= resident_ctas(dev, kVariants[variant], one + 1)) ++one;
+        while (one < kPortableCluster && one < pl.most_splits && pl.n_tiles * (one + 1) <= full(one + 1)) ++one;
     }
     // Beyond the portable size where that leaves SMs idle ((1, 4096, 1024) 4.0 -> 3.1 us, (8, 8192, 1024) 6.7 -> 4.7, (16, 8192, 1024) 8.3 -> 5.4,
     // (1, 11008, 512) 7.0 -> 4.8 instead of clusters that meet in the workspace), and where the runs are long: with few CTAs an SM a stage
@@ -761,7 +769,7 @@ DecodePlan plan_decode(int64_t M, int64_t N, int64_t K) {
         const int portable = pl.n_tiles * one;
         const bool narrow = M <= 8 ? portable <= sms : (M <= 16 ? portable * 3 <= sms * 2 : portable * 11 <= sms * 6), deep = k_iters >= (M <= 8 ? 12 : 16) * one && portable * 4 <= sms * 9;
         for (int wide = kMaxCluster; wide > kPortableCluster && (narrow || deep); --wide) {
-            if (!slices_fit(wide) || pl.n_tiles * wide > resident_ctas(dev, kVariants[variant], wide)) continue;
+            if (!slices_fit(wide) || pl.n_tiles * wide > full(wide)) continue;
             one = wide;
             break;
         }
