@@ -24,8 +24,7 @@
 // No kernel of this file lets the launch behind it start early: the small-M quantized linear asks for the codes of its weight
 // before it waits for the kernel in front, and is safe behind these only because it starts when they have ended.  They are themselves
 // launched as programmatic dependents, and every CTA waits for the kernel in front before it touches memory: what remains between two launches
-// is shorter so (300 x 512 per column 4.2 -> 2.8 us, 285 x 2992 per row 5.3 -> 3.4, 300 x 400 restored 4.2 -> 1.6, 4096 x 11008 per column
-// 33.4 -> 31.7).
+// is shorter so (300 x 512 per column 4.2 -> 2.8 us, 285 x 2992 per row 5.3 -> 3.4, 300 x 400 restored 4.2 -> 1.6).
 #include <cooperative_groups.h>
 #include <cfloat>
 
@@ -974,9 +973,9 @@ int launch_quantize_rows(const T *w, Q *wq, T *scale, int64_t rows, int64_t cols
         // A row of more than half of a CTA's share has the whole CTA (a warp has few loads in flight for it, and few warps fit an SM): 4147 x 8242
         // f32 53 -> 34 us, 4096 x 12288 f16 39 -> 28, 674 x 6912 f32 12.2 -> 7.6.  Whole rows beyond that share are faster in the kernel below,
         // which keeps the SMs full (2000 x 20480 f32 61 us so, 45 there; 300 x 40960 f16 21 and 15), odd ones only beyond kLongRowBytes.
-        // f32 rows that leave no SM more than one of them or two stay (64 x 24576 8.1 us so, 10.1 there; 1 x 12652 4.5 and 3.6).
+        // f32 rows that leave no SM more than one of them or two stay (120 x 24576 9.0 us so, 10.7 there; 64 x 12296 4.8 and 3.8).
         const int sms = sm_count() > 0 ? sm_count() : 148;
-        const bool few = sizeof(T) == 4 && rows * 4 > sms && rows * 2 <= 3 * (int64_t)sms;
+        const bool few = sizeof(T) == 4 && rows * 2 > sms && rows * 2 <= 3 * (int64_t)sms;
         if (row_bytes > kRowCtaBytes / 2 && row_bytes <= (whole && !few ? kRowCtaBytes : kLongRowBytes)) {
             auto kernel = quantize_rows_flat_kernel<T, Q, VEC, true>;
             if (row_bytes > kRowCtaBytes) B200Q_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongRowBytes));
