@@ -19,11 +19,11 @@
 //
 // The kernel is launched as a programmatic dependent of the kernel before it in the stream: weight
 // tiles do not depend on that kernel, so they are requested before waiting for it (the scales may, as the
-// activations do), and the kernel after this one may start as soon as that wait is over.
+// activations do; with 17 to 24 rows the weight may too, see below), and the kernel after this one may start as soon as that wait is over.
 //
 // Replaces the generated mma.sync kernel of python/hidet/graph/ops/quant/matmul_f16_i8.py:136-485
-// (f16 accumulation, 64x128 tiles, no split-K by default) for M <= 16, and serves larger M by
-// tiling M over blockIdx.z.
+// (f16 accumulation, 64x128 tiles, no split-K by default) for up to 24 rows, and serves more where the
+// kernels for more rows are not faster, by tiling M over blockIdx.z.
 #include <atomic>
 
 #include "common.cuh"
@@ -194,7 +194,7 @@ struct Params {
     bool late;                // the weight may be a result of the kernel in front (with two row blocks; three always take it so)
 };
 
-// MT: 8-row blocks of activations per CTA (1: up to 8 rows, 2: up to 16).
+// MT: 8-row blocks of activations per CTA (1: up to 8 rows, 2: up to 16, 3: up to 24).
 // NK: the weight is [N, K] with K contiguous (the layout torch.nn.Linear keeps) instead of the reference's
 //     [K, N]: a stage is then 128 weight rows of 64 k-bytes (64-byte swizzle) and the fragments come from
 //     plain matrix loads; everything else is shared.

@@ -163,8 +163,8 @@ __global__ void qlinear_u4_reduce_kernel(const float *partial, __half *c, int64_
 // the warp's run; a part of a group is a term like any other)
 //     sum += scale * (group sum - zero * activation sum)
 // goes to the lane's own place in shared memory, where the warps, and then the cluster, are summed in a fixed order.
-// What is left is not bytes: at (1, 4096, 12288) the schedulers issue in 10 300 of 25 000 clocks (mostly unpacking; an eighth fewer since the
-// constants are kept in registers), and four warps each, in chains of short dependent steps, do not hide the latency between; then the
+// What is left is not bytes: at (1, 4096, 12288) a scheduler issues 8 900 times (mostly unpacking; 10 300 before the constants were kept in
+// registers), in half of its active clocks, and four warps each, in chains of short dependent steps, do not hide the latency between; then the
 // exchange at the end.  (Built like the small-M int8 kernel, with a TMA producer and transposing matrix loads of bytes, it takes
 // 11.2 us there for 11.6, 6.4 for 6.0 at (1, 4096, 4096), and 16.3 for 11.7 where rows are not multiples of 16 bytes.)
 // Per launch in a replayed graph, with the kernel below it before: (1, 4096, 12288) 25.8 -> 11.6 us, (8, 4096, 4096) 28.7 ->

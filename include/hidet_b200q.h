@@ -18,13 +18,17 @@
  *     hidet_get_last_error).  Nothing aborts the process and no kernel traps.
  *   - the kernels of the quantized linears (int8 weights at any M, int8 weights whose rows are not multiples of 16
  *     bytes, 4-bit weights) are launched as programmatic dependents of the kernel in front of them in the stream, and let
- *     the kernel behind them start while they run if that is launched the same way.  All operands are read, and outputs
- *     and scratch touched, only after the stream dependency on the kernel in front is honoured, with one exception:
- *     the int8 kernel for small M requests the codes `wq` before it ([K, N] rows of 16-byte multiples, and [N, K]); the
- *     scales it reads after it.  The codes must be complete when the kernel in front may let its dependents start.
- *     Ordinary kernels (b200q_symmetric_quantize, the packing kernels and every other kernel of this library but the
- *     quantized linears, memcpy / memset nodes, anything that does not itself execute
- *     griddepcontrol.launch_dependents) let dependents start only when they have finished, so producing a weight with
+ *     the kernel behind them start while they run if that is launched the same way.  The quantize, dequantize and lookup
+ *     kernels are launched as programmatic dependents too, and let nothing start before their end.  All operands are read,
+ *     and outputs and scratch touched, only after the stream dependency on the kernel in front is honoured, with one
+ *     exception: the int8 kernel for small M requests the codes `wq` before it ([K, N] rows of 16-byte multiples, and
+ *     [N, K]); the scales it reads after it.  The codes must be complete when the kernel in front may let its dependents
+ *     start.  That kernel serves up to 16 rows, and up to 64 where the kernels for more rows are not faster; a caller that does
+ *     not want to rely on which it is takes the exception to hold for every M <= 64.  (It waits with its codes too at 17 to
+ *     24 rows on weights of 6 Mi codes and more.)
+ *     Kernels that do not themselves execute griddepcontrol.launch_dependents (b200q_symmetric_quantize, the packing
+ *     kernels and every other kernel of this library but the quantized linears, memcpy / memset nodes, ordinary
+ *     kernels) let dependents start only when they have finished, so producing a weight with
  *     b200q_symmetric_quantize and using it in the next call on the same stream is safe.  Not safe: writing the codes of
  *     an int8 weight from a kernel that triggers its dependents early when nothing but kernels of that kind lie between
  *     it and the quantized linear that reads them on the same stream (the quantized linears are themselves of that

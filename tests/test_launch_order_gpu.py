@@ -1,7 +1,7 @@
 """Operands that the kernel in front writes, where the kernels launched as programmatic dependents promise to wait for its end: 4-bit weights,
-int8 weights whose rows are not multiples of 16 bytes, int8 weights of any linear of 17 rows and more on 6 MB and more, the scales of every
-weight, and all operands of the quantize, dequantize and lookup kernels.  (With fewer rows the small-M int8 kernel asks for the codes of its weight
-earlier by contract, and is tested behind this library's own producers only.)"""
+int8 weights whose rows are not multiples of 16 bytes, int8 weights of the kernels for more than a few rows and of 17 to 24 rows on 6 MB and more, the
+scales of every weight, and all operands of the quantize, dequantize and lookup kernels.  (Otherwise the small-M int8 kernel asks for the codes of its
+weight earlier by contract, and is tested behind this library's own producers only.)"""
 import ctypes
 
 import pytest
